@@ -134,7 +134,8 @@ static void free_table(kspace_ctx* c) {
     IntegratorDev& I = c->I;
     void* ptrs[] = {I.scalefact, I.dtot, I.coef, I.nu_init, I.nu_last, I.wavenum, I.dcdm, I.dnu_s, I.dnu,
                     I.knot_invdiag, I.knot_fac, I.knot_invh, I.knot_h3, I.knot_ih3, I.nc_g, I.nc_fsl,
-                    I.nc_dx, I.nc_j, I.fs_x, I.fs_y, I.fs_c, I.fs_seg, I.t_logk, I.t_T, I.t_c, I.sc,
+                    I.nc_dx, I.nc_j, I.nc_inv, I.fs_x, I.fs_y, I.fs_c, I.fs_seg, I.fs_suf, I.fs_tot, I.t_logk, I.t_T,
+                    I.t_c, I.sc,
                     I.qag_max, I.qag_total, I.coef_unit};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -472,6 +473,9 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
     CK(dalloc(&I.fs_y, I.fs_cap));
     CK(dalloc(&I.fs_c, I.fs_cap));
     CK(dalloc(&I.fs_seg, I.fs_cap));
+    CK(dalloc(&I.fs_suf, I.fs_cap));
+    CK(dalloc(&I.fs_tot, I.fs_cap / 16 + 1));
+    CK(dalloc(&I.nc_inv, kNcNodes));
     CK(dalloc(&I.sc, 1));
     CK(dalloc(&I.qag_max, 1));
     CK(dalloc(&I.qag_total, 1));
@@ -482,6 +486,7 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
     S.prefac = 1.5 * Omega0 * kHubble * kHubble * pow(UnitTime_in_s, 2) / S.light;  // :53
     S.Omeganonu = Omega0 - omega_nu(c->hB, 1);                                 // :55
     c->Omeganonu = S.Omeganonu;
+    c->S0 = S;
     CK(cudaMemcpy(I.sc, &S, sizeof(S), cudaMemcpyHostToDevice));
     // step buffers
     c->buf_nb = nk_alloc;
@@ -703,6 +708,13 @@ extern "C" int kspace_gpu_save_nu_power(kspace_ctx* c, double Time, int snapnum,
 }
 
 // ------------------------------------------------------------------ integrator
+// A call's preparation with Na knots at scale factor a (launch_integrator_prepare).
+static void prepare_call(kspace_ctx* c, int Na, double a, double loga, int start_row, int write_knot, RowsMode rows,
+                         int nk, int update_row, cudaStream_t st, bool scalars_only = false) {
+    launch_integrator_prepare(c->I, c->hB, c->S0, Na, a, loga, c->loga0, c->TimeTransfer, start_row, write_knot,
+                              scalars_only, rows, nk, update_row, st);
+}
+
 // delta_tot_table.c:79-149 (host bookkeeping; numbers on the device)
 static int delta_tot_init(kspace_ctx* c, int nk_in, const double* keff_d, const double* dcdm_d, double Time) {
     for (int ik = 0; ik < c->ia; ik++) {
@@ -729,9 +741,9 @@ static int delta_tot_init(kspace_ctx* c, int nk_in, const double* keff_d, const 
     if (st) return st;
     // delta_nu_last = delta_nu at the last stored time (delta_tot_table.c:146)
     const double a_last = exp(c->h_scalefact[c->ia - 1]);
-    launch_delta_nu_combined(c->I, c->nk, c->ia, a_last, c->h_scalefact[c->ia - 1], c->loga0, c->TimeTransfer,
-                             0, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split);
-    g_launches += 8;
+    prepare_call(c, c->ia, a_last, c->h_scalefact[c->ia - 1], 0, 0, kRowsFull, c->nk, -1, c->stream);
+    launch_integrator_rest(c->I, c->nk, c->ia, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split);
+    g_launches += 4;
     CK(cudaMemcpyAsync(c->I.nu_last, c->I.dnu, sizeof(double) * c->nk, cudaMemcpyDeviceToDevice, c->stream));
     c->fact_valid = 0;
     c->init_done = 1;
@@ -788,21 +800,19 @@ static int update_device(kspace_ctx* c, double a, int nk_in, const double* keff_
         if (want_corr || dnu_out_d) {
             // scalars at a (kspace_prefac) without integrating, then the table from
             // delta_nu_last passed through unclamped, as the reference returns it
-            launch_delta_nu_combined(I, 0, 1, a, loga, c->loga0, c->TimeTransfer, -1, 0, c->spec_ids, c->qag_warps,
-                                     c->stream);
+            prepare_call(c, 1, a, loga, 0, 0, kRowsNone, 0, -1, c->stream, true);
             CK(cudaMemcpyAsync(I.dnu, I.nu_last, sizeof(double) * c->nk, cudaMemcpyDeviceToDevice, c->stream));
             launch_finish_update(I, c->nk, -2, a, loga, want_corr ? keff_d : nullptr, dnu_out_d,
                                  want_corr ? c->logk_d : nullptr, want_corr ? c->ratio_d : nullptr,
                                  want_corr ? c->corr : CorrTable{}, c->norm_d, c->stream);
-            g_launches += 3;
+            g_launches += 2;
         }
         return sync_status(c);
     }
     if (c->ia >= I.namax) return KSPACE_ERR_NAMAX;
-    // provisional row from delta_nu_last (delta_tot_table.c:222): written here, or, after
-    // the prepared scalars, as the rows' splines are solved
+    // provisional row from delta_nu_last (delta_tot_table.c:222): written, after the call's
+    // scalars, as the rows' splines are solved
     const int prov_row = c->ia;
-    if (!prepared) launch_update_row(I, c->nk, prov_row, a, loga, I.dcdm, I.nu_last, c->stream);
     c->h_scalefact[c->ia] = loga;
     c->ia++;
     const int Na = c->ia;
@@ -812,8 +822,8 @@ static int update_device(kspace_ctx* c, double a, int nk_in, const double* keff_
         launch_integrator_rest(I, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, prov_row,
                                true, fin, c->prep_base);
     } else {
-        launch_delta_nu_combined(I, c->nk, Na, a, loga, c->loga0, c->TimeTransfer, c->fact_valid, c->nspec,
-                                 c->spec_ids, c->qag_warps, c->stream, c->qag_split);
+        prepare_call(c, Na, a, loga, c->fact_valid, 1, kRowsFull, c->nk, prov_row, c->stream);
+        launch_integrator_rest(I, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, -1, true);
     }
     I.kq = nullptr;
     c->prep_valid = false;
@@ -821,8 +831,8 @@ static int update_device(kspace_ctx* c, double a, int nk_in, const double* keff_
     const bool commit = a >= exp(c->h_scalefact[Na - 2]) + 0.009;
     launch_finish_update(I, c->nk, commit ? Na - 1 : -1, a, loga, want_corr ? keff_d : nullptr, dnu_out_d,
                          want_corr ? c->logk_d : nullptr, want_corr ? c->ratio_d : nullptr,
-                         want_corr ? c->corr : CorrTable{}, c->norm_d, c->stream, prepared);
-    g_launches += 10;
+                         want_corr ? c->corr : CorrTable{}, c->norm_d, c->stream, true);
+    g_launches += prepared ? 3 : 4;
     if (commit) {
         c->fact_valid = Na - 2 > 0 ? Na - 2 : 0;
     } else {
@@ -876,10 +886,10 @@ static int integrate_stored(kspace_ctx* c, double a, int nk, const double* waven
     CK(cudaMemsetAsync(I.qag_total, 0, sizeof(long long), c->stream));
     I.kq = kd;
     // the knot factorisation is rebuilt from the first row: rows may have changed since
-    launch_delta_nu_combined(I, nk, c->ia, a, log(a), c->loga0, c->TimeTransfer, 0, nspec, spec_ids, c->qag_warps,
-                             c->stream, c->qag_split);
+    prepare_call(c, c->ia, a, log(a), 0, 0, kRowsFull, nk, -1, c->stream);
+    launch_integrator_rest(I, nk, c->ia, nspec, spec_ids, c->qag_warps, c->stream, c->qag_split);
     I.kq = nullptr;
-    g_launches += 8;
+    g_launches += 4;
     c->fact_valid = 0;
     return KSPACE_OK;
 }
@@ -1235,10 +1245,10 @@ static int start_prep(kspace_ctx* c, const Geo* G, double Time) {
     if (loga - c->h_scalefact[c->ia - 1] < kFloatAcc) return KSPACE_OK;
     const int Na = c->ia + 1;
     CK(cudaStreamWaitEvent(c->side, c->ev_fork, 0));  // recorded before the binning pass
-    launch_integrator_prepare(c->I, Na, Time, loga, c->loga0, c->TimeTransfer, c->fact_valid, 1, false, c->side);
-    c->prep_base = launch_dtot_base(c->I, c->nk, Na, c->side);
+    c->prep_base = Na > 2;
+    prepare_call(c, Na, Time, loga, c->fact_valid, 1, c->prep_base ? kRowsBase : kRowsNone, c->nk, -1, c->side);
     CK(cudaEventRecord(c->ev_join, c->side));
-    g_launches += c->prep_base ? 6 : 5;
+    g_launches += 2;
     c->prep_valid = true;
     c->prep_Na = Na;
     c->prep_loga = loga;
@@ -1691,7 +1701,6 @@ extern "C" int kspace_gpu_diff_forward(kspace_ctx* c, double Time, double BoxSiz
     if (c->ia >= c->I.namax) return KSPACE_ERR_NAMAX;
     IntegratorDev& I = c->I;
     const double loga = log(Time);
-    launch_update_row(I, c->nk, c->ia, Time, loga, I.dcdm, I.nu_last, c->stream);
     const int Na = c->ia + 1;
     int start = c->fact_valid < Na - 3 ? c->fact_valid : Na - 3;
     if (start < 0) start = 0;
@@ -1702,13 +1711,13 @@ extern "C" int kspace_gpu_diff_forward(kspace_ctx* c, double Time, double BoxSiz
     }
     CK(cudaMemsetAsync(I.qag_max, 0, sizeof(int), c->stream));
     CK(cudaMemsetAsync(I.qag_total, 0, sizeof(long long), c->stream));
-    launch_delta_nu_combined(Is, c->nk, Na, Time, loga, c->loga0, c->TimeTransfer, start, c->nspec, c->spec_ids,
-                             c->qag_warps, c->stream, c->qag_split);
+    prepare_call(c, Na, Time, loga, start, 1, kRowsFull, c->nk, c->ia, c->stream);
+    launch_integrator_rest(Is, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, -1, true);
     c->fact_valid = start;
     launch_finish_update(I, c->nk, -3, Time, loga, c->keff_d, c->dnu_out_d, c->logk_d, c->ratio_d, c->corr,
-                         c->norm_d, c->stream);
+                         c->norm_d, c->stream, true);
     k_square<<<(c->nk + 127) / 128, 128, 0, c->stream>>>(c->dnu_out_d, pnu_out, c->nk);
-    g_launches += 11;
+    g_launches += 5;
     const size_t bytes = sizeof(float) * 2 * (size_t)pmgrid * pmgrid * (pmgrid / 2 + 1);
     if (grid_out != grid_in) CK(cudaMemcpyAsync(grid_out, grid_in, bytes, cudaMemcpyDeviceToDevice, c->stream));
     st = correct_grid(c, G, reinterpret_cast<float*>(grid_out), BoxSize, c->nk);

@@ -7,11 +7,9 @@
 // delta_nu is the one a single-instance call returns:
 //   kb_prologue     block per instance: provisional history row (:222), call scalars,
 //                   knot factorisation of the history spline
-//   kb_fs_segments  every instance's fslength segments (4-point Gauss-Legendre)
-//   kb_fs_finish    block per instance: suffix sums of the segments -> fslength table
-//   kb_fs_coeffs    thread per (instance, unknown): natural spline of the table
+//   kb_fs_eval      a block per stretch of an instance's fslength segments
+//   kb_tables       the fslength tables and the node tables of the integrand
 //   kb_dtot_coeffs  thread per (instance, bin): history-row spline coefficients
-//   kb_nc_build     thread per (instance, node): node tables of the integrand
 //   kb_dnu_qag      persistent warps that pull (instance, species, bin) tasks from an
 //                   atomic queue; knots, row and coefficients staged into shared memory
 //                   by TMA bulk copies; QAG with the 61-point Gauss-Kronrod rule
@@ -23,6 +21,7 @@
 #include <float.h>
 #include <stdint.h>
 #include "ksp_batch.h"
+#include "ksp_prep.cuh"
 #include "ksp_ptx.cuh"
 
 namespace ksp {
@@ -40,8 +39,8 @@ __device__ __forceinline__ int owner_of(const int* off, int n, int v) {
 constexpr int kBatchSmallBlocks = 4 * 152;
 
 // ------------------------------------------------------------------ prologue
-// The call scalars (as k_scalars), update_delta_tot's provisional row (as k_update_row)
-// and the knot factorisation (as k_scalars).
+// The call scalars, update_delta_tot's provisional row (as k_update_row) and the knot
+// factorisation.
 __global__ void kb_prologue(BatchDev b) {
     if (blockIdx.x == 0 && threadIdx.x == 0) b.hdr->counter = 0;
     for (int i = blockIdx.x; i < b.M; i += gridDim.x) {
@@ -68,24 +67,12 @@ __global__ void kb_prologue(BatchDev b) {
             I.knot_h3[j] = h / 3.0;
             I.knot_ih3[j] = 1.0 / (3.0 * h);
         }
-        if (threadIdx.x != 0) continue;
-        if (P.nfs == 0) {
+        auto knot = [&](int j) { return xk[j]; };
+        for (int r = (P.start_row < 0 ? 0 : P.start_row) + threadIdx.x; r < Na - 2; r += blockDim.x)
+            knot_row(knot, r, I.knot_invdiag, I.knot_fac);
+        if (threadIdx.x == 0 && P.nfs == 0) {
             S.fsl_A0a = 0.0;
             S.Nfs = 0;
-        }
-        const double* x = I.scalefact;
-        if (Na > 2) {
-            const int m = Na - 2;
-            for (int r = P.start_row < 0 ? 0 : P.start_row; r < m; r++) {
-                const double h0 = x[r + 1] - x[r], h1 = x[r + 2] - x[r + 1];
-                double d = 2.0 * (h0 + h1);
-                if (r > 0) {
-                    const double f = h0 * I.knot_invdiag[r - 1];
-                    d -= f * h0;
-                    I.knot_fac[r] = f;
-                }
-                I.knot_invdiag[r] = 1.0 / d;
-            }
         }
     }
 }
@@ -93,90 +80,55 @@ __global__ void kb_prologue(BatchDev b) {
 // ------------------------------------------------------------------ fslength table
 struct GL4b { double x[2], w[2]; };
 
-// groups of 4 lanes over the fslength segments of all instances (flat, so that
-// instances of any length balance), as k_fs_segments
-__global__ void kb_fs_segments(BatchDev b, GL4b gl) {
-    const int total = b.hdr->total_segs;  // groups
-    const long long stride = (long long)gridDim.x * blockDim.x;  // a multiple of 4
-    const long long end = 4LL * total;
-    for (long long base = (long long)blockIdx.x * blockDim.x; base < end; base += stride) {
-        const long long gt = base + threadIdx.x;
-        const int gg = (int)(gt >> 2), q = (int)(gt & 3);
-        const bool live = gt < end;
-        int i = 0, g = 0;
-        if (live) {
-            i = owner_of(b.fs_off, b.M, gg);
-            g = gg - __ldg(b.fs_off + i);
-        }
+// the stretches of all instances' segments (flat, so that instances of any length balance),
+// as k_prep_eval
+__global__ void __launch_bounds__(kPrepThreads) kb_fs_eval(BatchDev b, GL4b gl) {
+    __shared__ double f[kPrepThreads], sg[kPrepThreads];
+    const int total = b.hdr->total_segs;
+    for (int g = blockIdx.x; g < total; g += gridDim.x) {
+        const int i = owner_of(b.fs_off, b.M, g);
         const BatchCall& P = b.calls[i];
-        const int Nfs = live ? P.nfs : 1;
-        const double loga0 = P.loga0, loga = P.loga;
-        const int npts = live ? fs_rule_points(Nfs, loga0, loga) : 4;
-        fs_group_eval(*b.insts[i].B, Nfs, loga0, loga, npts, g, q, live, gl.x, gl.w, b.insts[i].fs_x,
-                      b.insts[i].fs_seg);
+        const IntegratorDev& I = b.insts[i];
+        __syncthreads();  // the previous stretch's shared arrays
+        fs_eval_block(*I.B, P.nfs, P.loga0, P.loga, g - __ldg(b.fs_off + i), gl.x[0], gl.x[1], gl.w[0], gl.w[1], f, sg,
+                      I.fs_seg, I.fs_suf, I.fs_tot);
     }
 }
 
-// block of 1024 threads per instance: the partition and summation order of k_fs_finish
-// (which also runs with 1024 threads)
-__global__ void __launch_bounds__(1024) kb_fs_finish(BatchDev b) {
-    __shared__ double warp_tot[32];
-    const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, w = t >> 5;
-    for (int i = blockIdx.x; i < b.M; i += gridDim.x) {
+// the fslength tables and the node tables, 128 nodes per block, as k_prep_tables
+__global__ void __launch_bounds__(kBatchTable) kb_tables(BatchDev b) {
+    __shared__ double tsuf[kPrepThreads + 1];
+    const int total = b.hdr->total_fsc;
+    for (int g = blockIdx.x; g < total; g += gridDim.x) {
+        const int i = owner_of(b.fsc_off, b.M, g);
         const BatchCall& P = b.calls[i];
-        const int Nfs = P.nfs;
-        if (!P.active || P.commit_row == -2 || Nfs <= 0) continue;  // uniform over the block
         const IntegratorDev& I = b.insts[i];
-        const int per = (Nfs + nt - 1) / nt;
-        const int i0 = t * per, i1 = min(Nfs, i0 + per);
-        double loc = 0;
-        for (int k = i1 - 1; k >= i0; k--) loc += I.fs_seg[k];
-        double v = loc;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double n = __shfl_down_sync(0xffffffffu, v, o);
-            if (lane + o < 32) v += n;
-        }
-        __syncthreads();  // warp_tot reuse across instances
-        if (lane == 0) warp_tot[w] = v;
-        __syncthreads();
-        if (w == 0) {
-            const int nw = nt >> 5;
-            double u = lane < nw ? warp_tot[lane] : 0.0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const double n = __shfl_down_sync(0xffffffffu, u, o);
-                if (lane + o < 32) u += n;
+        int blk = g - __ldg(b.fsc_off + i);
+        __syncthreads();  // the previous table's sums
+        const FsTable F = fs_table(I, P.nfs, P.loga0, P.loga, I.sc->light, tsuf);
+        const int table_blocks = (P.nfs + kBatchTable - 1) / kBatchTable;
+        if (blk < table_blocks) {
+            const int n = blk * kBatchTable + threadIdx.x;
+            if (n >= P.nfs) continue;
+            I.fs_x[n] = fs_node(n, P.nfs, P.loga0, P.loga);
+            const double y = fs_table_y(F, n);
+            I.fs_y[n] = y;
+            I.fs_c[n] = fs_table_c(F, n);
+            if (n == 0) {
+                I.sc->fsl_A0a = y;
+                I.sc->Nfs = P.nfs;
             }
-            if (lane < nw) warp_tot[lane] = u;
+            continue;
         }
-        __syncthreads();
-        const double later = (w + 1 < (nt >> 5)) ? warp_tot[w + 1] : 0.0;
-        double run = v - loc + later;
-        const double light = I.sc->light;
-        for (int k = i1 - 1; k >= i0; k--) {
-            run += I.fs_seg[k];
-            I.fs_y[k] = light * run;
-        }
-        __syncthreads();
-        if (t == 0) {
-            I.sc->fsl_A0a = I.fs_y[0];
-            I.sc->Nfs = Nfs;
-            I.fs_c[0] = 0.0;
-            I.fs_c[Nfs - 1] = 0.0;
-        }
-    }
-}
-
-// warp per instance: the fslength table's spline coefficients, as k_fs_coeffs
-__global__ void kb_fs_coeffs(BatchDev b) {
-    const int nw = blockDim.x >> 5;
-    for (int i = blockIdx.x * nw + (threadIdx.x >> 5); i < b.M; i += gridDim.x * nw) {
-        const BatchCall& P = b.calls[i];
-        const int Nfs = P.nfs;
-        if (!P.active || P.commit_row == -2 || Nfs <= 2) continue;  // uniform over the warp
-        const IntegratorDev& I = b.insts[i];
-        uniform_spline_warp(I.fs_y, I.fs_c, Nfs, (P.loga - P.loga0) / (Nfs - 1.));
+        const int q = (blk - table_blocks) * kBatchTable + threadIdx.x;
+        if (q >= b.nc_slots * 61) continue;
+        const double x = nc_node_x(q, P.loga0, P.loga);
+        const double fsl = fs_table_at(F, P.loga0, P.loga, x);
+        const int j = seg_bsearch(I.scalefact, P.Na, x);
+        I.nc_fsl[q] = fsl;
+        I.nc_j[q] = j;
+        I.nc_dx[q] = x - I.scalefact[j];
+        I.nc_g[q] = fsl * node_inv_aH(I.B, x);
     }
 }
 
@@ -215,36 +167,6 @@ __global__ void kb_dtot_coeffs(BatchDev b) {
             next = (c[k + 1] - off * next) * I.knot_invdiag[k];
             c[k + 1] = next;
         }
-    }
-}
-
-// thread per (instance, slot, node): the node tables (as k_nc_build)
-__global__ void kb_nc_build(BatchDev b) {
-    const double XK[31] = KSP_GK61_XK_INIT;  // the abscissae of gk61_fill
-    const int per = b.nc_slots * 61;
-    const long long total = (long long)b.M * per;
-    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < total;
-         g += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(g / per);
-        const int q = (int)(g - (long long)i * per);
-        const BatchCall& P = b.calls[i];
-        if (!P.active || P.commit_row == -2 || P.nfs <= 0 || P.Na <= 1) continue;
-        const IntegratorDev& I = b.insts[i];
-        const StepScalars& S = *I.sc;
-        const int slot = q / 61, jn = q - 61 * slot;
-        double lo, hi;
-        nc_interval(slot, S.loga0, S.loga, &lo, &hi);
-        const double c = __dmul_rn(0.5, __dadd_rn(lo, hi));
-        const double h = __dmul_rn(0.5, __dsub_rn(hi, lo));
-        const double xk = jn < 30 ? -XK[jn] : (jn < 60 ? XK[jn - 30] : 0.0);
-        const double x = __dadd_rn(c, __dmul_rn(h, xk));
-        const double fs_inv = (S.Nfs - 1.) / (S.loga - S.loga0);
-        const NodeTerms t =
-            dnu_node_terms(I.B, I.fs_x, I.fs_y, I.fs_c, S.Nfs, S.loga0, fs_inv, I.scalefact, P.Na, x);
-        I.nc_g[q] = t.g;
-        I.nc_fsl[q] = t.fsl;
-        I.nc_dx[q] = t.dx;
-        I.nc_j[q] = t.j;
     }
 }
 
@@ -428,11 +350,9 @@ void launch_batch_update(const BatchDev& b, cudaStream_t st) {
     }
     const int nb = kBatchSmallBlocks;
     kb_prologue<<<b.M < nb ? b.M : nb, 128, 0, st>>>(b);
-    kb_fs_segments<<<nb, 256, 0, st>>>(b, gl);
-    kb_fs_finish<<<b.M < 2 * 152 ? b.M : 2 * 152, 1024, 0, st>>>(b);
-    kb_fs_coeffs<<<nb, 128, 0, st>>>(b);
+    kb_fs_eval<<<4 * nb, kPrepThreads, 0, st>>>(b, gl);
+    kb_tables<<<2 * nb, kBatchTable, 0, st>>>(b);
     kb_dtot_coeffs<<<nb, 128, 0, st>>>(b);
-    kb_nc_build<<<nb, 128, 0, st>>>(b);
     kb_dnu_qag<<<b.qag_blocks, 32 * b.wpb, batch_qag_smem(b.ldmax, b.wpb), st>>>(b);
     kb_finish<<<nb, 256, 0, st>>>(b);
 }

@@ -21,12 +21,14 @@ struct BatchCall {
     int spec[3];
 };
 
+constexpr int kBatchTable = 128;
+
 // Totals of the current call; the kernels are launched with fixed grids (so one
 // captured graph serves every call) and stride over these.
 struct BatchHeader {
     int M;
-    int total_segs;   // fslength segment groups (fs_groups of each instance)
-    int total_fsc;    // sum of max(nfs-2, 0): fslength spline unknowns
+    int total_segs;   // blocks of fslength segments (fs_blocks of each instance)
+    int total_fsc;    // blocks of fslength-table and node-table entries (kBatchTable each)
     int total_bins;   // sum of nk
     int total_tasks;  // sum of nspec*nk over integrating instances
     int counter;      // task queue of kb_dnu_qag (reset by kb_prologue)

@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <vector>
 #include "ksp_batch.h"
+#include "ksp_prep.cuh"
 #include "ksp_ctx.h"
 
 using namespace ksp;
@@ -403,8 +404,11 @@ static int plan_call(kspace_batch* b, const double* a, bool dry, std::vector<int
             }
         }
         const bool integ = P.active && P.commit_row != -2;
-        fs_off[i + 1] = fs_off[i] + (integ && P.nfs > 0 ? fs_groups(P.nfs, P.loga0, P.loga) : 0);
-        fsc_off[i + 1] = fsc_off[i] + (integ && P.nfs > 2 ? P.nfs - 2 : 0);
+        fs_off[i + 1] = fs_off[i] + (integ && P.nfs > 0 ? fs_blocks(P.nfs, P.loga0, P.loga) : 0);
+        fsc_off[i + 1] = fsc_off[i];
+        if (integ && P.nfs > 0)
+            fsc_off[i + 1] += (P.nfs + kBatchTable - 1) / kBatchTable +
+                              (P.Na > 1 ? (b->nc_slots * 61 + kBatchTable - 1) / kBatchTable : 0);
         bin_off[i + 1] = b->off[i + 1];
         task_off[i + 1] = task_off[i] + (integ ? P.nspec * P.nk : 0);
     }

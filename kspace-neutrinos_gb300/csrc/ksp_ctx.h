@@ -93,7 +93,8 @@ struct kspace_ctx {
     bool prep_valid = false;
     int prep_Na = 0;
     double prep_loga = 0;
-    bool prep_base = false;  // launch_dtot_base ran with the preparation
+    bool prep_base = false;  // the rows' splines were solved with the preparation (kRowsBase)
+    ksp::StepScalars S0{};        // the table's part of the scalars (light, prefac, Omeganonu)
     // the binning pass's normalisation, deferred into the row-spline kernel of a prepared
     // step (active = 0: already done)
     ksp::FinalizeArgs fin{};

@@ -355,14 +355,20 @@ struct Gk61Nodes {  // expanded 61-node table: slot j<30: -x_j, 30<=j<60: +x_{j-
     double x[61], wk[61], wg[61];
 };
 
+// the rule in memory: as arrays of the functions that index them they were copied to every
+// thread's stack first (744 bytes, half a microsecond of each integral kernel's start)
+static __device__ const double kGkXK[31] = KSP_GK61_XK_INIT;
+static __device__ const double kGkWK[31] = KSP_GK61_WK_INIT;
+static __device__ const double kGkWG[31] = KSP_GK61_WG_INIT;
+__device__ __forceinline__ double gk61_x(int j) {  // abscissa of slot j
+    return j < 30 ? -__ldg(kGkXK + j) : (j < 60 ? __ldg(kGkXK + j - 30) : 0.0);
+}
 __device__ __forceinline__ void gk61_fill(Gk61Nodes& n, int tid, int nthreads) {
-    const double XK[31] = KSP_GK61_XK_INIT;
-    const double WK[31] = KSP_GK61_WK_INIT;
-    const double WG[31] = KSP_GK61_WG_INIT;
     for (int j = tid; j < 61; j += nthreads) {
-        if (j < 30) { n.x[j] = -XK[j]; n.wk[j] = WK[j]; n.wg[j] = WG[j]; }
-        else if (j < 60) { n.x[j] = XK[j - 30]; n.wk[j] = WK[j - 30]; n.wg[j] = WG[j - 30]; }
-        else { n.x[j] = 0.0; n.wk[j] = WK[30]; n.wg[j] = 0.0; }
+        const int i = j < 30 ? j : j - 30;  // slot 60: the centre, i = 30
+        n.x[j] = gk61_x(j);
+        n.wk[j] = __ldg(kGkWK + i);
+        n.wg[j] = j < 60 ? __ldg(kGkWG + i) : 0.0;
     }
 }
 
@@ -1026,8 +1032,21 @@ struct NodeTerms {
     int j;       // history segment: knot[j] <= x < knot[j+1]
 };
 
-// Not inlined: the table builder and the uncached path run the same compiled code and
+// Not inlined: the table builders and the uncached path run the same compiled code and
 // produce the same numbers bit for bit.
+// 1 / (a H(a)) at x = log a, from 1 / (a^2 H) (one division and the rho_nu segments' stored
+// polynomials instead of hubble()'s ten divisions)
+static __device__ __noinline__ double node_inv_aH(const Background* B, double x) {
+    return exp(x) * fsl_integrand(*B, x);
+}
+// the fslength spline on the segment [x0, x1] at x
+static __device__ __noinline__ double fs_spline_eval(double x0, double x1, double y0, double y1, double c0, double c1,
+                                                     double x) {
+    const double h = x1 - x0, dx = x - x0;
+    const double bq = (y1 - y0) / h - h * (c1 + 2.0 * c0) / 3.0;
+    const double d = (c1 - c0) / (3.0 * h);
+    return y0 + dx * (bq + dx * (c0 + dx * d));
+}
 static __device__ __noinline__ NodeTerms dnu_node_terms(const Background* B, const double* fs_x, const double* fs_y,
                                                  const double* fs_c, int nfs, double fs_x0, double fs_inv,
                                                  const double* kx, int na, double x) {
@@ -1036,19 +1055,10 @@ static __device__ __noinline__ NodeTerms dnu_node_terms(const Background* B, con
     i = i < 0 ? 0 : (i > nfs - 2 ? nfs - 2 : i);
     while (i > 0 && x < fs_x[i]) i--;
     while (i < nfs - 2 && x >= fs_x[i + 1]) i++;
-    {
-        const double x0 = fs_x[i], x1 = fs_x[i + 1];
-        const double y0 = fs_y[i], y1 = fs_y[i + 1];
-        const double c0 = fs_c[i], c1 = fs_c[i + 1];
-        const double h = x1 - x0, dx = x - x0;
-        const double bq = (y1 - y0) / h - h * (c1 + 2.0 * c0) / 3.0;
-        const double d = (c1 - c0) / (3.0 * h);
-        t.fsl = y0 + dx * (bq + dx * (c0 + dx * d));
-    }
+    t.fsl = fs_spline_eval(fs_x[i], fs_x[i + 1], fs_y[i], fs_y[i + 1], fs_c[i], fs_c[i + 1], x);
     t.j = seg_bsearch(kx, na, x);
     t.dx = x - kx[t.j];
-    const double ai = exp(x);
-    t.g = t.fsl / (ai * hubble(*B, ai));
+    t.g = t.fsl * node_inv_aH(B, x);
     return t;
 }
 

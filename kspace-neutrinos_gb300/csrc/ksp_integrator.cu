@@ -4,15 +4,14 @@
 //   k_nufrac_low                hybrid-neutrino fractions (omega_nu_single.c:214-240)
 //   k_update_row                update_delta_tot (delta_tot_table.c:177-191)
 //   k_delta_tot_init            delta_tot_init's per-bin part (delta_tot_table.c:94-129)
-//   k_scalars                   per-call scalars + factorised knot spline system
-//   k_fs_segments/k_fs_finish   the fslength table (delta_tot_table.c:574-591): a
-//                               cumulative fixed-order Gauss-Legendre sum over the 16*Na
-//                               uniform nodes replaces 16*Na adaptive integrals; spline
-//                               coefficients by the closed-form inverse of tridiag(1,4,1)
-//   k_nc_build                  the integrand's bin-independent terms on QAG's right spine
-//   k_dtot_coeffs               natural spline of every history row (shared knots); in a
-//                               prepared step also the binning pass's normalisation and
-//                               the provisional row
+//   k_prep_eval, k_prep_tables  a call's preparation in two kernels (ksp_prep.cuh): the
+//                               scalars, the factorised knot spline system, the fslength
+//                               table (delta_tot_table.c:574-591: sums of fixed-order
+//                               segment integrals over the 16*Na uniform nodes replace 16*Na
+//                               adaptive integrals), the integrand's bin-independent terms on
+//                               QAG's right spine, the natural spline of every history row
+//   k_row_update                a prepared step's provisional row, with the binning pass's
+//                               normalisation
 //   k_dnu_qag                   one warp per (species, bin): history row staged into
 //                               shared memory by a TMA bulk copy, then QAG/GK61 of the
 //                               delta_nu time integral (delta_tot_table.c:492-500,592-599)
@@ -22,6 +21,7 @@
 #include <cuda_runtime.h>
 #include <stdio.h>
 #include "ksp_internal.h"
+#include "ksp_prep.cuh"
 #include "ksp_ptx.cuh"
 
 namespace ksp {
@@ -199,7 +199,7 @@ void launch_update_row(const IntegratorDev& I, int nk, int row, double a, double
     k_update_row<<<(nk + 255) / 256, 256, 0, st>>>(I, nk, row, a, loga, dcdm, dnu);
 }
 
-// the same row from the call's scalars (after k_scalars), delta_nu_last and delta_cdm
+// the same row from the call's scalars (after k_prep_eval), delta_nu_last and delta_cdm
 __global__ void k_update_row_s(IntegratorDev I, int nk, int row) {
     const StepScalars& S = *I.sc;
     for (int ik = blockIdx.x * blockDim.x + threadIdx.x; ik < nk; ik += gridDim.x * blockDim.x)
@@ -247,199 +247,141 @@ void launch_delta_tot_init(const IntegratorDev& I, int nk, const double* wavenum
     k_delta_tot_init<<<(nk + 255) / 256, 256, 0, st>>>(I, nk, wavenum, dcdm, fresh, TimeTransfer);
 }
 
-// ------------------------------------------------------------------ per-call scalars
-// Scalars of the call and the factorised natural-spline system of the history knots
-// x = scalefact[0..Na-1] (shared by every row).  Rows below `start_row` were factorised
-// by an earlier call with the same leading knots and are kept.  Reciprocals are stored
-// so the per-row sweeps need no divisions.
-__global__ void k_scalars(IntegratorDev I, int Na, double a, double loga, double loga0, double TimeTransfer,
-                          int start_row, int write_knot) {
-    if (threadIdx.x == 0) {  // this call's QAG statistics start from zero
-        *I.qag_max = 0;
-        *I.qag_total = 0;
-    }
-    if (write_knot) {  // the provisional knot (update_row writes the same value)
-        if (threadIdx.x == 0) I.scalefact[Na - 1] = loga;
-        __syncthreads();
-    }
-    const double* xk = I.scalefact;
-    for (int i = threadIdx.x; i + 1 < Na; i += blockDim.x) {
-        const double h = xk[i + 1] - xk[i];
-        I.knot_invh[i] = 1.0 / h;
-        I.knot_h3[i] = h / 3.0;
-        I.knot_ih3[i] = 1.0 / (3.0 * h);
-    }
-    if (threadIdx.x < 32) call_scalars_warp(*I.B, a, loga, loga0, TimeTransfer, Na, *I.sc);
-    if (threadIdx.x != 0) return;
-    const double* x = I.scalefact;
-    if (Na > 2) {
-        const int m = Na - 2;
-        for (int i = start_row < 0 ? 0 : start_row; i < m; i++) {
-            const double h0 = x[i + 1] - x[i], h1 = x[i + 2] - x[i + 1];
-            double d = 2.0 * (h0 + h1);
-            if (i > 0) {
-                const double f = h0 * I.knot_invdiag[i - 1];
-                d -= f * h0;
-                I.knot_fac[i] = f;
-            }
-            I.knot_invdiag[i] = 1.0 / d;
-        }
-    }
-}
-
-// ------------------------------------------------------------------ fslength table
+// ------------------------------------------------------------------ preparation of a call
+// Two kernels instead of the eight (scalars, segments, sums, coefficients, nodes, rows, first
+// row, species sum) whose launches and one-thread stretches were 120 of the 163 us of a call
+// with 64 bins and 16 rows.  Blocks by role; every role is parallel.
 struct GL4 { double x[2], w[2]; };  // positive half of the 4-point Gauss-Legendre rule
-
-struct FslIntegrand {  // delta_tot_table.c:378-383
-    const Background* B;
-    __device__ double operator()(double loga) const { return fsl_integrand(*B, loga); }
+struct PrepArgs {
+    StepScalars S;                 // the call's scalars
+    double loga, loga0;
+    int Na, Nfs, nodes;            // Nfs, nodes: 0 without a table
+    int start_row, write_knot;
+    int knot_blocks, fs_blocks, node_blocks;
 };
 
-// The segment integrals of the fslength table, 4 lanes per group (fs_group_eval).
-__global__ void k_fs_segments(IntegratorDev I, int Nfs, double loga0, double loga, GL4 gl, int npts, int ngroups) {
-    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-    fs_group_eval(*I.B, Nfs, loga0, loga, npts, gt >> 2, gt & 3, (gt >> 2) < ngroups, gl.x, gl.w, I.fs_x, I.fs_seg);
-}
-
-// One block: suffix sums of the segment integrals -> fslength at every node.
-__global__ void k_fs_finish(IntegratorDev I, int Nfs) {
-    __shared__ double warp_tot[32];
-    const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, w = t >> 5;
-    const int per = (Nfs + nt - 1) / nt;
-    const int i0 = t * per, i1 = min(Nfs, i0 + per);
-    double loc = 0;
-    for (int i = i1 - 1; i >= i0; i--) loc += I.fs_seg[i];
-    // inclusive suffix scan over the threads of a warp, then over warps
-    double v = loc;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double n = __shfl_down_sync(0xffffffffu, v, o);
-        if (lane + o < 32) v += n;
-    }
-    if (lane == 0) warp_tot[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        const int nwarps = nt >> 5;
-        double u = lane < nwarps ? warp_tot[lane] : 0.0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double n = __shfl_down_sync(0xffffffffu, u, o);
-            if (lane + o < 32) u += n;
+// Block 0: the call's scalars to the device.  Then the knots' spacings and factorised spline system
+// x = scalefact[0..Na-1] (shared by every row; rows below `start_row` were factorised by an
+// earlier call with the same leading knots and are kept), the fslength segments, and the
+// part of the node table that needs no fslength.
+__global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, PrepArgs P, GL4 gl) {
+    __shared__ double f[kPrepThreads], sg[kPrepThreads];
+    const int t = threadIdx.x, Na = P.Na;
+    int b = blockIdx.x;
+    if (b == 0) {
+        if (t == 0) {
+            *I.sc = P.S;
+            *I.qag_max = 0;  // this call's QAG statistics start from zero
+            *I.qag_total = 0;
+            if (P.write_knot) I.scalefact[Na - 1] = P.loga;  // the provisional knot
         }
-        if (lane < nwarps) warp_tot[lane] = u;  // inclusive suffix over warps
+        return;
     }
-    __syncthreads();
-    const double later_warps = (w + 1 < (nt >> 5)) ? warp_tot[w + 1] : 0.0;
-    double run = v - loc + later_warps;  // exclusive suffix of this thread's chunk
-    const double light = I.sc->light;
-    for (int i = i1 - 1; i >= i0; i--) {
-        run += I.fs_seg[i];
-        I.fs_y[i] = light * run;  // fslength(x_i, log a)
-    }
-    __syncthreads();
-    if (t == 0) {
-        I.sc->fsl_A0a = I.fs_y[0];
-        I.sc->Nfs = Nfs;
-        I.fs_c[0] = 0.0;
-        I.fs_c[Nfs - 1] = 0.0;
-    }
-}
-
-// Natural-spline coefficients of the (uniformly spaced) fslength table, one thread per
-// unknown.  The system is tridiag(1,4,1) c = 3 D^2 y / h^2 with known inverse: for
-// mu = 2 - sqrt(3) and 1-based i <= j,
-//   (T^-1)_{ij} = (-1)^{i+j} mu^{j-i} (1-mu^{2i}) (1-mu^{2(m+1-j)}) / (2 sqrt3 (1-mu^{2(m+1)})).
-// Terms with |i-j| > 40 are below 1e-22 relative and dropped.  (Fully parallel: a single
-// table is solved faster this way than by one warp's substitution, whose loads are
-// serial; the batch path, with thousands of tables, uses uniform_spline_warp.)
-__global__ void k_fs_coeffs(IntegratorDev I, int Nfs, double loga0, double loga) {
-    __shared__ double mupow[82];
-    for (int e = threadIdx.x; e < 82; e += blockDim.x) {  // any block size
-        const double mu = 2.0 - sqrt(3.0);
-        double p = 1.0;
-        for (int k = 0; k < e; k++) p *= mu;
-        mupow[e] = p;
-    }
-    __syncthreads();
-    const int m = Nfs - 2;
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= m) return;
-    const double h = (loga - loga0) / (Nfs - 1.);
-    const double scale = 3.0 / (h * h) / (2.0 * sqrt(3.0));
-    const double D = (2 * (m + 1) < 82) ? 1.0 - mupow[2 * (m + 1)] : 1.0;
-    const double* y = I.fs_y;
-    double acc = 0;
-    const int vlo = max(0, u - 40), vhi = min(m - 1, u + 40);
-    for (int v = vlo; v <= vhi; v++) {
-        const int d = v > u ? v - u : u - v;
-        const int lo1 = min(u, v) + 1, hi1 = max(u, v) + 1;
-        const double A = (2 * lo1 < 82) ? 1.0 - mupow[2 * lo1] : 1.0;
-        const int e2 = 2 * (m + 1 - hi1);
-        const double Bf = (e2 < 82) ? 1.0 - mupow[e2] : 1.0;
-        const double r = __ldg(y + v + 2) - 2.0 * __ldg(y + v + 1) + __ldg(y + v);
-        acc += ((d & 1) ? -mupow[d] : mupow[d]) * A * Bf * r;
-    }
-    I.fs_c[u + 1] = acc * scale / D;
-}
-
-// ------------------------------------------------------------------ history splines
-// Forward/back substitution of every history row against the shared factorisation,
-// warp per row (warp-parallel affine scans when the row fits in shared memory).
-__global__ void k_dtot_coeffs(IntegratorDev I, int nk, int Na, int staged, int update_row, FinalizeArgs fin) {
-    extern __shared__ __align__(16) double sdc[];
-    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    double* sy = staged ? sdc + (size_t)warp * 2 * I.ld : nullptr;
-    double* sc = staged ? sy + I.ld : nullptr;
-    for (int ik = blockIdx.x * nw + warp; ik < nk; ik += gridDim.x * nw) {
-        if (fin.active && (threadIdx.x & 31) == 0) finalize_bin(fin, ik);  // this bin's delta_cdm first
-        if (update_row >= 0) {  // update_delta_tot (delta_tot_table.c:177-191), as k_update_row
-            if ((threadIdx.x & 31) == 0) {
-                const StepScalars& S = *I.sc;
-                I.dtot[(size_t)ik * I.ld + update_row] =
-                    get_delta_tot(I.nu_last[ik], I.dcdm[ik], S.OmegaNua3, S.Omeganonu, S.OmegaNu1, S.partnu);
-            }
-            __syncwarp();
+    b--;
+    if (b < P.knot_blocks) {
+        const double* x = I.scalefact;
+        auto knot = [&](int j) { return P.write_knot && j == Na - 1 ? P.loga : x[j]; };
+        const int i = b * kPrepThreads + t;
+        if (i + 1 < Na) {
+            const double h = knot(i + 1) - knot(i);
+            I.knot_invh[i] = 1.0 / h;
+            I.knot_h3[i] = h / 3.0;
+            I.knot_ih3[i] = 1.0 / (3.0 * h);
         }
-        if (staged) dtot_row_coeffs_scan(I, ik, Na, sy, sc);
-        else dtot_row_coeffs_warp(I, ik, Na, nullptr, nullptr);
+        if (i < Na - 2 && i >= P.start_row) knot_row(knot, i, I.knot_invdiag, I.knot_fac);
+        return;
     }
+    b -= P.knot_blocks;
+    if (b < P.fs_blocks) {
+        fs_eval_block(*I.B, P.Nfs, P.loga0, P.loga, b, gl.x[0], gl.x[1], gl.w[0], gl.w[1], f, sg, I.fs_seg, I.fs_suf,
+                      I.fs_tot);
+        return;
+    }
+    b -= P.fs_blocks;
+    const int q = b * kPrepThreads + t;
+    if (q >= P.nodes) return;
+    const double x = nc_node_x(q, P.loga0, P.loga);
+    const int j = seg_bsearch(I.scalefact, Na, x);  // (the last knot is not read)
+    I.nc_j[q] = j;
+    I.nc_dx[q] = x - I.scalefact[j];
+    I.nc_inv[q] = node_inv_aH(I.B, x);
 }
 
-// ------------------------------------------------------------------ row splines in two parts
-// A history row's natural spline is linear in the row, and the provisional (last) knot
-// enters the spline system through its last right-hand side only, so
+// The fslength table, the node table, and the row splines.
+//
+// Rows (RowsMode): a history row's natural spline is linear in the row, and the
+// provisional (last) knot enters the spline system through its last right-hand side only, so
 //   c = c_base + (y_new - y_base) c_unit,
 // with c_base the coefficients of the row whose last knot is y_base (the knot before it)
 // and c_unit those of a unit last knot with all other knots zero.  Both depend only on
-// the committed rows and the knots: k_dtot_base solves them beside the binning pass
-// (block nk: c_unit).  After it, k_row_update forms y_new (update_delta_tot,
+// the committed rows and the knots: kRowsBase solves them beside the binning pass
+// (row nk: c_unit).  After it, k_row_update forms y_new (update_delta_tot,
 // delta_tot_table.c:177-191) from this step's delta_cdm and adds the correction, in
 // place of the solve.  y_new - y_base is one step's growth of delta_tot, so the sum does
-// not cancel.
-__global__ void k_dtot_base(IntegratorDev I, int nk, int Na) {
-    // in place in the coefficient rows (global memory, L1-cached): the binning pass holds
-    // nearly all of every SM's shared memory, and these blocks run beside it
-    const int lane = threadIdx.x & 31;
-    const int m = Na - 2;  // unknowns c[1..m]
-    const double* ih = I.knot_invh;
-    double* c;
-    if (blockIdx.x == nk) {
-        c = I.coef_unit;
-        for (int u = lane; u < m; u += 32) c[u + 1] = u == m - 1 ? 3.0 * ih[m] : 0.0;
-    } else {
-        const double* y = I.dtot + (size_t)blockIdx.x * I.ld;
-        c = I.coef + (size_t)blockIdx.x * I.ld;
-        for (int u = lane; u < m; u += 32) {
-            const double y2 = u == m - 1 ? y[m] : y[u + 2];  // the last knot taken equal to the one before
-            c[u + 1] = 3.0 * ((y2 - y[u + 1]) * ih[u + 1] - (y[u + 1] - y[u]) * ih[u]);
+// not cancel.  The solves work in place in the coefficient rows (global memory,
+// L1-cached): the binning pass holds nearly all of every SM's shared memory.
+constexpr int kTableThreads = 128;
+__global__ void __launch_bounds__(kTableThreads, 8)
+    k_prep_tables(IntegratorDev I, PrepArgs P, int rows, int nk, int update_row) {
+    __shared__ double tsuf[kPrepThreads + 1], sh[2 * kTableThreads / 32];
+    const int t = threadIdx.x, Na = P.Na;
+    int b = blockIdx.x;
+    const int nrow = rows == kRowsBase ? nk + 1 : (rows == kRowsFull ? nk : 0);
+    if (b < nrow) {
+        const int m = Na - 2;  // unknowns c[1..m]
+        const double* ih = I.knot_invh;
+        double* c;
+        if (b == nk) {
+            c = I.coef_unit;
+            for (int u = t; u < m; u += kTableThreads) c[u + 1] = u == m - 1 ? 3.0 * ih[m] : 0.0;
+        } else {
+            double* y = I.dtot + (size_t)b * I.ld;
+            c = I.coef + (size_t)b * I.ld;
+            if (update_row >= 0) {
+                if (t == 0) {
+                    const StepScalars& S = *I.sc;
+                    y[update_row] =
+                        get_delta_tot(I.nu_last[b], I.dcdm[b], S.OmegaNua3, S.Omeganonu, S.OmegaNu1, S.partnu);
+                }
+                __syncthreads();
+            }
+            for (int u = t; u < m; u += kTableThreads) {
+                // (base: the last knot taken equal to the one before)
+                const double y2 = rows == kRowsBase && u == m - 1 ? y[m] : y[u + 2];
+                c[u + 1] = 3.0 * ((y2 - y[u + 1]) * ih[u + 1] - (y[u + 1] - y[u]) * ih[u]);
+            }
         }
+        if (m < 1) return;
+        __syncthreads();
+        spline_solve_block<kTableThreads>(I, m, c, sh);
+        if (t == 0) {
+            c[0] = 0.0;
+            c[Na - 1] = 0.0;
+        }
+        return;
     }
-    __syncwarp();
-    spline_solve_scan(I, m, c);
-    if (lane == 0) {
-        c[0] = 0.0;
-        c[Na - 1] = 0.0;
+    b -= nrow;
+    const FsTable F = fs_table(I, P.Nfs, P.loga0, P.loga, P.S.light, tsuf);
+    const int table_blocks = (P.Nfs + kTableThreads - 1) / kTableThreads;
+    if (b < table_blocks) {
+        const int i = b * kTableThreads + t;
+        if (i >= P.Nfs) return;
+        I.fs_x[i] = fs_node(i, P.Nfs, P.loga0, P.loga);
+        const double y = fs_table_y(F, i);
+        I.fs_y[i] = y;
+        I.fs_c[i] = fs_table_c(F, i);
+        if (i == 0) {
+            I.sc->fsl_A0a = y;
+            I.sc->Nfs = P.Nfs;
+        }
+        return;
     }
+    const int q = (b - table_blocks) * kTableThreads + t;
+    if (q >= P.nodes) return;
+    const double x = nc_node_x(q, P.loga0, P.loga);
+    const double fsl = fs_table_at(F, P.loga0, P.loga, x);
+    I.nc_fsl[q] = fsl;
+    I.nc_g[q] = fsl * I.nc_inv[q];
 }
 
 // block per bin: this bin's delta_cdm (a deferred normalisation), the provisional row
@@ -459,35 +401,6 @@ __global__ void k_row_update(IntegratorDev I, int nk, int Na, int row, FinalizeA
     const double dy = s_dy;
     double* c = I.coef + (size_t)ik * I.ld;
     for (int k = 1 + threadIdx.x; k < Na - 1; k += blockDim.x) c[k] = fma(dy, __ldg(I.coef_unit + k), c[k]);
-}
-
-bool launch_dtot_base(const IntegratorDev& I, int nk, int Na, cudaStream_t st) {
-    if (Na <= 2 || nk <= 0) return false;
-    k_dtot_base<<<nk + 1, 32, 0, st>>>(I, nk, Na);
-    return cudaPeekAtLastError() == cudaSuccess;
-}
-
-// ------------------------------------------------------------------ node table
-// The k-independent terms of the delta_nu integrand at the 61 nodes of the first
-// kNcLevels levels of QAG's bisection of [log a0, log a]: thread per (slot, node).
-__global__ void k_nc_build(IntegratorDev I, int Na) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= I.nc_slots * 61) return;
-    const StepScalars& S = *I.sc;
-    const int slot = q / 61, jn = q - 61 * slot;
-    double lo, hi;
-    nc_interval(slot, S.loga0, S.loga, &lo, &hi);
-    const double c = __dmul_rn(0.5, __dadd_rn(lo, hi));
-    const double h = __dmul_rn(0.5, __dsub_rn(hi, lo));
-    const double XK[31] = KSP_GK61_XK_INIT;  // the abscissae of gk61_fill
-    const double xk = jn < 30 ? -XK[jn] : (jn < 60 ? XK[jn - 30] : 0.0);
-    const double x = __dadd_rn(c, __dmul_rn(h, xk));
-    const double fs_inv = (S.Nfs - 1.) / (S.loga - S.loga0);
-    const NodeTerms t = dnu_node_terms(I.B, I.fs_x, I.fs_y, I.fs_c, S.Nfs, S.loga0, fs_inv, I.scalefact, Na, x);
-    I.nc_g[q] = t.g;
-    I.nc_fsl[q] = t.fsl;
-    I.nc_dx[q] = t.dx;
-    I.nc_j[q] = t.j;
 }
 
 // ------------------------------------------------------------------ delta_nu integral
@@ -802,60 +715,52 @@ size_t dnu_qag_smem(int ld, int wpb) {
            wpb * (sizeof(QagList) + 4 * sizeof(double) * ld) + wpb * sizeof(uint64_t);
 }
 
-// The part of a call that does not depend on the current delta_cdm: the scalars and the
-// knot factorisation, the fslength table, the node table.  Can run concurrently with
-// the binning pass (write_knot = 1 also stores the provisional knot, log a).
-void launch_integrator_prepare(const IntegratorDev& I, int Na, double a, double loga, double loga0,
-                               double TimeTransfer, int start_row, int write_knot, bool scalars_only,
-                               cudaStream_t st) {
+// Blocks per role of a call's preparation.
+void launch_integrator_prepare(const IntegratorDev& I, const Background& B, const StepScalars& S, int Na, double a,
+                               double loga, double loga0, double TimeTransfer, int start_row, int write_knot,
+                               bool scalars_only, RowsMode rows, int nk, int update_row, cudaStream_t st) {
     static const GL4 gl = gl4_host();
-    k_scalars<<<1, 256, 0, st>>>(I, Na, a, loga, loga0, TimeTransfer, start_row, write_knot);
-    if (scalars_only) return;
-    // the fslength table (always built: it also gives fslength(log a0, log a))
-    const int Nfs = 16 * (Na > 1 ? Na : 1);
-    if (loga > loga0) {
-        const int npts = fs_rule_points(Nfs, loga0, loga), ngroups = fs_groups(Nfs, loga0, loga);
-        const long long threads = 4LL * ngroups;
-        k_fs_segments<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(I, Nfs, loga0, loga, gl, npts, ngroups);
-        k_fs_finish<<<1, 1024, 0, st>>>(I, Nfs);
-        if (Nfs > 2) k_fs_coeffs<<<(Nfs - 2 + 31) / 32, 32, 0, st>>>(I, Nfs, loga0, loga);
-    } else {
-        cudaMemsetAsync(&I.sc->fsl_A0a, 0, sizeof(double), st);
-        cudaMemsetAsync(&I.sc->Nfs, 0, sizeof(int), st);
+    PrepArgs P{};
+    P.S = S;
+    call_scalars(B, a, loga, loga0, TimeTransfer, Na, P.S);
+    P.loga = loga;
+    P.loga0 = loga0;
+    P.Na = Na;
+    P.start_row = start_row < 0 ? 0 : start_row;
+    P.write_knot = write_knot;
+    if (scalars_only) {  // block 0
+        k_prep_eval<<<1, kPrepThreads, 0, st>>>(I, P, gl);
+        return;
     }
-    if (loga > loga0 && Na > 1 && I.nc_slots > 0)
-        k_nc_build<<<(I.nc_slots * 61 + 63) / 64, 64, 0, st>>>(I, Na);
+    P.knot_blocks = (Na - 1 + kPrepThreads - 1) / kPrepThreads;
+    if (loga > loga0) {  // the fslength table also gives fslength(log a0, log a)
+        P.Nfs = 16 * (Na > 1 ? Na : 1);
+        P.fs_blocks = fs_blocks(P.Nfs, loga0, loga);
+        P.nodes = Na > 1 ? I.nc_slots * 61 : 0;
+        P.node_blocks = (P.nodes + kPrepThreads - 1) / kPrepThreads;
+    }
+    k_prep_eval<<<1 + P.knot_blocks + P.fs_blocks + P.node_blocks, kPrepThreads, 0, st>>>(I, P, gl);
+    const int nrow = rows == kRowsBase ? nk + 1 : (rows == kRowsFull && (Na > 2 || update_row >= 0) ? nk : 0);
+    const int blocks = nrow + (P.Nfs + kTableThreads - 1) / kTableThreads +
+                       (P.nodes + kTableThreads - 1) / kTableThreads;
+    if (blocks > 0)
+        k_prep_tables<<<blocks, kTableThreads, 0, st>>>(I, P, nrow > 0 ? (int)rows : (int)kRowsNone, nk, update_row);
 }
 
-// The rest, after the provisional history row: spline coefficients of the rows, the
-// integrals, the species sum.
+// The rest, after the rows' splines: the integrals, the species sum.
 void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, const int* spec_ids,
                             int warps_per_block, cudaStream_t st, int qag_split, int update_row, bool defer_combine,
                             const FinalizeArgs* fin, bool base_ready) {
-    // a deferred normalisation runs in the row-spline kernel, or on its own without one
-    FinalizeArgs fa{};
-    if (fin && fin->active) {
-        if (Na > 2) fa = *fin;
-        else
+    if (update_row >= 0 && base_ready) {
+        FinalizeArgs fa{};
+        if (fin && fin->active) fa = *fin;
+        k_row_update<<<nk, 128, 0, st>>>(I, nk, Na, update_row, fa);
+    } else if (update_row >= 0) {
+        // a history of two knots: no splines
+        if (fin && fin->active)
             launch_finalize_power(fin->bin_sum, fin->F0sq, fin->count, fin->ksum, fin->compact_bins, nk, fin->BoxSize,
                                   fin->power_out, fin->keff_out, fin->dcdm_out, fin->keffphys_out, st);
-    }
-    if (update_row >= 0 && Na <= 2) {
         launch_update_row_scalars(I, nk, update_row, st);
-        update_row = -1;
-    }
-    if (Na > 2 && base_ready && update_row == Na - 1) {
-        k_row_update<<<nk, 128, 0, st>>>(I, nk, Na, update_row, fa);
-    } else if (Na > 2) {
-        static bool dc_attr = false;
-        if (!dc_attr) {
-            raise_dynamic_smem_limit(reinterpret_cast<const void*>(k_dtot_coeffs));
-            dc_attr = true;
-        }
-        // a warp (one row at a time) per block: the latency-bound solves spread over SMs
-        const size_t smem = 2 * sizeof(double) * I.ld;
-        const int staged = smem <= 200 * 1024;
-        k_dtot_coeffs<<<nk, 32, staged ? smem : 0, st>>>(I, nk, Na, staged, update_row, fa);
     }
     int wpb = warps_per_block < 1 ? 1 : (warps_per_block > 4 ? 4 : warps_per_block);
     while (wpb > 1 && dnu_qag_smem(I.ld, wpb) > 227 * 1024 - 256) wpb--;
@@ -899,14 +804,6 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
         }
     }
     if (!defer_combine) k_combine<<<(nk + 255) / 256, 256, 0, st>>>(I, nk);
-}
-
-void launch_delta_nu_combined(const IntegratorDev& I, int nk, int Na, double a, double loga, double loga0,
-                              double TimeTransfer, int start_row, int nspec, const int* spec_ids,
-                              int warps_per_block, cudaStream_t st, int qag_split) {
-    launch_integrator_prepare(I, Na, a, loga, loga0, TimeTransfer, start_row, 0, nk <= 0, st);
-    if (nk <= 0) return;  // scalars only
-    launch_integrator_rest(I, nk, Na, nspec, spec_ids, warps_per_block, st, qag_split);
 }
 
 // ------------------------------------------------------------------ end of an update

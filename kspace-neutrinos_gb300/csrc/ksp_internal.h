@@ -8,7 +8,7 @@
 namespace ksp {
 
 // Scalars of one integrator call at scale factor a (delta_tot_table.c:153-172,507-548,
-// interface_common.c:139-145), computed on the device by k_scalars.
+// interface_common.c:139-145), formed by call_scalars.
 struct StepScalars {
     double a, loga, loga0;           // inputs (logs taken on the host, as the reference does)
     double light, prefac, Omeganonu; // delta_tot_table.c:52-57
@@ -52,7 +52,10 @@ struct IntegratorDev {
     double* fs_x;                    // [fs_cap]
     double* fs_y;                    // [fs_cap]
     double* fs_c;                    // [fs_cap]
-    double* fs_seg;                  // [fs_cap]
+    double* fs_seg;                  // [fs_cap] integrals of 1/(a^2 H) over the table's segments
+    double* fs_suf;                  // [fs_cap] their suffix sums within a block's stretch
+    double* fs_tot;                  // [fs_cap / 16 + 1] the stretches' totals
+    double* nc_inv;                  // [kNcNodes] 1/(a H) at the nodes
     int fs_cap;
     double* t_logk;                  // transfer table [ntrans]
     double* t_T;
@@ -65,13 +68,41 @@ struct IntegratorDev {
     double* ivals;                   // optional: final QAG intervals [kNuSpecies][nk_alloc][kQagLimit][2]
     int* nivals;                     // [kNuSpecies][nk_alloc]
     double* coef_unit;               // [ld] spline coefficients of a unit provisional (last) knot,
-                                     // the other knots zero (k_dtot_base)
+                                     // the other knots zero (kRowsBase)
 };
 
+// The part of StepScalars that a call sets (the rest is set with the table): on the host
+// for a single call, where it takes about a microsecond beside the launches (on the device
+// it was a chain of some 60 dependent FP64 divisions, 12 us of each call).
+inline void call_scalars(const Background& B, double a, double loga, double loga0, double TT, int Na, StepScalars& S) {
+    const double om_a = omega_nu(B, a), om_1 = omega_nu(B, 1), partnu = particle_nu_fraction(B, a, 0);
+    const double nop = om_a - om_1 * partnu / (a * a * a);  // omega_nu_nopart (omega_nu_single.c:69-74)
+    S.a = a;
+    S.loga = loga;
+    S.loga0 = loga0;
+    S.Na = Na;
+    S.OmegaNua3 = nop * (a * a * a);
+    S.OmegaNu1 = om_1;
+    S.partnu = partnu;
+    S.Omega_nu_tot = nop;
+    for (int mi = 0; mi < kNuSpecies; mi++) S.omeganu[mi] = B.deg[mi] > 0 ? B.deg[mi] * omega_nu_single(B, a, mi) : 0.0;
+    S.deriv_prefac = TT * (hubble(B, TT) / S.light) * TT;
+    S.relerr = 1e-6;
+    S.partnu_now = partnu;
+    S.skip_integral = 0;
+    if (S.partnu_now > 0) {
+        if (1 - S.partnu_now < 1e-3) S.skip_integral = 1;
+        S.relerr /= (1. + 1e-5 - S.partnu_now);
+    }
+    S.kspace_prefac = nop / (S.Omeganonu / (a * a * a) + (om_a - nop));
+    S.fsl_A0a = 0;
+    S.Nfs = 0;
+}
+
 #ifdef __CUDACC__
-// The scalars of a call at a (as k_scalars, delta_tot_table.c:153-172,507-548,
-// interface_common.c:139-145), by one warp: the background evaluations, which are long
-// FP64 dependency chains, run on different lanes; lane 0 combines them.
+// The same on the device, for batches: the scalars of a call at a (delta_tot_table.c:153-172,
+// 507-548, interface_common.c:139-145), by one warp: the background evaluations, which are
+// long FP64 dependency chains, run on different lanes; lane 0 combines them.
 __device__ __forceinline__ void call_scalars_warp(const Background& B, double a, double loga, double loga0,
                                                   double TT, int Na, StepScalars& S) {
     const int lane = threadIdx.x & 31;
@@ -108,198 +139,12 @@ __device__ __forceinline__ void call_scalars_warp(const Background& B, double a,
     S.kspace_prefac = nop / (S.Omeganonu / (a * a * a) + (om_a - nop));
 }
 
-// Natural-spline coefficients of one history row against the shared factorisation of
-// the knot system (knot_fac, knot_invdiag from k_scalars), by one warp: the row is
-// staged in shared memory with coalesced loads, lane 0 runs the forward and back
-// substitutions there, and the warp writes the coefficients back coalesced.
-// sy, sc: ld doubles of shared memory each, or null to work in global memory (rows
-// too long for shared memory).
-__device__ __forceinline__ void dtot_row_coeffs_warp(const IntegratorDev& I, int ik, int Na, double* sy,
-                                                     double* sc) {
-    const int lane = threadIdx.x & 31;
-    const double* y = I.dtot + (size_t)ik * I.ld;
-    double* c = I.coef + (size_t)ik * I.ld;
-    const bool staged = sy != nullptr;
-    if (staged) {
-        for (int k = lane; k < Na; k += 32) sy[k] = y[k];
-    } else {
-        sy = const_cast<double*>(y);
-        sc = c;
-    }
-    __syncwarp();
-    if (lane == 0) {
-        const double* ih = I.knot_invh;
-        const int m = Na - 2;
-        double prev = 0;
-        for (int k = 0; k < m; k++) {
-            double r = 3.0 * ((sy[k + 2] - sy[k + 1]) * ih[k + 1] - (sy[k + 1] - sy[k]) * ih[k]);
-            if (k > 0) r -= I.knot_fac[k] * prev;
-            prev = r;
-            sc[k + 1] = r;
-        }
-        sc[0] = 0.0;
-        sc[Na - 1] = 0.0;
-        double next = sc[m] * I.knot_invdiag[m - 1];
-        sc[m] = next;
-        const double* x = I.scalefact;
-        for (int k = m - 1; k-- > 0;) {
-            const double off = x[k + 2] - x[k + 1];
-            next = (sc[k + 1] - off * next) * I.knot_invdiag[k];
-            sc[k + 1] = next;
-        }
-    }
-    __syncwarp();
-    if (staged)
-        for (int k = lane; k < Na; k += 32) c[k] = sc[k];
-    __syncwarp();
-}
-
-// The fslength table's segment integrals (the segments between its 16*Na uniform knots
-// in log a): a group of 4 lanes takes one segment with the 4-point Gauss-Legendre rule
-// or, where the knots are closer than 1.5e-3 in log a (the 2-point rule's relative
-// error per segment is then below ~3e-14 for this smooth integrand), two segments with
-// the 2-point rule.
-__host__ __device__ inline int fs_rule_points(int Nfs, double loga0, double loga) {
-    return (loga - loga0) / (Nfs - 1.) < 1.5e-3 ? 2 : 4;
-}
-__host__ __device__ inline int fs_groups(int Nfs, double loga0, double loga) {
-    return fs_rule_points(Nfs, loga0, loga) == 4 ? Nfs : (Nfs + 1) / 2;
-}
-#ifdef __CUDACC__
-// lane q (0..3) of group g; called by whole warps (groups are aligned to 4 lanes).
-// gx, gw: the positive half of the 4-point rule.
-__device__ __forceinline__ void fs_group_eval(const Background& B, int Nfs, double loga0, double loga, int npts,
-                                              int g, int q, bool live, const double* gx, const double* gw,
-                                              double* fs_x, double* fs_seg) {
-    double v = 0.0;
-    int seg = -1;
-    if (live) {
-        const int node = npts == 4 ? q : (q & 1);
-        seg = npts == 4 ? g : 2 * g + (q >> 1);
-        if (seg < Nfs) {
-            const double xa = loga0 + seg * (loga - loga0) / (Nfs - 1.);
-            double xb = loga0 + (seg + 1) * (loga - loga0) / (Nfs - 1.);
-            if (seg == Nfs - 1) xb = loga;
-            if (xb > xa) {
-                const double c = 0.5 * (xa + xb), h = 0.5 * (xb - xa);
-                double x, w;
-                if (npts == 4) {
-                    const int j = node & 1;
-                    x = node < 2 ? c - h * gx[j] : c + h * gx[j];
-                    w = gw[j];
-                } else {
-                    x = node ? c + h * 0.57735026918962576451 : c - h * 0.57735026918962576451;  // 1/sqrt(3)
-                    w = 1.0;
-                }
-                v = w * h * fsl_integrand(B, x);
-            }
-            if (node == 0) fs_x[seg] = xa;
-        } else {
-            seg = -1;
-        }
-    }
-    const double s1 = v + __shfl_down_sync(0xffffffffu, v, 1, 4);
-    const double s2 = s1 + __shfl_down_sync(0xffffffffu, s1, 2, 4);
-    if (seg >= 0) {
-        if (npts == 4 && q == 0) fs_seg[seg] = s2;
-        if (npts == 2 && (q & 1) == 0) fs_seg[seg] = s1;
-    }
-}
-#endif
-
-// Natural-spline second derivatives c[0..n-1] of a table y on uniform spacing h, by
-// one warp: tridiag(1,4,1) c[1..n-2] = 3/h^2 (y[u+2] - 2 y[u+1] + y[u]), c[0] = c[n-1]
-// = 0.  Gaussian elimination has pivots d_0 = 4, d_u = 4 - 1/d_{u-1}; they reach
-// 2 + sqrt(3) to double precision by u = 40, and d_u = d_40 is used from there on.
-// Forward and back substitution are chains of affine maps, composed per lane over a
-// stretch of rows, then across lanes by a warp scan, then replayed (as
-// spline_solve_scan).  c holds the forward pass's results in between.
-struct UniformPivots {
-    double inv[41];  // 1 / d_u, u = 0..40
-    constexpr UniformPivots() : inv() {
-        double d = 4.0;
-        for (int u = 0; u <= 40; u++) {
-            if (u > 0) d = 4.0 - 1.0 / d;
-            inv[u] = 1.0 / d;
-        }
-    }
-};
-static __constant__ UniformPivots kUniformPivots{};
-__device__ __forceinline__ double uniform_inv_pivot(int u) { return kUniformPivots.inv[u < 40 ? u : 40]; }
-__device__ __forceinline__ void uniform_spline_warp(const double* y, double* c, int n, double h) {
-    const int lane = threadIdx.x & 31;
-    const int m = n - 2;
-    if (m >= 1) {
-        const double s3 = 3.0 / (h * h);
-        const int per = (m + 31) / 32;
-        const int u0 = min(m, lane * per), u1 = min(m, u0 + per);
-        // forward: z_u = r_u - z_{u-1} / d_{u-1}
-        double A = 1.0, B = 0.0;
-        for (int u = u0; u < u1; u++) {
-            const double f = u > 0 ? uniform_inv_pivot(u - 1) : 0.0;
-            B = s3 * (y[u + 2] - 2.0 * y[u + 1] + y[u]) - f * B;
-            A = -f * A;
-        }
-        double pa = A, pb = B;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const double qa = __shfl_up_sync(0xffffffffu, pa, d), qb = __shfl_up_sync(0xffffffffu, pb, d);
-            if (lane >= d) {
-                pb = pa * qb + pb;
-                pa = pa * qa;
-            }
-        }
-        double zin = __shfl_up_sync(0xffffffffu, pb, 1);
-        if (lane == 0) zin = 0.0;
-        for (int u = u0; u < u1; u++) {
-            const double f = u > 0 ? uniform_inv_pivot(u - 1) : 0.0;
-            zin = s3 * (y[u + 2] - 2.0 * y[u + 1] + y[u]) - f * zin;
-            c[u + 1] = zin;
-        }
-        __syncwarp();
-        // back: x_u = (z_u - x_{u+1}) / d_u, x_m = 0
-        A = 1.0;
-        B = 0.0;
-        for (int u = u1 - 1; u >= u0; u--) {
-            const double iv = uniform_inv_pivot(u);
-            const double off = u < m - 1 ? 1.0 : 0.0;
-            B = (c[u + 1] - off * B) * iv;
-            A = -off * iv * A;
-        }
-        pa = A;
-        pb = B;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const double qa = __shfl_down_sync(0xffffffffu, pa, d), qb = __shfl_down_sync(0xffffffffu, pb, d);
-            if (lane + d < 32) {
-                pb = pa * qb + pb;
-                pa = pa * qa;
-            }
-        }
-        double cin = __shfl_down_sync(0xffffffffu, pb, 1);
-        if (lane == 31) cin = 0.0;
-        __syncwarp();
-        for (int u = u1 - 1; u >= u0; u--) {
-            const double off = u < m - 1 ? 1.0 : 0.0;
-            cin = (c[u + 1] - off * cin) * uniform_inv_pivot(u);
-            c[u + 1] = cin;
-        }
-    }
-    if (lane == 0) {
-        c[0] = 0.0;
-        c[n - 1] = 0.0;
-    }
-    __syncwarp();
-}
-
-// The same solve with all 32 lanes: both substitutions are linear recurrences
-// z_u = r_u - f_u z_{u-1} and c_u = (z_u - o_u c_{u+1}) / d_u, i.e. chains of affine
-// maps; each lane composes the maps of its stretch of rows, a warp scan composes the
-// stretches, and each lane then replays its stretch from the value entering it.  The
-// results equal the sequential sweep's up to rounding.  sy, sc: ld doubles of shared
-// memory each (staged rows).
-// Solve the natural-spline system of the knots (factorised by k_scalars) for the
-// right-hand side sc[1..m], m = Na - 2, in place, with all 32 lanes of a warp.
+// Solve the natural-spline system of the knots (factorised by knot_row) for the
+// right-hand side sc[1..m], m = Na - 2, in place, with all 32 lanes of a warp: both
+// substitutions are linear recurrences z_u = r_u - f_u z_{u-1} and c_u = (z_u - o_u c_{u+1}) /
+// d_u, i.e. chains of affine maps; each lane composes the maps of its stretch of rows, a
+// warp scan composes the stretches, and each lane then replays its stretch from the
+// value entering it.
 __device__ __forceinline__ void spline_solve_scan(const IntegratorDev& I, int m, double* sc) {
     const int lane = threadIdx.x & 31;
     const double* x = I.scalefact;
@@ -356,29 +201,6 @@ __device__ __forceinline__ void spline_solve_scan(const IntegratorDev& I, int m,
         cin = (sc[u + 1] - off * cin) * I.knot_invdiag[u];
         sc[u + 1] = cin;
     }
-    __syncwarp();
-}
-
-// The same solve with all 32 lanes: both substitutions are linear recurrences
-// z_u = r_u - f_u z_{u-1} and c_u = (z_u - o_u c_{u+1}) / d_u, i.e. chains of affine
-// maps; each lane composes the maps of its stretch of rows, a warp scan composes the
-// stretches, and each lane then replays its stretch from the value entering it.  The
-// results equal the sequential sweep's up to rounding.  sy, sc: ld doubles of shared
-// memory each (staged rows).
-__device__ __forceinline__ void dtot_row_coeffs_scan(const IntegratorDev& I, int ik, int Na, double* sy,
-                                                     double* sc) {
-    const int lane = threadIdx.x & 31;
-    const double* y = I.dtot + (size_t)ik * I.ld;
-    double* c = I.coef + (size_t)ik * I.ld;
-    for (int k = lane; k < Na; k += 32) sy[k] = y[k];
-    __syncwarp();
-    const int m = Na - 2;  // unknowns c[1..m]
-    const double* ih = I.knot_invh;
-    for (int u = lane; u < m; u += 32)
-        sc[u + 1] = 3.0 * ((sy[u + 2] - sy[u + 1]) * ih[u + 1] - (sy[u + 1] - sy[u]) * ih[u]);
-    __syncwarp();
-    spline_solve_scan(I, m, sc);
-    for (int k = lane; k < Na; k += 32) c[k] = (k == 0 || k == Na - 1) ? 0.0 : sc[k];
     __syncwarp();
 }
 
@@ -489,30 +311,31 @@ void launch_update_row(const IntegratorDev& I, int nk, int row, double a, double
 // delta_tot_init part that needs the device (delta_tot_table.c:94-129)
 void launch_delta_tot_init(const IntegratorDev& I, int nk, const double* wavenum, const double* dcdm,
                            int fresh, double TimeTransfer, cudaStream_t st);
-// get_delta_nu_combined (delta_tot_table.c:153-172) with Na rows: writes I.dnu
-// start_row: leading rows of the knot factorisation still valid from an earlier call
-// qag_split: warps per (species, bin) task (1, 2 or 4; 0 = chosen by the task count)
-void launch_delta_nu_combined(const IntegratorDev& I, int nk, int Na, double a, double loga, double loga0,
-                              double TimeTransfer, int start_row, int nspec, const int* spec_ids,
-                              int warps_per_block, cudaStream_t st, int qag_split = 0);
-// the same in two parts: what does not depend on delta_cdm (may overlap the binning
-// pass; write_knot stores the provisional knot log a), and the rest
-void launch_integrator_prepare(const IntegratorDev& I, int Na, double a, double loga, double loga0,
-                               double TimeTransfer, int start_row, int write_knot, bool scalars_only,
-                               cudaStream_t st);
-// update_row >= 0: write the provisional row `update_row` (update_delta_tot, from
-// delta_nu_last and delta_cdm with the call's scalars) as each row's spline is solved;
+// A call's preparation (scalars, knot factorisation, fslength and node tables) and, with
+// it, the splines of the history rows.
+// start_row: leading rows of the knot factorisation still valid from an earlier call;
+// write_knot stores the provisional knot log a
+enum RowsMode {
+    kRowsNone,  // no row splines
+    kRowsBase,  // before the provisional row is known (beside the binning pass): every row's
+                // spline with its last knot equal to the one before, and that of a unit last
+                // knot; launch_integrator_rest adds the provisional row as a correction
+    kRowsFull   // every row's spline; update_row >= 0: after writing the provisional row
+                // `update_row` (update_delta_tot, from delta_nu_last and delta_cdm)
+};
+// S: the table's scalars (light, prefac, Omeganonu); B: the background's host copy
+void launch_integrator_prepare(const IntegratorDev& I, const Background& B, const StepScalars& S, int Na, double a,
+                               double loga, double loga0, double TimeTransfer, int start_row, int write_knot,
+                               bool scalars_only, RowsMode rows, int nk, int update_row, cudaStream_t st);
+// The rest: the integrals and the species sum (get_delta_nu_combined,
+// delta_tot_table.c:153-172, writes I.dnu).
+// update_row >= 0: with a prepared step's provisional row first (base_ready: kRowsBase ran);
+// qag_split: warps per (species, bin) task (1, 2, 4 or 8; 0 = chosen by the task count)
 // defer_combine: leave the species sum to launch_finish_update(..., combine = true)
-// base_ready: launch_dtot_base ran for this Na (the rows' splines then take the
-// provisional row as a correction)
 void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, const int* spec_ids,
                             int warps_per_block, cudaStream_t st, int qag_split, int update_row = -1,
                             bool defer_combine = false, const FinalizeArgs* fin = nullptr,
                             bool base_ready = false);
-// Before the provisional row is known (beside the binning pass, after
-// launch_integrator_prepare): every row's spline with its last knot equal to the one
-// before, and the spline of a unit last knot.  False for histories of two knots or fewer.
-bool launch_dtot_base(const IntegratorDev& I, int nk, int Na, cudaStream_t st);
 size_t dnu_qag_smem(int ld, int wpb);
 // end of get_delta_nu_update (delta_tot_table.c:226-248) + interface_common.c:134-146:
 // delta_nu_last, committed row, NaN check, clamp, ratio/log k/kspace_prefac, grid table

@@ -1,0 +1,368 @@
+// ksp_prep.cuh -- the preparation of an integrator call that does not depend on the
+// current delta_cdm: the knots' spline factorisation, the fslength table and the node
+// table, as device functions of one block (single calls and batches launch them over
+// their own block maps).
+//
+// The fslength table (delta_tot_table.c:574-591) has N = 16 Na uniform nodes x_i in
+// log a; fslength(x_i) = light * sum_{v >= i} s_v with s_v the integral of 1/(a^2 H) over
+// segment v, and its natural spline's coefficients follow from the s_v in closed form.
+// Two kernels make it: the first evaluates the segments, a block per stretch of them,
+// with their suffix sums within the stretch and the stretch's total; the second adds the
+// totals of the later stretches and forms the coefficients.  Nothing in it is serial in
+// N, and no block is larger than 64 threads or 128 registers a thread, so that the blocks
+// find room beside the binning pass, which holds most of every SM.
+#pragma once
+#include "ksp_internal.h"
+
+namespace ksp {
+
+constexpr int kPrepThreads = 64;
+
+// ------------------------------------------------------------------ segments
+// The rule by the node spacing h: the 4-point Gauss-Legendre rule per segment from 5e-3 on,
+// the 2-point rule below (fslength then within 1e-12, as the 4-point rule's: both are held up
+// by the jump of the rho_nu tables where they give way to the series), and below 1.5e-3 one
+// evaluation per node, a segment being the integral of the degree-7 interpolant through 8
+// neighbouring nodes (7e-13; at wider spacings the kinks of the rho_nu tables, a knot every
+// ~0.016, spread over its 8 segments: 2e-10 at h = 0.019).  An evaluation is an exp, a
+// square root, two divisions and the rho_nu tables, ~100 FP64 operations.
+constexpr double kFsNodeRule = 1.5e-3, kFsGauss2 = 5e-3;
+constexpr int kFsNodeSegs = kPrepThreads - 7;  // segments of a block by the node rule
+__host__ __device__ inline int fs_block_segs(int Nfs, double loga0, double loga) {
+    const double h = (loga - loga0) / (Nfs - 1.);
+    return h < kFsNodeRule ? kFsNodeSegs : (h < kFsGauss2 ? kPrepThreads / 2 : kPrepThreads / 4);
+}
+// blocks of a table of Nfs nodes (segments 0 .. Nfs - 2, and a last one of zero)
+__host__ __device__ inline int fs_blocks(int Nfs, double loga0, double loga) {
+    const int per = fs_block_segs(Nfs, loga0, loga);
+    return (Nfs + per - 1) / per;
+}
+
+#ifdef __CUDACC__
+// integrals over [o, o + 1], o = 0..3, of the Lagrange basis on the nodes 0..7, x 120960
+// (o = 4..6: mirrored)
+static __constant__ double kNodeRule[4][8] = {
+    {36799, 139849, -121797, 123133, -88547, 41499, -11351, 1375},
+    {-1375, 47799, 101349, -44797, 26883, -11547, 2999, -351},
+    {351, -4183, 57627, 81693, -20227, 7227, -1719, 191},
+    {-191, 1879, -9531, 68323, 68323, -9531, 1879, -191}};
+
+__device__ __noinline__ static double fsl_integrand_call(const Background& B, double x) { return fsl_integrand(B, x); }
+
+// Node i of the table.
+__device__ __forceinline__ double fs_node(int i, int Nfs, double loga0, double loga) {
+    return loga0 + i * (loga - loga0) / (Nfs - 1.);
+}
+
+// Block `blk` of the segments, by 64 threads: fs_seg[v] = s_v, fs_suf[v] = the sum of the
+// block's s from v on, fs_tot[blk] = the block's.  f: 64 doubles of shared memory, sg: 64.
+__device__ __forceinline__ void fs_eval_block(const Background& B, int Nfs, double loga0, double loga, int blk,
+                                              double gx0, double gx1, double gw0, double gw1, double* f, double* sg,
+                                              double* fs_seg, double* fs_suf, double* fs_tot) {
+    const int t = threadIdx.x;
+    const double h = (loga - loga0) / (Nfs - 1.);
+    int per, v;
+    double s = 0;
+    if (h < kFsNodeRule) {
+        per = kFsNodeSegs;
+        const int first = blk * per;
+        // nodes base .. base + 63, as many of the table as reach around the block's segments
+        int base = first - 3;
+        base = base > Nfs - kPrepThreads ? Nfs - kPrepThreads : base;
+        base = base < 0 ? 0 : base;
+        f[t] = base + t < Nfs ? fsl_integrand_call(B, fs_node(base + t, Nfs, loga0, loga)) : 0.0;
+        __syncthreads();
+        v = first + t;
+        if (t < per && v < Nfs - 1) {
+            int st = v - 3;
+            st = st > Nfs - 8 ? Nfs - 8 : st;
+            st = st < 0 ? 0 : st;
+            const int o = v - st;
+            const double* w = kNodeRule[o < 4 ? o : 6 - o];
+            const double* q = f + (st - base);
+            double acc = 0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) acc += w[o < 4 ? k : 7 - k] * q[k];
+            s = acc * (h / 120960.);
+        }
+    } else {
+        // a segment per pair or per four threads
+        const bool two = h < kFsGauss2;
+        const int w = two ? 2 : 4;
+        per = kPrepThreads / w;
+        const int u = blk * per + t / w, q = t % w;
+        double x = 0;
+        if (u < Nfs - 1) {
+            const double xa = fs_node(u, Nfs, loga0, loga), xb = u + 1 == Nfs - 1 ? loga : fs_node(u + 1, Nfs, loga0, loga);
+            const double c = 0.5 * (xa + xb), hh = 0.5 * (xb - xa);
+            const double gx = two ? 0.57735026918962576451 : ((q & 1) ? gx1 : gx0);  // 1 / sqrt 3
+            const double gw = two ? 1.0 : ((q & 1) ? gw1 : gw0);
+            x = gw * hh * fsl_integrand_call(B, 2 * q < w ? c - hh * gx : c + hh * gx);
+        }
+        x += __shfl_down_sync(0xffffffffu, x, 1, 4);
+        if (!two) x += __shfl_down_sync(0xffffffffu, x, 2, 4);
+        if (q == 0) f[t / w] = x;
+        __syncthreads();
+        v = blk * per + t;
+        if (t < per) s = f[t];
+    }
+    sg[t] = t < per ? s : 0.0;
+    __syncthreads();
+    // suffix sums: each thread of the first warp two neighbours
+    if (t < 32) {
+        const double b1 = sg[2 * t + 1], b0 = sg[2 * t];
+        const double own = b0 + b1;
+        double r = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double n = __shfl_down_sync(0xffffffffu, r, o);
+            if (t + o < 32) r += n;
+        }
+        double later = __shfl_down_sync(0xffffffffu, r, 1);
+        if (t == 31) later = 0;
+        f[2 * t + 1] = b1 + later;
+        f[2 * t] = r;
+        if (t == 0) fs_tot[blk] = r;
+    }
+    __syncthreads();
+    if (t < per && v < Nfs) {
+        fs_seg[v] = s;
+        fs_suf[v] = f[t];
+    }
+}
+
+// ------------------------------------------------------------------ table
+// The totals of the stretches from the one of thread t on: suf[t] = the totals of the blocks
+// t c, t c + 1, ... (c: blocks per thread), t <= 64.  suf: 65 doubles of shared memory.
+__device__ __forceinline__ void fs_totals_suffix(const double* fs_tot, int nblk, double* suf) {
+    const int t = threadIdx.x, c = (nblk + kPrepThreads - 1) / kPrepThreads;
+    double own = 0;
+    for (int b = min(nblk, (t + 1) * c) - 1; b >= t * c; b--) own += fs_tot[b];
+    double r = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double n = __shfl_down_sync(0xffffffffu, r, o);
+        if ((t & 31) + o < 32) r += n;
+    }
+    if (t >= 32) suf[t] = r;
+    __syncthreads();
+    if (t < 32) suf[t] = r + suf[32];
+    if (t == 0) suf[kPrepThreads] = 0;
+    __syncthreads();
+}
+
+struct FsTable {  // what the second kernel reads
+    const double* seg;
+    const double* suf;
+    const double* tot;
+    const double* tsuf;  // fs_totals_suffix
+    int Nfs, nblk, per;
+    double light, h;     // h: node spacing
+    double cscale;       // light * 3 / h^2 / (2 sqrt 3)
+};
+
+// fslength at node i: its stretch's suffix sum and the later stretches' totals
+__device__ __forceinline__ double fs_table_y(const FsTable& F, int i) {
+    const int b = i / F.per, c = (F.nblk + kPrepThreads - 1) / kPrepThreads, t = b / c;
+    double later = F.tsuf[t + 1];
+    for (int q = min(F.nblk, (t + 1) * c) - 1; q > b; q--) later += F.tot[q];
+    return F.light * (F.suf[i] + later);
+}
+
+// Spline coefficient (second derivative / 2) at node i of 0 .. Nfs-1.  The system is
+// tridiag(1,4,1) c = 3 D^2 y / h^2, D^2 y_v = light (s_{v-1} - s_v) (fslength falls by light s_v
+// from node v to v + 1), whose inverse on the whole line is nu^|d| / (2 sqrt 3),
+// nu = sqrt 3 - 2; the ends c = 0 are met by continuing the right-hand side oddly about them,
+// that is, the s evenly: s_{-1-k} = s_k, s_{n+k} = s_{n-1-k}, n = Nfs - 1.  The sums over the
+// neighbours are taken over the s themselves (summation by parts: one multiply-add per
+// term), D to a side: 20 where h < 0.02 (nu^20 = 4e-12 of a term below 4e-4 of fslength), 28
+// elsewhere (Nfs >= 16: one continuation reaches).
+__device__ __forceinline__ double fs_table_s(const FsTable& F, int i) {
+    const int n = F.Nfs - 1;
+    i = i < 0 ? -1 - i : i;
+    i = i >= n ? 2 * n - 1 - i : i;
+    return F.seg[i];
+}
+__device__ __forceinline__ double fs_table_c(const FsTable& F, int i) {
+    if (i == 0 || i == F.Nfs - 1) return 0.0;
+    const double nu = -0.26794919243112270647, k = 0.78867513459481288225;  // 1 / (1 - nu)
+    double l, r;
+    if (F.h < 0.02) {
+        constexpr int D = 20;
+        l = fs_table_s(F, i - D - 1) * k;
+        r = fs_table_s(F, i + D) * k;
+#pragma unroll
+        for (int d = D; d >= 2; d--) {
+            l = fma(nu, l, fs_table_s(F, i - d));
+            r = fma(nu, r, fs_table_s(F, i + d - 1));
+        }
+    } else {
+        constexpr int D = 28;
+        l = fs_table_s(F, i - D - 1) * k;
+        r = fs_table_s(F, i + D) * k;
+        for (int d = D; d >= 2; d--) {
+            l = fma(nu, l, fs_table_s(F, i - d));
+            r = fma(nu, r, fs_table_s(F, i + d - 1));
+        }
+    }
+    const double s0 = F.seg[i], s1 = F.seg[i - 1];
+    const double q = fma(1.0 - nu, l - r, s0 - s1);  // the two sides' sums of nu^(d-1) D^2 y
+    return F.cscale * fma(nu, q, s1 - s0);
+}
+
+// The table of a call as the second kernel's blocks read it.  Called by a whole block of at
+// least kPrepThreads threads; tsuf: kPrepThreads + 1 doubles of shared memory.
+__device__ __forceinline__ FsTable fs_table(const IntegratorDev& I, int Nfs, double loga0, double loga, double light,
+                                            double* tsuf) {
+    FsTable F;
+    F.seg = I.fs_seg;
+    F.suf = I.fs_suf;
+    F.tot = I.fs_tot;
+    F.tsuf = tsuf;
+    F.Nfs = Nfs;
+    F.nblk = fs_blocks(Nfs, loga0, loga);
+    F.per = fs_block_segs(Nfs, loga0, loga);
+    F.light = light;
+    F.h = (loga - loga0) / (Nfs - 1.);
+    F.cscale = light * (3.0 / (F.h * F.h) / (2.0 * 1.7320508075688772935));
+    if (threadIdx.x < kPrepThreads) {
+        fs_totals_suffix(I.fs_tot, F.nblk, tsuf);
+    } else {
+        __syncthreads();
+        __syncthreads();
+    }
+    return F;
+}
+
+// fslength at x, from the spline of the table
+__device__ __forceinline__ double fs_table_at(const FsTable& F, double loga0, double loga, double x) {
+    int i = (int)((x - loga0) * ((F.Nfs - 1.) / (loga - loga0)));
+    i = i < 0 ? 0 : (i > F.Nfs - 2 ? F.Nfs - 2 : i);
+    while (i > 0 && x < fs_node(i, F.Nfs, loga0, loga)) i--;
+    while (i < F.Nfs - 2 && x >= fs_node(i + 1, F.Nfs, loga0, loga)) i++;
+    return fs_spline_eval(fs_node(i, F.Nfs, loga0, loga), fs_node(i + 1, F.Nfs, loga0, loga), fs_table_y(F, i),
+                          fs_table_y(F, i + 1), fs_table_c(F, i), fs_table_c(F, i + 1), x);
+}
+
+// ------------------------------------------------------------------ knots
+// Row i of the factorised natural-spline system of the knots x[0..Na-1]: the pivot
+// d_i = b_i - h_i^2 / d_{i-1}, b_i = 2 (h_i + h_{i+1}), h_i = x_{i+1} - x_i, as a quotient
+// of two-term recurrences p / q carried from 28 rows before (an error in a pivot shrinks
+// by 4 or more per row, so the start does not show), with two divisions at the end instead
+// of one per row.  knot(j): knot j.
+template <class X>
+__device__ __forceinline__ void knot_row(const X& knot, int i, double* invdiag, double* fac) {
+    int r = i > 28 ? i - 28 : 0;
+    double x1 = knot(r + 1), x2 = knot(r + 2);
+    double h0 = x1 - knot(r), h1 = x2 - x1;
+    double p = 2.0 * (h0 + h1), q = 1.0, pp = 0, qp = 0;
+    while (r < i) {
+        r++;
+        pp = p;
+        qp = q;
+        x1 = x2;
+        x2 = knot(r + 2);
+        h0 = h1;
+        h1 = x2 - x1;
+        p = 2.0 * (h0 + h1) * pp - h0 * h0 * qp;
+        q = pp;
+        if ((r & 7) == 0) {  // both back to their first size
+            p /= q;
+            q = 1.0;
+        }
+    }
+    invdiag[i] = q / p;
+    if (i > 0) fac[i] = h0 * (qp / pp);
+}
+
+// ------------------------------------------------------------------ nodes
+// Node q = 61 slot + jn of the node table: its log a.
+__device__ __forceinline__ double nc_node_x(int q, double loga0, double loga) {
+    const int slot = q / 61, jn = q - 61 * slot;
+    double lo, hi;
+    nc_interval(slot, loga0, loga, &lo, &hi);
+    const double c = __dmul_rn(0.5, __dadd_rn(lo, hi));
+    const double h = __dmul_rn(0.5, __dsub_rn(hi, lo));
+    return __dadd_rn(c, __dmul_rn(h, gk61_x(jn)));
+}
+
+// The same solve as spline_solve_scan with all T threads of a block (T a multiple of 32):
+// warp scans of the affine maps, combined over the warps through sh (2 * T / 32 doubles of
+// shared memory).
+template <int T>
+__device__ __forceinline__ void spline_solve_block(const IntegratorDev& I, int m, double* sc, double* sh) {
+    constexpr int NW = T / 32;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const double* x = I.scalefact;
+    const int per = (m + T - 1) / T;
+    const int u0 = min(m, t * per), u1 = min(m, u0 + per);
+    // forward: z_u = r_u - fac_u z_{u-1} (fac_0 = 0)
+    double A = 1.0, B = 0.0;
+    for (int u = u0; u < u1; u++) {
+        const double f = u > 0 ? I.knot_fac[u] : 0.0;
+        B = sc[u + 1] - f * B;
+        A = -f * A;
+    }
+    double pa = A, pb = B;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const double qa = __shfl_up_sync(0xffffffffu, pa, d), qb = __shfl_up_sync(0xffffffffu, pb, d);
+        if (lane >= d) {
+            pb = pa * qb + pb;
+            pa = pa * qa;
+        }
+    }
+    if (lane == 31) {
+        sh[2 * warp] = pa;
+        sh[2 * warp + 1] = pb;
+    }
+    __syncthreads();
+    double win = 0.0;  // z entering this warp's stretch
+    for (int w = 0; w < warp; w++) win = sh[2 * w] * win + sh[2 * w + 1];
+    double ea = __shfl_up_sync(0xffffffffu, pa, 1), eb = __shfl_up_sync(0xffffffffu, pb, 1);
+    double zin = lane == 0 ? win : ea * win + eb;
+    for (int u = u0; u < u1; u++) {
+        const double f = u > 0 ? I.knot_fac[u] : 0.0;
+        zin = sc[u + 1] - f * zin;
+        sc[u + 1] = zin;
+    }
+    __syncthreads();
+    // backward: c_u = (z_u - off_u c_{u+1}) * invdiag_u, c_m = 0
+    A = 1.0;
+    B = 0.0;
+    for (int u = u1 - 1; u >= u0; u--) {
+        const double off = u < m - 1 ? x[u + 2] - x[u + 1] : 0.0;
+        const double iv = I.knot_invdiag[u];
+        B = (sc[u + 1] - off * B) * iv;
+        A = -off * iv * A;
+    }
+    pa = A;
+    pb = B;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const double qa = __shfl_down_sync(0xffffffffu, pa, d), qb = __shfl_down_sync(0xffffffffu, pb, d);
+        if (lane + d < 32) {
+            pb = pa * qb + pb;
+            pa = pa * qa;
+        }
+    }
+    if (lane == 0) {
+        sh[2 * warp] = pa;
+        sh[2 * warp + 1] = pb;
+    }
+    __syncthreads();
+    win = 0.0;
+    for (int w = NW - 1; w > warp; w--) win = sh[2 * w] * win + sh[2 * w + 1];
+    ea = __shfl_down_sync(0xffffffffu, pa, 1);
+    eb = __shfl_down_sync(0xffffffffu, pb, 1);
+    double cin = lane == 31 ? win : ea * win + eb;
+    for (int u = u1 - 1; u >= u0; u--) {
+        const double off = u < m - 1 ? x[u + 2] - x[u + 1] : 0.0;
+        cin = (sc[u + 1] - off * cin) * I.knot_invdiag[u];
+        sc[u + 1] = cin;
+    }
+    __syncthreads();
+}
+#endif  // __CUDACC__
+
+}  // namespace ksp

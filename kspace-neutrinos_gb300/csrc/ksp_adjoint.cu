@@ -453,7 +453,9 @@ __global__ void __launch_bounds__(128) k_dnu_adj(IntegratorDev I, DnuAdjArgs A, 
                 nint = A.nivals[(size_t)mi * I.nk_alloc + ik];
                 iv = A.ivals + ((size_t)mi * I.nk_alloc + ik) * kQagLimit * 2;
             } else {
-                const DnuIntegrandC f = dnu_integrand(I, S, k, mnubykT, qc, knots, row, rc, sb, sd, Na);
+                if (Na == 2 && lane < 2) rc[lane] = 0.0;
+                __syncwarp();
+                const DnuIntegrandW f = dnu_integrand_w(I, S, mi, k * S.inv_m[mi], row, rc, Na);
                 QagResult r = qag_warp_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit);
                 nint = r.nint;
             }
@@ -630,7 +632,9 @@ __global__ void __launch_bounds__(128) k_dnu_adj_blk(IntegratorDev I, DnuAdjArgs
                 nint = A.nivals[(size_t)mi * I.nk_alloc + ik];
                 iv = A.ivals + ((size_t)mi * I.nk_alloc + ik) * kQagLimit * 2;
             } else {
-                const DnuIntegrandC f = dnu_integrand(I, S, k, mnubykT, qc, knots, row, rc, sb, sd, Na);
+                if (Na == 2 && tid < 2) rc[tid] = 0.0;
+                __syncthreads();
+                const DnuIntegrandW f = dnu_integrand_w(I, S, mi, k * S.inv_m[mi], row, rc, Na);
                 const QagResult r = qag_block_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
                 nint = r.nint;
             }

@@ -134,7 +134,7 @@ static void free_table(kspace_ctx* c) {
     IntegratorDev& I = c->I;
     void* ptrs[] = {I.scalefact, I.dtot, I.coef, I.nu_init, I.nu_last, I.wavenum, I.dcdm, I.dnu_s, I.dnu,
                     I.knot_invdiag, I.knot_fac, I.knot_invh, I.knot_h3, I.knot_ih3, I.nc_g, I.nc_fsl,
-                    I.nc_dx, I.nc_j, I.nc_inv, I.fs_x, I.fs_y, I.fs_c, I.fs_seg, I.fs_suf, I.fs_tot, I.t_logk, I.t_T,
+                    I.nc_dx, I.nc_j, I.nc_inv, I.nc_ab, I.nc_cd, I.nc_jf, I.fs_x, I.fs_y, I.fs_c, I.fs_seg, I.fs_suf, I.fs_tot, I.t_logk, I.t_T,
                     I.t_c, I.sc,
                     I.qag_max, I.qag_total, I.coef_unit};
     for (void* p : ptrs)
@@ -467,6 +467,11 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
     CK(dalloc(&I.nc_fsl, kNcNodes));
     CK(dalloc(&I.nc_dx, kNcNodes));
     CK(dalloc(&I.nc_j, kNcNodes));
+    CK(dalloc(&I.nc_ab, kNcNodes));
+    CK(dalloc(&I.nc_cd, kNcNodes));
+    CK(dalloc(&I.nc_jf, kNcNodes));
+    I.jt = jfine_table();
+    NEED(I.jt, KSPACE_ERR_CUDA);
     I.nc_slots = c->nc_levels > 0 ? 1 + 2 * c->nc_levels : 0;
     I.fs_cap = 16 * (int)ld + 16;
     CK(dalloc(&I.fs_x, I.fs_cap));
@@ -710,9 +715,10 @@ extern "C" int kspace_gpu_save_nu_power(kspace_ctx* c, double Time, int snapnum,
 // ------------------------------------------------------------------ integrator
 // A call's preparation with Na knots at scale factor a (launch_integrator_prepare).
 static void prepare_call(kspace_ctx* c, int Na, double a, double loga, int start_row, int write_knot, RowsMode rows,
-                         int nk, int update_row, cudaStream_t st, bool scalars_only = false) {
+                         int nk, int update_row, cudaStream_t st, bool scalars_only = false,
+                         const FinalizeArgs* fin = nullptr) {
     launch_integrator_prepare(c->I, c->hB, c->S0, Na, a, loga, c->loga0, c->TimeTransfer, start_row, write_knot,
-                              scalars_only, rows, nk, update_row, st);
+                              scalars_only, rows, nk, update_row, fin, st);
 }
 
 // delta_tot_table.c:79-149 (host bookkeeping; numbers on the device)
@@ -753,7 +759,7 @@ static int delta_tot_init(kspace_ctx* c, int nk_in, const double* keff_d, const 
 // get_delta_nu_update (delta_tot_table.c:193-250) on device arrays.  Optionally
 // produces the correction table of interface_common.c:134-146.
 // fin: the binning pass's normalisation when it was deferred (see bin_grid): folded into
-// the row-spline kernel of a prepared step, else launched first.
+// the integral kernel of a prepared step, else launched first.
 // sync = false (a step whose correction pass follows on the stream): no host round trip
 // at the end; the correction pass reads the status word itself and leaves the grid as it
 // is after an error, which the step's final status check reports.
@@ -827,12 +833,13 @@ static int update_device(kspace_ctx* c, double a, int nk_in, const double* keff_
     }
     I.kq = nullptr;
     c->prep_valid = false;
+    const bool logk_ready = prepared && fin && fin->active && c->prep_base;
     // keep the row if far enough from the previous one (delta_tot_table.c:229-237)
     const bool commit = a >= exp(c->h_scalefact[Na - 2]) + 0.009;
     launch_finish_update(I, c->nk, commit ? Na - 1 : -1, a, loga, want_corr ? keff_d : nullptr, dnu_out_d,
                          want_corr ? c->logk_d : nullptr, want_corr ? c->ratio_d : nullptr,
-                         want_corr ? c->corr : CorrTable{}, c->norm_d, c->stream, true);
-    g_launches += prepared ? 3 : 4;
+                         want_corr ? c->corr : CorrTable{}, c->norm_d, c->stream, true, logk_ready);
+    g_launches += prepared ? 2 : 4;
     if (commit) {
         c->fact_valid = Na - 2 > 0 ? Na - 2 : 0;
     } else {
@@ -1246,7 +1253,8 @@ static int start_prep(kspace_ctx* c, const Geo* G, double Time) {
     const int Na = c->ia + 1;
     CK(cudaStreamWaitEvent(c->side, c->ev_fork, 0));  // recorded before the binning pass
     c->prep_base = Na > 2;
-    prepare_call(c, Na, Time, loga, c->fact_valid, 1, c->prep_base ? kRowsBase : kRowsNone, c->nk, -1, c->side);
+    prepare_call(c, Na, Time, loga, c->fact_valid, 1, c->prep_base ? kRowsBase : kRowsNone, c->nk, -1, c->side, false,
+                 &c->fin);
     CK(cudaEventRecord(c->ev_join, c->side));
     g_launches += 2;
     c->prep_valid = true;
@@ -1289,6 +1297,11 @@ static int bin_grid(kspace_ctx* c, Geo* G, const float* gd, int pmgrid, int slab
         }
     }
     if (c->prof) cudaEventRecord(c->ev[1], c->stream);
+    c->fin = FinalizeArgs{c->bin_sum_d, c->F0sq_d, G->count_d, G->ksum_d, G->compact_d, BoxSize, c->power_d,
+                          c->keffg_d, c->I.dcdm, c->keff_d, 1};
+    c->fin.scale = pow(BoxSize, -3.0);
+    c->fin.kfac = 2 * kPi / BoxSize;
+    c->fin.logk_out = c->logk_d;
     if (prep_time > 0) {
         const int sp = start_prep(c, G, prep_time);
         if (sp) return sp;
@@ -1299,12 +1312,8 @@ static int bin_grid(kspace_ctx* c, Geo* G, const float* gd, int pmgrid, int slab
         if (c->ar_fn(c->ar_h, nb + 1, c->ar_user) != 0) return KSPACE_ERR_ARG;
         CK(cudaMemcpyAsync(c->bin_sum_d, c->ar_h, sizeof(double) * (nb + 1), cudaMemcpyHostToDevice, c->stream));
     }
-    c->fin = FinalizeArgs{c->bin_sum_d, c->F0sq_d, G->count_d, G->ksum_d, G->compact_d, BoxSize, c->power_d,
-                          c->keffg_d, c->I.dcdm, c->keff_d, 1};
-    c->fin.scale = pow(BoxSize, -3.0);
-    c->fin.kfac = 2 * kPi / BoxSize;
     if (!(prep_time > 0 && c->prep_valid)) {
-        // a prepared step does it in its row-spline kernel instead (update_device)
+        // a prepared step does it in its integral kernel instead (update_device)
         launch_finalize_power(c->bin_sum_d, c->F0sq_d, G->count_d, G->ksum_d, G->compact_d, G->nk, BoxSize,
                               c->power_d, c->keffg_d, c->I.dcdm, c->keff_d, c->stream);
         g_launches += 1;

@@ -125,10 +125,7 @@ __global__ void __launch_bounds__(kBatchTable) kb_tables(BatchDev b) {
         const double x = nc_node_x(q, P.loga0, P.loga);
         const double fsl = fs_table_at(F, P.loga0, P.loga, x);
         const int j = seg_bsearch(I.scalefact, P.Na, x);
-        I.nc_fsl[q] = fsl;
-        I.nc_j[q] = j;
-        I.nc_dx[q] = x - I.scalefact[j];
-        I.nc_g[q] = fsl * node_inv_aH(I.B, x);
+        nc_store(I, q, fsl, node_inv_aH(I.B, x), x - I.scalefact[j], j, I.scalefact[j + 1] - I.scalefact[j], P.Na);
     }
 }
 
@@ -171,25 +168,21 @@ __global__ void kb_dtot_coeffs(BatchDev b) {
 }
 
 size_t batch_qag_smem(int ldmax, int wpb) {
-    return ((sizeof(Gk61Nodes) + 15) & ~size_t(15)) + wpb * (sizeof(QagList) + 5 * sizeof(double) * ldmax) +
+    return ((sizeof(Gk61Nodes) + 15) & ~size_t(15)) + wpb * (sizeof(QagList) + 2 * sizeof(double) * ldmax) +
            wpb * sizeof(uint64_t);
 }
 
-// Shared memory: Gk61Nodes | per warp: QagList, knots[ldmax], row[ldmax], coef[ldmax], seg_poly [2 ldmax] |
-// mbarriers
+// Shared memory: Gk61Nodes | per warp: QagList, row[ldmax], coef[ldmax] | mbarriers
 __global__ void __launch_bounds__(128) kb_dnu_qag(BatchDev b) {
     extern __shared__ __align__(16) unsigned char sm[];
     Gk61Nodes& N = *reinterpret_cast<Gk61Nodes*>(sm);
     const size_t off = (sizeof(Gk61Nodes) + 15) & ~size_t(15);
     const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t per_warp = sizeof(QagList) + 5 * sizeof(double) * b.ldmax;
+    const size_t per_warp = sizeof(QagList) + 2 * sizeof(double) * b.ldmax;
     unsigned char* wbase = sm + off + warp * per_warp;
     QagList& L = *reinterpret_cast<QagList*>(wbase);
-    double* knots = reinterpret_cast<double*>(wbase + sizeof(QagList));
-    double* row = knots + b.ldmax;
+    double* row = reinterpret_cast<double*>(wbase + sizeof(QagList));
     double* rc = row + b.ldmax;
-    double* sb = rc + b.ldmax;
-    double* sd = sb + b.ldmax;
     uint64_t* mybar = reinterpret_cast<uint64_t*>(sm + off + nw * per_warp) + warp;
     gk61_fill(N, threadIdx.x, blockDim.x);
     if (lane == 0) ptx::mbar_init(mybar, 1);
@@ -209,32 +202,23 @@ __global__ void __launch_bounds__(128) kb_dnu_qag(BatchDev b) {
         const int nk = P.nk;
         const int si = loc / nk, ik = loc - si * nk;
         const int mi = P.spec[si];
-        const Background* B = I.B;
         const StepScalars& S = *I.sc;
         const int Na = P.Na;
         const double k = I.wavenum[ik];
-        // the task's divisions on lane 0
-        double mnubykT = 0, kom = 0, fsi = 0;
-        if (lane == 0) {
-            mnubykT = B->mnu_J[mi] / B->kBtnu;
-            kom = k / mnubykT;
-            fsi = (S.Nfs - 1.) / (S.loga - S.loga0);
-        }
-        mnubykT = __shfl_sync(0xffffffffu, mnubykT, 0);
-        kom = __shfl_sync(0xffffffffu, kom, 0);
-        fsi = __shfl_sync(0xffffffffu, fsi, 0);
-        double integral = 0;
-        const bool integrate = !S.skip_integral && Na > 1 && mnubykT > 0;
+        const bool integrate = !S.skip_integral && Na > 1 && S.inv_m[mi] > 0;
         if (integrate) {
-            const unsigned bytes = (unsigned)(((Na + 1) & ~1) * sizeof(double));
             __syncwarp();
             if (lane == 0) {
+                const unsigned bytes = (unsigned)(((Na + 1) & ~1) * sizeof(double));
                 ptx::fence_async_smem();
-                ptx::mbar_expect_tx(mybar, Na > 2 ? 3 * bytes : 2 * bytes);
-                ptx::bulk_g2s(knots, I.scalefact, bytes, mybar);
+                ptx::mbar_expect_tx(mybar, Na > 2 ? 2 * bytes : bytes);
                 ptx::bulk_g2s(row, I.dtot + (size_t)ik * I.ld, bytes, mybar);
                 if (Na > 2) ptx::bulk_g2s(rc, I.coef + (size_t)ik * I.ld, bytes, mybar);
             }
+            if (Na == 2 && lane < 2) rc[lane] = 0.0;  // linear: no coefficients
+        }
+        double val = lane == 0 ? dnu_initial(I, S, ik, mi, k) : 0.0;
+        if (integrate) {
             const bool got = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(mybar, phase));  // warp-uniform
             phase ^= 1;
             if (!got) {
@@ -242,16 +226,13 @@ __global__ void __launch_bounds__(128) kb_dnu_qag(BatchDev b) {
                 ptx::mbar_wait_bounded(mybar, phase ^ 1);  // the copies still in flight
                 return;
             }
-            const KnotSeg ks{I.knot_invh, I.knot_h3, I.knot_ih3};
-            if (Na > 2) seg_poly(row, rc, Na, ks, sb, sd, lane, 32);
             __syncwarp();
-            const double qc = S.partnu_now > 0 ? B->vcrit * mnubykT : 0.0;
-            const DnuIntegrandC f = dnu_integrand_pre(I, S, kom, fsi, qc, knots, row, rc, sb, sd, Na);
+            const DnuIntegrandW f = dnu_integrand_w(I, S, mi, k * S.inv_m[mi], row, rc, Na);
             const QagResult r = qag_warp_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit);
-            integral = r.result;
+            val += S.prefac * r.result;
             if (!r.ok && lane == 0) atomicOr(I.status, kStGsl);
         }
-        if (lane == 0) I.dnu_s[(size_t)mi * I.nk_alloc + ik] = dnu_task_value(I, S, ik, k, mnubykT, integrate, integral);
+        if (lane == 0) I.dnu_s[(size_t)mi * I.nk_alloc + ik] = val;
     }
 }
 
@@ -273,7 +254,7 @@ __global__ void kb_finish(BatchDev b) {
         } else {
             double v = 0;
             for (int mi = 0; mi < kNuSpecies; mi++)
-                if (I.B->deg[mi] > 0) v += I.dnu_s[(size_t)mi * I.nk_alloc + ik] * S.omeganu[mi] / S.Omega_nu_tot;
+                if (S.wnu[mi] != 0.0) v += I.dnu_s[(size_t)mi * I.nk_alloc + ik] * S.wnu[mi];
             I.dnu[ik] = v;
             if (!P.dry) I.nu_last[ik] = v;
             if (P.commit_row >= 0 && !P.dry) {

@@ -304,24 +304,41 @@ KSP_HD double sinc_j0(double y) {
     return sin(y) / y;
 }
 
-// delta_tot_table.c:431-434
-KSP_HD double II(double x, double qc, int n) {
-    return (n * n + n * n * n * qc + n * qc * x * x - x * x) * qc * sinc_j0(qc * x) +
-           (2 * n + n * n * qc + qc * x * x) * cos(qc * x);
+// delta_tot_table.c:431-463 with qc > 0: sum over n = 1..19 of -(-1)^n e^{-n qc} /
+// (n^2 + x^2)^2 times
+//   (n^2 + n^3 qc + x^2 (n qc - 1)) qc sinc(qc x) + (2 n + n^2 qc + qc x^2) cos(qc x).
+// The sine and the cosine do not depend on n and are taken once; the weights e^{-n qc} are
+// powers; four terms share a division.  (Term by term, 19 exponentials, sines, cosines and
+// 38 divisions a node, a call with 151 bins took 3.1 ms in its integrals.)
+KSP_HD double specialJ_series(double x, double qc, double nufrac_low) {
+    const double x2 = x * x, e1 = exp(-qc), qx = qc * x;
+    double en = 1.0, A = 0.0, B = 0.0;
+    for (int n0 = 1; n0 < 20; n0 += 4) {
+        double d[4], w[4], a[4], c[4];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+        for (int j = 0; j < 4; j++) {
+            const double n = n0 + j;
+            en *= e1;
+            w[j] = n0 + j < 20 ? ((j & 1) ? -en : en) : 0.0;  // n0 is odd
+            const double t = n * n + x2;
+            d[j] = t * t;
+            a[j] = n * n * (1.0 + n * qc) + x2 * (n * qc - 1.0);
+            c[j] = n * (2.0 + n * qc) + qc * x2;
+        }
+        const double d01 = d[0] * d[1], d23 = d[2] * d[3], inv = 1.0 / (d01 * d23);
+        const double w0 = w[0] * d[1] * d23, w1 = w[1] * d[0] * d23, w2 = w[2] * d01 * d[3], w3 = w[3] * d01 * d[2];
+        A += inv * (w0 * a[0] + w1 * a[1] + w2 * a[2] + w3 * a[3]);
+        B += inv * (w0 * c[0] + w1 * c[1] + w2 * c[2] + w3 * c[3]);
+    }
+    const double integ = A * qc * sinc_j0(qx) + B * cos(qx);
+    return integ / (1.5 * kZeta3 * (1 - nufrac_low));
 }
 
 // delta_tot_table.c:442-463
 KSP_HD double specialJ(double x, double qc, double nufrac_low) {
-    if (qc > 0) {
-        double integ = 0;
-        for (int n = 1; n < 20; n++) {
-            const double s = (n & 1) ? 1.0 : -1.0;  // -(-1)^n
-            const double d = n * n + x * x;
-            integ += s * exp(-n * qc) / d / d * II(x, qc, n);
-        }
-        return integ / (1.5 * kZeta3 * (1 - nufrac_low));
-    }
-    return specialJ_fit(x);
+    return qc > 0 ? specialJ_series(x, qc, nufrac_low) : specialJ_fit(x);
 }
 
 // Index of the largest error among e[0..n) (lowest index on ties), on every lane of
@@ -380,14 +397,22 @@ __device__ __forceinline__ double warp_sum_to0(double v) {
 __device__ __forceinline__ double bcast0(double v) { return __shfl_sync(0xffffffffu, v, 0); }
 
 // QUADPACK error estimate: err = resasc * min(1, (200 |err|/resasc)^1.5), floored at
-// 50 eps resabs (Piessens et al. 1983, qk rules).  t^1.5 as t sqrt(t): within an ulp of
-// pow(t, 1.5), without pow's long FP64 dependency chain on the QAG's critical path.
+// 50 eps resabs (Piessens et al. 1983, qk rules).  With x = 200 |err| below resasc the estimate
+// is x sqrt(x / resasc), formed as x^2 / sqrt(x resasc): one reciprocal square root in place of
+// pow, or of a division and a square root, whose dependent FP64 chains are on the QAG's
+// critical path.
 __device__ __forceinline__ double rescale_error(double err, double resabs, double resasc) {
     err = fabs(err);
     if (resasc != 0.0 && err != 0.0) {
-        const double t = 200.0 * err / resasc;
-        const double s = t * sqrt(t);
-        err = s < 1.0 ? resasc * s : resasc;
+        const double x = 200.0 * err, p = x * resasc;
+        if (x >= resasc) {
+            err = resasc;
+        } else if (p > 1e-280) {
+            err = x * (x * rsqrt(p));
+        } else {
+            const double t = x / resasc;
+            err = resasc * (t * sqrt(t));
+        }
     }
     if (resabs > DBL_MIN / (50.0 * DBL_EPSILON)) {
         const double fl = 50.0 * DBL_EPSILON * resabs;
@@ -544,69 +569,58 @@ __device__ __forceinline__ int nc_child(int s, int right, int nslots) {
     return c < nslots ? c : -1;
 }
 
-// The GK61 sums of one or two intervals from the node values of a warp (lane holds the
-// values of slots lane, lane+32, lane+64, lane+96; slot s is node s%61 of interval s/61),
-// and the rule's outputs, identical on every lane.  The six sums (Kronrod, Gauss and
-// |f| sums of both intervals) are reduced together by a butterfly that halves the set of
-// values each lane carries at every step (9 additions per lane instead of 30), then
-// resasc's two sums likewise (5 instead of 10); the results are broadcast.
-__device__ __forceinline__ void gk61_lane_sums(const Gk61Nodes& N, const double* fv, int nslots, int nint,
-                                               const double* h, GkOut* out) {
+// The GK61 sums of one or two intervals from the node values of a warp (fv[2 t + m]: node
+// lane + 32 m of interval t, 0 past the 61st), and the rule's outputs, identical on every
+// lane.  The FP64 pipe takes 16 cycles a warp instruction whatever its lanes do, so the count
+// is what matters: the sums of both intervals are reduced together by a butterfly that
+// halves the set of values each lane carries at every step, and where no value is negative
+// (a density history's sign does not change: nearly always) |f| sums to what f does: the
+// Kronrod and Gauss sums take 6 additions per lane, resasc's two 5.
+__device__ __forceinline__ void gk61_lane_sums(const Gk61Nodes& N, const double* fv, int nint, const double* h,
+                                               GkOut* out) {
     const int lane = threadIdx.x & 31;
-    double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // rk0 rg0 ra0 - rk1 rg1 ra1 -
+    const bool two = lane < 29;  // the lane has a second node
+    const double k0 = N.wk[lane], k1 = two ? N.wk[32 + lane] : 0.0;
+    const double g0 = N.wg[lane], g1 = two ? N.wg[32 + lane] : 0.0;
+    const int b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+    double rk[2], rg[2];
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const int s = lane + 32 * m;
-        if (s < nslots) {
-            const int t = s >= 61 ? 1 : 0;
-            const int j = s - 61 * t;
-            const double x = fv[m];
-            if (t == 0) { v[0] += N.wk[j] * x; v[1] += N.wg[j] * x; v[2] += N.wk[j] * fabs(x); }
-            else { v[4] += N.wk[j] * x; v[5] += N.wg[j] * x; v[6] += N.wk[j] * fabs(x); }
-        }
+    for (int t = 0; t < 2; t++) {
+        rk[t] = fma(k1, fv[2 * t + 1], k0 * fv[2 * t]);
+        rg[t] = fma(g1, fv[2 * t + 1], g0 * fv[2 * t]);
     }
-    // value q ends in lanes with bits (4, 3, 2) = (q >> 2, (q >> 1) & 1, q & 1)
-    const int b4 = (lane >> 4) & 1, b3 = (lane >> 3) & 1, b2 = (lane >> 2) & 1;
-    double w[4];
+    const int signs = __double2hiint(fv[0]) | __double2hiint(fv[1]) | __double2hiint(fv[2]) | __double2hiint(fv[3]);
+    const bool negative = __any_sync(0xffffffffu, signs < 0);
+    // interval 0 goes to the lanes below 16, 1 to the others; there Kronrod below bit 3, Gauss above
+    const double ka = (b4 ? rk[1] : rk[0]) + __shfl_xor_sync(0xffffffffu, b4 ? rk[0] : rk[1], 16);
+    const double ga = (b4 ? rg[1] : rg[0]) + __shfl_xor_sync(0xffffffffu, b4 ? rg[0] : rg[1], 16);
+    double y = (b3 ? ga : ka) + __shfl_xor_sync(0xffffffffu, b3 ? ka : ga, 8);
+    double ra = 0.0;
+    if (negative) {  // warp-uniform
+        double r[2];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const double keep = b4 ? v[4 + k] : v[k], give = b4 ? v[k] : v[4 + k];
-        w[k] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
-    }
-    double x2[2];
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const double keep = b3 ? w[2 + k] : w[k], give = b3 ? w[k] : w[2 + k];
-        x2[k] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
-    }
-    double y;
-    {
-        const double keep = b2 ? x2[1] : x2[0], give = b2 ? x2[0] : x2[1];
+        for (int t = 0; t < 2; t++) r[t] = fma(k1, fabs(fv[2 * t + 1]), k0 * fabs(fv[2 * t]));
+        ra = (b4 ? r[1] : r[0]) + __shfl_xor_sync(0xffffffffu, b4 ? r[0] : r[1], 16);
+        ra += __shfl_xor_sync(0xffffffffu, ra, 8);
+        // one more value each: |f| on the lanes with bit 2
+        const double give = b2 ? y : ra, keep = b2 ? ra : y;
         y = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+    } else {
+        y += __shfl_xor_sync(0xffffffffu, y, 4);
     }
     y += __shfl_xor_sync(0xffffffffu, y, 2);
     y += __shfl_xor_sync(0xffffffffu, y, 1);
     const double rk0 = __shfl_sync(0xffffffffu, y, 0), rk1 = __shfl_sync(0xffffffffu, y, 16);
-    const double mean[2] = {0.5 * rk0, 0.5 * rk1};
-    double rs[2] = {0, 0};
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const int s = lane + 32 * m;
-        if (s < nslots) {
-            const int t = s >= 61 ? 1 : 0;
-            const int j = s - 61 * t;
-            const double d = N.wk[j] * fabs(fv[m] - mean[t]);
-            if (t == 0) rs[0] += d; else rs[1] += d;
-        }
-    }
-    double z = (b4 ? rs[1] : rs[0]) + __shfl_xor_sync(0xffffffffu, b4 ? rs[0] : rs[1], 16);
+    const double mean0 = 0.5 * rk0, mean1 = 0.5 * rk1;
+    const double s0 = fma(k1, fabs(fv[1] - mean0), k0 * fabs(fv[0] - mean0));
+    const double s1 = fma(k1, fabs(fv[3] - mean1), k0 * fabs(fv[2] - mean1));
+    double z = (b4 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, b4 ? s0 : s1, 16);
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-    // the outputs of interval t on lane t only (FP64 is issued per active lane), then
-    // broadcast
+    // the outputs of interval t on lane t, then broadcast
     const int t = lane & 1;
-    const double rgt = __shfl_sync(0xffffffffu, y, t ? 20 : 4);
-    const double rat = __shfl_sync(0xffffffffu, y, t ? 24 : 8);
+    const double rgt = __shfl_sync(0xffffffffu, y, t ? 24 : 8);
+    const double rat = __shfl_sync(0xffffffffu, y, (t ? 16 : 0) + (negative ? 4 : 0));
     const double rst = __shfl_sync(0xffffffffu, z, t ? 16 : 0);
     GkOut o = {0.0, 0.0, 0.0, 0.0};
     if (lane < nint) {
@@ -625,7 +639,7 @@ __device__ __forceinline__ void gk61_lane_sums(const Gk61Nodes& N, const double*
     }
 }
 
-// gk61_warp with interval slots (same arithmetic)
+// gk61_warp with interval slots
 template <class F>
 __device__ __forceinline__ void gk61_warp_c(const F& f, const Gk61Nodes& N, int nint, const double* a,
                                             const double* b, const int* slot, GkOut* out) {
@@ -644,18 +658,14 @@ __device__ __forceinline__ void gk61_warp_c(const F& f, const Gk61Nodes& N, int 
         h[t] = __shfl_sync(0xffffffffu, h[t], 0);
     }
     double fv[4];
-    const int nslots = 61 * nint;
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const int s = lane + 32 * m;
-        fv[m] = 0.0;
-        if (s < nslots) {
-            const int t = s >= 61 ? 1 : 0;
-            const int j = s - 61 * t;
-            fv[m] = f.node_at(slot[t], j, c[t], h[t], N.x[j]);
+    for (int t = 0; t < 2; t++)
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            const int j = lane + 32 * m;
+            fv[2 * t + m] = t < nint && j < 61 ? f.node_at(slot[t], j, c[t], h[t], N.x[j]) : 0.0;
         }
-    }
-    gk61_lane_sums(N, fv, nslots, nint, h, out);
+    gk61_lane_sums(N, fv, nint, h, out);
 }
 
 // qag_warp with interval slots (same decisions)
@@ -728,10 +738,8 @@ __device__ QagResult qag_warp_c(const F& f, const Gk61Nodes& N, QagList& L, doub
 
 // ------------------------------------------------------------------ block-cooperative QAG
 // The same rule and decisions with the node evaluations spread over the warps of a block
-// (blockDim.x = 32 * W, W = 2 or 4): thread t evaluates slot t, t + 32W, ...; warp 0
-// then forms every lane's partial sums over the slots lane + 32m in the order m = 0..3
-// and reduces them with the butterfly of gk61_warp_c: the arithmetic of qag_warp_c in
-// the same order (the compiler may contract multiply-adds differently per kernel, so the
+// (blockDim.x = 32 * W, W = 2 or 4): thread t evaluates node t, t + 32W, ...; warp 0
+// then sums them as gk61_warp_c does: the arithmetic of qag_warp_c in the same order (the compiler may contract multiply-adds differently per kernel, so the
 // results agree to the last bits).  Shared scratch: QagBlockSmem.
 struct QagBlockSmem {
     double fv[128];
@@ -762,11 +770,11 @@ __device__ __forceinline__ void gk61_block_c(const F& f, const Gk61Nodes& N, int
         double fv[4];
 #pragma unroll
         for (int m = 0; m < 4; m++) {
-            const int s = lane + 32 * m;
-            fv[m] = s < nslots ? sh.fv[s] : 0.0;
+            const int j = lane + 32 * (m & 1), t = m >> 1;
+            fv[m] = t < nint && j < 61 ? sh.fv[61 * t + j] : 0.0;
         }
         GkOut o[2];
-        gk61_lane_sums(N, fv, nslots, nint, h, o);
+        gk61_lane_sums(N, fv, nint, h, o);
         if (lane < nint) sh.out[lane] = o[lane];
     }
     __syncthreads();
@@ -899,12 +907,12 @@ __device__ __forceinline__ void gk61_block_groups(const F& f, const Gk61Nodes& N
         double fv[4];
 #pragma unroll
         for (int m = 0; m < 4; m++) {
-            const int sl = lane + 32 * m;
-            fv[m] = sl < 61 * ng ? fvg[sl] : 0.0;
+            const int j = lane + 32 * (m & 1), t = m >> 1;
+            fv[m] = t < ng && j < 61 ? fvg[61 * t + j] : 0.0;
         }
         const double hh[2] = {sh.ih[2 * warp], sh.ih[2 * warp + 1]};
         GkOut o[2];
-        gk61_lane_sums(N, fv, 61 * ng, ng, hh, o);
+        gk61_lane_sums(N, fv, ng, hh, o);
         if (lane == 0) {
             sh.out[2 * warp] = o[0];
             if (ng > 1) sh.out[2 * warp + 1] = o[1];
@@ -1021,6 +1029,8 @@ __device__ QagResult qag_block_spec_c(const F& f, const Gk61Nodes& N, QagList& L
 #include "ksp_jfit.cuh"
 namespace ksp {
 
+struct StepScalars;
+
 // ------------------------------------------------------------------ delta_nu integrand
 // delta_tot_table.c:492-500: fslength(x, log a) / (a H(a)) J(k fslength / (m/kT))
 // delta_tot(k, x) at x = log a_i.  Split into the part that depends only on x (and the
@@ -1069,23 +1079,9 @@ struct KnotSeg {
     const double* ih3;
 };
 
-// The history row's natural spline (or linear for 2 knots) at a node.
-__device__ __forceinline__ double dnu_S(const NodeTerms& t, const double* ky, const double* kc, int na,
-                                        const KnotSeg& ks) {
-    const int j = t.j;
-    const double y0 = ky[j], y1 = ky[j + 1];
-    if (na > 2) {
-        const double c0 = kc[j], c1 = kc[j + 1];
-        const double bq = (y1 - y0) * __ldg(ks.ih + j) - (c1 + 2.0 * c0) * __ldg(ks.h3 + j);
-        const double d = (c1 - c0) * __ldg(ks.ih3 + j);
-        return y0 + t.dx * (bq + t.dx * (c0 + t.dx * d));
-    }
-    return y0 + t.dx * ((y1 - y0) * __ldg(ks.ih + j));
-}
-
-// The node-independent part of dnu_S per segment of a history row, computed once per
-// (row, call) into sb / sd by threads t, t+nt, ...: the same expressions as dnu_S, so
-// that dnu_S_poly returns the same values with three FMAs per node.
+// The history row's natural spline (or linear for 2 knots) at a node: the node-independent
+// part per segment of a history row, computed once per (row, call) into sb / sd by threads
+// t, t+nt, ..., then three FMAs per node.
 __device__ __forceinline__ void seg_poly(const double* ky, const double* kc, int na, const KnotSeg& ks, double* sb,
                                          double* sd, int t, int nt) {
     for (int j = t; j < na - 1; j += nt) {
@@ -1101,18 +1097,6 @@ __device__ __forceinline__ double dnu_S_poly(const NodeTerms& t, const double* k
     return ky[j] + t.dx * ((ky[j + 1] - ky[j]) * __ldg(ks.ih + j));
 }
 
-// The per-bin rest: J and the history row's natural spline (or linear for 2 knots) at
-// the node.  Same for the cached and uncached paths.
-// k_over_m = k / (m / kT): J's argument is fslength * k_over_m (one division per bin
-// instead of one per node).
-__device__ __forceinline__ double dnu_combine(const NodeTerms& t, double k_over_m, double qc, double nfl,
-                                              const double* ky, const double* kc, const double* sb,
-                                              const double* sd, int na, const KnotSeg& ks) {
-    const double S = dnu_S_poly(t, ky, kc, sb, sd, na, ks);
-    const double J = specialJ_tab(t.fsl * k_over_m, qc, nfl);
-    return t.g * J * S;
-}
-
 // Node table of one instance for one call: nslots * 61 entries, slot-major.
 struct NodeCache {
     double* g;
@@ -1122,7 +1106,7 @@ struct NodeCache {
     int nslots;
 };
 
-// The full integrand with the node table.
+// The integrand's terms at the nodes, for the adjoint.
 struct DnuIntegrandC {
     const Background* B;
     double k_over_m, qc, nfl;
@@ -1131,34 +1115,6 @@ struct DnuIntegrandC {
     const double* sb; const double* sd;  // seg_poly of (ky, kc)
     KnotSeg ks;
     NodeCache nc;
-    __device__ double node(int slot, int jn, double x) const {
-        NodeTerms t;
-        if (slot >= 0) {
-            const int q = slot * 61 + jn;
-            t.g = __ldg(nc.g + q);
-            t.fsl = __ldg(nc.fsl + q);
-            t.dx = __ldg(nc.dx + q);
-            t.j = __ldg(nc.j + q);
-        } else {
-            t = dnu_node_terms(B, fs_x, fs_y, fs_c, nfs, fs_x0, fs_inv, kx, na, x);
-        }
-        return dnu_combine(t, k_over_m, qc, nfl, ky, kc, sb, sd, na, ks);
-    }
-    // node jn of the interval with centre c and half-length h: x = c + h x_jn is needed
-    // only where the node table has no entry
-    __device__ double node_at(int slot, int jn, double c, double h, double xj) const {
-        NodeTerms t;
-        if (slot >= 0) {
-            const int q = slot * 61 + jn;
-            t.g = __ldg(nc.g + q);
-            t.fsl = __ldg(nc.fsl + q);
-            t.dx = __ldg(nc.dx + q);
-            t.j = __ldg(nc.j + q);
-        } else {
-            t = dnu_node_terms(B, fs_x, fs_y, fs_c, nfs, fs_x0, fs_inv, kx, na, __dadd_rn(c, __dmul_rn(h, xj)));
-        }
-        return dnu_combine(t, k_over_m, qc, nfl, ky, kc, sb, sd, na, ks);
-    }
     __device__ NodeTerms terms(int slot, int jn, double x) const {
         if (slot >= 0) {
             const int q = slot * 61 + jn;
@@ -1171,6 +1127,64 @@ struct DnuIntegrandC {
         }
         return dnu_node_terms(B, fs_x, fs_y, fs_c, nfs, fs_x0, fs_inv, kx, na, x);
     }
+};
+
+// The integrand as the integrals evaluate it.  At a node in history segment j the natural
+// spline is S = A y_j + B y_{j+1} + C c_j + D c_{j+1} (c = S''/2 at the knots) with weights that
+// depend on the node only, so the node table holds g A, g B, g C, g D and a bin's value is
+// J (k fslength / (m / kT)) times their sum with its row: five FP64 operations and J's six,
+// against fourteen with the spline's polynomial per segment and J's first table, and no
+// per-bin pass over the segments.
+struct NodeWeights {
+    double a, b, c, d;
+};
+__device__ __forceinline__ NodeWeights node_weights(double g, double dx, double h, int na) {
+    NodeWeights w;
+    const double s = dx / h;
+    const double gs = __dmul_rn(g, s);
+    w.a = __dsub_rn(g, gs);
+    w.b = gs;
+    const double e = na > 2 ? __dmul_rn(__dmul_rn(g, dx), 1.0 / 3.0) : 0.0;  // two knots: linear
+    // C = dx (dx - 2 h / 3 - dx s / 3), D = dx (dx s - h) / 3
+    w.c = __dmul_rn(e, __dsub_rn(__dmul_rn(3.0, dx), __fma_rn(dx, s, __dmul_rn(2.0, h))));
+    w.d = __dmul_rn(e, __fma_rn(dx, s, -h));
+    return w;
+}
+// Node table entry: {g A, g B}, {g C, g D}, fslength, {j, fslength as a float}.
+struct NodeTable {
+    const double2* ab;
+    const double2* cd;
+    const double* fsl;
+    const int2* jf;
+    int nslots;
+};
+struct DnuIntegrandW {
+    const Background* B;
+    const double* jt;          // J's fine table
+    double kom;                // k / (m / kT)
+    float komf;
+    double qc, nfl;            // qc > 0: the series instead of the fit
+    const double* ky;          // the bin's history row and its spline coefficients
+    const double* kc;
+    NodeTable nc;
+    // for intervals that are not in the node table
+    const double* fs_x; const double* fs_y; const double* fs_c; const double* kx;
+    const StepScalars* S;
+    int na;
+    __device__ __forceinline__ double value(const NodeWeights& w, double fsl, float fslf, int j) const {
+        const double v = fma(w.d, kc[j + 1], fma(w.c, kc[j], fma(w.b, ky[j + 1], __dmul_rn(w.a, ky[j]))));
+        return __dmul_rn(v, specialJ_node(jt, fsl, fslf, kom, komf, qc, nfl));
+    }
+    __device__ __forceinline__ double node_at(int slot, int jn, double c, double h, double xj) const {
+        if (slot >= 0) {
+            const int q = slot * 61 + jn;
+            const double2 ab = __ldg(nc.ab + q), cd = __ldg(nc.cd + q);
+            const int2 jf = __ldg(nc.jf + q);
+            return value(NodeWeights{ab.x, ab.y, cd.x, cd.y}, __ldg(nc.fsl + q), __int_as_float(jf.y), jf.x);
+        }
+        return slow(__dadd_rn(c, __dmul_rn(h, xj)));
+    }
+    __device__ __noinline__ double slow(double x) const;  // (ksp_internal.h)
 };
 
 // Slot of the dyadic interval [a, b] of [lo, hi] in a node table of nslots slots (-1: not

@@ -22,9 +22,17 @@
 #include <stdio.h>
 #include "ksp_internal.h"
 #include "ksp_prep.cuh"
+#include "jfine_table.h"
 #include "ksp_ptx.cuh"
 
 namespace ksp {
+
+static __device__ const __align__(16) double g_jfine[KSP_JFINE_PIECES * KSP_JFINE_STRIDE] = KSP_JFINE_TABLE_INIT;
+static_assert(KSP_JFINE_SUB_BITS == 8 && KSP_JFINE_DEG == 5 && KSP_JFINE_STRIDE == 8, "specialJ_node");
+const double* jfine_table() {
+    void* p = nullptr;
+    return cudaGetSymbolAddress(&p, g_jfine) == cudaSuccess ? static_cast<const double*>(p) : nullptr;
+}
 
 // ------------------------------------------------------------------ background tables
 struct RhoIntegrand {  // omega_nu_single.c:89-96
@@ -300,11 +308,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, 
     b -= P.fs_blocks;
     const int q = b * kPrepThreads + t;
     if (q >= P.nodes) return;
-    const double x = nc_node_x(q, P.loga0, P.loga);
-    const int j = seg_bsearch(I.scalefact, Na, x);  // (the last knot is not read)
-    I.nc_j[q] = j;
-    I.nc_dx[q] = x - I.scalefact[j];
-    I.nc_inv[q] = node_inv_aH(I.B, x);
+    I.nc_inv[q] = node_inv_aH(I.B, nc_node_x(q, P.loga0, P.loga));
 }
 
 // The fslength table, the node table, and the row splines.
@@ -322,12 +326,13 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, 
 // L1-cached): the binning pass holds nearly all of every SM's shared memory.
 constexpr int kTableThreads = 128;
 __global__ void __launch_bounds__(kTableThreads, 8)
-    k_prep_tables(IntegratorDev I, PrepArgs P, int rows, int nk, int update_row) {
+    k_prep_tables(IntegratorDev I, PrepArgs P, int rows, int nk, int update_row, FinalizeArgs fin) {
     __shared__ double tsuf[kPrepThreads + 1], sh[2 * kTableThreads / 32];
     const int t = threadIdx.x, Na = P.Na;
     int b = blockIdx.x;
     const int nrow = rows == kRowsBase ? nk + 1 : (rows == kRowsFull ? nk : 0);
     if (b < nrow) {
+        if (fin.active && b < nk && t == kTableThreads - 1) finalize_keff(fin, b);
         const int m = Na - 2;  // unknowns c[1..m]
         const double* ih = I.knot_invh;
         double* c;
@@ -380,8 +385,9 @@ __global__ void __launch_bounds__(kTableThreads, 8)
     if (q >= P.nodes) return;
     const double x = nc_node_x(q, P.loga0, P.loga);
     const double fsl = fs_table_at(F, P.loga0, P.loga, x);
-    I.nc_fsl[q] = fsl;
-    I.nc_g[q] = fsl * I.nc_inv[q];
+    const double* kx = I.scalefact;
+    const int j = seg_bsearch(kx, Na, x);
+    nc_store(I, q, fsl, I.nc_inv[q], x - kx[j], j, kx[j + 1] - kx[j], Na);
 }
 
 // block per bin: this bin's delta_cdm (a deferred normalisation), the provisional row
@@ -390,7 +396,11 @@ __global__ void k_row_update(IntegratorDev I, int nk, int Na, int row, FinalizeA
     __shared__ double s_dy;
     const int ik = blockIdx.x;
     if (threadIdx.x == 0) {
-        if (fin.active) finalize_bin(fin, ik);
+        if (fin.active) {
+            double p;
+            I.dcdm[ik] = finalize_power(fin, ik, &p);
+            if (fin.power_out) fin.power_out[ik] = p;
+        }
         const StepScalars& S = *I.sc;
         double* y = I.dtot + (size_t)ik * I.ld;
         const double yn = get_delta_tot(I.nu_last[ik], I.dcdm[ik], S.OmegaNua3, S.Omeganonu, S.OmegaNu1, S.partnu);
@@ -404,32 +414,24 @@ __global__ void k_row_update(IntegratorDev I, int nk, int Na, int row, FinalizeA
 }
 
 // ------------------------------------------------------------------ delta_nu integral
-// Shared memory per CTA: Gk61Nodes | knots[ld] | per warp: QagList, row[ld], coef[ld], seg_poly [2 ld] |
-// mbarriers
+// Shared memory per CTA: Gk61Nodes | per warp: QagList, row[ld], coef[ld] | mbarriers
 __global__ void __launch_bounds__(128) k_dnu_qag(IntegratorDev I, int nk, int Na, int nspec, int4 spec_ids) {
     extern __shared__ __align__(16) unsigned char sm[];
     Gk61Nodes& N = *reinterpret_cast<Gk61Nodes*>(sm);
-    size_t off = (sizeof(Gk61Nodes) + 15) & ~size_t(15);
-    double* knots = reinterpret_cast<double*>(sm + off);
-    off += sizeof(double) * I.ld;
+    const size_t off = (sizeof(Gk61Nodes) + 15) & ~size_t(15);
     const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t per_warp = sizeof(QagList) + 4 * sizeof(double) * I.ld;
+    const size_t per_warp = sizeof(QagList) + 2 * sizeof(double) * I.ld;
     unsigned char* wbase = sm + off + warp * per_warp;
     QagList& L = *reinterpret_cast<QagList*>(wbase);
     double* row = reinterpret_cast<double*>(wbase + sizeof(QagList));
     double* rc = row + I.ld;
-    double* sb = rc + I.ld;
-    double* sd = sb + I.ld;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(sm + off + nw * per_warp);
-    uint64_t* mybar = bars + warp;
+    uint64_t* mybar = reinterpret_cast<uint64_t*>(sm + off + nw * per_warp) + warp;
 
     gk61_fill(N, threadIdx.x, blockDim.x);
-    for (int i = threadIdx.x; i < Na; i += blockDim.x) knots[i] = I.scalefact[i];
     if (lane == 0) ptx::mbar_init(mybar, 1);
     ptx::mbar_init_fence();
     __syncthreads();
 
-    const Background* B = I.B;
     const StepScalars& S = *I.sc;
     const int ntask = nspec * nk;
     const unsigned row_bytes = (unsigned)(((Na + 1) & ~1) * sizeof(double));
@@ -440,19 +442,8 @@ __global__ void __launch_bounds__(128) k_dnu_qag(IntegratorDev I, int nk, int Na
         const int si = task / nk, ik = task % nk;
         const int mi = si == 0 ? spec_ids.x : (si == 1 ? spec_ids.y : spec_ids.z);
         const double k = I.kq ? I.kq[ik] : I.wavenum[ik];
-        // the task's divisions on lane 0
-        double mnubykT = 0, kom = 0, fsi = 0;
-        if (lane == 0) {
-            mnubykT = B->mnu_J[mi] / B->kBtnu;
-            kom = k / mnubykT;
-            fsi = (S.Nfs - 1.) / (S.loga - S.loga0);
-        }
-        mnubykT = __shfl_sync(0xffffffffu, mnubykT, 0);
-        kom = __shfl_sync(0xffffffffu, kom, 0);
-        fsi = __shfl_sync(0xffffffffu, fsi, 0);
-        double integral = 0;
-        const bool integrate = !S.skip_integral && Na > 1 && mnubykT > 0;
-        if (integrate) {
+        double val = lane == 0 ? dnu_initial(I, S, ik, mi, k) : 0.0;
+        if (!S.skip_integral && Na > 1 && S.inv_m[mi] > 0) {
             // stage the history row and its spline coefficients (TMA bulk copies)
             __syncwarp();
             if (lane == 0) {
@@ -462,6 +453,7 @@ __global__ void __launch_bounds__(128) k_dnu_qag(IntegratorDev I, int nk, int Na
                 ptx::bulk_g2s(row, I.dtot + (size_t)ik * I.ld, row_bytes, mybar);
                 if (Na > 2) ptx::bulk_g2s(rc, I.coef + (size_t)ik * I.ld, row_bytes, mybar);
             }
+            if (Na == 2 && lane < 2) rc[lane] = 0.0;  // linear: no coefficients
             const bool got = __all_sync(0xffffffffu, ptx::mbar_wait_bounded(mybar, phase));  // warp-uniform
             phase ^= 1;
             if (!got) {
@@ -470,13 +462,10 @@ __global__ void __launch_bounds__(128) k_dnu_qag(IntegratorDev I, int nk, int Na
                 ptx::mbar_wait_bounded(mybar, phase ^ 1);
                 return;
             }
-            const KnotSeg ks{I.knot_invh, I.knot_h3, I.knot_ih3};
-            if (Na > 2) seg_poly(row, rc, Na, ks, sb, sd, lane, 32);
             __syncwarp();
-            const double qc = S.partnu_now > 0 ? B->vcrit * mnubykT : 0.0;
-            const DnuIntegrandC f = dnu_integrand_pre(I, S, kom, fsi, qc, knots, row, rc, sb, sd, Na);
+            const DnuIntegrandW f = dnu_integrand_w(I, S, mi, k * S.inv_m[mi], row, rc, Na);
             QagResult r = qag_warp_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit);
-            integral = r.result;
+            val += S.prefac * r.result;
             if (I.ivals) {  // keep the final subdivision for the adjoint
                 double* dst = I.ivals + ((size_t)mi * I.nk_alloc + ik) * kQagLimit * 2;
                 for (int q = lane; q < r.nint; q += 32) {
@@ -489,7 +478,7 @@ __global__ void __launch_bounds__(128) k_dnu_qag(IntegratorDev I, int nk, int Na
             my_max = max(my_max, r.nint);
             my_tot += r.nint;
         }
-        if (lane == 0) I.dnu_s[(size_t)mi * I.nk_alloc + ik] = dnu_task_value(I, S, ik, k, mnubykT, integrate, integral);
+        if (lane == 0) I.dnu_s[(size_t)mi * I.nk_alloc + ik] = val;
     }
     if (lane == 0 && my_tot) {
         atomicMax(I.qag_max, my_max);
@@ -503,7 +492,13 @@ __global__ void __launch_bounds__(128) k_dnu_qag(IntegratorDev I, int nk, int Na
 // per task leaves the SMs' FP64 pipes idle between the long dependent chains of a single
 // warp and the sequential QAG rounds set the time.
 // SPEC = false: blocks of 4 warps and qag_block_c (no look-ahead).
-// Shared memory: Gk61Nodes | knots[ld] | row[ld] | coef[ld] | QagList | QagSpecSmem or QagBlockSmem | mbarrier
+// upd.row >= 0: a prepared step's provisional row (k_row_update's arithmetic, per task, while
+// the row is on its way, instead of a launch of its own before this one: 7 us).
+// Shared memory: Gk61Nodes | row[ld] | coef[ld] | QagList | QagSpecSmem or QagBlockSmem | mbarrier
+struct RowUpdate {
+    int row;
+    FinalizeArgs fin;
+};
 template <bool SPEC>
 struct QagBlkSmemOf { typedef QagSpecSmem type; };
 template <>
@@ -511,58 +506,62 @@ struct QagBlkSmemOf<false> { typedef QagBlockSmem type; };
 
 template <bool SPEC>
 __global__ void __launch_bounds__(SPEC ? 256 : 128, SPEC ? 2 : 4)
-    k_dnu_qag_blk(IntegratorDev I, int nk, int Na, int nspec, int4 spec_ids) {
+    k_dnu_qag_blk(IntegratorDev I, int nk, int Na, int nspec, int4 spec_ids, RowUpdate upd) {
     typedef typename QagBlkSmemOf<SPEC>::type Smem;
     extern __shared__ __align__(16) unsigned char sm[];
     Gk61Nodes& N = *reinterpret_cast<Gk61Nodes*>(sm);
     size_t off = (sizeof(Gk61Nodes) + 15) & ~size_t(15);
-    double* knots = reinterpret_cast<double*>(sm + off);
-    off += sizeof(double) * I.ld;
     double* row = reinterpret_cast<double*>(sm + off);
-    off += sizeof(double) * I.ld;
-    double* rc = reinterpret_cast<double*>(sm + off);
-    off += sizeof(double) * I.ld;
-    double* sb = reinterpret_cast<double*>(sm + off);
-    double* sd = sb + I.ld;
+    double* rc = row + I.ld;
     off += 2 * sizeof(double) * I.ld;
     QagList& L = *reinterpret_cast<QagList*>(sm + off);
     off += (sizeof(QagList) + 15) & ~size_t(15);
     Smem& sh = *reinterpret_cast<Smem*>(sm + off);
     off += (sizeof(Smem) + 15) & ~size_t(15);
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + off);
-    __shared__ double s_task[4];  // m/kT, k/(m/kT), (Nfs-1)/(log a - log a0), integrate? of the current task
+    __shared__ double s_y, s_dy;  // the current task's provisional value, and what it adds
     const int tid = threadIdx.x;
-    const Background* B = I.B;
     const StepScalars& S = *I.sc;
     const int ntask = nspec * nk;
     const unsigned row_bytes = (unsigned)(((Na + 1) & ~1) * sizeof(double));
-    // Thread 0 starts a task: the copies of its history row and spline coefficients, then
-    // the task's divisions while they land.
+    // Thread 0 starts a task: the copies of its history row and spline coefficients, then the
+    // provisional value while they land; another warp's first thread leaves the
+    // initial-condition term where the integral will be added.
     auto start_task = [&](int task) {
         const int si = task / nk, ik = task % nk;
         const int mi = si == 0 ? spec_ids.x : (si == 1 ? spec_ids.y : spec_ids.z);
-        const double mnu = B->mnu_J[mi];
-        const bool integ = !S.skip_integral && Na > 1 && mnu / B->kBtnu > 0;
-        if (integ) {
+        if (tid == 32) I.dnu_s[(size_t)mi * I.nk_alloc + ik] = dnu_initial(I, S, ik, mi, I.kq ? I.kq[ik] : I.wavenum[ik]);
+        if (tid != 0) return;
+        if (!S.skip_integral && Na > 1 && S.inv_m[mi] > 0) {
             ptx::fence_async_smem();
             ptx::mbar_expect_tx(bar, Na > 2 ? 2 * row_bytes : row_bytes);
             ptx::bulk_g2s(row, I.dtot + (size_t)ik * I.ld, row_bytes, bar);
             if (Na > 2) ptx::bulk_g2s(rc, I.coef + (size_t)ik * I.ld, row_bytes, bar);
+            else rc[0] = rc[1] = 0.0;  // linear: no coefficients
         }
-        const double m = mnu / B->kBtnu;
-        s_task[0] = m;
-        s_task[1] = (I.kq ? I.kq[ik] : I.wavenum[ik]) / m;
-        s_task[2] = (S.Nfs - 1.) / (S.loga - S.loga0);
-        s_task[3] = integ ? 1.0 : 0.0;
+        if (upd.row >= 0) {
+            double d;
+            if (upd.fin.active) {
+                double p;
+                d = finalize_power(upd.fin, ik, &p);
+                if (si == 0) {
+                    I.dcdm[ik] = d;
+                    if (upd.fin.power_out) upd.fin.power_out[ik] = p;
+                }
+            } else {
+                d = I.dcdm[ik];
+            }
+            s_y = get_delta_tot(I.nu_last[ik], d, S.OmegaNua3, S.Omeganonu, S.OmegaNu1, S.partnu);
+            s_dy = s_y - I.dtot[(size_t)ik * I.ld + Na - 2];
+        }
     };
     // the first task's copies are in flight while the block fills its tables
     if (tid == 0) {
         ptx::mbar_init(bar, 1);
         ptx::mbar_init_fence();
-        if (blockIdx.x < ntask) start_task(ntask - 1 - (int)blockIdx.x);
     }
+    if (blockIdx.x < ntask) start_task(ntask - 1 - (int)blockIdx.x);
     gk61_fill(N, tid, blockDim.x);
-    for (int i = tid; i < Na; i += blockDim.x) knots[i] = I.scalefact[i];
     __syncthreads();
     unsigned phase = 0;
     int my_max = 0;
@@ -573,45 +572,43 @@ __global__ void __launch_bounds__(SPEC ? 256 : 128, SPEC ? 2 : 4)
     for (int task = blockIdx.x; task < ntask; task += gridDim.x) {
         const int si = (ntask - 1 - task) / nk, ik = (ntask - 1 - task) % nk;
         const int mi = si == 0 ? spec_ids.x : (si == 1 ? spec_ids.y : spec_ids.z);
-        const double k = I.kq ? I.kq[ik] : I.wavenum[ik];
         if (task != (int)blockIdx.x) {  // later tasks: after the previous task's reads of row / rc
             __syncthreads();
-            if (tid == 0) start_task(ntask - 1 - task);
+            start_task(ntask - 1 - task);
             __syncthreads();
         }
-        const double mnubykT = s_task[0];
-        double integral = 0;
-        const bool integrate = s_task[3] != 0.0;
-        if (integrate) {
-            const bool got = __syncthreads_and(ptx::mbar_wait_bounded(bar, phase));  // block-uniform
-            phase ^= 1;
-            if (!got) {
-                if (tid == 0) atomicOr(I.status, kStTimeout);
-                ptx::mbar_wait_bounded(bar, phase ^ 1);
-                return;
-            }
-            const KnotSeg ks{I.knot_invh, I.knot_h3, I.knot_ih3};
-            if (Na > 2) seg_poly(row, rc, Na, ks, sb, sd, tid, blockDim.x);
-            __syncthreads();
-            const double qc = S.partnu_now > 0 ? B->vcrit * mnubykT : 0.0;
-            const DnuIntegrandC f = dnu_integrand_pre(I, S, s_task[1], s_task[2], qc, knots, row, rc, sb, sd, Na);
-            QagResult r;
-            if constexpr (SPEC) r = qag_block_spec_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
-            else r = qag_block_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
-            integral = r.result;
-            if (I.ivals) {  // keep the final subdivision for the adjoint
-                double* dst = I.ivals + ((size_t)mi * I.nk_alloc + ik) * kQagLimit * 2;
-                for (int q = tid; q < r.nint; q += blockDim.x) {
-                    dst[2 * q] = L.a[q];
-                    dst[2 * q + 1] = L.b[q];
-                }
-                if (tid == 0) I.nivals[(size_t)mi * I.nk_alloc + ik] = r.nint;
-            }
-            if (!r.ok && tid == 0) atomicOr(I.status, kStGsl);
-            my_max = max(my_max, r.nint);
-            my_tot += r.nint;
+        if (S.skip_integral || Na <= 1 || !(S.inv_m[mi] > 0)) continue;  // block-uniform
+        const bool got = __syncthreads_and(ptx::mbar_wait_bounded(bar, phase));  // block-uniform
+        phase ^= 1;
+        if (!got) {
+            if (tid == 0) atomicOr(I.status, kStTimeout);
+            ptx::mbar_wait_bounded(bar, phase ^ 1);
+            return;
         }
-        if (tid == 0) I.dnu_s[(size_t)mi * I.nk_alloc + ik] = dnu_task_value(I, S, ik, k, mnubykT, integrate, integral);
+        if (upd.row >= 0) {
+            const double dy = s_dy;
+            for (int j = 1 + tid; j < Na - 1; j += blockDim.x) rc[j] = fma(dy, __ldg(I.coef_unit + j), rc[j]);
+            if (tid == 0) row[Na - 1] = s_y;
+            __syncthreads();
+        }
+        const double kom = (I.kq ? I.kq[ik] : I.wavenum[ik]) * S.inv_m[mi];
+        const DnuIntegrandW f = dnu_integrand_w(I, S, mi, kom, row, rc, Na);
+        QagResult r;
+        if constexpr (SPEC) r = qag_block_spec_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
+        else r = qag_block_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
+        if (I.ivals) {  // keep the final subdivision for the adjoint
+            double* dst = I.ivals + ((size_t)mi * I.nk_alloc + ik) * kQagLimit * 2;
+            for (int q = tid; q < r.nint; q += blockDim.x) {
+                dst[2 * q] = L.a[q];
+                dst[2 * q + 1] = L.b[q];
+            }
+            if (tid == 0) I.nivals[(size_t)mi * I.nk_alloc + ik] = r.nint;
+        }
+        if (!r.ok && tid == 0) atomicOr(I.status, kStGsl);
+        my_max = max(my_max, r.nint);
+        my_tot += r.nint;
+        // (the same block wrote the initial-condition term, before a barrier)
+        if (tid == 0) I.dnu_s[(size_t)mi * I.nk_alloc + ik] += S.prefac * r.result;
     }
     if (tid == 0 && my_tot) {
         atomicMax(I.qag_max, my_max);
@@ -620,7 +617,7 @@ __global__ void __launch_bounds__(SPEC ? 256 : 128, SPEC ? 2 : 4)
 }
 
 size_t dnu_qag_blk_smem(int ld, bool spec) {
-    return ((sizeof(Gk61Nodes) + 15) & ~size_t(15)) + 5 * sizeof(double) * ld + ((sizeof(QagList) + 15) & ~size_t(15)) +
+    return ((sizeof(Gk61Nodes) + 15) & ~size_t(15)) + 2 * sizeof(double) * ld + ((sizeof(QagList) + 15) & ~size_t(15)) +
            (((spec ? sizeof(QagSpecSmem) : sizeof(QagBlockSmem)) + 15) & ~size_t(15)) + sizeof(uint64_t);
 }
 
@@ -631,7 +628,7 @@ __global__ void k_combine(IntegratorDev I, int nk) {
     const StepScalars& S = *I.sc;
     double acc = 0;
     for (int mi = 0; mi < kNuSpecies; mi++)
-        if (I.B->deg[mi] > 0) acc += I.dnu_s[(size_t)mi * I.nk_alloc + ik] * S.omeganu[mi] / S.Omega_nu_tot;
+        if (S.wnu[mi] != 0.0) acc += I.dnu_s[(size_t)mi * I.nk_alloc + ik] * S.wnu[mi];
     I.dnu[ik] = acc;
 }
 
@@ -711,14 +708,15 @@ static GL4 gl4_host() {
 }
 
 size_t dnu_qag_smem(int ld, int wpb) {
-    return ((sizeof(Gk61Nodes) + 15) & ~size_t(15)) + sizeof(double) * ld +
-           wpb * (sizeof(QagList) + 4 * sizeof(double) * ld) + wpb * sizeof(uint64_t);
+    return ((sizeof(Gk61Nodes) + 15) & ~size_t(15)) + wpb * (sizeof(QagList) + 2 * sizeof(double) * ld) +
+           wpb * sizeof(uint64_t);
 }
 
 // Blocks per role of a call's preparation.
 void launch_integrator_prepare(const IntegratorDev& I, const Background& B, const StepScalars& S, int Na, double a,
                                double loga, double loga0, double TimeTransfer, int start_row, int write_knot,
-                               bool scalars_only, RowsMode rows, int nk, int update_row, cudaStream_t st) {
+                               bool scalars_only, RowsMode rows, int nk, int update_row, const FinalizeArgs* fin,
+                               cudaStream_t st) {
     static const GL4 gl = gl4_host();
     PrepArgs P{};
     P.S = S;
@@ -744,17 +742,19 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
     const int blocks = nrow + (P.Nfs + kTableThreads - 1) / kTableThreads +
                        (P.nodes + kTableThreads - 1) / kTableThreads;
     if (blocks > 0)
-        k_prep_tables<<<blocks, kTableThreads, 0, st>>>(I, P, nrow > 0 ? (int)rows : (int)kRowsNone, nk, update_row);
+        k_prep_tables<<<blocks, kTableThreads, 0, st>>>(I, P, nrow > 0 ? (int)rows : (int)kRowsNone, nk, update_row,
+                                                     fin ? *fin : FinalizeArgs{});
 }
 
 // The rest, after the rows' splines: the integrals, the species sum.
 void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, const int* spec_ids,
                             int warps_per_block, cudaStream_t st, int qag_split, int update_row, bool defer_combine,
                             const FinalizeArgs* fin, bool base_ready) {
+    RowUpdate upd{};
+    upd.row = -1;
     if (update_row >= 0 && base_ready) {
-        FinalizeArgs fa{};
-        if (fin && fin->active) fa = *fin;
-        k_row_update<<<nk, 128, 0, st>>>(I, nk, Na, update_row, fa);
+        upd.row = update_row;
+        if (fin && fin->active) upd.fin = *fin;
     } else if (update_row >= 0) {
         // a history of two knots: no splines
         if (fin && fin->active)
@@ -795,9 +795,10 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
                 blk_attr = true;
             }
             const int4 sp = make_int4(spec_ids[0], spec_ids[1], spec_ids[2], 0);
-            if (spec) k_dnu_qag_blk<true><<<ntask, 256, bsmem, st>>>(I, nk, Na, nspec, sp);
-            else k_dnu_qag_blk<false><<<ntask, split >= 4 ? 128 : 64, bsmem, st>>>(I, nk, Na, nspec, sp);
+            if (spec) k_dnu_qag_blk<true><<<ntask, 256, bsmem, st>>>(I, nk, Na, nspec, sp, upd);
+            else k_dnu_qag_blk<false><<<ntask, split >= 4 ? 128 : 64, bsmem, st>>>(I, nk, Na, nspec, sp, upd);
         } else {
+            if (upd.row >= 0) k_row_update<<<nk, 128, 0, st>>>(I, nk, Na, upd.row, upd.fin);
             const int blocks = (ntask + wpb - 1) / wpb;
             k_dnu_qag<<<blocks, 32 * wpb, smem, st>>>(I, nk, Na, nspec,
                                                       make_int4(spec_ids[0], spec_ids[1], spec_ids[2], 0));
@@ -813,7 +814,7 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
 // -3: a differentiable step: like -1 but delta_nu_last is left unchanged.
 __global__ void k_finish(IntegratorDev I, int nk, int commit_row, double a, double loga, const double* keff,
                          double* dnu_out, double* logk_out, double* ratio_out, CorrTable corr, double* norm_out,
-                         int combine) {
+                         int combine, int logk_ready) {
     const StepScalars& S = *I.sc;
     const bool pass = commit_row == -2;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -826,7 +827,7 @@ __global__ void k_finish(IntegratorDev I, int nk, int commit_row, double a, doub
         if (!combine) return I.dnu[ik];
         double acc = 0;
         for (int mi = 0; mi < kNuSpecies; mi++)
-            if (I.B->deg[mi] > 0) acc += I.dnu_s[(size_t)mi * I.nk_alloc + ik] * S.omeganu[mi] / S.Omega_nu_tot;
+            if (S.wnu[mi] != 0.0) acc += I.dnu_s[(size_t)mi * I.nk_alloc + ik] * S.wnu[mi];
         return acc;
     };
     // Bin ik's slope needs bin ik+1's final value: recomputed here rather than read back,
@@ -846,9 +847,9 @@ __global__ void k_finish(IntegratorDev I, int nk, int commit_row, double a, doub
         }
         dnu_out[ik] = out;
         if (keff) {
-            const double lk = log(keff[ik]);
+            const double lk = logk_ready ? logk_out[ik] : log(keff[ik]);
             const double r = out / I.dcdm[ik];
-            if (logk_out) logk_out[ik] = lk;
+            if (logk_out && !logk_ready) logk_out[ik] = lk;
             if (ratio_out) ratio_out[ik] = r;
             if (corr.xf) {
                 corr.xf[ik] = (float)lk;
@@ -857,7 +858,7 @@ __global__ void k_finish(IntegratorDev I, int nk, int commit_row, double a, doub
                 if (ik + 1 < nk) {
                     const double v1 = dnu_of(ik + 1);
                     const double out1 = pass ? v1 : (v1 < 0 ? 0.0 : v1);
-                    const double lk1 = log(keff[ik + 1]);
+                    const double lk1 = logk_ready ? logk_out[ik + 1] : log(keff[ik + 1]);
                     const double r1 = out1 / I.dcdm[ik + 1];
                     sl = norm * (r1 - r) / (lk1 - lk);
                 }
@@ -870,10 +871,10 @@ __global__ void k_finish(IntegratorDev I, int nk, int commit_row, double a, doub
 
 void launch_finish_update(const IntegratorDev& I, int nk, int commit_row, double a, double loga,
                           const double* keff, double* dnu_out, double* logk_out, double* ratio_out,
-                          CorrTable corr, double* norm_out, cudaStream_t st, bool combine) {
+                          CorrTable corr, double* norm_out, cudaStream_t st, bool combine, bool logk_ready) {
     k_finish<<<(nk + 31) / 32 > 0 ? (nk + 31) / 32 : 1, 32, 0, st>>>(I, nk, commit_row, a, loga, keff, dnu_out,
                                                                      logk_out, ratio_out, corr, norm_out,
-                                                                     combine ? 1 : 0);
+                                                                     combine ? 1 : 0, logk_ready ? 1 : 0);
 }
 
 }  // namespace ksp

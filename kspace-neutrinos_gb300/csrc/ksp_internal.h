@@ -15,6 +15,9 @@ struct StepScalars {
     double OmegaNua3, OmegaNu1, partnu;  // get_delta_tot coefficients at a (:179-181)
     double Omega_nu_tot;             // get_omega_nu_nopart(a) (:155)
     double omeganu[kNuSpecies];      // deg * omega_nu_single(a, mi) (:162)
+    double wnu[kNuSpecies];          // omeganu / Omega_nu_tot: the species' weights (0: none)
+    double inv_m[kNuSpecies];        // 1 / (m / kT) of the mass inside J (0: massless)
+    double qc[kNuSpecies];           // the momentum cut of J's series (0: the fit)
     double fsl_A0a;                  // fslength(log a0, log a) (:522)
     double deriv_prefac;             // a0 * H(a0)/c * a0 (:524)
     double relerr;                   // 1e-6, loosened for hybrid neutrinos (:547)
@@ -48,6 +51,10 @@ struct IntegratorDev {
     double* nc_fsl;
     double* nc_dx;
     int* nc_j;
+    double2* nc_ab;                  // [kNcNodes] the same as weights of the row (NodeTable)
+    double2* nc_cd;
+    int2* nc_jf;
+    const double* jt;                // J's fine table (one per device)
     int nc_slots;                    // slots of the node table in use (1 + 2 levels, 0 = none)
     double* fs_x;                    // [fs_cap]
     double* fs_y;                    // [fs_cap]
@@ -71,6 +78,15 @@ struct IntegratorDev {
                                      // the other knots zero (kRowsBase)
 };
 
+// What the integrals and the species sum need of a species, from its omeganu, Omega_nu_tot and
+// partnu.
+KSP_HD void species_scalars(const Background& B, int mi, StepScalars& S) {
+    const double mnubykT = B.mnu_J[mi] / B.kBtnu;
+    S.wnu[mi] = B.deg[mi] > 0 ? S.omeganu[mi] / S.Omega_nu_tot : 0.0;
+    S.inv_m[mi] = mnubykT > 0 ? 1.0 / mnubykT : 0.0;
+    S.qc[mi] = S.partnu > 0 ? B.vcrit * mnubykT : 0.0;
+}
+
 // The part of StepScalars that a call sets (the rest is set with the table): on the host
 // for a single call, where it takes about a microsecond beside the launches (on the device
 // it was a chain of some 60 dependent FP64 divisions, 12 us of each call).
@@ -85,7 +101,10 @@ inline void call_scalars(const Background& B, double a, double loga, double loga
     S.OmegaNu1 = om_1;
     S.partnu = partnu;
     S.Omega_nu_tot = nop;
-    for (int mi = 0; mi < kNuSpecies; mi++) S.omeganu[mi] = B.deg[mi] > 0 ? B.deg[mi] * omega_nu_single(B, a, mi) : 0.0;
+    for (int mi = 0; mi < kNuSpecies; mi++) {
+        S.omeganu[mi] = B.deg[mi] > 0 ? B.deg[mi] * omega_nu_single(B, a, mi) : 0.0;
+        species_scalars(B, mi, S);
+    }
     S.deriv_prefac = TT * (hubble(B, TT) / S.light) * TT;
     S.relerr = 1e-6;
     S.partnu_now = partnu;
@@ -127,7 +146,10 @@ __device__ __forceinline__ void call_scalars_warp(const Background& B, double a,
     S.OmegaNu1 = om_1;
     S.partnu = partnu;
     S.Omega_nu_tot = nop;
-    for (int mi = 0; mi < kNuSpecies; mi++) S.omeganu[mi] = om_s[mi];
+    for (int mi = 0; mi < kNuSpecies; mi++) {
+        S.omeganu[mi] = om_s[mi];
+        species_scalars(B, mi, S);
+    }
     S.deriv_prefac = TT * (h_tt / S.light) * TT;
     S.relerr = 1e-6;
     S.partnu_now = partnu;
@@ -229,15 +251,40 @@ __device__ __forceinline__ DnuIntegrandC dnu_integrand(const IntegratorDev& I, c
                                                        const double* sd, int Na) {
     return dnu_integrand_pre(I, S, k / mnubykT, (S.Nfs - 1.) / (S.loga - S.loga0), qc, knots, row, rc, sb, sd, Na);
 }
-// The delta_nu of one (species, bin) task (delta_tot_table.c:525-535 and :597-603): the
-// initial-condition term plus prefac times the integral; one lane forms it (FP64 log and
-// exp of the J fit are issued per active lane).
-__device__ __forceinline__ double dnu_task_value(const IntegratorDev& I, const StepScalars& S, int ik,
-                                                 double k, double mnubykT, bool integrated, double integral) {
-    const double specJ0 = specialJ(k * S.fsl_A0a / (mnubykT > 0 ? mnubykT : 1), 0.0, I.B->nufrac_low[0]);
-    double val = specJ0 * I.nu_init[ik] * (1. + S.deriv_prefac * S.fsl_A0a);
-    if (integrated) val += S.prefac * integral;
-    return val;
+// The integrand of one (species mi, bin) from its row and spline coefficients (shared memory).
+__device__ __forceinline__ DnuIntegrandW dnu_integrand_w(const IntegratorDev& I, const StepScalars& S, int mi, double kom,
+                                                         const double* row, const double* rc, int Na) {
+    DnuIntegrandW f;
+    f.B = I.B; f.jt = I.jt; f.kom = kom; f.komf = (float)kom;
+    f.qc = S.qc[mi]; f.nfl = I.B->nufrac_low[0];
+    f.ky = row; f.kc = rc;
+    f.nc = NodeTable{I.nc_ab, I.nc_cd, I.nc_fsl, I.nc_jf, I.nc_slots};
+    f.fs_x = I.fs_x; f.fs_y = I.fs_y; f.fs_c = I.fs_c; f.kx = I.scalefact;
+    f.S = &S; f.na = Na;
+    return f;
+}
+// A node outside the node table: its terms evaluated here, then the same arithmetic.
+__device__ __noinline__ inline double DnuIntegrandW::slow(double x) const {
+    const NodeTerms t = dnu_node_terms(B, fs_x, fs_y, fs_c, S->Nfs, S->loga0, (S->Nfs - 1.) / (S->loga - S->loga0), kx, na, x);
+    return value(node_weights(t.g, t.dx, kx[t.j + 1] - kx[t.j], na), t.fsl, (float)t.fsl, t.j);
+}
+// Node q of the node table.
+__device__ __forceinline__ void nc_store(const IntegratorDev& I, int q, double fsl, double inv_aH, double dx, int j,
+                                         double h, int Na) {
+    const double g = fsl * inv_aH;
+    const NodeWeights w = node_weights(g, dx, h, Na);
+    I.nc_g[q] = g;
+    I.nc_fsl[q] = fsl;
+    I.nc_dx[q] = dx;
+    I.nc_j[q] = j;
+    I.nc_ab[q] = make_double2(w.a, w.b);
+    I.nc_cd[q] = make_double2(w.c, w.d);
+    I.nc_jf[q] = make_int2(j, __float_as_int((float)fsl));
+}
+// The initial-condition term of one (species, bin) task (delta_tot_table.c:525-535).
+__device__ __forceinline__ double dnu_initial(const IntegratorDev& I, const StepScalars& S, int ik, int mi, double k) {
+    const double specJ0 = specialJ_fit_tab(k * S.fsl_A0a * (S.inv_m[mi] > 0 ? S.inv_m[mi] : 1.0));
+    return specJ0 * I.nu_init[ik] * (1. + S.deriv_prefac * S.fsl_A0a);
 }
 #endif
 
@@ -262,19 +309,32 @@ struct FinalizeArgs {
     // formed on the host, as the reference forms them there (interface_gadget.c:84,96-99):
     // scale = BoxSize^-3 (pow), kfac = 2 pi / BoxSize
     double scale, kfac;
+    double* logk_out;  // log of the physical keff (finalize_keff)
 };
 #ifdef __CUDACC__
-__device__ __forceinline__ void finalize_bin(const FinalizeArgs& f, int c) {
+// the part that depends on the sums, and the part that is the geometry's alone (a prepared
+// step forms the latter beside the binning pass); p: the bin's power, returned: delta_cdm
+__device__ __forceinline__ double finalize_power(const FinalizeArgs& f, int c, double* p_out) {
     const int b = f.compact_bins[c];
     double p = f.bin_sum[b];
     p /= *f.F0sq;
-    const double cnt = (double)f.count[b];
-    const double ke = f.ksum[b] / cnt;
-    p /= cnt;
-    if (f.power_out) f.power_out[c] = p;
+    p /= (double)f.count[b];
+    *p_out = p;
+    return sqrt(p / f.scale);
+}
+__device__ __forceinline__ void finalize_keff(const FinalizeArgs& f, int c) {
+    const int b = f.compact_bins[c];
+    const double ke = f.ksum[b] / (double)f.count[b], kp = ke * f.kfac;
     if (f.keff_out) f.keff_out[c] = ke;
-    if (f.dcdm_out) f.dcdm_out[c] = sqrt(p / f.scale);
-    if (f.keffphys_out) f.keffphys_out[c] = ke * f.kfac;
+    if (f.keffphys_out) f.keffphys_out[c] = kp;
+    if (f.logk_out) f.logk_out[c] = log(kp);
+}
+__device__ __forceinline__ void finalize_bin(const FinalizeArgs& f, int c) {
+    double p;
+    const double d = finalize_power(f, c, &p);
+    if (f.power_out) f.power_out[c] = p;
+    if (f.dcdm_out) f.dcdm_out[c] = d;
+    finalize_keff(f, c);
 }
 #endif
 
@@ -295,6 +355,8 @@ int raise_dynamic_smem_limit(const void* kernel);
 void launch_background_tables(Background* dB, double a0, cudaStream_t st, unsigned* status);
 void launch_spline_coeffs_1thread(const double* x, const double* y, double* c, double* scratch, int n,
                                   cudaStream_t st);
+// J's fine table on the current device
+const double* jfine_table();
 void launch_nufrac_low(Background* dB, double light, double vcrit, cudaStream_t st, unsigned* status);
 // natural cubic spline of log H on n uniform knots of spacing h: coef[4 (n-1)], scratch[n]
 void launch_hubble_table(const double* H, int n, double h, double* coef, double* scratch, cudaStream_t st);
@@ -324,9 +386,11 @@ enum RowsMode {
                 // `update_row` (update_delta_tot, from delta_nu_last and delta_cdm)
 };
 // S: the table's scalars (light, prefac, Omeganonu); B: the background's host copy
+// fin (kRowsBase): the binning pass's normalisation, whose geometry part (keff) is formed here
 void launch_integrator_prepare(const IntegratorDev& I, const Background& B, const StepScalars& S, int Na, double a,
                                double loga, double loga0, double TimeTransfer, int start_row, int write_knot,
-                               bool scalars_only, RowsMode rows, int nk, int update_row, cudaStream_t st);
+                               bool scalars_only, RowsMode rows, int nk, int update_row, const FinalizeArgs* fin,
+                               cudaStream_t st);
 // The rest: the integrals and the species sum (get_delta_nu_combined,
 // delta_tot_table.c:153-172, writes I.dnu).
 // update_row >= 0: with a prepared step's provisional row first (base_ready: kRowsBase ran);
@@ -339,9 +403,11 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
 size_t dnu_qag_smem(int ld, int wpb);
 // end of get_delta_nu_update (delta_tot_table.c:226-248) + interface_common.c:134-146:
 // delta_nu_last, committed row, NaN check, clamp, ratio/log k/kspace_prefac, grid table
+// combine: the species sum first; logk_ready: logk_out holds the logs already
 void launch_finish_update(const IntegratorDev& I, int nk, int commit_row, double a, double loga,
                           const double* keff, double* dnu_out, double* logk_out, double* ratio_out,
-                          CorrTable corr, double* norm_out, cudaStream_t st, bool combine = false);
+                          CorrTable corr, double* norm_out, cudaStream_t st, bool combine = false,
+                          bool logk_ready = false);
 
 // ---- adjoint (ksp_adjoint.cu)
 struct AdjBinsHost {

@@ -8,6 +8,11 @@
 #include <cuda_runtime.h>
 #include "jfit_table.h"
 
+// the fine table (jfine_table.h): pieces of 64 bytes, in one translation unit, handed around
+// by pointer
+#define KSP_JFINE_E0 (-12)
+#define KSP_JFINE_PIECES 6400
+
 namespace ksp {
 
 static __device__ const double g_jfit[KSP_JFIT_PIECES * KSP_JFIT_STRIDE] = KSP_JFIT_TABLE_INIT;
@@ -61,6 +66,21 @@ __device__ __forceinline__ void specialJ_fit_tab_d(double x, double& J, double& 
     }
     J = v;
     Jd = dv;
+}
+
+// J at the node of a bin's integral, x = fslength k / (m / kT): the piece from x in single
+// precision (a piece's polynomial holds a rounding beyond its ends too), its variable
+// x - centre in one multiply-add, five more for the polynomial.  Arguments below 2^-12 or from
+// 2^13 on go to the first table and the formula.
+__device__ __forceinline__ double specialJ_node(const double* jt, double fsl, float fslf, double kom, float komf,
+                                                double qc, double nfl) {
+    if (qc > 0) return specialJ_series(fsl * kom, qc, nfl);
+    const int idx = (int)(__float_as_uint(fslf * komf) >> 15) - ((127 + KSP_JFINE_E0) << 8);
+    if ((unsigned)idx >= KSP_JFINE_PIECES) return specialJ_fit_tab(fsl * kom);
+    const double2* p = reinterpret_cast<const double2*>(jt) + 4 * idx;
+    const double2 p0 = __ldg(p), p1 = __ldg(p + 1), p2 = __ldg(p + 2), p3 = __ldg(p + 3);
+    const double t = fma(fsl, kom, -p0.x);
+    return fma(t, fma(t, fma(t, fma(t, fma(t, p3.x, p2.y), p2.x), p1.y), p1.x), p0.y);
 }
 
 // specialJ (delta_tot_table.c:442-463) with the tabulated fit

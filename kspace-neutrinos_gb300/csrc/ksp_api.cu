@@ -134,7 +134,7 @@ static void free_table(kspace_ctx* c) {
     IntegratorDev& I = c->I;
     void* ptrs[] = {I.scalefact, I.dtot, I.coef, I.nu_init, I.nu_last, I.wavenum, I.dcdm, I.dnu_s, I.dnu,
                     I.knot_invdiag, I.knot_fac, I.knot_invh, I.knot_h3, I.knot_ih3, I.nc_g, I.nc_fsl,
-                    I.nc_dx, I.nc_j, I.nc_inv, I.nc_ab, I.nc_cd, I.nc_jf, I.fs_x, I.fs_y, I.fs_c, I.fs_seg, I.fs_suf, I.fs_tot, I.t_logk, I.t_T,
+                    I.nc_dx, I.nc_j, I.nc_inv, I.nc_ab, I.nc_cd, I.nc_jf, I.hyb, I.fs_x, I.fs_y, I.fs_c, I.fs_seg, I.fs_suf, I.fs_tot, I.t_logk, I.t_T,
                     I.t_c, I.sc,
                     I.qag_max, I.qag_total, I.coef_unit};
     for (void* p : ptrs)
@@ -717,6 +717,12 @@ extern "C" int kspace_gpu_save_nu_power(kspace_ctx* c, double Time, int snapnum,
 static void prepare_call(kspace_ctx* c, int Na, double a, double loga, int start_row, int write_knot, RowsMode rows,
                          int nk, int update_row, cudaStream_t st, bool scalars_only = false,
                          const FinalizeArgs* fin = nullptr) {
+    // hybrid neutrinos: room for J's tables, with the first call that can need them (without it
+    // the integrals evaluate the series)
+    if (c->hB.hyb_enabled && !c->I.hyb && dalloc(&c->I.hyb, (size_t)kNuSpecies * kHybTable) != cudaSuccess) {
+        cudaGetLastError();
+        c->I.hyb = nullptr;
+    }
     launch_integrator_prepare(c->I, c->hB, c->S0, Na, a, loga, c->loga0, c->TimeTransfer, start_row, write_knot,
                               scalars_only, rows, nk, update_row, fin, st);
 }

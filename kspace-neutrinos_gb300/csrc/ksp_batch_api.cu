@@ -218,6 +218,7 @@ static int lay_out(kspace_batch* b, const int* nk_in) {
         desc[i] = b->ctx[i]->I;
         desc[i].dcdm = b->dcdm_pool + b->off[i];  // the instance's delta_cdm lives in the pool
         desc[i].status = b->status_d + i;
+        desc[i].hyb = nullptr;  // (the tables of a single call)
         desc[i].ivals = nullptr;
         desc[i].nivals = nullptr;
         desc[i].nc_slots = b->nc_slots;

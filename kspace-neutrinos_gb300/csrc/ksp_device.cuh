@@ -307,11 +307,9 @@ KSP_HD double sinc_j0(double y) {
 // delta_tot_table.c:431-463 with qc > 0: sum over n = 1..19 of -(-1)^n e^{-n qc} /
 // (n^2 + x^2)^2 times
 //   (n^2 + n^3 qc + x^2 (n qc - 1)) qc sinc(qc x) + (2 n + n^2 qc + qc x^2) cos(qc x).
-// The sine and the cosine do not depend on n and are taken once; the weights e^{-n qc} are
-// powers; four terms share a division.  (Term by term, 19 exponentials, sines, cosines and
-// 38 divisions a node, a call with 151 bins took 3.1 ms in its integrals.)
-KSP_HD double specialJ_series(double x, double qc, double nufrac_low) {
-    const double x2 = x * x, e1 = exp(-qc), qx = qc * x;
+// The sine and the cosine do not depend on n: A and B are their factors' sums.  The weights
+// e^{-n qc} are powers of e1 = e^{-qc}; four terms share a division.
+KSP_HD void specialJ_sums(double x2, double qc, double e1, double* A_out, double* B_out) {
     double en = 1.0, A = 0.0, B = 0.0;
     for (int n0 = 1; n0 < 20; n0 += 4) {
         double d[4], w[4], a[4], c[4];
@@ -332,8 +330,13 @@ KSP_HD double specialJ_series(double x, double qc, double nufrac_low) {
         A += inv * (w0 * a[0] + w1 * a[1] + w2 * a[2] + w3 * a[3]);
         B += inv * (w0 * c[0] + w1 * c[1] + w2 * c[2] + w3 * c[3]);
     }
-    const double integ = A * qc * sinc_j0(qx) + B * cos(qx);
-    return integ / (1.5 * kZeta3 * (1 - nufrac_low));
+    *A_out = A;
+    *B_out = B;
+}
+KSP_HD double specialJ_series(double x, double qc, double nufrac_low) {
+    double A, B;
+    specialJ_sums(x * x, qc, exp(-qc), &A, &B);
+    return (A * qc * sinc_j0(qc * x) + B * cos(qc * x)) / (1.5 * kZeta3 * (1 - nufrac_low));
 }
 
 // delta_tot_table.c:442-463
@@ -1163,7 +1166,8 @@ struct DnuIntegrandW {
     const double* jt;          // J's fine table
     double kom;                // k / (m / kT)
     float komf;
-    double qc, nfl;            // qc > 0: the series instead of the fit
+    double qc, nfl;            // qc > 0: the series instead of the fit,
+    const double* hyb;         // from its table (or null)
     const double* ky;          // the bin's history row and its spline coefficients
     const double* kc;
     NodeTable nc;
@@ -1173,7 +1177,8 @@ struct DnuIntegrandW {
     int na;
     __device__ __forceinline__ double value(const NodeWeights& w, double fsl, float fslf, int j) const {
         const double v = fma(w.d, kc[j + 1], fma(w.c, kc[j], fma(w.b, ky[j + 1], __dmul_rn(w.a, ky[j]))));
-        return __dmul_rn(v, specialJ_node(jt, fsl, fslf, kom, komf, qc, nfl));
+        return __dmul_rn(v, qc > 0 ? specialJ_cut(hyb, fsl * kom, qc, nfl)
+                                   : specialJ_node(jt, fsl, fslf, kom, komf));
     }
     __device__ __forceinline__ double node_at(int slot, int jn, double c, double h, double xj) const {
         if (slot >= 0) {

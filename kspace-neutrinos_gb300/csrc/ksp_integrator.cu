@@ -265,13 +265,13 @@ struct PrepArgs {
     double loga, loga0;
     int Na, Nfs, nodes;            // Nfs, nodes: 0 without a table
     int start_row, write_knot;
-    int knot_blocks, fs_blocks, node_blocks;
+    int knot_blocks, fs_blocks, node_blocks, hyb_blocks;  // hyb_blocks: per species
 };
 
 // Block 0: the call's scalars to the device.  Then the knots' spacings and factorised spline system
 // x = scalefact[0..Na-1] (shared by every row; rows below `start_row` were factorised by an
-// earlier call with the same leading knots and are kept), the fslength segments, and the
-// part of the node table that needs no fslength.
+// earlier call with the same leading knots and are kept), the fslength segments, J's tables
+// where hybrid neutrinos cut it, and the part of the node table that needs no fslength.
 __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, PrepArgs P, GL4 gl) {
     __shared__ double f[kPrepThreads], sg[kPrepThreads];
     const int t = threadIdx.x, Na = P.Na;
@@ -306,6 +306,13 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, 
         return;
     }
     b -= P.fs_blocks;
+    if (b < kNuSpecies * P.hyb_blocks) {
+        const int mi = b / P.hyb_blocks;
+        if (P.S.qc[mi] > 0 && I.B->deg[mi] > 0)
+            hyb_table_block(I.hyb + (size_t)mi * kHybTable, b - mi * P.hyb_blocks, P.S.qc[mi], I.B->nufrac_low[0]);
+        return;
+    }
+    b -= kNuSpecies * P.hyb_blocks;
     const int q = b * kPrepThreads + t;
     if (q >= P.nodes) return;
     I.nc_inv[q] = node_inv_aH(I.B, nc_node_x(q, P.loga0, P.loga));
@@ -736,8 +743,9 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
         P.fs_blocks = fs_blocks(P.Nfs, loga0, loga);
         P.nodes = Na > 1 ? I.nc_slots * 61 : 0;
         P.node_blocks = (P.nodes + kPrepThreads - 1) / kPrepThreads;
+        if (I.hyb && P.S.partnu > 0 && !P.S.skip_integral) P.hyb_blocks = kHybPieces / 8;
     }
-    k_prep_eval<<<1 + P.knot_blocks + P.fs_blocks + P.node_blocks, kPrepThreads, 0, st>>>(I, P, gl);
+    k_prep_eval<<<1 + P.knot_blocks + P.fs_blocks + kNuSpecies * P.hyb_blocks + P.node_blocks, kPrepThreads, 0, st>>>(I, P, gl);
     const int nrow = rows == kRowsBase ? nk + 1 : (rows == kRowsFull && (Na > 2 || update_row >= 0) ? nk : 0);
     const int blocks = nrow + (P.Nfs + kTableThreads - 1) / kTableThreads +
                        (P.nodes + kTableThreads - 1) / kTableThreads;

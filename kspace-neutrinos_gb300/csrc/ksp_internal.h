@@ -55,6 +55,7 @@ struct IntegratorDev {
     double2* nc_cd;
     int2* nc_jf;
     const double* jt;                // J's fine table (one per device)
+    double* hyb;                     // optional: [kNuSpecies][kHybTable] the tables of J with a cut
     int nc_slots;                    // slots of the node table in use (1 + 2 levels, 0 = none)
     double* fs_x;                    // [fs_cap]
     double* fs_y;                    // [fs_cap]
@@ -257,6 +258,7 @@ __device__ __forceinline__ DnuIntegrandW dnu_integrand_w(const IntegratorDev& I,
     DnuIntegrandW f;
     f.B = I.B; f.jt = I.jt; f.kom = kom; f.komf = (float)kom;
     f.qc = S.qc[mi]; f.nfl = I.B->nufrac_low[0];
+    f.hyb = I.hyb ? I.hyb + (size_t)mi * kHybTable : nullptr;
     f.ky = row; f.kc = rc;
     f.nc = NodeTable{I.nc_ab, I.nc_cd, I.nc_fsl, I.nc_jf, I.nc_slots};
     f.fs_x = I.fs_x; f.fs_y = I.fs_y; f.fs_c = I.fs_c; f.kx = I.scalefact;

@@ -1279,6 +1279,7 @@ static int bin_grid(kspace_ctx* c, Geo* G, const float* gd, int pmgrid, int slab
     G->g.slab0 = slab0;
     G->g.nslab = nslab;
     G->g.nmodes = (long long)nslab * pmgrid * (pmgrid / 2 + 1);
+    G->g.beside = prep_time > 0 && !ch;
     CK(cudaMemsetAsync(c->bin_sum_d, 0, sizeof(double) * (nb + 1), c->stream));
     c->F0sq_d = c->bin_sum_d + nb;
     if (c->prof) cudaEventRecord(c->ev[0], c->stream);

@@ -430,7 +430,9 @@ struct GridGeom {
     int* cmap;                      // device [nrbins]: bin -> compact index (-1 empty)
     float bin_c1;                   // binsperunit * ln2 / 2 (approximate bin estimate)
     unsigned* runtab = nullptr;     // device run table of the binning pass (or null)
-    int run_Rp = 0;                 // its row length: runs of 17 modes per grid row, rounded up to 4
+    int run_Rp = 0;                 // its row length: runs per grid row, rounded up to 4
+    int run_K = 0;                  // modes per run
+    int beside = 0;                 // the integrator's preparation runs beside this binning pass
 };
 // the run table of a geometry (ksp_stream.cu): 0 built, 1 not applicable (2^15 bins or
 // more, or over 1 GiB), -1 error

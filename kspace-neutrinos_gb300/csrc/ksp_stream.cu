@@ -22,11 +22,12 @@
 // hand each closed run to the CTA's float-pair totals (compensated atomics) and the
 // CTA totals to the global FP64 sums once.
 //
-// The default binning kernel is k_bin_mirror (further down): 17-mode runs of a grid row
-// and of its mirror row (ky and -ky fall in the same bins), moved by 1-D bulk copies
-// with their run-table rows, the two modes of a pair summed exactly before they are
-// binned.  k_bin_rows, over tiles of whole grid rows and runs of one row, bins grids of
-// more than 32 runs per row (N > 1086) and works without a run table.
+// The default binning kernel is k_bin_mirror (further down): runs of up to 17 modes of a
+// grid row and of its mirror row (ky and -ky fall in the same bins), moved by 1-D bulk
+// copies with their run-table rows, the two modes of a pair summed exactly before they
+// are binned, and the sums of up to four row pairs of the same bins flushed together.
+// k_bin_rows, over tiles of whole grid rows and runs of one row, works without a run table
+// (the allocation-free entry point).
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -946,55 +947,128 @@ __global__ void __launch_bounds__(WARPS * 32)
 // ------------------------------------------------------------------ K1 over mirrored rows
 // The rows ky and -ky of a plane (grid rows j and N - j) hold, at every z, modes of the
 // same |k|, the same window factor and the same multiplicity: they fall in the same bins
-// at the same z.  So a lane takes one 17-mode run of both rows at once.  The two |F|^2
+// at the same z.  So a lane takes one run of K <= 17 modes of both rows at once.  The two |F|^2
 // (each rounded in float as the reference forms it) are added exactly (Fast2Sum of the
 // larger and the smaller), and the pair goes through the window product, the crossing and
 // the compensated run sum once: the sum of the two double products the reference adds,
-// to float-pair precision.  Crossings come from the run table, as in k_bin_rows; a run
-// and its closed bins now cover 34 modes.
-// A tile is P consecutive |ky| = q of one plane (P = 32 / runs per row): rows q0..q0+P-1
-// (one copy) and their mirrors N-q (one copy, q descending).  q = 0 and q = N/2 are
-// their own mirrors: their lanes pair the row with zeros (the stage's zeroed tail).  A
-// copy starts at the 16-byte boundary at or below its first row and ends at the one at
-// or above its last row end (a row is 8 (N/2+1) bytes, so odd rows start 8 bytes past a
-// boundary).  Each warp owns a ring of two stages.
-// zeroed bytes after a stage's rows: reads past the last row end, and the zero partner
-// (17 modes) of a row that is its own mirror
+// to float-pair precision.  Crossings come from the run table, as in k_bin_rows.
+//
+// The same holds for the planes kx and -kx, and for kx and ky exchanged: up to four row
+// pairs, (kx, +-ky), (-kx, +-ky), (ky, +-kx) and (-ky, +-kx), cross the same bins at the
+// same z.  They are a group: one warp takes its tiles one after the other, each adding
+// to the sums of its lanes' spill slots, and the group's closed bins go to the CTA's
+// totals once, after its last tile: the flush (dependent shared-memory atomics) had been
+// 0.2 ms of the 0.89 ms at N=1024 with one flush per row pair.
+// A lane takes its run into registers before it sums (two stretches of it in turn where the
+// integrator's preparation runs beside the pass): a store to a spill slot no longer holds up
+// the next modes' loads, and with the whole run in registers the stage is on its way again
+// during the sums.
+// Together, kernel alone: N=1024 889 -> 697 us (0.92 of the measured copy bandwidth, 534
+// million warp instructions, issue slots 63 % busy: 11 warps by shared memory, mostly
+// waiting for fixed latencies; in two stretches 735), N=512 137 -> 124 us.  Two steps' arithmetic packed
+// (f32x2) took fewer instructions and more time (N=1024 +80 us): the chain of the run sum
+// stays, and the packing's register pairs lengthen the rest.
+//
+// A tile is P consecutive |ky| = q of one plane (P = 32 / runs per row) and its rows'
+// mirrors: two copies where the rows are neighbours in memory (tiles 0 and 1), a copy per
+// row for the exchanged tiles (2 and 3), whose rows lie in P planes.  Rows of more than
+// 32 runs (N > 1086) are cut into parts, a part per warp (the row kernel's stages do not
+// fit shared memory there, and the plain kernel that was left took 45.5 ms at N=1280).
+// Rows q = 0 and q = N/2 are their own mirrors: their lanes pair the row with zeros (the
+// stage's zeroed tail).  A copy starts at the 16-byte boundary at or below its first mode
+// and ends at the one at or above its last (a row is 8 (N/2+1) bytes, so odd rows start
+// 8 bytes past a boundary).  Each warp owns a ring of two stages.
+// zeroed bytes after a stage's rows: the zero partner (up to 17 modes) of a row that is its own
+// mirror, and what a short last run reads past the last row
 constexpr int kMirrorTail = 144;
-constexpr int kMirrorMaxWarps = 12;
-// Spill slots per lane: a run closing more than kMirrorSlots - 1 bins (low k only) takes
-// the warp-cooperative path; the shared memory saved holds one more warp per SM.
-constexpr int kMirrorSlots = 9;
+// Warps of a CTA, by the registers of a run of K modes (WHOLE: the run's modes all in
+// registers at once).  Beside the integrator's preparation (!WHOLE) the pass leaves room for a
+// block of it on every SM: 12 warps of 128 registers, three per quarter of the register
+// file, and 4 KB of shared memory.  (With 160 registers the preparation waited for the pass
+// to end: N=512 564 us a step against 541, N=300 230 against 211.)
+constexpr int mirror_max_warps(int K, bool whole) { return whole && K <= 11 ? 14 : 12; }
+constexpr size_t kMirrorSmem = 224 * 1024;
+// Spill slots per lane: a run closing more than kMirrorSlots - 2 bins (low k only) takes
+// the warp-cooperative path; the shared memory saved holds one more warp per SM.  The
+// last slot is never a bin's: the step reads one slot ahead.
+constexpr int kMirrorSlots = 10;
 
 struct MirrorTiling {
-    int R;            // 17-mode runs per row
+    int K, R;         // modes per run, runs per row
+    int parts;        // parts of a row (1 up to 32 runs)
+    int Rt;           // runs of a part (a multiple of 4 where parts > 1: the table rows' alignment)
     int P;            // |ky| values (row pairs) per tile
     int Rp;           // run-table row length
     int tpp;          // tiles per plane: ceil((N/2 + 1) / P)
+    int full;         // groups of up to four tiles; else of planes kx and -kx only,
+    int pairs;        // or (0) every tile a group of its own
+    int ngroups;
     FastDiv fd_tpp;
+    // slab ranges: |kx| of the planes kx >= 0 [a0, a1) and kx < 0 [b0, b1); nA = a1 - a0 groups
+    // of planes start with the former, then nBl from b0, then the rest from br0
+    int a0, a1, b0, b1, nA, nBl, br0;
     int tab_bytes;    // run-table rows of a tile, rounded to 16
-    int blk;          // bytes of the region one copy lands in: P rows + 16, rounded to 16
+    int slot;         // bytes of one row's (or part's) region
+    int blk;          // bytes of P rows' regions
     int stage_bytes;  // table rows | rows q | mirror rows | tail
     int copies;       // copies of the CTA's bin totals: pair p adds to copy p % copies
 };
 
-inline MirrorTiling make_mirror_tiling(int nz) {
+inline MirrorTiling make_mirror_tiling(int K, int N, int nz, int slab0, int nslab) {
     MirrorTiling t{};
-    t.R = (nz + kRun - 1) / kRun;
-    t.P = t.R <= 32 ? 32 / t.R : 0;
-    if (t.P > nz) t.P = nz;
+    t.R = (nz + K - 1) / K;
     t.Rp = (t.R + 3) & ~3;
-    t.tpp = t.P > 0 ? (nz + t.P - 1) / t.P : 0;
-    t.fd_tpp = make_fastdiv((uint32_t)(t.tpp > 0 ? t.tpp : 1));
-    t.tab_bytes = (t.P * t.Rp * 4 + 15) & ~15;
-    t.blk = (t.P * nz * 8 + 16 + 15) & ~15;
+    t.K = K;
+    t.parts = (t.R + 31) / 32;
+    t.Rt = t.parts > 1 ? ((t.R + t.parts - 1) / t.parts + 3) & ~3 : t.R;
+    if (t.parts > 1) t.parts = (t.R + t.Rt - 1) / t.Rt;
+    t.P = 32 / t.Rt;
+    if (t.P > nz) t.P = nz;
+    if (t.parts > 1) t.P = 1;
+    t.tpp = (nz + t.P - 1) / t.P;
+    t.fd_tpp = make_fastdiv((uint32_t)t.tpp);
+    const int half = N / 2;
+    // A warp adds the tiles of a group one after the other, so groups need many times more
+    // tiles than the chip has warps: below eight tiles per warp every tile is a group of its
+    // own (N=192, at 2.3: 72 us against 84 in pairs, the call's 45 included), and kx and ky are
+    // exchanged from eight groups of four per warp on (N=340, at 4.4: 110 us with it, 97
+    // without).  Exchanged tiles also take a copy per row and are partly empty on the
+    // diagonal: with three or more rows per tile that is more than the flush it saves (N=300:
+    // 109 us with it, 96 without; N=1024, a row per tile: 756 us against 797).
+    constexpr long long kWarps = 152 * 11;
+    long long tri = 0;  // (|kx|, tile of |ky| <= |kx|): floor(kx / P) + 1 tiles
+    for (int ax = 0; ax <= half; ax++) tri += ax / t.P + 1;
+    t.full = slab0 == 0 && nslab == N && t.P <= 2 && tri >= 8 * kWarps;
+    t.pairs = (long long)nslab * t.tpp * t.parts >= 8 * kWarps;
+    if (t.full) {
+        t.ngroups = (int)tri;
+    } else {
+        const int s1 = slab0 + nslab;
+        t.a0 = slab0 < half + 1 ? slab0 : half + 1;
+        t.a1 = s1 < half + 1 ? s1 : half + 1;
+        const int lo = slab0 > half + 1 ? slab0 : half + 1;
+        t.b0 = s1 > lo ? N - s1 + 1 : 0;
+        t.b1 = s1 > lo ? N - lo + 1 : 0;
+        t.nA = t.a1 - t.a0;
+        // the kx < 0 planes whose +kx plane is not in the range
+        const bool both = t.pairs && t.nA > 0;
+        const int e = both ? (t.b1 < t.a0 ? t.b1 : t.a0) : t.b1;
+        t.nBl = e > t.b0 ? e - t.b0 : 0;
+        t.br0 = both ? (t.b0 > t.a1 ? t.b0 : t.a1) : t.b1;
+        const int nBr = t.b1 > t.br0 ? t.b1 - t.br0 : 0;
+        t.ngroups = (t.nA + t.nBl + nBr) * t.tpp;
+    }
+    const int seg = t.parts > 1 ? t.Rt * K : nz;
+    t.tab_bytes = t.parts > 1 ? t.Rt * 4 : (t.P * t.Rp * 4 + 15) & ~15;
+    t.slot = (seg * 8 + 16 + 15) & ~15;
+    t.blk = t.P * t.slot;
     t.stage_bytes = (t.tab_bytes + 2 * t.blk + kMirrorTail + 127) & ~127;
     t.copies = 1;
     return t;
 }
 
 // stage rings (two stages per warp) | mbarriers | per-warp spill slots | float-pair bin
-// totals (T.copies copies) | thresholds | {w1[z], multiplicity} for z < nz + 17 (zero past nz)
+// totals (T.copies copies) | thresholds | {w1[z], multiplicity} for z < nz + 17 Rt (zero past nz)
 __host__ __device__ inline StreamPlan plan_bin_mirror(int warps, int nrbins, int nz, bool exact,
                                                       const MirrorTiling& T) {
     StreamPlan p{};
@@ -1012,7 +1086,7 @@ __host__ __device__ inline StreamPlan plan_bin_mirror(int warps, int nrbins, int
     o += sizeof(int) * (size_t)(nrbins + 1);
     o = (o + 15) & ~size_t(15);
     p.tab_off = o;
-    o += sizeof(float2) * (size_t)(nz + kRun);
+    o += sizeof(float2) * (size_t)(nz + T.K);
     p.total = o + 128;  // alignment slack
     return p;
 }
@@ -1021,20 +1095,45 @@ __device__ __forceinline__ float spill_hi(float2 v) { return v.x; }
 __device__ __forceinline__ float spill_lo(float2 v) { return v.y; }
 __device__ __forceinline__ float spill_hi(float v) { return v; }
 __device__ __forceinline__ float spill_lo(float) { return 0.f; }
+__device__ __forceinline__ void spill_set(float2* p, float h, float l) { *p = make_float2(h, l); }
+__device__ __forceinline__ void spill_set(float* p, float h, float) { *p = h; }
 
-// One mode pair of a fast run (z of row q and of its mirror): close the current bin if
-// the run table marks a crossing, then add m (|F_a|^2 + |F_b|^2) inv^2 to the (new)
-// current bin.  m (0, 1 or 2) multiplies exactly inside the fused multiply-adds.
+// Where e has the bit: the sum (h, l) to the slot sp, the next slot's taken up, and the one after that read.  Predicated, not branched over: nearly every
+// step has a lane that crosses.
+__device__ __forceinline__ void mirror_cross(unsigned e, unsigned bit, uint32_t& sp, float2& next, float& h, float& l) {
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .u32 t;\n and.b32 t, %5, %6;\n setp.ne.u32 p, t, 0;\n"
+        " @p st.shared.v2.f32 [%0], {%1, %2};\n"
+        " @p mov.f32 %1, %3;\n @p mov.f32 %2, %4;\n"
+        " @p add.u32 %0, %0, 256;\n"
+        " @p ld.shared.v2.f32 {%3, %4}, [%0 + 256];\n}"
+        : "+r"(sp), "+f"(h), "+f"(l), "+f"(next.x), "+f"(next.y)
+        : "r"(e), "r"(bit)
+        : "memory");
+}
+__device__ __forceinline__ void mirror_cross(unsigned e, unsigned bit, uint32_t& sp, float& next, float& h, float&) {
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .u32 t;\n and.b32 t, %3, %4;\n setp.ne.u32 p, t, 0;\n"
+        " @p st.shared.f32 [%0], %1;\n @p mov.f32 %1, %2;\n"
+        " @p add.u32 %0, %0, 128;\n @p ld.shared.f32 %2, [%0 + 128];\n}"
+        : "+r"(sp), "+f"(h), "+f"(next)
+        : "r"(e), "r"(bit)
+        : "memory");
+}
+
+// One mode pair of a fast run (z of row q and of its mirror): at a crossing the current
+// bin's sum goes to its slot and the next slot's (of the group's earlier tiles) is taken
+// up, read one crossing ahead; then m (|F_a|^2 + |F_b|^2) inv^2 is added.  m (1 or 2)
+// multiplies exactly inside the fused multiply-adds.
 template <bool EXACT>
-__device__ __forceinline__ void mirror_step(float2 a, float2 b, float iwxy, float wz, float m, bool c,
-                                            typename SpillOf<EXACT>::type*& sp, float& h, float& l) {
+__device__ __forceinline__ void mirror_step(float2 a, float2 b, float iwxy, float wz, float m, unsigned e, unsigned bit,
+                                            uint32_t& sp, typename SpillOf<EXACT>::type& next, float& h, float& l) {
     const float Fa = __fadd_rn(__fmul_rn(a.x, a.x), __fmul_rn(a.y, a.y));
     const float Fb = __fadd_rn(__fmul_rn(b.x, b.x), __fmul_rn(b.y, b.y));
     const float t = __fmul_rn(iwxy, wz);
     const float inv = __fmul_rn(t, t);
     const float fh = __fmul_rn(inv, inv);
-    sp += c ? 32 : 0;
-    const float h0 = c ? 0.f : h;
+    if (bit > 1u) mirror_cross(e, bit, sp, next, h, l);
     if constexpr (EXACT) {
         const float mx = ptx::fmax_nan(Fa, Fb), mn = ptx::fmin_nan(Fa, Fb);
         const float sh = __fadd_rn(mx, mn);
@@ -1042,51 +1141,122 @@ __device__ __forceinline__ void mirror_step(float2 a, float2 b, float iwxy, floa
         const float fl = fmaf(inv, inv, -fh);
         const float hi = __fmul_rn(sh, fh);
         const float lo = fmaf(sh, fl, fmaf(sl, fh, fmaf(sh, fh, -hi)));
-        const float l0 = c ? 0.f : l;
-        const float s = fmaf(hi, m, h0);
-        const float bb = __fsub_rn(s, h0);
-        const float e = __fadd_rn(__fsub_rn(h0, __fsub_rn(s, bb)), fmaf(hi, m, -bb));
+        const float s = fmaf(hi, m, h);
+        const float bb = __fsub_rn(s, h);
+        const float e = __fadd_rn(__fsub_rn(h, __fsub_rn(s, bb)), fmaf(hi, m, -bb));
         h = s;
-        l = __fadd_rn(l0, fmaf(lo, m, e));
-        *sp = make_float2(h, l);
+        l = __fadd_rn(l, fmaf(lo, m, e));
     } else {
-        h = fmaf(__fmul_rn(__fadd_rn(Fa, Fb), fh), m, h0);
-        *sp = h;
+        h = fmaf(__fmul_rn(__fadd_rn(Fa, Fb), fh), m, h);
     }
 }
 
-// Tile t into a stage: its run-table rows, rows q0.. and their mirrors, on one mbarrier.
+// A warp's walk over its groups and their tiles (warp-uniform).
+struct MirrorWalk {
+    int gi;         // group
+    int ax, q0;     // |kx|, first |ky| of the group's tiles
+    int nA;         // |ky| values in the tiles
+    unsigned left;  // tiles still to come (bits 0..3)
+    bool first;     // the group's first tile: the one that brings the run-table rows
+    __device__ __forceinline__ int sub() const { return __ffs(left) - 1; }
+    __device__ __forceinline__ void open(const GridArgs& g, const MirrorTiling& T) {
+        if (gi >= T.ngroups) return;
+        first = true;
+        if (T.full) {
+            // group = (ax, j), ax / P = m: P m (m+1) / 2 groups lie before the block of P
+            // values ax with m + 1 tiles each
+            int m = (int)(0.5f * (sqrtf(8.f * (float)gi / (float)T.P + 1.f) - 1.f));
+            while (m > 0 && T.P * (m * (m + 1) / 2) > gi) m--;
+            while (T.P * ((m + 1) * (m + 2) / 2) <= gi) m++;
+            const int rem = gi - T.P * (m * (m + 1) / 2);
+            const int i = rem / (m + 1);
+            ax = m * T.P + i;
+            q0 = (rem - i * (m + 1)) * T.P;
+            nA = min(T.P, ax - q0 + 1);
+            const int qhi = min(q0 + nA - 1, ax - 1);  // the exchanged tiles hold |ky| < |kx|
+            left = 1u | (ax > 0 && ax < g.half ? 2u : 0u) | (q0 < ax ? 4u : 0u) | (max(q0, 1) <= qhi ? 8u : 0u);
+        } else {
+            const int u = (int)fdiv((uint32_t)gi, T.fd_tpp);
+            q0 = (gi - u * T.tpp) * T.P;
+            nA = min(T.P, g.nz - q0);
+            if (u < T.nA) {
+                ax = T.a0 + u;
+                left = 1u | (T.pairs && ax >= T.b0 && ax < T.b1 ? 2u : 0u);
+            } else {
+                const int v = u - T.nA;
+                ax = v < T.nBl ? T.b0 + v : T.br0 + (v - T.nBl);
+                left = 2u;
+            }
+        }
+    }
+    __device__ __forceinline__ void next(const GridArgs& g, const MirrorTiling& T, int step) {
+        left &= left - 1;
+        first = false;
+        if (!left) {
+            gi += step;
+            open(g, T);
+        }
+    }
+};
+
+// The walk's tile into a stage, on one mbarrier: the group's run-table rows with its
+// first tile, the rows and their mirrors.  Called by a whole warp.
 __device__ __forceinline__ void issue_mirror_tile(const GridArgs& g, const MirrorTiling& T, const unsigned* runtab,
                                                   const unsigned char* gsrc, unsigned char* dst, uint64_t* bar,
-                                                  long long t) {
-    const int plane = (int)fdiv((uint32_t)t, T.fd_tpp);
-    const int q0 = ((int)t - plane * T.tpp) * T.P;
-    const int nA = min(T.P, g.nz - q0);
-    const int qlo = max(q0, 1), qhi = min(q0 + nA - 1, g.half - 1);
+                                                  const MirrorWalk& w, int part) {
+    const int lane = threadIdx.x & 31;
     const size_t rb = (size_t)g.nz * 8;
-    const size_t a0 = ((size_t)plane * g.N + q0) * rb;
-    const size_t as = a0 & ~size_t(15), ae = (a0 + (size_t)nA * rb + 15) & ~size_t(15);
-    size_t bs = 0, be = 0;
-    if (qhi >= qlo) {
-        const size_t b0 = ((size_t)plane * g.N + g.N - qhi) * rb;
-        bs = b0 & ~size_t(15);
-        be = (b0 + (size_t)(qhi - qlo + 1) * rb + 15) & ~size_t(15);
+    const int z0 = part * T.Rt * T.K;
+    const int zn = T.parts > 1 ? min(g.nz - z0, T.Rt * T.K) : g.nz;
+    const int sub = w.sub();
+    const unsigned tb = w.first ? (unsigned)(T.parts > 1 ? min(T.Rp - part * T.Rt, T.Rt) * 4 : w.nA * T.Rp * 4) : 0u;
+    if (sub < 2) {
+        if (lane == 0) {
+            const int plane = (sub == 0 ? w.ax : g.N - w.ax) - g.slab0;
+            const int qlo = max(w.q0, 1), qhi = min(w.q0 + w.nA - 1, g.half - 1);
+            const size_t a0 = ((size_t)plane * g.N + w.q0) * rb + (size_t)z0 * 8;
+            const size_t la = (size_t)(w.nA - 1) * rb + (size_t)zn * 8;
+            const size_t as = a0 & ~size_t(15), ae = (a0 + la + 15) & ~size_t(15);
+            size_t bs = 0, be = 0;
+            if (qhi >= qlo) {
+                const size_t b0 = ((size_t)plane * g.N + g.N - qhi) * rb + (size_t)z0 * 8;
+                bs = b0 & ~size_t(15);
+                be = (b0 + (size_t)(qhi - qlo) * rb + (size_t)zn * 8 + 15) & ~size_t(15);
+            }
+            ptx::fence_async_smem();
+            ptx::mbar_expect_tx(bar, (unsigned)(ae - as + be - bs) + tb);
+            // grid rows are read once: their lines leave L2 first (the run table's stay)
+            const uint64_t pol = ptx::policy_evict_first();
+            ptx::bulk_g2s_hint(dst + T.tab_bytes, gsrc + as, (unsigned)(ae - as), bar, pol);
+            if (be > bs) ptx::bulk_g2s_hint(dst + T.tab_bytes + T.blk, gsrc + bs, (unsigned)(be - bs), bar, pol);
+        }
+    } else {
+        // lane p: row |kx| of plane +-(q0 + p), and its mirror
+        const int q = w.q0 + lane;
+        const bool live = lane < w.nA && q < w.ax && (sub == 2 || q > 0);
+        const bool pair = live && w.ax > 0 && w.ax < g.half;
+        const int plane = sub == 2 ? q : g.N - q;
+        const size_t a0 = live ? ((size_t)plane * g.N + w.ax) * rb + (size_t)z0 * 8 : 0;
+        const size_t b0 = pair ? ((size_t)plane * g.N + g.N - w.ax) * rb + (size_t)z0 * 8 : 0;
+        const size_t as = a0 & ~size_t(15), bs = b0 & ~size_t(15);
+        const unsigned na = live ? (unsigned)(((a0 + (size_t)zn * 8 + 15) & ~size_t(15)) - as) : 0u;
+        const unsigned nb = pair ? (unsigned)(((b0 + (size_t)zn * 8 + 15) & ~size_t(15)) - bs) : 0u;
+        const unsigned total = __reduce_add_sync(kFull, na + nb);
+        ptx::fence_async_smem();
+        if (lane == 0) ptx::mbar_expect_tx(bar, total + tb);
+        __syncwarp();
+        const uint64_t pol = ptx::policy_evict_first();
+        if (live) ptx::bulk_g2s_hint(dst + T.tab_bytes + lane * T.slot, gsrc + as, na, bar, pol);
+        if (pair) ptx::bulk_g2s_hint(dst + T.tab_bytes + T.blk + lane * T.slot, gsrc + bs, nb, bar, pol);
     }
-    const int kx = kval(g.slab0 + plane, g.N), ax = kx < 0 ? -kx : kx;
-    const unsigned tb = (unsigned)(nA * T.Rp * 4);
-    ptx::fence_async_smem();
-    ptx::mbar_expect_tx(bar, (unsigned)(ae - as + be - bs) + tb);
-    ptx::bulk_g2s(dst, runtab + ((size_t)ax * (g.half + 1) + q0) * T.Rp, tb, bar);
-    // grid rows are read once: their lines leave L2 first (the run table's stay)
-    const uint64_t pol = ptx::policy_evict_first();
-    ptx::bulk_g2s_hint(dst + T.tab_bytes, gsrc + as, (unsigned)(ae - as), bar, pol);
-    if (be > bs) ptx::bulk_g2s_hint(dst + T.tab_bytes + T.blk, gsrc + bs, (unsigned)(be - bs), bar, pol);
+    if (tb && lane == 0)
+        ptx::bulk_g2s(dst, runtab + ((size_t)w.ax * (g.half + 1) + w.q0) * T.Rp + part * T.Rt, tb, bar);
 }
 
-template <bool EXACT>
-__global__ void __launch_bounds__(kMirrorMaxWarps * 32)
+template <int K, bool EXACT, bool WHOLE>
+__global__ void __launch_bounds__(WHOLE ? mirror_max_warps(K, true) * 32 : 512)
     k_bin_mirror(GridArgs g, MirrorTiling T, const int* __restrict__ thresh, const float* __restrict__ w1g,
-                 const float* __restrict__ grid, double* bin_sum, double* F0sq, unsigned* status, long long ntiles,
+                 const float* __restrict__ grid, double* bin_sum, double* F0sq, unsigned* status,
                  const unsigned* __restrict__ runtab) {
     typedef typename SpillOf<EXACT>::type Spill;
     extern __shared__ unsigned char sm_raw[];
@@ -1103,13 +1273,13 @@ __global__ void __launch_bounds__(kMirrorMaxWarps * 32)
     const int hstride = totals_stride(g.nrbins);
     for (int i = tid; i < hstride * T.copies; i += blockDim.x) s_H0[i] = 0.f;
     for (int i = tid; i < g.nrbins; i += blockDim.x) s_thr[i] = thresh[i];
-    for (int i = tid; i < g.nz + kRun; i += blockDim.x)
+    for (int i = tid; i < g.nz + K; i += blockDim.x)
         s_wt[i] = i < g.nz ? make_float2(w1g[i], (i == 0 || i == g.half) ? 1.f : 2.f) : make_float2(0.f, 0.f);
-    // the stages start zeroed: bytes a lane reads past a row end that no copy wrote are 0
-    {
-        uint4* st4 = reinterpret_cast<uint4*>(base + Pl.stage_off);
-        for (int i = tid; i < W * 2 * T.stage_bytes / 16; i += blockDim.x) st4[i] = make_uint4(0, 0, 0, 0);
-        ptx::fence_async_smem();
+    // the tails of the stages are zero and stay so (no copy reaches them)
+    for (int i = tid; i < W * 2 * (kMirrorTail / 16); i += blockDim.x) {
+        unsigned char* tail = base + Pl.stage_off + (size_t)(i / (kMirrorTail / 16)) * T.stage_bytes + T.tab_bytes +
+                              2 * T.blk;
+        reinterpret_cast<uint4*>(tail)[i % (kMirrorTail / 16)] = make_uint4(0, 0, 0, 0);
     }
     if (tid == 0) s_thr[g.nrbins] = 0x7fffffff;
     if (lane == 0) {
@@ -1119,93 +1289,134 @@ __global__ void __launch_bounds__(kMirrorMaxWarps * 32)
     }
     __syncthreads();
 
+    // a warp keeps to one part of the rows, so a lane's run is at the same z in every tile
+    const int TW = (int)(gridDim.x * W) / T.parts;  // walks per part
+    const int gw = (int)(blockIdx.x * W) + warp;
+    const int part = gw % T.parts;
     // this lane's pair and run within every tile; its window factors and multiplicities
-    const int p = lane / T.R, r = lane - p * T.R;
-    const bool lane_ok = p < T.P;
-    const int z0 = r * kRun;
-    float wz[kRun], mz[kRun];
+    const int p = lane / T.Rt, r = lane - p * T.Rt;
+    const bool lane_ok = p < T.P && part * T.Rt + r < T.R;
+    const int zl = r * K, z0 = part * T.Rt * K + zl;
+    float wz[K], mz[K];
 #pragma unroll
-    for (int i = 0; i < kRun; i++) {
-        const float2 w = s_wt[z0 + i];
+    for (int i = 0; i < K; i++) {
+        const float2 w = lane_ok ? s_wt[z0 + i] : make_float2(0.f, 0.f);
         wz[i] = w.x;
         mz[i] = w.y;
     }
+    // A short last run: its first mode past the row end opens a slot that is never flushed,
+    // which keeps what lies there out of the sums.
+    const int nv = g.nz - z0;
+    const unsigned stop = lane_ok && nv < K ? 1u << nv : 0u;
     float* s_H = s_H0 + (size_t)(p % T.copies) * hstride;
     float* s_L = s_H + g.nrbins;
     const size_t rb = (size_t)g.nz * 8;
-
-    const long long gw = (long long)blockIdx.x * W + warp, TW = (long long)gridDim.x * W;
-    const long long my_n = gw < ntiles ? (ntiles - 1 - gw) / TW + 1 : 0;
     const unsigned char* gsrc = reinterpret_cast<const unsigned char*>(grid);
-    if (lane == 0)
-        for (int s = 0; s < 2 && s < my_n; s++)
-            issue_mirror_tile(g, T, runtab, gsrc, wst + s * T.stage_bytes, &wbar[s], gw + s * TW);
+
+    MirrorWalk cur;
+    cur.gi = gw / T.parts < TW ? gw / T.parts : T.ngroups;
+    cur.open(g, T);
+    MirrorWalk ahead = cur;
+    int flying = 0;
+    for (; flying < 2 && ahead.gi < T.ngroups; flying++) {
+        issue_mirror_tile(g, T, runtab, gsrc, wst + flying * T.stage_bytes, &wbar[flying], ahead, part);
+        ahead.next(g, T, TW);
+    }
     bool ok = true;
-    long long k = 0;
     int s = 0;
-    unsigned phase = 0;
-    for (; k < my_n; k++) {
-        const bool got = ptx::mbar_wait_bounded_n(&wbar[s], phase, k == 0 ? g.first_wait : (1 << 22));
+    unsigned phase = 0, e = 1u;
+    int b = 0, nsp = 0;  // the lane's first bin, and how many more its run closes
+    bool have = false, fast = false;
+    int limit = g.first_wait;
+    while (cur.gi < T.ngroups) {
+        const bool got = ptx::mbar_wait_bounded_n(&wbar[s], phase, limit);
+        limit = 1 << 22;
         if (!__all_sync(kFull, got)) {
             ok = false;
             break;
         }
         const unsigned char* st = wst + s * T.stage_bytes;
-        const uint32_t t = (uint32_t)(gw + k * TW);
-        const int plane = (int)fdiv(t, T.fd_tpp);
-        const int q0 = ((int)t - plane * T.tpp) * T.P;
-        const int nA = min(T.P, g.nz - q0);
-        const bool valid = lane_ok && p < nA;
-        const int q = valid ? q0 + p : 0;
-        const int kx = kval(g.slab0 + plane, g.N), ax = kx < 0 ? -kx : kx;
-        const float iwxy = __fmul_rn(s_wt[ax].x, s_wt[q].x);
-        const bool single = q == 0 || q == g.half;
-        const int qhi = min(q0 + nA - 1, g.half - 1);
-        const size_t a0 = ((size_t)plane * g.N + q0) * rb, b0 = ((size_t)plane * g.N + g.N - qhi) * rb;
-        const unsigned offA = (unsigned)T.tab_bytes + (unsigned)(a0 & 15) + (unsigned)(p * g.nz + z0) * 8u;
-        // a row that is its own mirror pairs with the stage's zeroed tail
-        const unsigned offB = !valid ? offA
-                              : single ? (unsigned)(T.tab_bytes + 2 * T.blk)
-                                       : (unsigned)(T.tab_bytes + T.blk) + (unsigned)(b0 & 15) +
-                                             (unsigned)((qhi - q) * g.nz + z0) * 8u;
-        unsigned e = 1u;
-        if (valid) e = reinterpret_cast<const unsigned*>(st)[p * T.Rp + r];
-        const bool fast = valid && (e & 1u) == 0 && __popc(e & 0x1fffeu) < kMirrorSlots;
-        const int b = (int)(e >> 17);
-        const int nsp = fast ? __popc(e & 0x1fffeu) : 0;  // the run's closed bins
-        if (fast) {
-            Spill* sp = my_spill;
-            float h = 0.f, l = 0.f;
-            const float2* va = reinterpret_cast<const float2*>(st + offA);
-            const float2* vb = reinterpret_cast<const float2*>(st + offB);
+        const int ax = cur.ax, sub = cur.sub();
+        const int q = lane_ok && p < cur.nA ? cur.q0 + p : 0;
+        if (cur.first) {
+            have = lane_ok && p < cur.nA;
+            e = have ? reinterpret_cast<const unsigned*>(st)[p * T.Rp + r] : 1u;
+            nsp = __popc(e & 0x1fffeu);
+            b = (int)(e >> 17);
+            e |= stop;
+            fast = have && (e & 1u) == 0 && __popc(e & 0x1fffeu) <= kMirrorSlots - 2;
+            if (!fast) nsp = 0;
+            // the group's sums start at zero (a loop of its own for the first tile, without
+            // these stores and the reads ahead, made the code larger and the pass 6 % slower)
+            Spill zero;
+            spill_set(&zero, 0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < kRun; i++)
-                mirror_step<EXACT>(va[i], vb[i], iwxy, wz[i], mz[i], i > 0 && ((e >> i) & 1u), sp, h, l);
+            for (int i = 0; i < kMirrorSlots; i++) my_spill[32 * i] = zero;
         }
-        // The next lane's run continues this one: where it starts in the bin this run ends
-        // in and has a later bin of its own, its first sum joins this run's last one here.
-        float fx = 0.f, fy = 0.f;
-        if (fast) {
-            const Spill f0 = my_spill[0];
-            fx = spill_hi(f0);
-            fy = spill_lo(f0);
+        const float iwxy = __fmul_rn(s_wt[ax].x, s_wt[q].x);
+        bool live, single;
+        unsigned offA, offB;
+        if (sub < 2) {
+            const int plane = (sub == 0 ? ax : g.N - ax) - g.slab0;
+            const int qhi = min(cur.q0 + cur.nA - 1, g.half - 1);
+            const size_t zb = (size_t)part * T.Rt * K * 8;
+            const size_t a0 = ((size_t)plane * g.N + cur.q0) * rb + zb, b0 = ((size_t)plane * g.N + g.N - qhi) * rb + zb;
+            live = have;
+            single = q == 0 || q == g.half;
+            offA = (unsigned)(a0 & 15) + (unsigned)(p * g.nz + zl) * 8u;
+            offB = (unsigned)(b0 & 15) + (unsigned)((qhi - q) * g.nz + zl) * 8u;
+        } else {
+            const int plane = sub == 2 ? q : g.N - q;
+            const size_t zb = (size_t)part * T.Rt * K * 8;
+            const size_t a0 = ((size_t)plane * g.N + ax) * rb + zb, b0 = ((size_t)plane * g.N + g.N - ax) * rb + zb;
+            live = have && q < ax && (sub == 2 || q > 0);
+            single = ax == 0 || ax == g.half;
+            offA = (unsigned)(a0 & 15) + (unsigned)(p * T.slot + zl * 8);
+            offB = (unsigned)(b0 & 15) + (unsigned)(p * T.slot + zl * 8);
         }
-        const int info = fast ? (p << 8) | (nsp + 1) : 0;  // pair, items; 0: no run
-        const int nb_info = __shfl_down_sync(kFull, info, 1);
-        const int nb_b = __shfl_down_sync(kFull, b, 1);
-        const float nfx = __shfl_down_sync(kFull, fx, 1), nfy = __shfl_down_sync(kFull, fy, 1);
-        const bool take = fast && lane < 31 && (nb_info >> 8) == p && (nb_info & 255) >= 2 && nb_b == b + nsp;
-        const bool given = __shfl_up_sync(kFull, take ? 1 : 0, 1) != 0 && lane > 0;
-        if (take) {
-            const Spill v = my_spill[32 * nsp];
-            float vh = spill_hi(v), vl = spill_lo(v);
-            pair_add(vh, vl, nfx, nfy);
-            if constexpr (EXACT) my_spill[32 * nsp] = make_float2(vh, vl);
-            else my_spill[32 * nsp] = vh;
+        offA += (unsigned)T.tab_bytes;
+        // a row that is its own mirror pairs with the stage's zeroed tail
+        offB = !live ? offA : single ? (unsigned)(T.tab_bytes + 2 * T.blk) : offB + (unsigned)(T.tab_bytes + T.blk);
+        // !WHOLE: the run in two stretches, summed here; WHOLE: all of it into registers, summed
+        // below, after the stage is given its next tile
+        constexpr int C = WHOLE ? K : (K + 1) / 2;
+        float2 va[C], vb[C];
+        const float2* pa = reinterpret_cast<const float2*>(st + offA);
+        const float2* pb = reinterpret_cast<const float2*>(st + offB);
+        uint32_t sp = ptx::smem_u32(my_spill);
+        Spill next;
+        float h = 0.f, l = 0.f;
+        auto load = [&](int i0) {
+#pragma unroll
+            for (int i = 0; i < C; i++)
+                if (i0 + i < K) {
+                    va[i] = pa[i0 + i];
+                    vb[i] = pb[i0 + i];
+                }
+        };
+        auto sum = [&](int i0) {
+            if (i0 == 0) {
+                next = my_spill[32];
+                h = spill_hi(my_spill[0]);
+                l = spill_lo(my_spill[0]);
+            }
+#pragma unroll
+            for (int i = 0; i < C; i++)
+                if (i0 + i < K)
+                    mirror_step<EXACT>(va[i], vb[i], iwxy, wz[i0 + i], mz[i0 + i], e, 1u << (i0 + i), sp, next, h, l);
+            if (i0 + C >= K) spill_set(&my_spill[(sp - ptx::smem_u32(my_spill)) / (unsigned)sizeof(Spill)], h, l);
+        };
+        if (fast && live) {
+            load(0);
+            if constexpr (!WHOLE) {
+                sum(0);
+                load(C);
+                sum(C);
+            }
         }
         // slow runs (the k = 0 mode; a bin skipped between two modes; more closed bins than
         // spill slots): one run at a time, a mode of both rows per lane
-        unsigned slow = __ballot_sync(kFull, valid && !fast);
+        unsigned slow = __ballot_sync(kFull, live && !fast);
         while (slow) {
             const int L = __ffs(slow) - 1;
             slow &= slow - 1;
@@ -1218,7 +1429,7 @@ __global__ void __launch_bounds__(kMirrorMaxWarps * 32)
             float phi = 0.f, plo = 0.f;
             const int zz = zL + lane;
             const int k2m = kxyL + zz * zz;
-            if (lane < kRun && zz < g.nz && k2m != 0) {
+            if (lane < K && zz < g.nz && k2m != 0) {
                 const float2 va = *reinterpret_cast<const float2*>(st + oaL + 8 * lane);
                 mode_value<EXACT>(va.x, va.y, iwL, s_wt[zz], phi, plo);
                 if (!sgL) {
@@ -1234,16 +1445,45 @@ __global__ void __launch_bounds__(kMirrorMaxWarps * 32)
             if (tail && key >= 0) add_pair(s_H, s_L, key, phi, plo);
         }
         __syncwarp();
-        if (lane == 0 && k + 2 < my_n)
-            issue_mirror_tile(g, T, runtab, gsrc, wst + s * T.stage_bytes, &wbar[s], gw + (k + 2) * TW);
-        // the closed bins of the fast runs go to the totals from the spill slots, after the
-        // stage is on its way again
-        if (fast) {
-            for (int qq = given ? 1 : 0; qq <= nsp; qq++) {
-                const Spill v = my_spill[32 * qq];
-                add_pair(s_H, s_L, b + qq, spill_hi(v), spill_lo(v));
+        flying--;
+        if (ahead.gi < T.ngroups) {
+            issue_mirror_tile(g, T, runtab, gsrc, wst + s * T.stage_bytes, &wbar[s], ahead, part);
+            ahead.next(g, T, TW);
+            flying++;
+        }
+        if constexpr (WHOLE)
+            if (fast && live) sum(0);
+        const bool last = (cur.left & (cur.left - 1)) == 0;
+        if (last) {
+            // The next lane's run continues this one: where it starts in the bin this run ends
+            // in and has a later bin of its own, its first sum joins this run's last one here.
+            float fx = 0.f, fy = 0.f;
+            if (fast) {
+                const Spill f0 = my_spill[0];
+                fx = spill_hi(f0);
+                fy = spill_lo(f0);
+            }
+            const int info = fast ? (p << 8) | (nsp + 1) : 0;  // pair, items; 0: no run
+            const int nb_info = __shfl_down_sync(kFull, info, 1);
+            const int nb_b = __shfl_down_sync(kFull, b, 1);
+            const float nfx = __shfl_down_sync(kFull, fx, 1), nfy = __shfl_down_sync(kFull, fy, 1);
+            const bool take = fast && lane < 31 && (nb_info >> 8) == p && (nb_info & 255) >= 2 && nb_b == b + nsp;
+            const bool given = __shfl_up_sync(kFull, take ? 1 : 0, 1) != 0 && lane > 0;
+            if (take) {
+                const Spill v = my_spill[32 * nsp];
+                float vh = spill_hi(v), vl = spill_lo(v);
+                pair_add(vh, vl, nfx, nfy);
+                spill_set(&my_spill[32 * nsp], vh, vl);
+            }
+            // the closed bins of the fast runs go to the totals from the spill slots
+            if (fast) {
+                for (int qq = given ? 1 : 0; qq <= nsp; qq++) {
+                    const Spill v = my_spill[32 * qq];
+                    add_pair(s_H, s_L, b + qq, spill_hi(v), spill_lo(v));
+                }
             }
         }
+        cur.next(g, T, TW);
         if (++s == 2) {
             s = 0;
             phase ^= 1;
@@ -1251,7 +1491,7 @@ __global__ void __launch_bounds__(kMirrorMaxWarps * 32)
     }
     if (!ok && lane == 0) {
         atomicOr(status, kStTimeout);
-        for (long long kk = k; kk < my_n && kk < k + 2; kk++) {
+        for (; flying > 0; flying--) {  // the copies still in flight
             ptx::mbar_wait_bounded(&wbar[s], phase);
             if (++s == 2) {
                 s = 0;
@@ -1429,15 +1669,15 @@ int run_bin_rows(const GridGeom& g, const GridArgs& a, const float* grid, double
 template <int WARPS, int STAGES, bool EXACT>
 int run_bin_rows_any(const GridGeom& g, const GridArgs& a, const float* grid, double* bin_sum, double* F0sq,
                      unsigned* status, cudaStream_t st) {
-    if (EXACT && g.runtab && g.run_Rp == ((a.nz + kRun - 1) / kRun + 3) / 4 * 4)
+    if (EXACT && g.runtab && g.run_K == kRun && g.run_Rp == ((a.nz + kRun - 1) / kRun + 3) / 4 * 4)
         return run_bin_rows<WARPS, STAGES, EXACT, EXACT>(g, a, grid, bin_sum, F0sq, status, st);
     return run_bin_rows<WARPS, STAGES, EXACT, false>(g, a, grid, bin_sum, F0sq, status, st);
 }
 
-// The mirrored-row pass needs the geometry's run table and rows of at most 32 runs
-// (N <= 1086).  Warps per CTA: the most resident warps per SM, then the largest CTA
+// The mirrored-row pass needs the geometry's run table (up to 1 GiB of it: N <= 3200).
+// Warps per CTA: the most resident warps per SM, then the largest CTA
 // (KSPACE_GPU_MIRROR_WARPS fixes it).
-template <bool EXACT>
+template <int K, bool EXACT, bool WHOLE>
 int run_bin_mirror(const GridGeom& g, const GridArgs& a, const float* grid, double* bin_sum, double* F0sq,
                    unsigned* status, cudaStream_t st) {
     static const int force_w = [] {
@@ -1447,16 +1687,15 @@ int run_bin_mirror(const GridGeom& g, const GridArgs& a, const float* grid, doub
     if ((reinterpret_cast<uintptr_t>(grid) & 15) != 0) return -1;
     // rows q = 0 and N/2 are their own mirrors only for even N (the geometry requires it)
     if (a.N & 1) return -1;
-    MirrorTiling T = make_mirror_tiling(a.nz);
-    if (T.P < 1 || !g.runtab || g.run_Rp != T.Rp || g.nslab <= 0) return -1;
-    const long long ntiles = (long long)g.nslab * T.tpp;
-    if (ntiles >= (1LL << 31)) return -1;
-    auto kern = k_bin_mirror<EXACT>;
+    if (!g.runtab || g.nslab <= 0 || g.slab0 < 0 || g.slab0 + g.nslab > a.N) return -1;
+    MirrorTiling T = make_mirror_tiling(K, a.N, a.nz, g.slab0, g.nslab);
+    if (g.run_Rp != T.Rp) return -1;
+    auto kern = k_bin_mirror<K, EXACT, WHOLE>;
     int best_w = 0, best_occ = 0;
-    for (int w = kMirrorMaxWarps; w >= 2; w--) {
+    for (int w = mirror_max_warps(K, WHOLE); w >= 2; w--) {
         if (force_w > 0 && w != force_w) continue;
         const StreamPlan p = plan_bin_mirror(w, g.nrbins, a.nz, EXACT, T);
-        if (p.total > (size_t)kMaxSmemPass) continue;
+        if (p.total > kMirrorSmem) continue;
         const int occ = resident_blocks(kern, w * 32, p.total);
         if (occ * w > best_occ * best_w) {
             best_w = w;
@@ -1469,17 +1708,31 @@ int run_bin_mirror(const GridGeom& g, const GridArgs& a, const float* grid, doub
         MirrorTiling t2 = T;
         t2.copies = c;
         const StreamPlan p = plan_bin_mirror(best_w, g.nrbins, a.nz, EXACT, t2);
-        if (p.total <= (size_t)kMaxSmemPass && resident_blocks(kern, best_w * 32, p.total) == best_occ) {
+        if (p.total <= kMirrorSmem && resident_blocks(kern, best_w * 32, p.total) == best_occ) {
             T = t2;
             break;
         }
     }
     const StreamPlan P = plan_bin_mirror(best_w, g.nrbins, a.nz, EXACT, T);
     long long n = (long long)sm_count_s() * best_occ;
-    const long long need = (ntiles + best_w - 1) / best_w;
+    const long long need = ((long long)T.ngroups * T.parts + best_w - 1) / best_w;
     if (n > need) n = need > 0 ? need : 1;
-    kern<<<(int)n, best_w * 32, P.total, st>>>(a, T, g.thresh, g.w1, grid, bin_sum, F0sq, status, ntiles, g.runtab);
+    if (n * best_w < T.parts) n = (T.parts + best_w - 1) / best_w;  // a walk for every part
+    kern<<<(int)n, best_w * 32, P.total, st>>>(a, T, g.thresh, g.w1, grid, bin_sum, F0sq, status, g.runtab);
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -2;
+}
+
+template <bool EXACT, bool WHOLE>
+int run_bin_mirror_any(const GridGeom& g, const GridArgs& a, const float* grid, double* bin_sum, double* F0sq,
+                       unsigned* status, cudaStream_t st) {
+    switch (g.run_K) {
+    case 9: return run_bin_mirror<9, EXACT, WHOLE>(g, a, grid, bin_sum, F0sq, status, st);
+    case 11: return run_bin_mirror<11, EXACT, WHOLE>(g, a, grid, bin_sum, F0sq, status, st);
+    case 13: return run_bin_mirror<13, EXACT, WHOLE>(g, a, grid, bin_sum, F0sq, status, st);
+    case 15: return run_bin_mirror<15, EXACT, WHOLE>(g, a, grid, bin_sum, F0sq, status, st);
+    case 17: return run_bin_mirror<17, EXACT, WHOLE>(g, a, grid, bin_sum, F0sq, status, st);
+    default: return -1;
+    }
 }
 
 template <int WARPS, int STAGES>
@@ -1496,13 +1749,45 @@ int run_corr_stream(const GridArgs& a, float* grid, CorrTable corr, unsigned* st
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -2;
 }
 
-// Run table of a geometry: for |kx|, |ky| in [0, N/2] and run r (modes z = 17r .. 17r+16
-// of a grid row), entry = b_start << 17 | bit i (i = 1..16) set where mode i opens the next
+// KSPACE_GPU_MIRROR=0: the row pass only (read once)
+bool use_mirror() {
+    static const bool on = [] {
+        const char* e = getenv("KSPACE_GPU_MIRROR");
+        return e ? atoi(e) != 0 : true;
+    }();
+    return on;
+}
+
+// Modes per run of a geometry (odd: the lanes' 8-byte reads are then free of bank
+// conflicts; at most 17: the crossing bits of a table entry).  A tile costs about K steps
+// and 8 more whatever K is; the K of the least cost for the tiles of a whole grid, at
+// least one per warp.  (N=768: 23 runs of 17 leave 9 of 32 lanes idle, 30 runs of 13 two:
+// 423 -> 382 us with the call's 45; N=1280: 2001 -> 1657 us with runs of 11.)
+int mirror_run_length(int nz) {
+    if (!use_mirror()) return kRun;
+    int best = kRun;
+    double least = 1e30;
+    const int parts = (nz + 32 * kRun - 1) / (32 * kRun);
+    for (int K = kRun; K >= 9; K -= 2) {
+        const MirrorTiling t = make_mirror_tiling(K, 2 * (nz - 1), nz, 0, 1);
+        if (t.parts > parts) break;
+        const double tiles = 2.0 * (nz - 1) * t.tpp * t.parts / (152 * 11);
+        const double c = (K + 8.0) * (tiles < 1 ? 1 : tiles);
+        if (c < least) {
+            least = c;
+            best = K;
+        }
+    }
+    return best;
+}
+
+// Run table of a geometry: for |kx|, |ky| in [0, N/2] and run r (modes z = Kr .. Kr+K-1
+// of a grid row), entry = b_start << 17 | bit i (i = 1..K-1) set where mode i opens the next
 // bin | bit 0 "slow".  Slow: the run holds the k = 0 mode (excluded, powerspectrum.c:65)
 // or skips a bin between two consecutive modes (low k, a bin narrower than one k^2 step).
 // Rows of Rp = R rounded up to 4 entries (16-byte rows); entries past R are slow.
-__global__ void k_run_table(const int* __restrict__ thr, int nrbins, float c1, int half, int nz, int R, int Rp,
-                            unsigned* __restrict__ tab) {
+__global__ void k_run_table(const int* __restrict__ thr, int nrbins, float c1, int half, int nz, int K, int R,
+                            int Rp, unsigned* __restrict__ tab) {
     const long long n = (long long)(half + 1) * (half + 1) * Rp;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < n;
          e += (long long)gridDim.x * blockDim.x) {
@@ -1517,8 +1802,8 @@ __global__ void k_run_table(const int* __restrict__ thr, int nrbins, float c1, i
         unsigned mask = 0;
         int bprev = -1, bstart = 0;
         bool slow = false;
-        for (int i = 0; i < kRun; i++) {
-            const int z = kRun * r + i;
+        for (int i = 0; i < K; i++) {
+            const int z = K * r + i;
             if (z >= nz) break;
             const int k2 = kxy2 + z * z;
             if (k2 == 0) {
@@ -1542,22 +1827,23 @@ __global__ void k_run_table(const int* __restrict__ thr, int nrbins, float c1, i
 
 int build_run_table(GridGeom& g, cudaStream_t st) {
     g.runtab = nullptr;
-    g.run_Rp = 0;
+    g.run_Rp = g.run_K = 0;
     const int half = g.N / 2, nz = half + 1;
-    const int R = (nz + kRun - 1) / kRun, Rp = (R + 3) & ~3;
+    const int K = mirror_run_length(nz), R = (nz + K - 1) / K, Rp = (R + 3) & ~3;
     const size_t n = (size_t)(half + 1) * (half + 1) * Rp;
     if (g.nrbins >= (1 << 15) || n * sizeof(unsigned) > (size_t(1) << 30)) return 1;
     unsigned* tab = nullptr;
     if (cudaMalloc(&tab, n * sizeof(unsigned)) != cudaSuccess) return -1;
     long long blocks = ((long long)n + 255) / 256;
     if (blocks > 8LL * sm_count_s()) blocks = 8LL * sm_count_s();
-    k_run_table<<<(int)blocks, 256, 0, st>>>(g.thresh, g.nrbins, g.bin_c1, half, nz, R, Rp, tab);
+    k_run_table<<<(int)blocks, 256, 0, st>>>(g.thresh, g.nrbins, g.bin_c1, half, nz, K, R, Rp, tab);
     if (cudaPeekAtLastError() != cudaSuccess) {
         cudaFree(tab);
         return -1;
     }
     g.runtab = tab;
     g.run_Rp = Rp;
+    g.run_K = K;
     return 0;
 }
 
@@ -1578,13 +1864,10 @@ int launch_bin_rows(const GridGeom& g, const GridArgs& a, const float* grid, dou
                     unsigned* status, int warps, int stages, bool exact, cudaStream_t st) {
     if (a.N >= 32768) return -1;
     // the mirrored-row pass where it applies (KSPACE_GPU_MIRROR=0: the row pass only)
-    static const int mirror = [] {
-        const char* e = getenv("KSPACE_GPU_MIRROR");
-        return e ? atoi(e) : 1;
-    }();
-    if (mirror) {
-        const int r = exact ? run_bin_mirror<true>(g, a, grid, bin_sum, F0sq, status, st)
-                            : run_bin_mirror<false>(g, a, grid, bin_sum, F0sq, status, st);
+    if (use_mirror()) {
+        const int r = !exact     ? run_bin_mirror_any<false, false>(g, a, grid, bin_sum, F0sq, status, st)
+                      : g.beside ? run_bin_mirror_any<true, false>(g, a, grid, bin_sum, F0sq, status, st)
+                                 : run_bin_mirror_any<true, true>(g, a, grid, bin_sum, F0sq, status, st);
         if (r != -1) return r;
     }
 #define KSP_BR(W, S)                                                                            \

@@ -199,3 +199,33 @@ def test_row_kernel_without_mirrors(gpu, oracle):
         nk_o, p_o, c_o, _ = oracle.total_powerspectrum(g, N, nb)
         assert nk == nk_o and np.array_equal(np.asarray(c), c_o)
         assert cases.rel_err(np.asarray(p), p_o) < (TOL_EXACT if tma == 5 else TOL_LEAN), (N, tma)
+
+
+@pytest.mark.parametrize("N,nb", [(64, 40), (300, 90), (1088, 200), (1640, 300)])
+@pytest.mark.parametrize("where", ["zero", "pair", "negative"])
+def test_mirrored_rows_of_slab_ranges(gpu, oracle, N, nb, where):
+    """The mirrored-row pass on slab ranges: only planes kx >= 0, planes kx and -kx together
+    (one flush for both), only planes kx < 0; rows of up to 32 runs (several row pairs per
+    tile) and beyond (N > 1086: rows in parts, 1640 with a short last one).  Per-bin sums as
+    the exchange between ranks sees them, 1e-12 of the oracle's double sums as above."""
+    import torch
+    s0, n = {"zero": (0, 2), "pair": (N // 2 - 1, 3), "negative": (N // 2 + 2, 2)}[where]
+    rng = np.random.default_rng(N + s0)
+    nz = N // 2 + 1
+    g = (rng.standard_normal((n, N, nz)) + 1j * rng.standard_normal((n, N, nz))).astype(np.complex64)
+    po, _, _, fo = oracle.total_powerspectrum(g, N, nb, startslab=s0, nslab=n, partial=True)
+    k = _instance(gpu, nb)
+    got = []
+
+    def exchange(sums):
+        got.append(sums.copy())
+        sums[-1] = 1.0
+
+    k.set_allreduce(exchange)
+    k.total_powerspectrum(N, torch.as_tensor(g).cuda(), nb, s0, n)
+    k.close()
+    sums = got[0]
+    assert np.array_equal(sums[:nb] == 0, po == 0)
+    m = po != 0
+    assert cases.rel_err(sums[:nb][m], po[m]) < TOL_EXACT
+    assert sums[nb] == (fo if s0 == 0 else 0.0)

@@ -542,7 +542,7 @@ extern "C" int kspace_gpu_set_transfer(kspace_ctx* c, const double* logk, const 
     I.ntrans = n;
     CK(cudaMemcpy(I.t_logk, logk, sizeof(double) * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(I.t_T, T, sizeof(double) * n, cudaMemcpyHostToDevice));
-    launch_spline_coeffs_1thread(I.t_logk, I.t_T, I.t_c, I.t_c + n, n, c->stream);
+    launch_spline_coeffs(I.t_logk, I.t_T, I.t_c, I.t_c + n, n, c->stream);
     g_launches += 1;
     CK(cudaStreamSynchronize(c->stream));
     return KSPACE_OK;

@@ -100,33 +100,6 @@ KSP_HD double linear_seg(const double* x, const double* y, int i, double v) {
     return y[i] + (v - x[i]) * ((y[i + 1] - y[i]) / (x[i + 1] - x[i]));
 }
 
-// Natural cubic spline coefficients by Gaussian elimination (sequential; small n).
-// scratch: 2*(n-2) doubles.  Same equations as a natural spline anywhere.
-KSP_HD void natural_spline_coeffs(const double* x, const double* y, int n, double* c, double* scratch) {
-    const int m = n - 2;
-    c[0] = 0.0;
-    c[n - 1] = 0.0;
-    if (m <= 0) return;
-    double* diag = scratch;
-    double* rhs = scratch + m;
-    for (int i = 0; i < m; i++) {
-        const double h0 = x[i + 1] - x[i], h1 = x[i + 2] - x[i + 1];
-        diag[i] = 2.0 * (h0 + h1);
-        rhs[i] = 3.0 * ((y[i + 2] - y[i + 1]) / h1 - (y[i + 1] - y[i]) / h0);
-    }
-    for (int i = 1; i < m; i++) {
-        const double off = x[i + 1] - x[i];
-        const double f = off / diag[i - 1];
-        diag[i] -= f * off;
-        rhs[i] -= f * rhs[i - 1];
-    }
-    c[m] = rhs[m - 1] / diag[m - 1];
-    for (int i = m - 1; i-- > 0;) {
-        const double off = x[i + 2] - x[i + 1];
-        c[i + 1] = (rhs[i] - off * c[i + 2]) / diag[i];
-    }
-}
-
 // ------------------------------------------------------------------ background
 // omega_nu_single.c:100-114 (rho_nu conversion factor)
 KSP_HD double rho_nu_conversion() {
@@ -426,60 +399,94 @@ __device__ __forceinline__ double rescale_error(double err, double resabs, doubl
 
 struct GkOut { double result, abserr, resabs, resasc; };
 
+// The GK61 sums of one or two intervals from the node values of a warp (fv[2 t + m]: node
+// lane + 32 m of interval t, 0 past the 61st), and the rule's outputs, identical on every
+// lane.  The FP64 pipe takes 16 cycles a warp instruction whatever its lanes do, so the count
+// is what matters: the sums of both intervals are reduced together by a butterfly that
+// halves the set of values each lane carries at every step, and where no value is negative
+// (a density history's sign does not change: nearly always) |f| sums to what f does: the
+// Kronrod and Gauss sums take 6 additions per lane, resasc's two 5.
+__device__ __forceinline__ void gk61_lane_sums(const Gk61Nodes& N, const double* fv, int nint, const double* h,
+                                               GkOut* out) {
+    const int lane = threadIdx.x & 31;
+    const bool two = lane < 29;  // the lane has a second node
+    const double k0 = N.wk[lane], k1 = two ? N.wk[32 + lane] : 0.0;
+    const double g0 = N.wg[lane], g1 = two ? N.wg[32 + lane] : 0.0;
+    const int b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+    double rk[2], rg[2];
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+        rk[t] = fma(k1, fv[2 * t + 1], k0 * fv[2 * t]);
+        rg[t] = fma(g1, fv[2 * t + 1], g0 * fv[2 * t]);
+    }
+    const int signs = __double2hiint(fv[0]) | __double2hiint(fv[1]) | __double2hiint(fv[2]) | __double2hiint(fv[3]);
+    const bool negative = __any_sync(0xffffffffu, signs < 0);
+    // interval 0 goes to the lanes below 16, 1 to the others; there Kronrod below bit 3, Gauss above
+    const double ka = (b4 ? rk[1] : rk[0]) + __shfl_xor_sync(0xffffffffu, b4 ? rk[0] : rk[1], 16);
+    const double ga = (b4 ? rg[1] : rg[0]) + __shfl_xor_sync(0xffffffffu, b4 ? rg[0] : rg[1], 16);
+    double y = (b3 ? ga : ka) + __shfl_xor_sync(0xffffffffu, b3 ? ka : ga, 8);
+    double ra = 0.0;
+    if (negative) {  // warp-uniform
+        double r[2];
+#pragma unroll
+        for (int t = 0; t < 2; t++) r[t] = fma(k1, fabs(fv[2 * t + 1]), k0 * fabs(fv[2 * t]));
+        ra = (b4 ? r[1] : r[0]) + __shfl_xor_sync(0xffffffffu, b4 ? r[0] : r[1], 16);
+        ra += __shfl_xor_sync(0xffffffffu, ra, 8);
+        // one more value each: |f| on the lanes with bit 2
+        const double give = b2 ? y : ra, keep = b2 ? ra : y;
+        y = keep + __shfl_xor_sync(0xffffffffu, give, 4);
+    } else {
+        y += __shfl_xor_sync(0xffffffffu, y, 4);
+    }
+    y += __shfl_xor_sync(0xffffffffu, y, 2);
+    y += __shfl_xor_sync(0xffffffffu, y, 1);
+    const double rk0 = __shfl_sync(0xffffffffu, y, 0), rk1 = __shfl_sync(0xffffffffu, y, 16);
+    const double mean0 = 0.5 * rk0, mean1 = 0.5 * rk1;
+    const double s0 = fma(k1, fabs(fv[1] - mean0), k0 * fabs(fv[0] - mean0));
+    const double s1 = fma(k1, fabs(fv[3] - mean1), k0 * fabs(fv[2] - mean1));
+    double z = (b4 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, b4 ? s0 : s1, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+    // the outputs of interval t on lane t, then broadcast
+    const int t = lane & 1;
+    const double rgt = __shfl_sync(0xffffffffu, y, t ? 24 : 8);
+    const double rat = __shfl_sync(0xffffffffu, y, (t ? 16 : 0) + (negative ? 4 : 0));
+    const double rst = __shfl_sync(0xffffffffu, z, t ? 16 : 0);
+    GkOut o = {0.0, 0.0, 0.0, 0.0};
+    if (lane < nint) {
+        const double ht = t ? h[1] : h[0];
+        const double rkt = t ? rk1 : rk0;
+        o.result = rkt * ht;
+        o.resabs = rat * fabs(ht);
+        o.resasc = rst * fabs(ht);
+        o.abserr = rescale_error((rkt - rgt) * ht, o.resabs, o.resasc);
+    }
+    for (int u = 0; u < nint; u++) {
+        out[u].result = __shfl_sync(0xffffffffu, o.result, u);
+        out[u].resabs = __shfl_sync(0xffffffffu, o.resabs, u);
+        out[u].resasc = __shfl_sync(0xffffffffu, o.resasc, u);
+        out[u].abserr = __shfl_sync(0xffffffffu, o.abserr, u);
+    }
+}
+
 // Evaluate the GK61 rule on `nint` (1 or 2) intervals [a_t, b_t] with one warp.
-// Every lane returns identical values (sums are reduced to lane 0 and broadcast).
+// Every lane returns identical values.
 template <class F>
 __device__ __forceinline__ void gk61_warp(const F& f, const Gk61Nodes& N, int nint, const double* a, const double* b,
                                           GkOut* out) {
     const int lane = threadIdx.x & 31;
-    double c[2], h[2];
+    double h[2], fv[4];
+#pragma unroll
     for (int t = 0; t < 2; t++) {
-        c[t] = __dmul_rn(0.5, __dadd_rn(a[t], b[t]));
+        const double c = __dmul_rn(0.5, __dadd_rn(a[t], b[t]));
         h[t] = __dmul_rn(0.5, __dsub_rn(b[t], a[t]));
-    }
-    double fv[4];
-    double rk[2] = {0, 0}, rg[2] = {0, 0}, ra[2] = {0, 0};
-    const int nslots = 61 * nint;
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const int s = lane + 32 * m;
-        fv[m] = 0.0;
-        if (s < nslots) {
-            const int t = s >= 61 ? 1 : 0;
-            const int j = s - 61 * t;
-            const double x = __dadd_rn(c[t], __dmul_rn(h[t], N.x[j]));
-            const double v = f(x);
-            fv[m] = v;
-            if (t == 0) { rk[0] += N.wk[j] * v; rg[0] += N.wg[j] * v; ra[0] += N.wk[j] * fabs(v); }
-            else { rk[1] += N.wk[j] * v; rg[1] += N.wg[j] * v; ra[1] += N.wk[j] * fabs(v); }
+        for (int m = 0; m < 2; m++) {
+            const int j = lane + 32 * m;
+            fv[2 * t + m] = t < nint && j < 61 ? f(__dadd_rn(c, __dmul_rn(h[t], N.x[j]))) : 0.0;
         }
     }
-    double mean[2];
-    for (int t = 0; t < nint; t++) {
-        rk[t] = bcast0(warp_sum_to0(rk[t]));
-        rg[t] = bcast0(warp_sum_to0(rg[t]));
-        ra[t] = bcast0(warp_sum_to0(ra[t]));
-        mean[t] = 0.5 * rk[t];
-    }
-    double rs[2] = {0, 0};
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const int s = lane + 32 * m;
-        if (s < nslots) {
-            const int t = s >= 61 ? 1 : 0;
-            const int j = s - 61 * t;
-            const double d = N.wk[j] * fabs(fv[m] - mean[t]);
-            if (t == 0) rs[0] += d; else rs[1] += d;
-        }
-    }
-    for (int t = 0; t < nint; t++) {
-        rs[t] = bcast0(warp_sum_to0(rs[t]));
-        const double err = (rk[t] - rg[t]) * h[t];
-        out[t].result = rk[t] * h[t];
-        out[t].resabs = ra[t] * fabs(h[t]);
-        out[t].resasc = rs[t] * fabs(h[t]);
-        out[t].abserr = rescale_error(err, out[t].resabs, out[t].resasc);
-    }
+    gk61_lane_sums(N, fv, nint, h, out);
 }
 
 struct QagList {  // per-warp interval list in shared memory
@@ -570,76 +577,6 @@ __device__ __forceinline__ int nc_child(int s, int right, int nslots) {
     const int d = s / 2 + 1;                      // depth of the children
     const int c = 2 * d - 1 + right;
     return c < nslots ? c : -1;
-}
-
-// The GK61 sums of one or two intervals from the node values of a warp (fv[2 t + m]: node
-// lane + 32 m of interval t, 0 past the 61st), and the rule's outputs, identical on every
-// lane.  The FP64 pipe takes 16 cycles a warp instruction whatever its lanes do, so the count
-// is what matters: the sums of both intervals are reduced together by a butterfly that
-// halves the set of values each lane carries at every step, and where no value is negative
-// (a density history's sign does not change: nearly always) |f| sums to what f does: the
-// Kronrod and Gauss sums take 6 additions per lane, resasc's two 5.
-__device__ __forceinline__ void gk61_lane_sums(const Gk61Nodes& N, const double* fv, int nint, const double* h,
-                                               GkOut* out) {
-    const int lane = threadIdx.x & 31;
-    const bool two = lane < 29;  // the lane has a second node
-    const double k0 = N.wk[lane], k1 = two ? N.wk[32 + lane] : 0.0;
-    const double g0 = N.wg[lane], g1 = two ? N.wg[32 + lane] : 0.0;
-    const int b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-    double rk[2], rg[2];
-#pragma unroll
-    for (int t = 0; t < 2; t++) {
-        rk[t] = fma(k1, fv[2 * t + 1], k0 * fv[2 * t]);
-        rg[t] = fma(g1, fv[2 * t + 1], g0 * fv[2 * t]);
-    }
-    const int signs = __double2hiint(fv[0]) | __double2hiint(fv[1]) | __double2hiint(fv[2]) | __double2hiint(fv[3]);
-    const bool negative = __any_sync(0xffffffffu, signs < 0);
-    // interval 0 goes to the lanes below 16, 1 to the others; there Kronrod below bit 3, Gauss above
-    const double ka = (b4 ? rk[1] : rk[0]) + __shfl_xor_sync(0xffffffffu, b4 ? rk[0] : rk[1], 16);
-    const double ga = (b4 ? rg[1] : rg[0]) + __shfl_xor_sync(0xffffffffu, b4 ? rg[0] : rg[1], 16);
-    double y = (b3 ? ga : ka) + __shfl_xor_sync(0xffffffffu, b3 ? ka : ga, 8);
-    double ra = 0.0;
-    if (negative) {  // warp-uniform
-        double r[2];
-#pragma unroll
-        for (int t = 0; t < 2; t++) r[t] = fma(k1, fabs(fv[2 * t + 1]), k0 * fabs(fv[2 * t]));
-        ra = (b4 ? r[1] : r[0]) + __shfl_xor_sync(0xffffffffu, b4 ? r[0] : r[1], 16);
-        ra += __shfl_xor_sync(0xffffffffu, ra, 8);
-        // one more value each: |f| on the lanes with bit 2
-        const double give = b2 ? y : ra, keep = b2 ? ra : y;
-        y = keep + __shfl_xor_sync(0xffffffffu, give, 4);
-    } else {
-        y += __shfl_xor_sync(0xffffffffu, y, 4);
-    }
-    y += __shfl_xor_sync(0xffffffffu, y, 2);
-    y += __shfl_xor_sync(0xffffffffu, y, 1);
-    const double rk0 = __shfl_sync(0xffffffffu, y, 0), rk1 = __shfl_sync(0xffffffffu, y, 16);
-    const double mean0 = 0.5 * rk0, mean1 = 0.5 * rk1;
-    const double s0 = fma(k1, fabs(fv[1] - mean0), k0 * fabs(fv[0] - mean0));
-    const double s1 = fma(k1, fabs(fv[3] - mean1), k0 * fabs(fv[2] - mean1));
-    double z = (b4 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, b4 ? s0 : s1, 16);
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-    // the outputs of interval t on lane t, then broadcast
-    const int t = lane & 1;
-    const double rgt = __shfl_sync(0xffffffffu, y, t ? 24 : 8);
-    const double rat = __shfl_sync(0xffffffffu, y, (t ? 16 : 0) + (negative ? 4 : 0));
-    const double rst = __shfl_sync(0xffffffffu, z, t ? 16 : 0);
-    GkOut o = {0.0, 0.0, 0.0, 0.0};
-    if (lane < nint) {
-        const double ht = t ? h[1] : h[0];
-        const double rkt = t ? rk1 : rk0;
-        o.result = rkt * ht;
-        o.resabs = rat * fabs(ht);
-        o.resasc = rst * fabs(ht);
-        o.abserr = rescale_error((rkt - rgt) * ht, o.resabs, o.resasc);
-    }
-    for (int u = 0; u < nint; u++) {
-        out[u].result = __shfl_sync(0xffffffffu, o.result, u);
-        out[u].resabs = __shfl_sync(0xffffffffu, o.resabs, u);
-        out[u].resasc = __shfl_sync(0xffffffffu, o.resasc, u);
-        out[u].abserr = __shfl_sync(0xffffffffu, o.abserr, u);
-    }
 }
 
 // gk61_warp with interval slots

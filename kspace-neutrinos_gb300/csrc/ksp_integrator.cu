@@ -66,20 +66,22 @@ __global__ void k_rho_points(Background* B, unsigned* status) {
     }
 }
 
-__global__ void k_rho_splines(Background* B, double* scratch) {
-    const int s = threadIdx.x;
-    if (s >= kNuSpecies) return;
-    RhoTable& T = B->tab[s];
-    T.imnu = 1.0 / T.mnu;
-    if (!B->deg[s] || !T.has_table) return;
-    natural_spline_coeffs(T.loga, T.rhonu, kNRhoTab, T.c, scratch + s * 2 * kNRhoTab);
+// a block per species: the table's natural spline and its segments' polynomials (one thread per
+// species swept the system in 574 us)
+constexpr int kSplineThreads = 128;
+__global__ void __launch_bounds__(kSplineThreads) k_rho_splines(Background* B) {
+    __shared__ double fac[kNRhoTab], inv[kNRhoTab], sh[2 * kSplineThreads / 32];
+    RhoTable& T = B->tab[blockIdx.x];
+    if (threadIdx.x == 0) T.imnu = 1.0 / T.mnu;
+    if (!B->deg[blockIdx.x] || !T.has_table) return;
+    natural_spline_block<kSplineThreads>(T.loga, T.rhonu, kNRhoTab, T.c, fac, inv, sh);
     // the node-independent terms of cspline_seg, per segment
-    for (int i = 0; i + 1 < kNRhoTab; i++) {
+    for (int i = threadIdx.x; i + 1 < kNRhoTab; i += kSplineThreads) {
         const double h = T.loga[i + 1] - T.loga[i];
         T.sb[i] = (T.rhonu[i + 1] - T.rhonu[i]) / h - h * (T.c[i + 1] + 2.0 * T.c[i]) / 3.0;
         T.sd[i] = (T.c[i + 1] - T.c[i]) / (3.0 * h);
     }
-    T.inv_dx = (kNRhoTab - 1) / (T.loga[kNRhoTab - 1] - T.loga[0]);
+    if (threadIdx.x == 0) T.inv_dx = (kNRhoTab - 1) / (T.loga[kNRhoTab - 1] - T.loga[0]);
 }
 
 void launch_background_tables(Background* dB, double a0, cudaStream_t st, unsigned* status) {
@@ -87,10 +89,7 @@ void launch_background_tables(Background* dB, double a0, cudaStream_t st, unsign
     const int warps = 4;
     const int tasks = kNuSpecies * kNRhoTab;
     k_rho_points<<<(tasks + warps - 1) / warps, 32 * warps, warps * sizeof(QagList), st>>>(dB, status);
-    double* scratch = nullptr;
-    cudaMallocAsync(&scratch, sizeof(double) * 2 * kNRhoTab * kNuSpecies, st);
-    k_rho_splines<<<1, 32, 0, st>>>(dB, scratch);
-    cudaFreeAsync(scratch, st);
+    k_rho_splines<<<kNuSpecies, kSplineThreads, 0, st>>>(dB);
 }
 
 // Natural cubic spline of log H on n uniform knots (spacing h), as per-segment
@@ -126,12 +125,14 @@ void launch_hubble_table(const double* H, int n, double h, double* coef, double*
     k_hubble_table<<<1, 32, 0, st>>>(H, n, h, coef, scratch);
 }
 
-__global__ void k_spline1(const double* x, const double* y, double* c, double* scratch, int n) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) natural_spline_coeffs(x, y, n, c, scratch);
+// natural spline of one table of n >= 3 knots; scratch: 2 n
+__global__ void __launch_bounds__(kSplineThreads) k_spline1(const double* x, const double* y, double* c,
+                                                            double* scratch, int n) {
+    __shared__ double sh[2 * kSplineThreads / 32];
+    natural_spline_block<kSplineThreads>(x, y, n, c, scratch, scratch + n, sh);
 }
-void launch_spline_coeffs_1thread(const double* x, const double* y, double* c, double* scratch, int n,
-                                  cudaStream_t st) {
-    k_spline1<<<1, 32, 0, st>>>(x, y, c, scratch, n);
+void launch_spline_coeffs(const double* x, const double* y, double* c, double* scratch, int n, cudaStream_t st) {
+    k_spline1<<<1, kSplineThreads, 0, st>>>(x, y, c, scratch, n);
 }
 
 struct FermiDirac {  // omega_nu_single.c:207-210
@@ -365,7 +366,7 @@ __global__ void __launch_bounds__(kTableThreads, 8)
         }
         if (m < 1) return;
         __syncthreads();
-        spline_solve_block<kTableThreads>(I, m, c, sh);
+        spline_solve_block<kTableThreads>(I.scalefact, I.knot_fac, I.knot_invdiag, m, c, sh);
         if (t == 0) {
             c[0] = 0.0;
             c[Na - 1] = 0.0;

@@ -355,8 +355,8 @@ int raise_dynamic_smem_limit(const void* kernel);
 
 // ---- integrator launchers (ksp_integrator.cu)
 void launch_background_tables(Background* dB, double a0, cudaStream_t st, unsigned* status);
-void launch_spline_coeffs_1thread(const double* x, const double* y, double* c, double* scratch, int n,
-                                  cudaStream_t st);
+// natural cubic spline coefficients c[n] of y on the knots x, n >= 3; scratch[2 n]
+void launch_spline_coeffs(const double* x, const double* y, double* c, double* scratch, int n, cudaStream_t st);
 // J's fine table on the current device
 const double* jfine_table();
 void launch_nufrac_low(Background* dB, double light, double vcrit, cudaStream_t st, unsigned* status);

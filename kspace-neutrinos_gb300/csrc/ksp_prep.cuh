@@ -288,18 +288,18 @@ __device__ __forceinline__ double nc_node_x(int q, double loga0, double loga) {
 
 // The same solve as spline_solve_scan with all T threads of a block (T a multiple of 32):
 // warp scans of the affine maps, combined over the warps through sh (2 * T / 32 doubles of
-// shared memory).
+// shared memory).  x, fac, invdiag: the knots and their factorised system (knot_row).
 template <int T>
-__device__ __forceinline__ void spline_solve_block(const IntegratorDev& I, int m, double* sc, double* sh) {
+__device__ __forceinline__ void spline_solve_block(const double* x, const double* fac, const double* invdiag, int m,
+                                                   double* sc, double* sh) {
     constexpr int NW = T / 32;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const double* x = I.scalefact;
     const int per = (m + T - 1) / T;
     const int u0 = min(m, t * per), u1 = min(m, u0 + per);
     // forward: z_u = r_u - fac_u z_{u-1} (fac_0 = 0)
     double A = 1.0, B = 0.0;
     for (int u = u0; u < u1; u++) {
-        const double f = u > 0 ? I.knot_fac[u] : 0.0;
+        const double f = u > 0 ? fac[u] : 0.0;
         B = sc[u + 1] - f * B;
         A = -f * A;
     }
@@ -322,7 +322,7 @@ __device__ __forceinline__ void spline_solve_block(const IntegratorDev& I, int m
     double ea = __shfl_up_sync(0xffffffffu, pa, 1), eb = __shfl_up_sync(0xffffffffu, pb, 1);
     double zin = lane == 0 ? win : ea * win + eb;
     for (int u = u0; u < u1; u++) {
-        const double f = u > 0 ? I.knot_fac[u] : 0.0;
+        const double f = u > 0 ? fac[u] : 0.0;
         zin = sc[u + 1] - f * zin;
         sc[u + 1] = zin;
     }
@@ -332,7 +332,7 @@ __device__ __forceinline__ void spline_solve_block(const IntegratorDev& I, int m
     B = 0.0;
     for (int u = u1 - 1; u >= u0; u--) {
         const double off = u < m - 1 ? x[u + 2] - x[u + 1] : 0.0;
-        const double iv = I.knot_invdiag[u];
+        const double iv = invdiag[u];
         B = (sc[u + 1] - off * B) * iv;
         A = -off * iv * A;
     }
@@ -358,8 +358,28 @@ __device__ __forceinline__ void spline_solve_block(const IntegratorDev& I, int m
     double cin = lane == 31 ? win : ea * win + eb;
     for (int u = u1 - 1; u >= u0; u--) {
         const double off = u < m - 1 ? x[u + 2] - x[u + 1] : 0.0;
-        cin = (sc[u + 1] - off * cin) * I.knot_invdiag[u];
+        cin = (sc[u + 1] - off * cin) * invdiag[u];
         sc[u + 1] = cin;
+    }
+    __syncthreads();
+}
+
+// Natural cubic spline of y on the knots x (n >= 3) by a block of T threads: c = S''/2 at the
+// knots.  fac, invdiag: n doubles of scratch each; sh as spline_solve_block's.
+template <int T>
+__device__ __forceinline__ void natural_spline_block(const double* x, const double* y, int n, double* c, double* fac,
+                                                     double* invdiag, double* sh) {
+    const int t = threadIdx.x;
+    auto knot = [&](int j) { return x[j]; };
+    for (int u = t; u < n - 2; u += T) {
+        knot_row(knot, u, invdiag, fac);
+        c[u + 1] = 3.0 * ((y[u + 2] - y[u + 1]) / (x[u + 2] - x[u + 1]) - (y[u + 1] - y[u]) / (x[u + 1] - x[u]));
+    }
+    __syncthreads();
+    spline_solve_block<T>(x, fac, invdiag, n - 2, c, sh);
+    if (t == 0) {
+        c[0] = 0.0;
+        c[n - 1] = 0.0;
     }
     __syncthreads();
 }

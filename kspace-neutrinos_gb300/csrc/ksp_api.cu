@@ -16,6 +16,7 @@
 #include <mutex>
 #include <set>
 #include <string>
+#include <type_traits>
 #include <vector>
 #include "ksp_ctx.h"
 
@@ -54,7 +55,8 @@ int ksp::map_status(unsigned s) {
     return KSPACE_OK;
 }
 
-// Synchronise with the stream and convert the device status word.
+// Synchronise with the stream and convert the device status word.  Results that a call has
+// queued for pinned memory before it are then there too.
 static int sync_status(kspace_ctx* c) {
     CK(cudaMemcpyAsync(c->status_h, c->status_d, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
@@ -93,6 +95,19 @@ bool ksp::is_device_ptr(const void* p) {
     return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
+// The copy stream and the events of host grids, with the first of them.
+static int ensure_copy_stream(kspace_ctx* c) {
+    if (c->ev_copy_end) return KSPACE_OK;
+    if (!c->copy) CK(cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking));
+    for (int i = 0; i < kspace_ctx::kChunks; i++) {
+        if (!c->ev_up[i]) CK(cudaEventCreateWithFlags(&c->ev_up[i], cudaEventDisableTiming));
+        if (!c->ev_done[i]) CK(cudaEventCreateWithFlags(&c->ev_done[i], cudaEventDisableTiming));
+    }
+    if (!c->ev_copy_start) CK(cudaEventCreateWithFlags(&c->ev_copy_start, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&c->ev_copy_end, cudaEventDisableTiming));
+    return KSPACE_OK;
+}
+
 // ------------------------------------------------------------------ lifecycle
 extern "C" int kspace_gpu_create(kspace_ctx** out, int device) {
     NEED(out, KSPACE_ERR_ARG);
@@ -105,15 +120,7 @@ extern "C" int kspace_gpu_create(kspace_ctx** out, int device) {
     CK(cudaMemset(c->status_d, 0, sizeof(unsigned)));
     CK(cudaMallocHost(reinterpret_cast<void**>(&c->status_h), sizeof(unsigned)));
     CK(dalloc(&c->dB, 1));
-    for (int i = 0; i < 5; i++) CK(cudaEventCreate(&c->ev[i]));
     CK(cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking));
-    for (int i = 0; i < kspace_ctx::kChunks; i++) {
-        CK(cudaEventCreateWithFlags(&c->ev_up[i], cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&c->ev_done[i], cudaEventDisableTiming));
-    }
-    CK(cudaEventCreateWithFlags(&c->ev_copy_start, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&c->ev_copy_end, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
     if (const char* e = getenv("KSPACE_GPU_TMA")) c->tma = atoi(e);
@@ -132,23 +139,16 @@ extern "C" int kspace_gpu_create(kspace_ctx** out, int device) {
 
 static void free_table(kspace_ctx* c) {
     IntegratorDev& I = c->I;
-    void* ptrs[] = {I.scalefact, I.dtot, I.coef, I.nu_init, I.nu_last, I.wavenum, I.dcdm, I.dnu_s, I.dnu,
-                    I.knot_invdiag, I.knot_fac, I.knot_invh, I.knot_h3, I.knot_ih3, I.nc_g, I.nc_fsl,
-                    I.nc_dx, I.nc_j, I.nc_inv, I.nc_ab, I.nc_cd, I.nc_jf, I.hyb, I.fs_x, I.fs_y, I.fs_c, I.fs_seg, I.fs_suf, I.fs_tot, I.t_logk, I.t_T,
-                    I.t_c, I.sc,
-                    I.qag_max, I.qag_total, I.coef_unit};
+    void* ptrs[] = {c->arena_d, I.hyb, I.t_logk};  // (t_T and t_c lie behind t_logk)
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    c->arena_d = nullptr;
     memset(&I, 0, sizeof(I));
-    void* bufs[] = {c->bin_sum_d, c->power_d, c->keffg_d, c->keff_d, c->logk_d, c->ratio_d,
-                    c->norm_d, c->dnu_out_d, c->io_d, c->corr.xf, c->corr.rn, c->corr.sn};
-    for (void* p : bufs)
-        if (p) cudaFree(p);
     c->bin_sum_d = c->F0sq_d = c->power_d = c->keffg_d = c->keff_d = nullptr;
     c->logk_d = c->ratio_d = c->norm_d = c->dnu_out_d = c->io_d = nullptr;
     c->corr = CorrTable{};
     if (c->ar_h) cudaFreeHost(c->ar_h);
-    c->ar_h = nullptr;
+    c->ar_h = c->io_h = nullptr;
     void* adj[] = {c->ivals_d, c->adj_node_d, c->adj_Dbar_d, c->adj_mbar_d, c->adj_Q_d, c->adj_dcsum_d,
                    c->adj_dnubar_d, c->adj_rbar_d, c->nivals_d};
     for (void* p : adj)
@@ -446,44 +446,76 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
     NEED(I.namax > 1, KSPACE_ERR_ARG);
     I.ld = (I.namax + 1) & ~1;  // even: every row starts on a 16-byte boundary
     const size_t nk = nk_alloc, ld = I.ld;
-    CK(dalloc(&I.scalefact, ld));
-    CK(dalloc(&I.dtot, nk * ld));
-    CK(dalloc(&I.coef, nk * ld));
-    CK(cudaMemset(I.dtot, 0, sizeof(double) * nk * ld));
-    CK(cudaMemset(I.coef, 0, sizeof(double) * nk * ld));
-    CK(dalloc(&I.coef_unit, ld));
-    CK(dalloc(&I.nu_init, nk));
-    CK(dalloc(&I.nu_last, nk));
-    CK(dalloc(&I.wavenum, nk));
-    CK(dalloc(&I.dcdm, nk));
-    CK(dalloc(&I.dnu_s, kNuSpecies * nk));
-    CK(dalloc(&I.dnu, nk));
-    CK(dalloc(&I.knot_invdiag, ld));
-    CK(dalloc(&I.knot_fac, ld));
-    CK(dalloc(&I.knot_invh, ld));
-    CK(dalloc(&I.knot_h3, ld));
-    CK(dalloc(&I.knot_ih3, ld));
-    CK(dalloc(&I.nc_g, kNcNodes));
-    CK(dalloc(&I.nc_fsl, kNcNodes));
-    CK(dalloc(&I.nc_dx, kNcNodes));
-    CK(dalloc(&I.nc_j, kNcNodes));
-    CK(dalloc(&I.nc_ab, kNcNodes));
-    CK(dalloc(&I.nc_cd, kNcNodes));
-    CK(dalloc(&I.nc_jf, kNcNodes));
-    I.jt = jfine_table();
-    NEED(I.jt, KSPACE_ERR_CUDA);
     I.nc_slots = c->nc_levels > 0 ? 1 + 2 * c->nc_levels : 0;
     I.fs_cap = 16 * (int)ld + 16;
-    CK(dalloc(&I.fs_x, I.fs_cap));
-    CK(dalloc(&I.fs_y, I.fs_cap));
-    CK(dalloc(&I.fs_c, I.fs_cap));
-    CK(dalloc(&I.fs_seg, I.fs_cap));
-    CK(dalloc(&I.fs_suf, I.fs_cap));
-    CK(dalloc(&I.fs_tot, I.fs_cap / 16 + 1));
-    CK(dalloc(&I.nc_inv, kNcNodes));
-    CK(dalloc(&I.sc, 1));
-    CK(dalloc(&I.qag_max, 1));
-    CK(dalloc(&I.qag_total, 1));
+    // all of the table's arrays and the step's buffers in one allocation, each from a 256-byte
+    // boundary (one call each, they were two thirds of closing an instance)
+    const size_t fs = I.fs_cap;
+    size_t at = 0;
+    char* base = nullptr;
+    auto take = [&](auto** p, size_t n) {
+        *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + at);
+        at = (at + sizeof(**p) * n + 255) & ~size_t(255);
+    };
+    for (int pass = 0; pass < 2; pass++) {
+        at = 0;
+        take(&I.dtot, nk * ld);  // first: these two are cleared
+        take(&I.coef, nk * ld);
+        take(&I.scalefact, ld);
+        take(&I.coef_unit, ld);
+        take(&I.nu_init, nk);
+        take(&I.nu_last, nk);
+        take(&I.wavenum, nk);
+        take(&I.dcdm, nk);
+        take(&I.dnu_s, kNuSpecies * nk);
+        take(&I.dnu, nk);
+        take(&I.knot_invdiag, ld);
+        take(&I.knot_fac, ld);
+        take(&I.knot_invh, ld);
+        take(&I.knot_h3, ld);
+        take(&I.knot_ih3, ld);
+        take(&I.nc_g, kNcNodes);
+        take(&I.nc_fsl, kNcNodes);
+        take(&I.nc_dx, kNcNodes);
+        take(&I.nc_j, kNcNodes);
+        take(&I.nc_ab, kNcNodes);
+        take(&I.nc_cd, kNcNodes);
+        take(&I.nc_jf, kNcNodes);
+        take(&I.nc_inv, kNcNodes);
+        take(&I.fs_x, fs);
+        take(&I.fs_y, fs);
+        take(&I.fs_c, fs);
+        take(&I.fs_seg, fs);
+        take(&I.fs_suf, fs);
+        take(&I.fs_tot, fs / 16 + 1);
+        take(&I.sc, 1);
+        take(&I.qag_max, 1);
+        take(&I.qag_total, 1);
+        take(&c->bin_sum_d, nk + 1);
+        take(&c->power_d, nk);
+        take(&c->keffg_d, nk);
+        take(&c->keff_d, nk);
+        take(&c->logk_d, nk);
+        take(&c->ratio_d, nk);
+        take(&c->norm_d, 1);
+        take(&c->dnu_out_d, nk);
+        take(&c->io_d, 4 * nk);
+        take(&c->corr.xf, nk);
+        take(&c->corr.rn, nk);
+        take(&c->corr.sn, nk);
+        if (pass == 0) {
+            const cudaError_t e = cudaMalloc(&c->arena_d, at);
+            if (e != cudaSuccess) {
+                c->arena_d = nullptr;
+                free_table(c);
+                CK(e);
+            }
+            base = static_cast<char*>(c->arena_d);
+        }
+    }
+    CK(cudaMemset(c->arena_d, 0, reinterpret_cast<char*>(I.scalefact) - base));  // dtot, coef
+    I.jt = jfine_table();
+    NEED(I.jt, KSPACE_ERR_CUDA);
     I.status = c->status_d;
     StepScalars S;
     memset(&S, 0, sizeof(S));
@@ -493,22 +525,10 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
     c->Omeganonu = S.Omeganonu;
     c->S0 = S;
     CK(cudaMemcpy(I.sc, &S, sizeof(S), cudaMemcpyHostToDevice));
-    // step buffers
     c->buf_nb = nk_alloc;
-    CK(dalloc(&c->bin_sum_d, nk + 1));
     c->F0sq_d = c->bin_sum_d + nk;
-    CK(dalloc(&c->power_d, nk));
-    CK(dalloc(&c->keffg_d, nk));
-    CK(dalloc(&c->keff_d, nk));
-    CK(dalloc(&c->logk_d, nk));
-    CK(dalloc(&c->ratio_d, nk));
-    CK(dalloc(&c->norm_d, 1));
-    CK(dalloc(&c->dnu_out_d, nk));
-    CK(dalloc(&c->io_d, 4 * nk));
-    CK(dalloc(&c->corr.xf, nk));
-    CK(dalloc(&c->corr.rn, nk));
-    CK(dalloc(&c->corr.sn, nk));
-    CK(cudaMallocHost(reinterpret_cast<void**>(&c->ar_h), sizeof(double) * (nk + 1)));
+    CK(cudaMallocHost(reinterpret_cast<void**>(&c->ar_h), sizeof(double) * (3 * nk + 1)));
+    c->io_h = c->ar_h + nk + 1;
     c->TimeTransfer = TimeTransfer;
     c->loga0 = log(TimeTransfer);
     c->nk = nk_alloc;
@@ -534,11 +554,10 @@ extern "C" int kspace_gpu_set_transfer(kspace_ctx* c, const double* logk, const 
     if (!c->table_ready) return KSPACE_OK;
     IntegratorDev& I = c->I;
     if (I.t_logk) cudaFree(I.t_logk);
-    if (I.t_T) cudaFree(I.t_T);
-    if (I.t_c) cudaFree(I.t_c);
-    CK(dalloc(&I.t_logk, n));
-    CK(dalloc(&I.t_T, n));
-    CK(dalloc(&I.t_c, 3 * n));
+    I.t_logk = I.t_T = I.t_c = nullptr;
+    CK(dalloc(&I.t_logk, 5 * (size_t)n));
+    I.t_T = I.t_logk + n;
+    I.t_c = I.t_T + n;
     I.ntrans = n;
     CK(cudaMemcpy(I.t_logk, logk, sizeof(double) * n, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(I.t_T, T, sizeof(double) * n, cudaMemcpyHostToDevice));
@@ -798,15 +817,13 @@ static int update_device(kspace_ctx* c, double a, int nk_in, const double* keff_
     if (nk_in != c->nk) return KSPACE_ERR_NK_MISMATCH;
     if (c->nk < 2) return KSPACE_ERR_NK_SMALL;
     const double loga = log(a);
-    // the delta_cdm-independent part already ran beside the binning pass (it also zeroes
-    // the QAG statistics)
+    // the delta_cdm-independent part already ran beside the binning pass (the preparation also
+    // zeroes the QAG statistics)
     const bool prepared = c->prep_valid && c->prep_Na == c->ia + 1 && c->prep_loga == loga &&
                           !(loga - c->h_scalefact[c->ia - 1] < kFloatAcc) && c->ia < I.namax;
-    if (!prepared) {
+    if (loga - c->h_scalefact[c->ia - 1] < kFloatAcc) {
         CK(cudaMemsetAsync(I.qag_max, 0, sizeof(int), c->stream));
         CK(cudaMemsetAsync(I.qag_total, 0, sizeof(long long), c->stream));
-    }
-    if (loga - c->h_scalefact[c->ia - 1] < kFloatAcc) {
         // same scale factor: return delta_nu_last unchanged (delta_tot_table.c:209-213)
         CK(cudaMemcpyAsync(I.dnu, I.nu_last, sizeof(double) * c->nk, cudaMemcpyDeviceToDevice, c->stream));
         if (want_corr || dnu_out_d) {
@@ -819,7 +836,7 @@ static int update_device(kspace_ctx* c, double a, int nk_in, const double* keff_
                                  want_corr ? c->corr : CorrTable{}, c->norm_d, c->stream);
             g_launches += 2;
         }
-        return sync_status(c);
+        return sync ? sync_status(c) : KSPACE_OK;
     }
     if (c->ia >= I.namax) return KSPACE_ERR_NAMAX;
     // provisional row from delta_nu_last (delta_tot_table.c:222): written, after the call's
@@ -861,12 +878,29 @@ extern "C" int kspace_gpu_get_delta_nu_update(kspace_ctx* c, double a, int nk, c
     NEED(c->table_ready, KSPACE_ERR_ORDER);
     NEED(nk <= c->I.nk_alloc, KSPACE_ERR_NK_ALLOC);
     double* kd = c->io_d;
-    double* dd = c->io_d + c->I.nk_alloc;
-    CK(cudaMemcpyAsync(kd, keff, sizeof(double) * nk, cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(dd, P_cdm_sqrt, sizeof(double) * nk, cudaMemcpyHostToDevice, c->stream));
-    int st = update_device(c, a, nk, kd, dd, c->dnu_out_d, false);
+    const size_t n = nk;
+    // through pinned memory: one copy in, one wait for the result and the status (copies from
+    // and to the caller's pageable memory took a wait of their own).  Anything else than plain
+    // host memory is left to the copies themselves.
+    const bool pinned = !is_device_ptr(keff) && !is_device_ptr(P_cdm_sqrt) && !is_device_ptr(delta_nu);
+    if (pinned) {
+        memcpy(c->io_h, keff, sizeof(double) * n);
+        memcpy(c->io_h + n, P_cdm_sqrt, sizeof(double) * n);
+        CK(cudaMemcpyAsync(kd, c->io_h, sizeof(double) * 2 * n, cudaMemcpyHostToDevice, c->stream));
+    } else {
+        CK(cudaMemcpyAsync(kd, keff, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(kd + n, P_cdm_sqrt, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
+    }
+    int st = update_device(c, a, nk, kd, kd + n, c->dnu_out_d, false, nullptr, false);
+    if (st) {
+        cudaStreamSynchronize(c->stream);  // the inputs are free again
+        return st;
+    }
+    if (pinned) CK(cudaMemcpyAsync(c->io_h, c->dnu_out_d, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+    st = sync_status(c);
     if (st) return st;
-    CK(cudaMemcpy(delta_nu, c->dnu_out_d, sizeof(double) * nk, cudaMemcpyDeviceToHost));
+    if (pinned) memcpy(delta_nu, c->io_h, sizeof(double) * n);
+    else CK(cudaMemcpy(delta_nu, c->dnu_out_d, sizeof(double) * n, cudaMemcpyDeviceToHost));
     return KSPACE_OK;
 }
 
@@ -895,8 +929,6 @@ static int integrate_stored(kspace_ctx* c, double a, int nk, const double* waven
     IntegratorDev& I = c->I;
     double* kd = c->io_d + 2 * (size_t)I.nk_alloc;
     CK(cudaMemcpyAsync(kd, wavenum, sizeof(double) * nk, cudaMemcpyDefault, c->stream));
-    CK(cudaMemsetAsync(I.qag_max, 0, sizeof(int), c->stream));
-    CK(cudaMemsetAsync(I.qag_total, 0, sizeof(long long), c->stream));
     I.kq = kd;
     // the knot factorisation is rebuilt from the first row: rows may have changed since
     prepare_call(c, c->ia, a, log(a), 0, 0, kRowsFull, nk, -1, c->stream);
@@ -1344,10 +1376,13 @@ extern "C" int kspace_gpu_total_powerspectrum(kspace_ctx* c, int dims, const voi
     if (st) return st;
     st = bin_grid(c, G, gd, dims, startslab, nslab, 1.0);
     if (st) return st;
+    const size_t n = G->nk;
+    CK(cudaMemcpyAsync(c->io_h, c->power_d, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(c->io_h + n, c->keffg_d, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
     st = sync_status(c);
     if (st) return st;
-    CK(cudaMemcpy(power, c->power_d, sizeof(double) * G->nk, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(keffs, c->keffg_d, sizeof(double) * G->nk, cudaMemcpyDeviceToHost));
+    memcpy(power, c->io_h, sizeof(double) * n);
+    memcpy(keffs, c->io_h + n, sizeof(double) * n);
     for (int i = 0; i < G->nk; i++) count[i] = G->count[G->compact[i]];
     // like the reference: entries beyond nk keep the pre-compaction values; we zero them
     for (int i = G->nk; i < nrbins; i++) {
@@ -1410,6 +1445,8 @@ extern "C" int kspace_gpu_add_nu_power_to_rhogrid(kspace_ctx* c, double Time, do
     if (staged) {
         // a host grid: upload in slab chunks on the copy stream (after the work queued so
         // far on the context's stream, which may still read the staging buffer)
+        st = ensure_copy_stream(c);
+        if (st) return st;
         st = stage_alloc(c, bytes);
         if (st) return st;
         gd = reinterpret_cast<float*>(c->stage_d);
@@ -1625,6 +1662,10 @@ extern "C" int kspace_gpu_last_correction(kspace_ctx* c, int* nk, double* logk, 
 
 extern "C" int kspace_gpu_set_profiling(kspace_ctx* c, int on) {
     NEED(c, KSPACE_ERR_ARG);
+    if (on) CK(cudaSetDevice(c->device));
+    if (on)
+        for (int i = 0; i < 5; i++)
+            if (!c->ev[i]) CK(cudaEventCreate(&c->ev[i]));
     c->prof = on != 0;
     return KSPACE_OK;
 }
@@ -1663,13 +1704,21 @@ extern "C" int kspace_gpu_set_vectors(kspace_ctx* c, const double* nu_init, cons
     return KSPACE_OK;
 }
 
+// The values travel as kernel arguments: nothing of the host's is read after the call.
+__global__ void k_set_jmass(Background* B, double m0, double m1, double m2) {
+    B->mnu_J[0] = m0;
+    B->mnu_J[1] = m1;
+    B->mnu_J[2] = m2;
+}
+
 extern "C" int kspace_gpu_set_jmass(kspace_ctx* c, const double* MNu) {
     NEED(c, KSPACE_ERR_ARG);
     NEED(c->bg_ready, KSPACE_ERR_ORDER);
     for (int i = 0; i < kNuSpecies; i++) c->hB.mnu_J[i] = MNu ? MNu[i] : c->hB.mnu[i];
-    CK(cudaMemcpyAsync(&c->dB->mnu_J[0], &c->hB.mnu_J[0], sizeof(double) * kNuSpecies, cudaMemcpyHostToDevice,
-                       c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    static_assert(kNuSpecies == 3, "one argument per species");
+    k_set_jmass<<<1, 1, 0, c->stream>>>(c->dB, c->hB.mnu_J[0], c->hB.mnu_J[1], c->hB.mnu_J[2]);
+    g_launches += 1;
+    CK(cudaGetLastError());
     return KSPACE_OK;
 }
 
@@ -1725,8 +1774,6 @@ extern "C" int kspace_gpu_diff_forward(kspace_ctx* c, double Time, double BoxSiz
         Is.ivals = c->ivals_d;
         Is.nivals = c->nivals_d;
     }
-    CK(cudaMemsetAsync(I.qag_max, 0, sizeof(int), c->stream));
-    CK(cudaMemsetAsync(I.qag_total, 0, sizeof(long long), c->stream));
     prepare_call(c, Na, Time, loga, start, 1, kRowsFull, c->nk, c->ia, c->stream);
     launch_integrator_rest(Is, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, -1, true);
     c->fact_valid = start;

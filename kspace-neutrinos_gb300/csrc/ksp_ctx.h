@@ -61,7 +61,9 @@ struct kspace_ctx {
     CorrTable corr{};
     unsigned* status_d = nullptr;
     unsigned* status_h = nullptr;
-    double* ar_h = nullptr;
+    void* arena_d = nullptr;   // the table's device arrays (alloc_table), one allocation
+    double* ar_h = nullptr;    // pinned: [nk_alloc + 1] for the exchange, then [2 nk_alloc] for a call's in- and outputs
+    double* io_h = nullptr;
     int last_nk = 0;
     double last_BoxSize = 0;
     // geometry cache keyed by (N, nrbins)

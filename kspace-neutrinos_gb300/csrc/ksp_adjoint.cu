@@ -17,7 +17,7 @@
 //                            d/d(row) through the spline (cubic basis + transposed
 //                            natural-spline solve) and d/dm through J's argument
 //   B2c k_adj_bins2          dcdm/P cotangents -> per-bin Q_b and the DC term
-//   B3  k_adj_grid_plain     xbar_m = gbar_m smth_m + Q_b w_m W_m^4 x_m   (reads gbar, x; writes xbar)
+//   B3  k_adj_grid           xbar_m = gbar_m smth_m + Q_b w_m W_m^4 x_m   (reads gbar, x; writes xbar)
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "ksp_internal.h"
@@ -64,15 +64,22 @@ __device__ __forceinline__ void corr_weights(int k2, const GridArgs& g, const Co
 // x = log k (as the correction pass does), and a run of modes in one segment j
 // accumulates A = sum u and B = sum u t (u = gbar . x, t the position in the segment) in
 // FP32, so d/dr_j gets A - B and d/dr_{j+1} gets B once per run, into the warp's own
-// float totals; each block adds its warps' totals to the FP64 node sums once.
+// float totals; each block adds its warps' totals to the FP64 node sums once.  Some lane of a
+// warp leaves its segment at nearly every step: the next segment is tried before a search
+// (256^3, 128 nodes: 52 us, 67 with a search and a division each time; the reads' floor
+// is 20).
 __global__ void __launch_bounds__(256) k_adj_reduce8(GridArgs g, CorrTable corr, const float* __restrict__ gbar,
                                                      const float* __restrict__ x, double* node_sum, long long nchunks,
                                                      int adv_il, int adv_j, int adv_z) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5;
     float* s_xf = reinterpret_cast<float*>(sm_raw);
-    float* s_acc = s_xf + g.nk;  // [nw][nk]
-    for (int i = threadIdx.x; i < g.nk; i += blockDim.x) s_xf[i] = corr.xf[i];
+    float* s_inv = s_xf + g.nk;
+    float* s_acc = s_inv + g.nk;  // [nw][nk]
+    for (int i = threadIdx.x; i < g.nk; i += blockDim.x) {
+        s_xf[i] = corr.xf[i];
+        s_inv[i] = i < g.nk - 1 ? 1.f / (corr.xf[i + 1] - corr.xf[i]) : 0.f;
+    }
     for (int i = threadIdx.x; i < nw * g.nk; i += blockDim.x) s_acc[i] = 0.f;
     __syncthreads();
     float* acc = s_acc + warp * g.nk;
@@ -89,19 +96,28 @@ __global__ void __launch_bounds__(256) k_adj_reduce8(GridArgs g, CorrTable corr,
         A = 0.f;
         B = 0.f;
     };
+    int seg = nk;  // -1 below the first node, nk - 1 from the last on
+    auto set = [&](int lo) {
+        seg = lo;
+        const bool below = lo < 0, above = lo >= nk - 1;  // constant there: all to node 0, to node nk-1
+        j0 = below ? 0 : (above ? nk - 2 : lo);
+        xlo = below ? -3.0e38f : s_xf[lo];
+        xhi = above ? 3.0e38f : s_xf[lo + 1];
+        x0 = below || above ? 0.f : xlo;
+        inv = below || above ? 0.f : s_inv[lo];
+        tadd = above ? 1.f : 0.f;
+    };
     auto locate = [&](float xm) {
+        if (xm >= xhi && seg < nk - 1) {
+            set(seg + 1);
+            if (xm < xhi) return;
+        }
         int lo = -1, hi = nk;  // largest j with xf[j] <= xm
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             if (s_xf[mid] <= xm) lo = mid; else hi = mid;
         }
-        if (lo < 0) {  // constant below the first node: all to node 0
-            j0 = 0; xlo = -3.0e38f; xhi = s_xf[0]; x0 = 0.f; inv = 0.f; tadd = 0.f;
-        } else if (lo >= nk - 1) {  // constant from the last node: all to node nk-1
-            j0 = nk - 2; xlo = s_xf[nk - 1]; xhi = 3.0e38f; x0 = 0.f; inv = 0.f; tadd = 1.f;
-        } else {
-            j0 = lo; xlo = s_xf[lo]; xhi = s_xf[lo + 1]; x0 = xlo; inv = 1.f / (xhi - xlo); tadd = 0.f;
-        }
+        set(lo);
     };
     const long long stride = (long long)gridDim.x * blockDim.x;
     long long ci = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -258,7 +274,7 @@ __global__ void k_adj_bins(AdjBins A, int nk) {
 }
 
 __global__ void k_adj_bins2(AdjBins A, int nk) {
-    __shared__ double red[256];
+    __shared__ double red[8];
     double acc = 0;
     for (int b = threadIdx.x; b < nk; b += blockDim.x) {
         const double v = A.dnu[b];
@@ -270,11 +286,12 @@ __global__ void k_adj_bins2(AdjBins A, int nk) {
         A.Q[bin] = 2.0 * Pbar / (*A.F0sq * (double)A.count[bin]);
         acc += Pbar * A.power[b];
     }
-    red[threadIdx.x] = acc;
+    acc = warp_sum_to0(acc);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
         double s = 0;
-        for (int i = 0; i < (int)blockDim.x; i++) s += red[i];
+        for (int i = 0; i < (int)blockDim.x / 32; i++) s += red[i];
         *A.dc_sum = s;
     }
 }
@@ -490,58 +507,108 @@ __global__ void __launch_bounds__(128) k_dnu_adj(IntegratorDev I, DnuAdjArgs A, 
 }
 
 // ------------------------------------------------------------------ B3
-__global__ void k_adj_grid_plain(GridArgs g, const int* __restrict__ thresh, const int* __restrict__ cmapg,
-                                 const float* __restrict__ w1g, CorrTable corr, const float* __restrict__ gbar,
-                                 const float* __restrict__ x, float* xbar, const double* __restrict__ Q,
-                                 const double* dc_sum, const double* F0sq) {
+// By columns of equal |kx|, |ky|, z: a warp takes 32 consecutive z of one |kx|, |ky|, and the
+// up to four rows (+-kx, +-ky) that share its k^2.  A mode's bin, its segment of the ratio
+// table and its window are found once for the four, and a lane's eight reads (four rows of
+// gbar and of x) are in flight together.  Bound by its traffic: 256^3, 203 MB, takes 31 us (a
+// thread per mode: 63 us).
+
+// Grid rows of (+-kx, +-ky): row q = 0..3 has -ky for odd q, -kx from q = 2; a row that is
+// its own mirror image has only one of the two.
+struct MirrorRows {
+    long long first, dx, dy;
+    bool mx, my;
+    __device__ __forceinline__ MirrorRows(const GridArgs& g, int ax, int ay)
+        : first(((long long)ax * g.N + ay) * g.nz), dx((long long)(g.N - 2 * ax) * g.N * g.nz),
+          dy((long long)(g.N - 2 * ay) * g.nz), mx(ax != 0 && 2 * ax != g.N), my(ay != 0 && 2 * ay != g.N) {}
+    __device__ __forceinline__ bool has(int q) const { return (!(q & 1) || my) && (!(q & 2) || mx); }
+    __device__ __forceinline__ long long mode(int q, int z) const {
+        return first + ((q & 1) ? dy : 0) + ((q & 2) ? dx : 0) + z;
+    }
+};
+
+// A warp's column block: |kx|, |ky| and its first z, from a task number below
+// (N/2+1)^2 ceil(nz/32) (2^31 of them would be a grid of 2 TB).
+struct ColumnTasks {
+    FastDiv fd_chunk, fd_half;
+    unsigned n;
+};
+__device__ __forceinline__ void column_task(const ColumnTasks& T, unsigned t, int& ax, int& ay, int& z0) {
+    const unsigned p = fdiv(t, T.fd_chunk);
+    z0 = 32 * (int)(t - p * T.fd_chunk.d);
+    ax = (int)fdiv(p, T.fd_half);
+    ay = (int)(p - (unsigned)ax * T.fd_half.d);
+}
+
+// Segment of the ratio table that holds x = log k: its lower node, -1 below the first, nk-1
+// from the last one on (delta_pow.c:19-37).  A bin's modes lie about the bin's own node.
+__device__ __forceinline__ int mode_segment(float x, int bin, const int* cmap, const float* xf) {
+    const int c = max(cmap[bin], 0);
+    return x < xf[c] ? c - 1 : c;
+}
+
+__global__ void __launch_bounds__(256, 4)
+    k_adj_grid(GridArgs g, ColumnTasks T, const int* __restrict__ thresh, const int* __restrict__ cmapg,
+               const float* __restrict__ w1g, CorrTable corr, const float* __restrict__ gbar,
+               const float* __restrict__ x, float* xbar, const double* __restrict__ Q,
+               const double* dc_sum, const double* F0sq) {
     extern __shared__ unsigned char sm_raw[];
+    const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nk = g.nk;
     int* s_thr = reinterpret_cast<int*>(sm_raw);
     int* s_cmap = s_thr + g.nrbins + 1;
-    float* s_tab = reinterpret_cast<float*>(s_cmap + g.nrbins);
-    float* s_w1 = s_tab + 3 * g.nk;
+    float* s_xf = reinterpret_cast<float*>(s_cmap + g.nrbins);
+    float* s_rn = s_xf + nk;
+    float* s_sn = s_rn + nk;
+    float* s_w1 = s_sn + nk;
     float* s_Q = s_w1 + g.nz;
     for (int i = threadIdx.x; i <= g.nrbins; i += blockDim.x) s_thr[i] = thresh[i];
     for (int i = threadIdx.x; i < g.nrbins; i += blockDim.x) {
         s_cmap[i] = cmapg[i];
         s_Q[i] = (float)Q[i];
     }
-    for (int i = threadIdx.x; i < g.nk; i += blockDim.x) {
-        s_tab[i] = corr.xf[i];
-        s_tab[g.nk + i] = corr.rn[i];
-        s_tab[2 * g.nk + i] = corr.sn[i];
+    for (int i = threadIdx.x; i < nk; i += blockDim.x) {
+        s_xf[i] = corr.xf[i];
+        s_rn[i] = corr.rn[i];
+        s_sn[i] = corr.sn[i];
     }
     for (int i = threadIdx.x; i < g.nz; i += blockDim.x) s_w1[i] = w1g[i];
     __syncthreads();
-    CorrSmem T{s_thr, s_cmap, s_tab, s_tab + g.nk, s_tab + 2 * g.nk};
-    unsigned flags = 0;
-    for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < g.nmodes;
-         m += (long long)gridDim.x * blockDim.x) {
-        const long long r = m / g.nz;
-        ModeCursor c;
-        c.z = (int)(m - r * g.nz);
-        c.il = (int)(r / g.N);
-        c.j = (int)(r - (long long)c.il * g.N);
-        c.set_row(g, s_w1);
-        const int k2 = c.kxy2 + c.z * c.z;
-        const float2 gv = reinterpret_cast<const float2*>(gbar)[m];
-        const float2 xv = reinterpret_cast<const float2*>(x)[m];
-        float2 o;
+    for (unsigned task = blockIdx.x * nw + warp; task < T.n; task += gridDim.x * nw) {
+        int ax, ay, z0;
+        column_task(T, task, ax, ay, z0);
+        const MirrorRows R(g, ax, ay);
+        const int z = z0 + lane;
+        if (z >= g.nz) continue;
+        float2 gv[4], xv[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (R.has(q)) {
+                gv[q] = __ldcs(reinterpret_cast<const float2*>(gbar) + R.mode(q, z));
+                xv[q] = __ldcs(reinterpret_cast<const float2*>(x) + R.mode(q, z));
+            }
+        const int k2 = ax * ax + ay * ay + z * z;
         if (k2 == 0) {
             // DC: y_0 = x_0, and |x_0|^2 normalises every P_b
             const double f = -2.0 * (*dc_sum) / (*F0sq);
-            o.x = (float)(gv.x + f * xv.x);
-            o.y = (float)(gv.y + f * xv.y);
-        } else {
-            const float d = corr_delta(k2, g, T, flags);
-            const float t = __fmul_rn(c.iwxy, s_w1[c.z]);
-            const float inv = __fmul_rn(t, t);
-            float wW = __fmul_rn(inv, inv);
-            if (c.z != 0 && c.z != g.half) wW = wW + wW;
-            const float q = s_Q[bin_of(k2, g.c1, s_thr, g.nrbins)] * wW;
-            o.x = fmaf(gv.x, d, gv.x) + q * xv.x;
-            o.y = fmaf(gv.y, d, gv.y) + q * xv.y;
+            reinterpret_cast<float2*>(xbar)[0] =
+                make_float2((float)(gv[0].x + f * xv[0].x), (float)(gv[0].y + f * xv[0].y));
+            continue;
         }
-        reinterpret_cast<float2*>(xbar)[m] = o;
+        const int bin = bin_of(k2, g.c1, s_thr, g.nrbins);
+        const float xm = fmaf(0.5f, __logf((float)k2), g.lnscale);
+        const int j = mode_segment(xm, bin, s_cmap, s_xf);
+        const float d = j < 0 ? s_rn[0] : (j >= nk - 1 ? s_rn[nk - 1] : fmaf(xm - s_xf[j], s_sn[j], s_rn[j]));
+        const float t = __fmul_rn(__fmul_rn(s_w1[ax], s_w1[ay]), s_w1[z]);
+        const float inv = __fmul_rn(t, t);
+        float wW = __fmul_rn(inv, inv);
+        if (z != 0 && z != g.half) wW = wW + wW;
+        const float qw = s_Q[bin] * wW;
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (R.has(q))
+                __stcs(reinterpret_cast<float2*>(xbar) + R.mode(q, z),
+                       make_float2(fmaf(gv[q].x, d, gv[q].x) + qw * xv[q].x,
+                                   fmaf(gv[q].y, d, gv[q].y) + qw * xv[q].y));
     }
 }
 
@@ -699,6 +766,23 @@ static int sm_count_a() {
     return n;
 }
 
+static ColumnTasks column_tasks(const GridArgs& a) {
+    ColumnTasks T;
+    T.fd_chunk = make_fastdiv((uint32_t)((a.nz + 31) / 32));
+    T.fd_half = make_fastdiv((uint32_t)(a.half + 1));
+    T.n = (unsigned)T.fd_half.d * T.fd_half.d * T.fd_chunk.d;
+    return T;
+}
+
+// Blocks of nw warps over the column tasks: as many as the chip holds at a time.
+template <typename K>
+static int column_blocks(K kern, int nw, size_t smem, unsigned ntask) {
+    int occ = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * nw, smem) != cudaSuccess || occ < 1) occ = 1;
+    const unsigned need = (ntask + nw - 1) / nw, have = (unsigned)(occ * sm_count_a());
+    return (int)(need < have ? need : have);
+}
+
 void launch_adj_reduce(const GridGeom& gg, CorrTable corr, float lnscale, const float* gbar, const float* x,
                        double* node_sum, cudaStream_t st) {
     GridArgs a = make_grid_args(gg, corr.nk, lnscale);
@@ -710,7 +794,7 @@ void launch_adj_reduce(const GridGeom& gg, CorrTable corr, float lnscale, const 
         if (blocks < 1) blocks = 1;
         const long long adv = blocks * 256 * 8;  // modes per grid stride
         const int nz = gg.N / 2 + 1;
-        const size_t smem = sizeof(float) * corr.nk * (1 + 8);
+        const size_t smem = sizeof(float) * corr.nk * (2 + 8);
         cudaFuncSetAttribute(k_adj_reduce8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         const long long adv_rows = adv / nz;
         k_adj_reduce8<<<(int)blocks, 256, smem, st>>>(a, corr, gbar, x, node_sum, nchunks, (int)(adv_rows / gg.N),
@@ -768,13 +852,12 @@ void launch_dnu_adj(const IntegratorDev& I, const double* dnu_bar, double* Dbar,
 
 void launch_adj_grid(const GridGeom& gg, CorrTable corr, float lnscale, const float* gbar, const float* x, float* xbar,
                      const double* Q, const double* dc_sum, const double* F0sq, cudaStream_t st) {
-    GridArgs a = make_grid_args(gg, corr.nk, lnscale);
-    const size_t smem = sizeof(int) * (2 * gg.nrbins + 1) + sizeof(float) * (3 * corr.nk + a.nz + gg.nrbins) + 64;
-    cudaFuncSetAttribute(k_adj_grid_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    long long blocks = (gg.nmodes + 255) / 256;
-    if (blocks > 8LL * sm_count_a()) blocks = 8LL * sm_count_a();
-    k_adj_grid_plain<<<(int)(blocks > 0 ? blocks : 1), 256, smem, st>>>(a, gg.thresh, gg.cmap, gg.w1, corr, gbar, x,
-                                                                        xbar, Q, dc_sum, F0sq);
+    const GridArgs a = make_grid_args(gg, corr.nk, lnscale);
+    const ColumnTasks T = column_tasks(a);
+    const size_t smem = sizeof(int) * (2 * gg.nrbins + 1) + sizeof(float) * (3 * corr.nk + a.nz + gg.nrbins);
+    cudaFuncSetAttribute(k_adj_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_adj_grid<<<column_blocks(k_adj_grid, 8, smem, T.n), 256, smem, st>>>(a, T, gg.thresh, gg.cmap, gg.w1, corr,
+                                                                           gbar, x, xbar, Q, dc_sum, F0sq);
 }
 
 }  // namespace ksp

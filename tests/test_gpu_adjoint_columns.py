@@ -1,0 +1,31 @@
+"""The adjoint's gradient pass goes through columns of 32 consecutive z of one |kx|, |ky|:
+gradients at grids whose rows end before, at and after a column's end, with all rows that
+are their own mirror image (kx or ky of 0 and N/2), against the FP64 reference adjoint.
+
+Tolerance 1e-5 of the largest gradient, as in test_gpu_adjoint.py: a mode's cotangent is
+formed in single precision from its inputs (about ten roundings of 6e-8), a bin's total
+from at most 1e5 of them in sums of 32."""
+import numpy as np
+import pytest
+
+from test_gpu_adjoint import gpu_grads, setup
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N,nb", [(30, 20), (62, 40), (66, 90)])
+def test_column_edges(gpu, oracle, N, nb):
+    c, ref, k, a = setup(oracle, gpu, N, nb, 16, (0.05, 0.05, 0.05), seed=N)
+    wb = np.random.default_rng(N).random(c["nk"])
+    xg, Dg, mg, out, pnu = gpu_grads(k, c, a, wb, recompute=False)
+    adj = ref.adjoint(c["grid"].astype(np.complex128), c["delta_tot"], np.array(c["MNu"]), wb)
+    xr, Dr = adj["xbar"], adj["Dbar"]
+    err = np.abs(xg - xr)
+    half = N // 2
+    for kx in (0, 1, half, half + 1, N - 1):
+        for z in (0, min(31, half), half):
+            assert err[kx, :, z].max() <= 1e-5 * np.max(np.abs(xr)), (kx, z)
+    assert err.max() <= 1e-5 * np.max(np.abs(xr))
+    assert np.max(np.abs(Dg - Dr)) <= 1e-5 * np.max(np.abs(Dr))
+    assert abs(mg[0] / adj["mbar"][0] - 1) < 1e-5
+    k.close()

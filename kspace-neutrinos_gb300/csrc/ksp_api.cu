@@ -1394,14 +1394,16 @@ extern "C" int kspace_gpu_total_powerspectrum(kspace_ctx* c, int dims, const voi
     return KSPACE_OK;
 }
 
+// in: the grid to read where it is not gd itself.
 static int correct_grid(kspace_ctx* c, Geo* G, float* gd, double BoxSize, int nk, const SlabChunks* ch = nullptr,
-                        void* host = nullptr) {
+                        void* host = nullptr, const float* in = nullptr) {
     CorrTable corr = c->corr;
     corr.nk = nk;
     const float lnscale = (float)log(2 * kPi / BoxSize);
     if (c->prof) cudaEventRecord(c->ev[2], c->stream);
     if (!ch) {
-        if (launch_apply_correction(G->g, gd, corr, lnscale, c->status_d, c->tma, c->rows, c->stages, c->stream) < 0)
+        if (launch_apply_correction(G->g, gd, corr, lnscale, c->status_d, c->tma, c->rows, c->stages, c->stream, in) <
+            0)
             return KSPACE_ERR_CUDA;
         g_launches += 1;
     } else {
@@ -1760,30 +1762,44 @@ extern "C" int kspace_gpu_diff_forward(kspace_ctx* c, double Time, double BoxSiz
     if (st) return st;
     st = ensure_adj_buffers(c, G->g.nrbins);
     if (st) return st;
-    st = bin_grid(c, G, reinterpret_cast<const float*>(grid_in), pmgrid, 0, pmgrid, BoxSize);
-    if (st) return st;
-    if (G->nk != c->nk) return KSPACE_ERR_NK_MISMATCH;
-    if (c->ia >= c->I.namax) return KSPACE_ERR_NAMAX;
     IntegratorDev& I = c->I;
     const double loga = log(Time);
     const int Na = c->ia + 1;
     int start = c->fact_valid < Na - 3 ? c->fact_valid : Na - 3;
     if (start < 0) start = 0;
+    c->fact_valid = start;
+    // the integrator's delta_cdm-independent work runs beside the binning pass (start_prep)
+    c->prep_valid = false;
+    CK(cudaEventRecord(c->ev_fork, c->stream));
+    st = bin_grid(c, G, reinterpret_cast<const float*>(grid_in), pmgrid, 0, pmgrid, BoxSize, nullptr, Time);
+    const bool prepared = c->prep_valid;
+    c->prep_valid = false;  // its base coefficients become this call's
+    if (prepared) CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+    if (st) return st;
+    if (G->nk != c->nk) return KSPACE_ERR_NK_MISMATCH;
+    if (c->ia >= c->I.namax) return KSPACE_ERR_NAMAX;
     IntegratorDev Is = I;
     if (store_intervals) {
         Is.ivals = c->ivals_d;
         Is.nivals = c->nivals_d;
     }
-    prepare_call(c, Na, Time, loga, start, 1, kRowsFull, c->nk, c->ia, c->stream);
-    launch_integrator_rest(Is, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, -1, true);
-    c->fact_valid = start;
+    // the adjoint reads the rows and their splines: stored before the integrals
+    bool logk_ready = false;
+    if (prepared) {
+        logk_ready = c->fin.active && c->prep_base;
+        launch_integrator_rest(Is, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, c->ia,
+                               true, c->fin.active ? &c->fin : nullptr, c->prep_base, true);
+    } else {
+        prepare_call(c, Na, Time, loga, start, 1, kRowsFull, c->nk, c->ia, c->stream);
+        launch_integrator_rest(Is, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, -1, true);
+    }
+    c->fin.active = 0;
     launch_finish_update(I, c->nk, -3, Time, loga, c->keff_d, c->dnu_out_d, c->logk_d, c->ratio_d, c->corr,
-                         c->norm_d, c->stream, true);
+                         c->norm_d, c->stream, true, logk_ready);
     k_square<<<(c->nk + 127) / 128, 128, 0, c->stream>>>(c->dnu_out_d, pnu_out, c->nk);
     g_launches += 5;
-    const size_t bytes = sizeof(float) * 2 * (size_t)pmgrid * pmgrid * (pmgrid / 2 + 1);
-    if (grid_out != grid_in) CK(cudaMemcpyAsync(grid_out, grid_in, bytes, cudaMemcpyDeviceToDevice, c->stream));
-    st = correct_grid(c, G, reinterpret_cast<float*>(grid_out), BoxSize, c->nk);
+    st = correct_grid(c, G, reinterpret_cast<float*>(grid_out), BoxSize, c->nk, nullptr, nullptr,
+                      reinterpret_cast<const float*>(grid_in));
     if (st) return st;
     st = sync_status(c);
     if (st) return st;

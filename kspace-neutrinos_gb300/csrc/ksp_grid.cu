@@ -562,13 +562,18 @@ static int corr_variant(const GridGeom& g, const GridArgs& a, float* grid, CorrT
 }
 
 int launch_apply_correction(const GridGeom& g, float* grid, CorrTable corr, float lnscale, unsigned* status, int tma,
-                            int rows_per_cta, int stages, cudaStream_t st) {
+                            int rows_per_cta, int stages, cudaStream_t st, const float* in) {
     const GridArgs a = make_grid_args(g, corr.nk, lnscale);
     if (tma >= 3) {
-        const int r = launch_correct_stream(a, grid, corr, status, rows_per_cta / 32, stages, st);
+        const int r = launch_correct_stream(a, in ? in : grid, grid, corr, status, rows_per_cta / 32, stages, st);
         if (r == 0) return 0;
         if (r == -2) return -2;
-    } else if (tma && a.nrows16 > 0) {
+    }
+    // the other kernels work in place
+    if (in && in != grid && cudaMemcpyAsync(grid, in, sizeof(float) * 2 * (size_t)g.nmodes, cudaMemcpyDeviceToDevice,
+                                            st) != cudaSuccess)
+        return -2;
+    if (tma && tma < 3 && a.nrows16 > 0) {
         const int r = corr_variant(g, a, grid, corr, status, rows_per_cta, stages, tma == 2 ? 8 : 16, st);
         if (r == 0) return 0;
         if (r == -2) return -2;

@@ -758,12 +758,16 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
 // The rest, after the rows' splines: the integrals, the species sum.
 void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, const int* spec_ids,
                             int warps_per_block, cudaStream_t st, int qag_split, int update_row, bool defer_combine,
-                            const FinalizeArgs* fin, bool base_ready) {
+                            const FinalizeArgs* fin, bool base_ready, bool rows_stored) {
     RowUpdate upd{};
     upd.row = -1;
     if (update_row >= 0 && base_ready) {
         upd.row = update_row;
         if (fin && fin->active) upd.fin = *fin;
+        if (rows_stored) {  // for a reader after the integrals
+            k_row_update<<<nk, 128, 0, st>>>(I, nk, Na, update_row, upd.fin);
+            upd.row = -1;
+        }
     } else if (update_row >= 0) {
         // a history of two knots: no splines
         if (fin && fin->active)

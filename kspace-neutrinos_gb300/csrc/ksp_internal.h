@@ -401,7 +401,7 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
 void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, const int* spec_ids,
                             int warps_per_block, cudaStream_t st, int qag_split, int update_row = -1,
                             bool defer_combine = false, const FinalizeArgs* fin = nullptr,
-                            bool base_ready = false);
+                            bool base_ready = false, bool rows_stored = false);
 size_t dnu_qag_smem(int ld, int wpb);
 // end of get_delta_nu_update (delta_tot_table.c:226-248) + interface_common.c:134-146:
 // delta_nu_last, committed row, NaN check, clamp, ratio/log k/kspace_prefac, grid table
@@ -446,7 +446,7 @@ int launch_bin_power(const GridGeom& g, const float* grid, double* bin_sum, doub
 // K3: grid *= 1 + norm * interp(log k)
 // Every variant leaves the grid as it is when the status word holds an error (kStAbort).
 int launch_apply_correction(const GridGeom& g, float* grid, CorrTable corr, float lnscale, unsigned* status, int tma,
-                            int rows_per_cta, int stages, cudaStream_t st);
+                            int rows_per_cta, int stages, cudaStream_t st, const float* in = nullptr);
 // normalisation of K1's sums into P(k), delta_cdm, keff (powerspectrum.c:98-115,
 // interface_gadget.c:96-100)
 void launch_finalize_power(const double* bin_sum, const double* F0sq, const long long* count, const double* ksum,

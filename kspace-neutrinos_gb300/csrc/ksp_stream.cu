@@ -435,8 +435,9 @@ __device__ __forceinline__ int seg_of(int k2, const int* k2t, int nk) {
 
 template <int WARPS, int STAGES>
 __global__ void __launch_bounds__(WARPS * 32)
-    k_correct_stream(const __grid_constant__ CUtensorMap tmap, GridArgs g, CorrTable corr, float* grid,
-                     unsigned* status, long long ntiles, int adv_r, int adv_z) {
+    k_correct_stream(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap omap, GridArgs g,
+                     CorrTable corr, const float* grid, float* out, unsigned* status, long long ntiles, int adv_r,
+                     int adv_z) {
     extern __shared__ unsigned char sm_raw[];
     __shared__ int s_gap, s_abort;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -462,7 +463,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         }
     }
     // an error of the step so far (the reference terminates before the multiply): the
-    // grid stays as it is
+    // grid stays as it is, and goes to another output unchanged
     if (tid == 0) s_abort = (*reinterpret_cast<volatile unsigned*>(status) & kStAbort) != 0u;
     // segment s covers k^2 in [k2t[s-1], k2t[s]): s = 0 below the first node (value of
     // node 0), 1..nk-1 the linear pieces between nodes, nk from the last node on (its
@@ -478,7 +479,8 @@ __global__ void __launch_bounds__(WARPS * 32)
         s_gap = -1;
     }
     __syncthreads();
-    if (s_abort) {
+    const bool keep = s_abort;
+    if (keep && out == grid) {
         if (lane == 0)
             for (int s = 0; s < STAGES - 1 && s < my_n; s++) ptx::mbar_wait_bounded(&my_bar[s], 0);
         return;
@@ -516,7 +518,7 @@ __global__ void __launch_bounds__(WARPS * 32)
             break;
         }
         unsigned char* tb = my_stage + s * kTileBytes;
-        const bool valid = tile * kRowsPerWarp + lane < g.nrows16;
+        const bool valid = tile * kRowsPerWarp + lane < g.nrows16 && !keep;
         const uint32_t o = (uint32_t)(zb + 16 * lane);
         const uint32_t dr = fdiv(o, g.fd_nz);
         const int z = (int)(o - dr * (uint32_t)g.nz);
@@ -581,7 +583,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         ptx::fence_async_smem();
         __syncwarp();
         if (lane == 0) {
-            ptx::tma_store_2d_hint(&tmap, tb, 0, (int)(tile * kRowsPerWarp), pol);
+            ptx::tma_store_2d_hint(&omap, tb, 0, (int)(tile * kRowsPerWarp), pol);
             ptx::bulk_commit();
             if (k + STAGES - 1 < my_n) {
                 ptx::bulk_wait_read_le1();  // the store from stage s2 (one tile ago) has read it
@@ -623,13 +625,18 @@ __global__ void __launch_bounds__(WARPS * 32)
             const int il2 = (int)(rr / g.N);
             const int kx2 = kval(g.slab0 + il2, g.N), ky2 = kval((int)(rr - (long long)il2 * g.N), g.N);
             const int k2m = kx2 * kx2 + ky2 * ky2 + zz * zz;
-            if (k2m == 0) continue;
-            const float x = fmaf(__log2f((float)k2m), kHalfLn2, g.lnscale);
-            const float4 cs = s_seg[seg_of(k2m, s_k2t, nk)];
-            if (x < xwarn) flags |= kStKWarn;
-            const float f = fmaf(x - cs.x, cs.y, cs.z);
-            grid[2 * m] = fmaf(grid[2 * m], f, grid[2 * m]);
-            grid[2 * m + 1] = fmaf(grid[2 * m + 1], f, grid[2 * m + 1]);
+            float f = 0.f;
+            if (k2m != 0 && !keep) {
+                const float x = fmaf(__log2f((float)k2m), kHalfLn2, g.lnscale);
+                const float4 cs = s_seg[seg_of(k2m, s_k2t, nk)];
+                if (x < xwarn) flags |= kStKWarn;
+                f = fmaf(x - cs.x, cs.y, cs.z);
+            } else if (out == grid) {
+                continue;
+            }
+            const float re = grid[2 * m], im = grid[2 * m + 1];
+            out[2 * m] = k2m != 0 && !keep ? fmaf(re, f, re) : re;
+            out[2 * m + 1] = k2m != 0 && !keep ? fmaf(im, f, im) : im;
         }
     }
     if (flags) atomicOr(status, flags);
@@ -1736,16 +1743,19 @@ int run_bin_mirror_any(const GridGeom& g, const GridArgs& a, const float* grid, 
 }
 
 template <int WARPS, int STAGES>
-int run_corr_stream(const GridArgs& a, float* grid, CorrTable corr, unsigned* status, cudaStream_t st) {
-    CUtensorMap map;
+int run_corr_stream(const GridArgs& a, const float* grid, float* out, CorrTable corr, unsigned* status,
+                    cudaStream_t st) {
+    CUtensorMap map, omap;
     if (!grid_tmap_cached(&map, grid, a.nrows16, kRowsPerWarp)) return -1;
+    if (out == grid) omap = map;
+    else if (!grid_tmap_cached(&omap, out, a.nrows16, kRowsPerWarp)) return -1;
     const StreamPlan P = plan_corr_stream(WARPS, STAGES, a.nk);
     if (P.total > 220 * 1024) return -1;
     auto kern = k_correct_stream<WARPS, STAGES>;
     const long long ntiles = (a.nrows16 + kRowsPerWarp - 1) / kRowsPerWarp;
     int grid_n = 1, adv_r = 0, adv_z = 0;
     if (!stream_grid(kern, WARPS, P.total, ntiles, a.nz, grid_n, adv_r, adv_z)) return -1;
-    kern<<<grid_n, WARPS * 32, P.total, st>>>(map, a, corr, grid, status, ntiles, adv_r, adv_z);
+    kern<<<grid_n, WARPS * 32, P.total, st>>>(map, omap, a, corr, grid, out, status, ntiles, adv_r, adv_z);
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -1880,14 +1890,14 @@ int launch_bin_rows(const GridGeom& g, const GridArgs& a, const float* grid, dou
                  : run_bin_rows_any<8, 2, false>(g, a, grid, bin_sum, F0sq, status, st);
 }
 
-int launch_correct_stream(const GridArgs& a, float* grid, CorrTable corr, unsigned* status, int warps, int stages,
-                          cudaStream_t st) {
+int launch_correct_stream(const GridArgs& a, const float* grid, float* out, CorrTable corr, unsigned* status,
+                          int warps, int stages, cudaStream_t st) {
     if (a.nrows16 <= 0 || a.nk < 2 || a.N >= 32768) return -1;
 #define KSP_CS(W, S) \
-    if (warps == W && stages == S) return run_corr_stream<W, S>(a, grid, corr, status, st);
+    if (warps == W && stages == S) return run_corr_stream<W, S>(a, grid, out, corr, status, st);
     KSP_CS(4, 2) KSP_CS(4, 3) KSP_CS(4, 4) KSP_CS(8, 2) KSP_CS(8, 3) KSP_CS(8, 4)
 #undef KSP_CS
-    return run_corr_stream<8, 2>(a, grid, corr, status, st);
+    return run_corr_stream<8, 2>(a, grid, out, corr, status, st);
 }
 
 }  // namespace ksp

@@ -29,3 +29,22 @@ def test_column_edges(gpu, oracle, N, nb):
     assert np.max(np.abs(Dg - Dr)) <= 1e-5 * np.max(np.abs(Dr))
     assert abs(mg[0] / adj["mbar"][0] - 1) < 1e-5
     k.close()
+
+
+@pytest.mark.parametrize("N,nb,Na", [(30, 20, 16), (66, 90, 2), (66, 90, 40)])
+def test_output_beside_the_input(gpu, oracle, N, nb, Na):
+    """The corrected grid written to another tensor, the history's splines completed after the
+    binning pass (with two rows there are none): the same grid as in place (the ratio table
+    is in single precision; P_nu's last bits follow the order of the binning pass's FP64 atomic adds), and
+    the input as it was."""
+    import torch
+    c, ref, k, a = setup(oracle, gpu, N, nb, Na, (0.05, 0.05, 0.05), seed=N)
+    g = torch.as_tensor(c["grid"]).cuda()
+    g0, out, work = g.clone(), torch.full_like(g, float("nan")), g.clone()
+    p1, p2 = (torch.empty(c["nk"], dtype=torch.float64, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    k.diff_forward(a, c["L"], g, out, N, p1, True)
+    k.diff_forward(a, c["L"], work, work, N, p2, True)
+    assert torch.equal(g, g0) and torch.equal(out, work)
+    assert out[0, 0, 0] == g[0, 0, 0] and not torch.equal(out, g)
+    k.close()

@@ -481,6 +481,7 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
         take(&I.nc_ab, kNcNodes);
         take(&I.nc_cd, kNcNodes);
         take(&I.nc_jf, kNcNodes);
+        take(&I.nc_half, kNcMaxSlots);
         take(&I.nc_inv, kNcNodes);
         take(&I.fs_x, fs);
         take(&I.fs_y, fs);

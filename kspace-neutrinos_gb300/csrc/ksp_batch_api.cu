@@ -49,7 +49,7 @@ struct kspace_batch {
     BatchGridCorr* gcorr_d = nullptr;
     int total_bins = 0, ldmax = 0;
     // tuning
-    int wpb = 4, blocks_per_sm = 2, use_graph = 1;
+    int wpb = 4, blocks_per_sm = 3, use_graph = 1;
     int nc_slots = 17;  // node-table slots per instance (8 levels of the right spine)
     bool eager_done = false;
     cudaGraph_t graph = nullptr;

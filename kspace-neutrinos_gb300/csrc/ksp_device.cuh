@@ -377,22 +377,26 @@ __device__ __forceinline__ double bcast0(double v) { return __shfl_sync(0xffffff
 // is x sqrt(x / resasc), formed as x^2 / sqrt(x resasc): one reciprocal square root in place of
 // pow, or of a division and a square root, whose dependent FP64 chains are on the QAG's
 // critical path.
+// Values that are not negative are compared by their bits, on the integer pipe: an FP64
+// comparison takes the FP64 pipe's 16 cycles.
+__device__ __forceinline__ long long bits_of(double v) { return __double_as_longlong(v); }
 __device__ __forceinline__ double rescale_error(double err, double resabs, double resasc) {
     err = fabs(err);
-    if (resasc != 0.0 && err != 0.0) {
+    if (bits_of(resasc) != 0 && bits_of(err) != 0) {
         const double x = 200.0 * err, p = x * resasc;
-        if (x >= resasc) {
+        const int hp = __double2hiint(p);
+        if (hp >= 0x05d00000 && hp < 0x7ff00000) {  // 2^-930 <= p, finite: neither is a NaN
+            err = bits_of(x) >= bits_of(resasc) ? resasc : x * (x * rsqrt(p));
+        } else if (x >= resasc) {
             err = resasc;
-        } else if (p > 1e-280) {
-            err = x * (x * rsqrt(p));
         } else {
             const double t = x / resasc;
             err = resasc * (t * sqrt(t));
         }
     }
-    if (resabs > DBL_MIN / (50.0 * DBL_EPSILON)) {
+    if (bits_of(resabs) > bits_of(DBL_MIN / (50.0 * DBL_EPSILON))) {
         const double fl = 50.0 * DBL_EPSILON * resabs;
-        if (fl > err) err = fl;
+        if (bits_of(fl) > bits_of(err)) err = fl;  // (a NaN among them: err was one)
     }
     return err;
 }
@@ -441,9 +445,9 @@ __device__ __forceinline__ void gk61_lane_sums(const Gk61Nodes& N, const double*
     y += __shfl_xor_sync(0xffffffffu, y, 2);
     y += __shfl_xor_sync(0xffffffffu, y, 1);
     const double rk0 = __shfl_sync(0xffffffffu, y, 0), rk1 = __shfl_sync(0xffffffffu, y, 16);
-    const double mean0 = 0.5 * rk0, mean1 = 0.5 * rk1;
-    const double s0 = fma(k1, fabs(fv[1] - mean0), k0 * fabs(fv[0] - mean0));
-    const double s1 = fma(k1, fabs(fv[3] - mean1), k0 * fabs(fv[2] - mean1));
+    // distances from the mean, half the Kronrod sum
+    const double s0 = fma(k1, fabs(fma(-0.5, rk0, fv[1])), k0 * fabs(fma(-0.5, rk0, fv[0])));
+    const double s1 = fma(k1, fabs(fma(-0.5, rk1, fv[3])), k0 * fabs(fma(-0.5, rk1, fv[2])));
     double z = (b4 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, b4 ? s0 : s1, 16);
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
@@ -496,6 +500,39 @@ struct QagList {  // per-warp interval list in shared memory
 
 struct QagResult { double result, abserr; int ok; int nint; };
 
+// QUADPACK's bookkeeping of a bisection: interval k (result r_i, error e_i) into halves with
+// the rule results g[0], g[1]; whether to go on.  The round-off and tiny-interval tests, whose
+// outcome a comparison of high words nearly always settles, are then left out.
+struct QagSums {
+    double area, errsum, tol;
+    int n, roundoff1, roundoff2, error_type;
+};
+__device__ __forceinline__ bool qag_account(QagSums& q, const GkOut* g, double r_i, double e_i, double a1, double a2,
+                                            double b2, double epsabs, double epsrel, int limit) {
+    const double area12 = g[0].result + g[1].result, error12 = g[0].abserr + g[1].abserr;
+    q.errsum += error12 - e_i;
+    q.area += area12 - r_i;
+    // below half of e_i the error has fallen as it should
+    if (__double2hiint(error12) >= __double2hiint(e_i) - 0x00100000 && g[0].resasc != g[0].abserr &&
+        g[1].resasc != g[1].abserr) {
+        if (fabs(r_i - area12) <= 1.0e-5 * fabs(area12) && error12 >= 0.99 * e_i) q.roundoff1++;
+        if (q.n >= 10 && error12 > e_i) q.roundoff2++;
+    }
+    const double t = epsrel * fabs(q.area);  // fmax(epsabs, t)
+    q.tol = bits_of(t) > bits_of(epsabs) && bits_of(t) <= 0x7ff0000000000000LL ? t : epsabs;
+    const bool more = q.errsum > q.tol;
+    if (more) {
+        if (q.roundoff1 >= 6 || q.roundoff2 >= 20) q.error_type = 2;
+        const int h1 = __double2hiint(fabs(a1)), h2 = __double2hiint(fabs(a2));
+        if (h1 <= h2 + 1 || h2 < 0x01000000) {  // else |a1| is well above |a2|, and that above 1e-303
+            const double tiny = (1 + 100 * DBL_EPSILON) * (fabs(a2) + 1000 * DBL_MIN);
+            if (fabs(a1) <= tiny && fabs(b2) <= tiny) q.error_type = 3;
+        }
+    }
+    q.n++;
+    return q.n < limit && !q.error_type && more;
+}
+
 // QUADPACK QAG (Piessens et al. 1983) with the 61-point rule, run by one warp:
 // bisect the interval with the largest error estimate until the summed error is
 // below max(epsabs, epsrel |area|); QUADPACK's round-off and tiny-interval checks.
@@ -518,44 +555,30 @@ __device__ QagResult qag_warp(const F& f, const Gk61Nodes& N, QagList& L, double
     if (g[0].abserr <= round_off && g[0].abserr > tol) { R.ok = 0; return R; }
     if ((g[0].abserr <= tol && g[0].abserr != g[0].resasc) || g[0].abserr == 0.0) { R.ok = 1; return R; }
     if (limit == 1) { R.ok = 0; return R; }
-    double area = g[0].result, errsum = g[0].abserr;
-    int n = 1, roundoff1 = 0, roundoff2 = 0, error_type = 0;
+    QagSums q = {g[0].result, g[0].abserr, tol, 1, 0, 0, 0};
+    bool cont;
     do {
         // argmax of the error list (lowest index on ties)
-        const int bk = warp_argmax_err(L.e, n);
-        const int k = bk;
+        const int n = q.n, k = warp_argmax_err(L.e, n);
         const double a_i = L.a[k], b_i = L.b[k], r_i = L.r[k], e_i = L.e[k];
         const double a1 = a_i, b1 = 0.5 * (a_i + b_i), a2 = b1, b2 = b_i;
         aa[0] = a1; bb[0] = b1; aa[1] = a2; bb[1] = b2;
         gk61_warp(f, N, 2, aa, bb, g);
-        const double area12 = g[0].result + g[1].result, error12 = g[0].abserr + g[1].abserr;
-        errsum += error12 - e_i;
-        area += area12 - r_i;
-        if (g[0].resasc != g[0].abserr && g[1].resasc != g[1].abserr) {
-            if (fabs(r_i - area12) <= 1.0e-5 * fabs(area12) && error12 >= 0.99 * e_i) roundoff1++;
-            if (n >= 10 && error12 > e_i) roundoff2++;
-        }
-        tol = fmax(epsabs, epsrel * fabs(area));
-        if (errsum > tol) {
-            if (roundoff1 >= 6 || roundoff2 >= 20) error_type = 2;
-            const double tiny = (1 + 100 * DBL_EPSILON) * (fabs(a2) + 1000 * DBL_MIN);
-            if (fabs(a1) <= tiny && fabs(b2) <= tiny) error_type = 3;
-        }
+        cont = qag_account(q, g, r_i, e_i, a1, a2, b2, epsabs, epsrel, limit);
         __syncwarp();
         if (lane == 0) {
             L.b[k] = b1; L.r[k] = g[0].result; L.e[k] = g[0].abserr;
             L.a[n] = a2; L.b[n] = b2; L.r[n] = g[1].result; L.e[n] = g[1].abserr;
         }
         __syncwarp();
-        n++;
-    } while (n < limit && !error_type && errsum > tol);
+    } while (cont);
     double sum = 0;
     if (lane == 0)
-        for (int i = 0; i < n; i++) sum += L.r[i];
+        for (int i = 0; i < q.n; i++) sum += L.r[i];
     R.result = bcast0(sum);
-    R.abserr = errsum;
-    R.nint = n;
-    R.ok = errsum <= tol;
+    R.abserr = q.errsum;
+    R.nint = q.n;
+    R.ok = q.errsum <= q.tol;
     __syncwarp();
     return R;
 }
@@ -579,24 +602,27 @@ __device__ __forceinline__ int nc_child(int s, int right, int nslots) {
     return c < nslots ? c : -1;
 }
 
+// Centre and half-width of an interval.  A cached one's nodes need no centre, and its half-width
+// is in the table.
+template <class F>
+__device__ __forceinline__ void gk61_geometry(const F& f, int slot, double a, double b, double& c, double& h) {
+    c = 0.0;
+    if (slot >= 0) {
+        h = __ldg(f.nc.half + slot);
+    } else {
+        c = __dmul_rn(0.5, __dadd_rn(a, b));
+        h = __dmul_rn(0.5, __dsub_rn(b, a));
+    }
+}
+
 // gk61_warp with interval slots
 template <class F>
 __device__ __forceinline__ void gk61_warp_c(const F& f, const Gk61Nodes& N, int nint, const double* a,
                                             const double* b, const int* slot, GkOut* out) {
     const int lane = threadIdx.x & 31;
-    // the intervals' geometry on lane 0, broadcast (FP64 is issued per active lane)
-    double c[2] = {0.0, 0.0}, h[2] = {0.0, 0.0};
-    if (lane == 0) {
-        for (int t = 0; t < 2; t++) {
-            c[t] = __dmul_rn(0.5, __dadd_rn(a[t], b[t]));
-            h[t] = __dmul_rn(0.5, __dsub_rn(b[t], a[t]));
-        }
-    }
+    double c[2], h[2];
 #pragma unroll
-    for (int t = 0; t < 2; t++) {
-        c[t] = __shfl_sync(0xffffffffu, c[t], 0);
-        h[t] = __shfl_sync(0xffffffffu, h[t], 0);
-    }
+    for (int t = 0; t < 2; t++) gk61_geometry(f, slot[t], a[t], b[t], c[t], h[t]);
     double fv[4];
 #pragma unroll
     for (int t = 0; t < 2; t++)
@@ -628,11 +654,10 @@ __device__ QagResult qag_warp_c(const F& f, const Gk61Nodes& N, QagList& L, doub
     if (g[0].abserr <= round_off && g[0].abserr > tol) { R.ok = 0; return R; }
     if ((g[0].abserr <= tol && g[0].abserr != g[0].resasc) || g[0].abserr == 0.0) { R.ok = 1; return R; }
     if (limit == 1) { R.ok = 0; return R; }
-    double area = g[0].result, errsum = g[0].abserr;
-    int n = 1, roundoff1 = 0, roundoff2 = 0, error_type = 0, cont = 0;
+    QagSums q = {g[0].result, g[0].abserr, tol, 1, 0, 0, 0};
+    int n = 1, cont = 0;
     do {
-        const int bk = warp_argmax_err(L.e, n);
-        const int k = bk;
+        const int k = warp_argmax_err(L.e, n);
         const double a_i = L.a[k], b_i = L.b[k], r_i = L.r[k], e_i = L.e[k];
         const int s_i = L.slot[k];
         const double a1 = a_i, b1 = 0.5 * (a_i + b_i), a2 = b1, b2 = b_i;
@@ -644,22 +669,9 @@ __device__ QagResult qag_warp_c(const F& f, const Gk61Nodes& N, QagList& L, doub
         cont = 0;
         __syncwarp();
         if (lane == 0) {
-            const double area12 = g[0].result + g[1].result, error12 = g[0].abserr + g[1].abserr;
-            errsum += error12 - e_i;
-            area += area12 - r_i;
-            if (g[0].resasc != g[0].abserr && g[1].resasc != g[1].abserr) {
-                if (fabs(r_i - area12) <= 1.0e-5 * fabs(area12) && error12 >= 0.99 * e_i) roundoff1++;
-                if (n >= 10 && error12 > e_i) roundoff2++;
-            }
-            tol = fmax(epsabs, epsrel * fabs(area));
-            if (errsum > tol) {
-                if (roundoff1 >= 6 || roundoff2 >= 20) error_type = 2;
-                const double tiny = (1 + 100 * DBL_EPSILON) * (fabs(a2) + 1000 * DBL_MIN);
-                if (fabs(a1) <= tiny && fabs(b2) <= tiny) error_type = 3;
-            }
+            cont = qag_account(q, g, r_i, e_i, a1, a2, b2, epsabs, epsrel, limit);
             L.b[k] = b1; L.r[k] = g[0].result; L.e[k] = g[0].abserr; L.slot[k] = ss[0];
             L.a[n] = a2; L.b[n] = b2; L.r[n] = g[1].result; L.e[n] = g[1].abserr; L.slot[n] = ss[1];
-            cont = n + 1 < limit && !error_type && errsum > tol;
         }
         cont = __shfl_sync(0xffffffffu, cont, 0);
         __syncwarp();
@@ -669,9 +681,9 @@ __device__ QagResult qag_warp_c(const F& f, const Gk61Nodes& N, QagList& L, doub
     if (lane == 0)
         for (int i = 0; i < n; i++) sum += L.r[i];
     R.result = bcast0(sum);
-    R.abserr = bcast0(errsum);
+    R.abserr = bcast0(q.errsum);
     R.nint = n;
-    R.ok = __shfl_sync(0xffffffffu, (int)(errsum <= tol), 0);
+    R.ok = __shfl_sync(0xffffffffu, (int)(q.errsum <= q.tol), 0);
     __syncwarp();
     return R;
 }
@@ -695,10 +707,7 @@ __device__ __forceinline__ void gk61_block_c(const F& f, const Gk61Nodes& N, int
                                              const double* b, const int* slot, GkOut* out, QagBlockSmem& sh) {
     const int tid = threadIdx.x, lane = tid & 31;
     double c[2], h[2];
-    for (int t = 0; t < 2; t++) {
-        c[t] = __dmul_rn(0.5, __dadd_rn(a[t], b[t]));
-        h[t] = __dmul_rn(0.5, __dsub_rn(b[t], a[t]));
-    }
+    for (int t = 0; t < 2; t++) gk61_geometry(f, slot[t], a[t], b[t], c[t], h[t]);
     const int nslots = 61 * nint;
     for (int s = tid; s < nslots; s += blockDim.x) {
         const int t = s >= 61 ? 1 : 0;
@@ -742,8 +751,8 @@ __device__ QagResult qag_block_c(const F& f, const Gk61Nodes& N, QagList& L, dou
     if (g[0].abserr <= round_off && g[0].abserr > tol) { R.ok = 0; return R; }
     if ((g[0].abserr <= tol && g[0].abserr != g[0].resasc) || g[0].abserr == 0.0) { R.ok = 1; return R; }
     if (limit == 1) { R.ok = 0; return R; }
-    double area = g[0].result, errsum = g[0].abserr;
-    int n = 1, roundoff1 = 0, roundoff2 = 0, error_type = 0;
+    QagSums q = {g[0].result, g[0].abserr, tol, 1, 0, 0, 0};
+    int n = 1;
     do {
         // warp 0 finds the interval of largest error (lowest index on ties)
         if (tid < 32) {
@@ -761,24 +770,11 @@ __device__ QagResult qag_block_c(const F& f, const Gk61Nodes& N, QagList& L, dou
         gk61_block_c(f, N, 2, aa, bb, ss, g, sh);
         // QUADPACK's bookkeeping on thread 0
         if (tid == 0) {
-            const double area12 = g[0].result + g[1].result, error12 = g[0].abserr + g[1].abserr;
-            errsum += error12 - e_i;
-            area += area12 - r_i;
-            if (g[0].resasc != g[0].abserr && g[1].resasc != g[1].abserr) {
-                if (fabs(r_i - area12) <= 1.0e-5 * fabs(area12) && error12 >= 0.99 * e_i) roundoff1++;
-                if (n >= 10 && error12 > e_i) roundoff2++;
-            }
-            tol = fmax(epsabs, epsrel * fabs(area));
-            if (errsum > tol) {
-                if (roundoff1 >= 6 || roundoff2 >= 20) error_type = 2;
-                const double tiny = (1 + 100 * DBL_EPSILON) * (fabs(a2) + 1000 * DBL_MIN);
-                if (fabs(a1) <= tiny && fabs(b2) <= tiny) error_type = 3;
-            }
+            sh.cont = qag_account(q, g, r_i, e_i, a1, a2, b2, epsabs, epsrel, limit);
             L.b[k] = b1; L.r[k] = g[0].result; L.e[k] = g[0].abserr; L.slot[k] = ss[0];
             L.a[n] = a2; L.b[n] = b2; L.r[n] = g[1].result; L.e[n] = g[1].abserr; L.slot[n] = ss[1];
-            sh.cont = n + 1 < limit && !error_type && errsum > tol;
-            sh.errsum = errsum;
-            sh.ok = errsum <= tol;
+            sh.errsum = q.errsum;
+            sh.ok = q.errsum <= q.tol;
         }
         __syncthreads();
         n++;
@@ -816,12 +812,12 @@ struct QagSpecSmem {
     double errsum;
 };
 
-// The geometry of interval q of the next evaluation, formed once (one thread) as every
-// GK61 call forms it: c = (a + b) / 2, h = (b - a) / 2.
+// Interval q of the next evaluation: its slot, or its geometry, formed once (one thread).
 __device__ __forceinline__ void spec_set_interval(QagSpecSmem& sh, int q, double a, double b, int slot) {
+    sh.isl[q] = slot;
+    if (slot >= 0) return;
     sh.ic[q] = __dmul_rn(0.5, __dadd_rn(a, b));
     sh.ih[q] = __dmul_rn(0.5, __dsub_rn(b, a));
-    sh.isl[q] = slot;
 }
 
 // Rule results of two groups of intervals, nA in {1, 2} (intervals 0, 1) and nB in
@@ -850,7 +846,12 @@ __device__ __forceinline__ void gk61_block_groups(const F& f, const Gk61Nodes& N
             const int j = lane + 32 * (m & 1), t = m >> 1;
             fv[m] = t < ng && j < 61 ? fvg[61 * t + j] : 0.0;
         }
-        const double hh[2] = {sh.ih[2 * warp], sh.ih[2 * warp + 1]};
+        double hh[2];
+#pragma unroll
+        for (int t = 0; t < 2; t++) {
+            const int q = 2 * warp + t, slot = t < ng ? sh.isl[q] : -1;
+            hh[t] = slot >= 0 ? __ldg(f.nc.half + slot) : sh.ih[q];
+        }
         GkOut o[2];
         gk61_lane_sums(N, fv, ng, hh, o);
         if (lane == 0) {
@@ -890,8 +891,8 @@ __device__ QagResult qag_block_spec_c(const F& f, const Gk61Nodes& N, QagList& L
     if (g0.abserr <= round_off && g0.abserr > tol) { R.ok = 0; return R; }
     if ((g0.abserr <= tol && g0.abserr != g0.resasc) || g0.abserr == 0.0) { R.ok = 1; return R; }
     if (limit == 1) { R.ok = 0; return R; }
-    double area = g0.result, errsum = g0.abserr;
-    int n = 1, roundoff1 = 0, roundoff2 = 0, error_type = 0;
+    QagSums q = {g0.result, g0.abserr, tol, 1, 0, 0, 0};
+    int n = 1;
     do {
         // warp 0 finds the interval of largest error (lowest index on ties); its lane 0
         // notes whether the halves are already evaluated and, if not, lays out the halves
@@ -925,19 +926,7 @@ __device__ QagResult qag_block_spec_c(const F& f, const Gk61Nodes& N, QagList& L
             const int s_i = L.slot[k];
             const double a1 = a_i, b1 = 0.5 * (a_i + b_i), a2 = b1, b2 = b_i;
             const GkOut g[2] = {hit ? sh.pg[0] : sh.out[0], hit ? sh.pg[1] : sh.out[1]};
-            const double area12 = g[0].result + g[1].result, error12 = g[0].abserr + g[1].abserr;
-            errsum += error12 - e_i;
-            area += area12 - r_i;
-            if (g[0].resasc != g[0].abserr && g[1].resasc != g[1].abserr) {
-                if (fabs(r_i - area12) <= 1.0e-5 * fabs(area12) && error12 >= 0.99 * e_i) roundoff1++;
-                if (n >= 10 && error12 > e_i) roundoff2++;
-            }
-            tol = fmax(epsabs, epsrel * fabs(area));
-            if (errsum > tol) {
-                if (roundoff1 >= 6 || roundoff2 >= 20) error_type = 2;
-                const double tiny = (1 + 100 * DBL_EPSILON) * (fabs(a2) + 1000 * DBL_MIN);
-                if (fabs(a1) <= tiny && fabs(b2) <= tiny) error_type = 3;
-            }
+            sh.cont = qag_account(q, g, r_i, e_i, a1, a2, b2, epsabs, epsrel, limit);
             L.b[k] = b1; L.r[k] = g[0].result; L.e[k] = g[0].abserr; L.slot[k] = nc_child(s_i, 0, ns);
             L.a[n] = a2; L.b[n] = b2; L.r[n] = g[1].result; L.e[n] = g[1].abserr; L.slot[n] = nc_child(s_i, 1, ns);
             if (hit) {
@@ -947,9 +936,8 @@ __device__ QagResult qag_block_spec_c(const F& f, const Gk61Nodes& N, QagList& L
                 sh.pg[0] = sh.out[2];
                 sh.pg[1] = sh.out[3];
             }
-            sh.cont = n + 1 < limit && !error_type && errsum > tol;
-            sh.errsum = errsum;
-            sh.ok = errsum <= tol;
+            sh.errsum = q.errsum;
+            sh.ok = q.errsum <= q.tol;
         }
         __syncthreads();
         n++;
@@ -1090,12 +1078,14 @@ __device__ __forceinline__ NodeWeights node_weights(double g, double dx, double 
     w.d = __dmul_rn(e, __fma_rn(dx, s, -h));
     return w;
 }
-// Node table entry: {g A, g B}, {g C, g D}, fslength, {j, fslength as a float}.
+// Node table entry: {g A, g B}, {g C, g D}, fslength, {j, fslength as a float}; a slot's 61
+// entries share a half-width.
 struct NodeTable {
     const double2* ab;
     const double2* cd;
     const double* fsl;
     const int2* jf;
+    const double* half;  // half-width of a slot's interval
     int nslots;
 };
 struct DnuIntegrandW {

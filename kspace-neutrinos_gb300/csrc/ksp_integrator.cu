@@ -316,7 +316,8 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, 
     b -= kNuSpecies * P.hyb_blocks;
     const int q = b * kPrepThreads + t;
     if (q >= P.nodes) return;
-    I.nc_inv[q] = node_inv_aH(I.B, nc_node_x(q, P.loga0, P.loga));
+    double half;
+    I.nc_inv[q] = node_inv_aH(I.B, nc_node_x(q, P.loga0, P.loga, &half));
 }
 
 // The fslength table, the node table, and the row splines.
@@ -391,11 +392,12 @@ __global__ void __launch_bounds__(kTableThreads, 8)
     }
     const int q = (b - table_blocks) * kTableThreads + t;
     if (q >= P.nodes) return;
-    const double x = nc_node_x(q, P.loga0, P.loga);
+    double half;
+    const double x = nc_node_x(q, P.loga0, P.loga, &half);
     const double fsl = fs_table_at(F, P.loga0, P.loga, x);
     const double* kx = I.scalefact;
     const int j = seg_bsearch(kx, Na, x);
-    nc_store(I, q, fsl, I.nc_inv[q], x - kx[j], j, kx[j + 1] - kx[j], Na);
+    nc_store(I, q, fsl, I.nc_inv[q], x - kx[j], j, kx[j + 1] - kx[j], Na, half);
 }
 
 // block per bin: this bin's delta_cdm (a deferred normalisation), the provisional row

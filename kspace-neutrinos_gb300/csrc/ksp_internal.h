@@ -54,6 +54,7 @@ struct IntegratorDev {
     double2* nc_ab;                  // [kNcNodes] the same as weights of the row (NodeTable)
     double2* nc_cd;
     int2* nc_jf;
+    double* nc_half;                 // [kNcMaxSlots]
     const double* jt;                // J's fine table (one per device)
     double* hyb;                     // optional: [kNuSpecies][kHybTable] the tables of J with a cut
     int nc_slots;                    // slots of the node table in use (1 + 2 levels, 0 = none)
@@ -260,7 +261,7 @@ __device__ __forceinline__ DnuIntegrandW dnu_integrand_w(const IntegratorDev& I,
     f.qc = S.qc[mi]; f.nfl = I.B->nufrac_low[0];
     f.hyb = I.hyb ? I.hyb + (size_t)mi * kHybTable : nullptr;
     f.ky = row; f.kc = rc;
-    f.nc = NodeTable{I.nc_ab, I.nc_cd, I.nc_fsl, I.nc_jf, I.nc_slots};
+    f.nc = NodeTable{I.nc_ab, I.nc_cd, I.nc_fsl, I.nc_jf, I.nc_half, I.nc_slots};
     f.fs_x = I.fs_x; f.fs_y = I.fs_y; f.fs_c = I.fs_c; f.kx = I.scalefact;
     f.S = &S; f.na = Na;
     return f;
@@ -270,9 +271,10 @@ __device__ __noinline__ inline double DnuIntegrandW::slow(double x) const {
     const NodeTerms t = dnu_node_terms(B, fs_x, fs_y, fs_c, S->Nfs, S->loga0, (S->Nfs - 1.) / (S->loga - S->loga0), kx, na, x);
     return value(node_weights(t.g, t.dx, kx[t.j + 1] - kx[t.j], na), t.fsl, (float)t.fsl, t.j);
 }
-// Node q of the node table.
+// Node q of the node table, in an interval of half-width `half`.
 __device__ __forceinline__ void nc_store(const IntegratorDev& I, int q, double fsl, double inv_aH, double dx, int j,
-                                         double h, int Na) {
+                                         double h, int Na, double half) {
+    if (q % 61 == 0) I.nc_half[q / 61] = half;
     const double g = fsl * inv_aH;
     const NodeWeights w = node_weights(g, dx, h, Na);
     I.nc_g[q] = g;

@@ -9,7 +9,7 @@
 //                   knot factorisation of the history spline
 //   kb_fs_eval      a block per stretch of an instance's fslength segments
 //   kb_tables       the fslength tables and the node tables of the integrand
-//   kb_dtot_coeffs  thread per (instance, bin): history-row spline coefficients
+//   kb_dtot_coeffs  warp per 32 bins of an instance: history-row spline coefficients
 //   kb_dnu_qag      persistent warps that pull (instance, species, bin) tasks from an
 //                   atomic queue; knots, row and coefficients staged into shared memory
 //                   by TMA bulk copies; QAG with the 61-point Gauss-Kronrod rule
@@ -131,40 +131,130 @@ __global__ void __launch_bounds__(kBatchTable) kb_tables(BatchDev b) {
 }
 
 // ------------------------------------------------------------------ history splines
-// thread per (instance, bin): the same substitutions as k_dtot_coeffs, each thread
-// sweeping its own row in global memory.  With a million rows in flight the latency of
-// the strided loads is hidden by parallelism, which a warp-per-row solve (one active
-// lane per row) cannot match at this size.
-__global__ void kb_dtot_coeffs(BatchDev b) {
-    const int total = b.hdr->total_bins;
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-        const int i = owner_of(b.bin_off, b.M, g);
-        const int ik = g - __ldg(b.bin_off + i);
+// A warp per 32 rows of one instance, a lane per row, 32 knots at a time: the rows' next 32
+// values are on their way to shared memory (lane = knot: whole lines) while the lanes step
+// through the present ones.  With g_k = r_k / diag_k the forward step is
+//   g_k = A_k (y_{k+2} - y_{k+1}) + B_k (y_{k+1} - y_k) + W_k g_{k-1}
+// and the backward one c_k = g_k + V_k c_{k+1}, the factors of a knot formed by one lane for
+// all rows: five FP64 operations per knot and row, which is the bound (a row by the warp's
+// scans costs twice that, a thread per row with its row in global memory waits for every
+// knot: 24 members, 446 us, now 197; 256 members, 687 us, now 374).
+constexpr int kRowTile = 32, kRowPitch = kRowTile + 1, kRowWarps = 4;
+struct RowSmem {
+    double y[2][32 * kRowPitch];  // [row][knot of the tile], a pitch free of bank conflicts
+    double2 ab[kRowTile], wv[kRowTile];
+};
+__device__ __forceinline__ void cp_async8(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(ptx::smem_u32(dst)), "l"(src) : "memory");
+}
+__global__ void __launch_bounds__(32 * kRowWarps) kb_dtot_coeffs(BatchDev b) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    RowSmem& sh = reinterpret_cast<RowSmem*>(sm)[warp];
+    const int total = b.hdr->total_rows;
+    for (int g = blockIdx.x * kRowWarps + warp; g < total; g += gridDim.x * kRowWarps) {
+        const int i = owner_of(b.row_off, b.M, g);
         const BatchCall& P = b.calls[i];
-        const int Na = P.Na;
-        if (!P.active || P.commit_row == -2 || Na <= 2) continue;
         const IntegratorDev& I = b.insts[i];
-        const double* y = I.dtot + (size_t)ik * I.ld;
-        double* c = I.coef + (size_t)ik * I.ld;
-        const double* ih = I.knot_invh;
-        const int m = Na - 2;
-        double prev = 0;
-        for (int k = 0; k < m; k++) {
-            double r = 3.0 * ((y[k + 2] - y[k + 1]) * ih[k + 1] - (y[k + 1] - y[k]) * ih[k]);
-            if (k > 0) r -= I.knot_fac[k] * prev;
-            prev = r;
-            c[k + 1] = r;
+        const int Na = P.Na, m = Na - 2, nt = (m + kRowTile - 1) / kRowTile;  // Na > 2
+        const int r0 = 32 * (g - __ldg(b.row_off + i)), nr = min(32, P.nk - r0);
+        const double* y = I.dtot + (size_t)r0 * I.ld;
+        double* c = I.coef + (size_t)r0 * I.ld;
+        const int my = min(lane, nr - 1);
+        // knots k0 + 2 .. k0 + 33 of the rows (the unknowns k0 + 1 .. k0 + 32 with them)
+        auto fetch = [&](int t, const double* src, int first, int buf) {
+            const int k = kRowTile * t + lane;
+            if (k < m)
+                for (int r = 0; r < nr; r++)
+                    cp_async8(&sh.y[buf][r * kRowPitch + lane], src + (size_t)r * I.ld + first + k);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        auto arrived = [&](bool later) {
+            if (later) asm volatile("cp.async.wait_group 1;" ::: "memory");
+            else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        };
+        // the factors of unknown k (of a tile, by its lane; zero past the last)
+        auto factors = [&](int t) {
+            const int k = kRowTile * t + lane;
+            double2 ab = make_double2(0.0, 0.0), wv = ab;
+            if (k < m) {
+                const double inv = I.knot_invdiag[k], i3 = 3.0 * inv;
+                const double h0 = I.scalefact[k + 1] - I.scalefact[k], h1 = I.scalefact[k + 2] - I.scalefact[k + 1];
+                ab = make_double2(i3 * I.knot_invh[k + 1], -i3 * I.knot_invh[k]);
+                wv = make_double2(-h0 * inv, -h1 * inv);
+            }
+            sh.ab[lane] = ab;
+            sh.wv[lane] = wv;
+        };
+        auto store = [&](int t, int buf) {
+            const int k = kRowTile * t + lane;
+            if (k < m)
+                for (int r = 0; r < nr; r++) c[(size_t)r * I.ld + 1 + k] = sh.y[buf][r * kRowPitch + lane];
+            __threadfence_block();  // read back by an asynchronous copy
+        };
+        __syncwarp();  // the previous group's reads
+        fetch(0, y, 2, 0);
+        const double* yr = y + (size_t)my * I.ld;
+        double y1 = yr[1], d0 = y1 - yr[0], gp = 0.0;
+        for (int t = 0; t < nt; t++) {
+            const int buf = t & 1, n = min(kRowTile, m - kRowTile * t);
+            if (t + 1 < nt) fetch(t + 1, y, 2, buf ^ 1);
+            factors(t);
+            arrived(t + 1 < nt);
+            __syncwarp();
+            double* q = sh.y[buf] + my * kRowPitch;
+            if (lane < nr) {
+                for (int k = 0; k < n; k += 4) {
+                    double2 ab[4];
+                    double w[4], y2[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        ab[u] = sh.ab[k + u];
+                        w[u] = sh.wv[k + u].x;
+                        y2[u] = q[k + u];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const double d1 = y2[u] - y1;
+                        gp = fma(w[u], gp, fma(ab[u].x, d1, ab[u].y * d0));
+                        q[k + u] = k + u < n ? gp : 0.0;
+                        y1 = y2[u];
+                        d0 = d1;
+                    }
+                }
+            }
+            __syncwarp();
+            if (t + 1 < nt) store(t, buf);  // the last one stays
+            __syncwarp();
         }
-        c[0] = 0.0;
-        c[Na - 1] = 0.0;
-        double next = c[m] * I.knot_invdiag[m - 1];
-        c[m] = next;
-        const double* x = I.scalefact;
-        for (int k = m - 1; k-- > 0;) {
-            const double off = x[k + 2] - x[k + 1];
-            next = (c[k + 1] - off * next) * I.knot_invdiag[k];
-            c[k + 1] = next;
+        double next = 0.0;
+        for (int t = nt - 1; t >= 0; t--) {
+            const int buf = t & 1, n = min(kRowTile, m - kRowTile * t);
+            if (t > 0) fetch(t - 1, c, 1, buf ^ 1);
+            if (t < nt - 1) factors(t);
+            arrived(t > 0);
+            __syncwarp();
+            double* q = sh.y[buf] + my * kRowPitch;
+            if (lane < nr) {
+                for (int k = (n - 1) & ~3; k >= 0; k -= 4) {
+                    double v[4], gk[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        v[u] = sh.wv[k + u].y;
+                        gk[u] = q[k + u];
+                    }
+#pragma unroll
+                    for (int u = 3; u >= 0; u--) {
+                        next = fma(v[u], next, gk[u]);
+                        q[k + u] = next;
+                    }
+                }
+            }
+            __syncwarp();
+            store(t, buf);
+            __syncwarp();
         }
+        if (lane < nr) c[(size_t)lane * I.ld] = c[(size_t)lane * I.ld + Na - 1] = 0.0;
     }
 }
 
@@ -321,6 +411,7 @@ static void gl_nodes_b(int n, double* X, double* Wt) {  // Newton on P_n, positi
 
 void batch_set_attributes() {
     raise_dynamic_smem_limit(reinterpret_cast<const void*>(kb_dnu_qag));
+    raise_dynamic_smem_limit(reinterpret_cast<const void*>(kb_dtot_coeffs));
 }
 
 void launch_batch_update(const BatchDev& b, cudaStream_t st) {
@@ -334,7 +425,7 @@ void launch_batch_update(const BatchDev& b, cudaStream_t st) {
     kb_prologue<<<b.M < nb ? b.M : nb, 128, 0, st>>>(b);
     kb_fs_eval<<<4 * nb, kPrepThreads, 0, st>>>(b, gl);
     kb_tables<<<2 * nb, kBatchTable, 0, st>>>(b);
-    kb_dtot_coeffs<<<nb, 128, 0, st>>>(b);
+    kb_dtot_coeffs<<<nb, 32 * kRowWarps, kRowWarps * sizeof(RowSmem), st>>>(b);
     kb_dnu_qag<<<b.qag_blocks, 32 * b.wpb, batch_qag_smem(b.ldmax, b.wpb), st>>>(b);
     kb_finish<<<nb, 256, 0, st>>>(b);
 }

@@ -30,9 +30,10 @@ struct BatchHeader {
     int total_segs;   // blocks of fslength segments (fs_blocks of each instance)
     int total_fsc;    // blocks of fslength-table and node-table entries (kBatchTable each)
     int total_bins;   // sum of nk
+    int total_rows;   // groups of 32 history rows of one instance
     int total_tasks;  // sum of nspec*nk over integrating instances
     int counter;      // task queue of kb_dnu_qag (reset by kb_prologue)
-    int pad[2];
+    int pad;
 };
 
 // Device arrays of the batch (offsets have M+1 entries).
@@ -42,6 +43,7 @@ struct BatchDev {
     BatchHeader* hdr;
     const int* fs_off;
     const int* fsc_off;
+    const int* row_off;
     const int* bin_off;
     const int* task_off;
     double* dnu_pool;   // [total_bins] delta_nu returned by every instance

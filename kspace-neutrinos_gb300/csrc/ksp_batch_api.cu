@@ -39,7 +39,7 @@ struct kspace_batch {
     // device
     IntegratorDev* insts_d = nullptr;
     BatchHeader* hdr_d = nullptr;
-    unsigned char* upload_d = nullptr;  // calls | fs_off | fsc_off | bin_off | task_off | header
+    unsigned char* upload_d = nullptr;  // calls | fs_off | fsc_off | row_off | bin_off | task_off | header
     unsigned char* upload_h = nullptr;  // pinned mirror
     size_t upload_bytes = 0;
     double* dcdm_pool = nullptr;
@@ -154,7 +154,7 @@ extern "C" int kspace_gpu_batch_bind_grid(kspace_batch* b, int inst, void* grid,
 
 // Per-call upload layout (one pinned buffer, one copy).
 struct UploadPlan {
-    size_t calls, fs_off, fsc_off, bin_off, task_off, hdr, total;
+    size_t calls, fs_off, fsc_off, row_off, bin_off, task_off, hdr, total;
 };
 static UploadPlan plan_upload(int M) {
     UploadPlan p;
@@ -167,6 +167,7 @@ static UploadPlan plan_upload(int M) {
     p.calls = take(sizeof(BatchCall) * M);
     p.fs_off = take(sizeof(int) * (M + 1));
     p.fsc_off = take(sizeof(int) * (M + 1));
+    p.row_off = take(sizeof(int) * (M + 1));
     p.bin_off = take(sizeof(int) * (M + 1));
     p.task_off = take(sizeof(int) * (M + 1));
     p.hdr = take(sizeof(BatchHeader));
@@ -182,6 +183,7 @@ static BatchDev dev_view(kspace_batch* b) {
     d.hdr = reinterpret_cast<BatchHeader*>(b->upload_d + p.hdr);
     d.fs_off = reinterpret_cast<const int*>(b->upload_d + p.fs_off);
     d.fsc_off = reinterpret_cast<const int*>(b->upload_d + p.fsc_off);
+    d.row_off = reinterpret_cast<const int*>(b->upload_d + p.row_off);
     d.bin_off = reinterpret_cast<const int*>(b->upload_d + p.bin_off);
     d.task_off = reinterpret_cast<const int*>(b->upload_d + p.task_off);
     d.dnu_pool = b->dnu_pool;
@@ -362,11 +364,12 @@ static int plan_call(kspace_batch* b, const double* a, bool dry, std::vector<int
     BatchCall* calls = reinterpret_cast<BatchCall*>(b->upload_h + p.calls);
     int* fs_off = reinterpret_cast<int*>(b->upload_h + p.fs_off);
     int* fsc_off = reinterpret_cast<int*>(b->upload_h + p.fsc_off);
+    int* row_off = reinterpret_cast<int*>(b->upload_h + p.row_off);
     int* bin_off = reinterpret_cast<int*>(b->upload_h + p.bin_off);
     int* task_off = reinterpret_cast<int*>(b->upload_h + p.task_off);
     BatchHeader* hdr = reinterpret_cast<BatchHeader*>(b->upload_h + p.hdr);
     after.assign(M, 0);
-    fs_off[0] = fsc_off[0] = bin_off[0] = task_off[0] = 0;
+    fs_off[0] = fsc_off[0] = row_off[0] = bin_off[0] = task_off[0] = 0;
     for (int i = 0; i < M; i++) {
         kspace_ctx* c = b->ctx[i];
         BatchCall& P = calls[i];
@@ -410,6 +413,7 @@ static int plan_call(kspace_batch* b, const double* a, bool dry, std::vector<int
         if (integ && P.nfs > 0)
             fsc_off[i + 1] += (P.nfs + kBatchTable - 1) / kBatchTable +
                               (P.Na > 1 ? (b->nc_slots * 61 + kBatchTable - 1) / kBatchTable : 0);
+        row_off[i + 1] = row_off[i] + (integ && P.Na > 2 ? (P.nk + 31) / 32 : 0);
         bin_off[i + 1] = b->off[i + 1];
         task_off[i + 1] = task_off[i] + (integ ? P.nspec * P.nk : 0);
     }
@@ -417,6 +421,7 @@ static int plan_call(kspace_batch* b, const double* a, bool dry, std::vector<int
     hdr->M = M;
     hdr->total_segs = fs_off[M];
     hdr->total_fsc = fsc_off[M];
+    hdr->total_rows = row_off[M];
     hdr->total_bins = bin_off[M];
     hdr->total_tasks = task_off[M];
     return KSPACE_OK;

@@ -306,45 +306,6 @@ struct DnuAdjArgs {
     int recompute;
 };
 
-// Node quantities of the delta_nu integrand for one bin (delta_tot_table.c:492-500).
-struct DnuNode {
-    double g, J, Jd, S, xj;
-    int seg;
-    double dx, h;
-};
-
-__device__ __forceinline__ DnuNode dnu_node(const Background* B, double k, double mnubykT, double qc, double nfl,
-                                            const double* fs_x, const double* fs_y, const double* fs_c, int nfs,
-                                            double fs_x0, double fs_inv, const double* kx, const double* ky,
-                                            const double* kc, int na, double logai) {
-    DnuNode o;
-    int i = (int)((logai - fs_x0) * fs_inv);
-    i = i < 0 ? 0 : (i > nfs - 2 ? nfs - 2 : i);
-    while (i > 0 && logai < __ldg(fs_x + i)) i--;
-    while (i < nfs - 2 && logai >= __ldg(fs_x + i + 1)) i++;
-    double fsl;
-    {
-        const double x0 = __ldg(fs_x + i), x1 = __ldg(fs_x + i + 1);
-        const double y0 = __ldg(fs_y + i), y1 = __ldg(fs_y + i + 1);
-        const double c0 = __ldg(fs_c + i), c1 = __ldg(fs_c + i + 1);
-        const double h = x1 - x0, dx = logai - x0;
-        const double b = (y1 - y0) / h - h * (c1 + 2.0 * c0) / 3.0;
-        const double d = (c1 - c0) / (3.0 * h);
-        fsl = y0 + dx * (b + dx * (c0 + dx * d));
-    }
-    const int j = seg_bsearch(kx, na, logai);
-    o.seg = j;
-    o.h = kx[j + 1] - kx[j];
-    o.dx = logai - kx[j];
-    o.S = na > 2 ? cspline_seg(kx, ky, kc, j, logai) : linear_seg(kx, ky, j, logai);
-    o.xj = k * fsl / mnubykT;
-    o.J = specialJ(o.xj, qc, nfl);
-    o.Jd = qc > 0 ? 0.0 : specialJ_fit_deriv(o.xj);
-    const double ai = exp(logai);
-    o.g = fsl / (ai * hubble(*B, ai));
-    return o;
-}
-
 // The 61 nodes of one interval [a_i, b_i] of the final subdivision, by one warp (lane
 // order = ascending x): each node's weight w g J times the spline weights of its
 // history segment goes to ybar / cbar (cotangents of the delta_tot row values and of

@@ -354,6 +354,7 @@ extern "C" int kspace_gpu_set_hubble(kspace_ctx* c, double Omega0, double OmegaL
     B.OmegaLambda = OmegaLambda;
     B.OmegaK = 1.0 - Omega0 - OmegaLambda;
     B.hubble = kHubble * UnitTime_in_s;
+    B.ihubble = 1.0 / B.hubble;
     B.radiation = radiation;
     upload_background(c);
     CK(cudaStreamSynchronize(c->stream));
@@ -483,7 +484,6 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
         take(&I.nc_jf, kNcNodes);
         take(&I.nc_half, kNcMaxSlots);
         take(&I.nc_inv, kNcNodes);
-        take(&I.fs_x, fs);
         take(&I.fs_y, fs);
         take(&I.fs_c, fs);
         take(&I.fs_seg, fs);

@@ -70,7 +70,7 @@ __global__ void kb_prologue(BatchDev b) {
         auto knot = [&](int j) { return xk[j]; };
         for (int r = (P.start_row < 0 ? 0 : P.start_row) + threadIdx.x; r < Na - 2; r += blockDim.x)
             knot_row(knot, r, I.knot_invdiag, I.knot_fac);
-        if (threadIdx.x == 0 && P.nfs == 0) {
+        if (threadIdx.x == 0 && P.fs.n == 0) {
             S.fsl_A0a = 0.0;
             S.Nfs = 0;
         }
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(kPrepThreads) kb_fs_eval(BatchDev b, GL4b gl) 
         const BatchCall& P = b.calls[i];
         const IntegratorDev& I = b.insts[i];
         __syncthreads();  // the previous stretch's shared arrays
-        fs_eval_block(*I.B, P.nfs, P.loga0, P.loga, g - __ldg(b.fs_off + i), gl.x[0], gl.x[1], gl.w[0], gl.w[1], f, sg,
+        fs_eval_block(*I.B, P.fs, P.loga, g - __ldg(b.fs_off + i), gl.x[0], gl.x[1], gl.w[0], gl.w[1], f, sg,
                       I.fs_seg, I.fs_suf, I.fs_tot);
     }
 }
@@ -105,28 +105,20 @@ __global__ void __launch_bounds__(kBatchTable) kb_tables(BatchDev b) {
         const IntegratorDev& I = b.insts[i];
         int blk = g - __ldg(b.fsc_off + i);
         __syncthreads();  // the previous table's sums
-        const FsTable F = fs_table(I, P.nfs, P.loga0, P.loga, I.sc->light, tsuf);
-        const int table_blocks = (P.nfs + kBatchTable - 1) / kBatchTable;
+        const FsTable F = fs_table(I, P.fs, I.sc->light, tsuf);
+        const int table_blocks = fs_table_blocks(P.fs.n, kBatchTable);
         if (blk < table_blocks) {
-            const int n = blk * kBatchTable + threadIdx.x;
-            if (n >= P.nfs) continue;
-            I.fs_x[n] = fs_node(n, P.nfs, P.loga0, P.loga);
-            const double y = fs_table_y(F, n);
-            I.fs_y[n] = y;
-            I.fs_c[n] = fs_table_c(F, n);
-            if (n == 0) {
-                I.sc->fsl_A0a = y;
-                I.sc->Nfs = P.nfs;
-            }
+            fs_table_store(I, F, blk * kBatchTable + threadIdx.x);
             continue;
         }
         const int q = (blk - table_blocks) * kBatchTable + threadIdx.x;
         if (q >= b.nc_slots * 61) continue;
         double half;
         const double x = nc_node_x(q, P.loga0, P.loga, &half);
-        const double fsl = fs_table_at(F, P.loga0, P.loga, x);
+        const double fsl = fs_table_at(F, x);
         const int j = seg_bsearch(I.scalefact, P.Na, x);
-        nc_store(I, q, fsl, node_inv_aH(I.B, x), x - I.scalefact[j], j, I.scalefact[j + 1] - I.scalefact[j], P.Na, half);
+        nc_store(I, q, fsl, node_inv_aH(I.B, x), x - I.scalefact[j], j, I.scalefact[j + 1] - I.scalefact[j],
+                 I.knot_invh[j], P.Na, half);
     }
 }
 

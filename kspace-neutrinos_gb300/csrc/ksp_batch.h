@@ -12,7 +12,7 @@ struct BatchCall {
     double a, loga, loga0, TimeTransfer;
     int Na;          // history rows used by this call (the provisional row included)
     int nk;          // bins of the instance
-    int nfs;         // fslength table nodes (16*Na, 0 when log a <= log a0)
+    FsGrid fs;       // fslength table (16*Na nodes, 0 when log a <= log a0)
     int start_row;   // leading rows of the knot factorisation still valid
     int commit_row;  // >= 0 keep that row, -1 drop the provisional row, -2 same scale factor
     int active;      // 0: instance not advanced in this call

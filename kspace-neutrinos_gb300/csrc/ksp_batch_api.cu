@@ -401,17 +401,17 @@ static int plan_call(kspace_batch* b, const double* a, bool dry, std::vector<int
                 const int Na = c->ia + 1;
                 P.Na = Na;
                 P.start_row = c->fact_valid;
-                P.nfs = loga > c->loga0 ? 16 * Na : 0;
+                P.fs = fs_grid(loga > c->loga0 ? 16 * Na : 0, c->loga0, loga);
                 const bool commit = a[i] >= exp(c->h_scalefact[Na - 2]) + 0.009;  // :229-237
                 P.commit_row = commit ? Na - 1 : -1;
                 after[i] = dry ? 0 : (commit ? 1 : 2);
             }
         }
         const bool integ = P.active && P.commit_row != -2;
-        fs_off[i + 1] = fs_off[i] + (integ && P.nfs > 0 ? fs_blocks(P.nfs, P.loga0, P.loga) : 0);
+        fs_off[i + 1] = fs_off[i] + (integ && P.fs.n > 0 ? fs_blocks(P.fs) : 0);
         fsc_off[i + 1] = fsc_off[i];
-        if (integ && P.nfs > 0)
-            fsc_off[i + 1] += (P.nfs + kBatchTable - 1) / kBatchTable +
+        if (integ && P.fs.n > 0)
+            fsc_off[i + 1] += fs_table_blocks(P.fs.n, kBatchTable) +
                               (P.Na > 1 ? (b->nc_slots * 61 + kBatchTable - 1) / kBatchTable : 0);
         row_off[i + 1] = row_off[i] + (integ && P.Na > 2 ? (P.nk + 31) / 32 : 0);
         bin_off[i + 1] = b->off[i + 1];

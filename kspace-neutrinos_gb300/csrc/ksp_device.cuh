@@ -58,7 +58,7 @@ struct RhoTable {
 // hubble_function (delta_tot_table_test.c:33-45; curvature as gadget-2/0003 patch:38).
 struct Background {
     double rhocrit, kBtnu, tcmb0, conv, omegag0;
-    double irhocrit;  // 1 / rhocrit
+    double irhocrit, ihubble;  // 1 / rhocrit, 1 / hubble
     int deg[kNuSpecies];
     double mnu[kNuSpecies];
     double mnu_J[kNuSpecies];  // mass inside J's argument (get_delta_nu's mnu, delta_tot_table.c:507)
@@ -78,12 +78,26 @@ struct Background {
 };
 
 // ------------------------------------------------------------------ splines
+#ifdef __CUDACC__
+// Integers in the order of the doubles: an FP64 comparison takes the FP64 pipe's 16 cycles.
+__device__ __forceinline__ long long order_key(double v) {
+    const long long b = __double_as_longlong(v);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+#endif
 // Segment i with x[i] <= v < x[i+1] (v == x[n-1] -> n-2), as GSL's bsearch.
 KSP_HD int seg_bsearch(const double* x, int n, double v) {
     int lo = 0, hi = n - 1;
+#ifdef __CUDA_ARCH__
+    const long long k = order_key(v);
+#endif
     while (hi > lo + 1) {
         const int mid = (lo + hi) >> 1;
+#ifdef __CUDA_ARCH__
+        if (order_key(x[mid]) > k) hi = mid; else lo = mid;
+#else
         if (x[mid] > v) hi = mid; else lo = mid;
+#endif
     }
     return lo;
 }
@@ -204,52 +218,52 @@ KSP_HD double hubble(const Background& B, double a, double loga = NAN) {
 }
 
 #ifdef __CUDACC__
-// rho_nu for fsl_integrand: the same branches as rho_nu, with 1/a given and the table
-// spline in per-segment polynomial form (RhoTable::sb, sd).
-__device__ __forceinline__ double rho_nu_ia(const RhoTable& T, double a, double ia, double loga, double kT,
-                                            double conv) {
-    const double amnu = a * T.mnu;
-    const double kTamnu = kT * ia * T.imnu, kTamnu2 = kTamnu * kTamnu;
-    bool nonrel = kNuSw * kNuSw * kTamnu2 < 1;
-    bool rel = !nonrel && amnu < 1e-6 * kT;
+// rho_nu for fsl_integrand: the same branches as rho_nu, of kT / (a m), with 1/a given and the
+// table spline in per-segment polynomial form (RhoTable::sb, sd).
+__device__ __forceinline__ double rho_nu_ia(const RhoTable& T, double ia, double loga, double kT, double conv) {
+    const double kTamnu = kT * ia * T.imnu;
+    bool nonrel = kNuSw * kTamnu < 1;
+    bool rel = !nonrel && kTamnu > 1e6;
     if (!nonrel && !rel && (!T.has_table || loga < T.loga[0])) {
-        rel = amnu < 1e-4 * kT;
+        rel = kTamnu > 1e4;
         nonrel = !rel;
     }
     if (nonrel) {
-        const double ia4 = (ia * ia) * (ia * ia);
-        return amnu * (kT * kT * kT) * ia4 *
-               (1.5 * kZeta3 + kTamnu2 * 45. / 4. * 1.0369277551433704 +
-                2835. / 32. * kTamnu2 * kTamnu2 * 1.0083492773819229 +
-                80325 / 32. * kTamnu2 * kTamnu2 * kTamnu2 * 1.0020083928260826) * conv;
+        const double t = kTamnu * kTamnu;
+        return T.mnu * (kT * kT * kT) * (ia * ia * ia) *
+               (1.5 * kZeta3 + t * (45. / 4. * 1.0369277551433704 +
+                                    t * (2835. / 32. * 1.0083492773819229 + t * (80325 / 32. * 1.0020083928260826)))) *
+               conv;
     }
     if (rel) {
         const double t = kPi * kT * ia, t2 = t * t;
         return 7 * (t2 * t2) / 120. * conv;
     }
+    // a rounding across a knot is harmless: the segments' polynomials meet there
     int i = (int)((loga - T.loga[0]) * T.inv_dx);
     i = i < 0 ? 0 : (i > kNRhoTab - 2 ? kNRhoTab - 2 : i);
-    while (i > 0 && loga < T.loga[i]) i--;
-    while (i < kNRhoTab - 2 && loga >= T.loga[i + 1]) i++;
     const double dx = loga - T.loga[i];
     return T.rhonu[i] + dx * (T.sb[i] + dx * (T.c[i] + dx * T.sd[i]));
 }
 
-// The fslength integrand 1/(a^2 H(a)) at a = e^x (delta_tot_table.c:378-383) with H as
-// hubble() forms it, 1/a computed once (one exp, one sqrt, two divisions per node).
-__device__ __forceinline__ double fsl_integrand(const Background& B, double x) {
-    if (B.htab_n > 0) return exp(-2.0 * x - hubble_tab_log(B, x));
-    const double a = exp(x);
-    const double ia = 1.0 / a;
+// 1 / H at a = 1 / ia with H as hubble() forms it.
+__device__ __forceinline__ double inv_hubble_ia(const Background& B, double x, double ia) {
     const double ia2 = ia * ia, ia3 = ia2 * ia;
     double om = B.Omega_nonu_H * ia3 + B.OmegaLambda;
     if (B.OmegaK != 0.0) om += B.OmegaK * ia2;
     double rhonu = 0;
     for (int mi = 0; mi < kNuSpecies; mi++)
-        if (B.deg[mi] > 0) rhonu += B.deg[mi] * rho_nu_ia(B.tab[mi], a, ia, x, B.kBtnu, B.conv);
+        if (B.deg[mi] > 0) rhonu += B.deg[mi] * rho_nu_ia(B.tab[mi], ia, x, B.kBtnu, B.conv);
     om += rhonu * B.irhocrit;
     if (B.radiation) om += B.omegag0 * (ia3 * ia);
-    return ia2 / (B.hubble * sqrt(om));
+    return rsqrt(om) * B.ihubble;
+}
+// The fslength integrand 1/(a^2 H(a)) at a = e^x (delta_tot_table.c:378-383): one exp, one
+// reciprocal square root and no division, ~60 FP64 operations (with 1/a and 1/H divided out, 90).
+__device__ __forceinline__ double fsl_integrand(const Background& B, double x) {
+    if (B.htab_n > 0) return exp(-2.0 * x - hubble_tab_log(B, x));
+    const double ia = exp(-x);
+    return ia * ia * inv_hubble_ia(B, x, ia);
 }
 #endif
 
@@ -970,30 +984,40 @@ struct NodeTerms {
     int j;       // history segment: knot[j] <= x < knot[j+1]
 };
 
-// Not inlined: the table builders and the uncached path run the same compiled code and
-// produce the same numbers bit for bit.
-// 1 / (a H(a)) at x = log a, from 1 / (a^2 H) (one division and the rho_nu segments' stored
-// polynomials instead of hubble()'s ten divisions)
+// 1 / (a H(a)) at x = log a
 static __device__ __noinline__ double node_inv_aH(const Background* B, double x) {
-    return exp(x) * fsl_integrand(*B, x);
+    if (B->htab_n > 0) return exp(-x - hubble_tab_log(*B, x));
+    const double ia = exp(-x);
+    return ia * inv_hubble_ia(*B, x, ia);
 }
-// the fslength spline on the segment [x0, x1] at x
-static __device__ __noinline__ double fs_spline_eval(double x0, double x1, double y0, double y1, double c0, double c1,
-                                                     double x) {
-    const double h = x1 - x0, dx = x - x0;
-    const double bq = (y1 - y0) / h - h * (c1 + 2.0 * c0) / 3.0;
-    const double d = (c1 - c0) / (3.0 * h);
-    return y0 + dx * (bq + dx * (c0 + dx * d));
+// The uniform nodes of the fslength table: log a of the first, their spacing and its inverse.
+struct FsGrid {
+    int n;
+    double x0, h, ih;
+    __host__ __device__ __forceinline__ double node(int i) const { return x0 + i * h; }
+    // the segment of x (a rounding across a node is harmless: the cubics meet there)
+    __device__ __forceinline__ int segment(double x) const {
+        const int i = (int)((x - x0) * ih);
+        return i < 0 ? 0 : (i > n - 2 ? n - 2 : i);
+    }
+};
+__host__ __device__ inline FsGrid fs_grid(int n, double loga0, double loga) {
+    if (n < 2) return FsGrid{n, loga0, 0.0, 0.0};
+    return FsGrid{n, loga0, (loga - loga0) / (n - 1.), (n - 1.) / (loga - loga0)};
 }
-static __device__ __noinline__ NodeTerms dnu_node_terms(const Background* B, const double* fs_x, const double* fs_y,
-                                                 const double* fs_c, int nfs, double fs_x0, double fs_inv,
-                                                 const double* kx, int na, double x) {
+// the table's spline dx past the lower node of a segment, from the values and coefficients of
+// its nodes (dy: the values' difference)
+__device__ __forceinline__ double fs_spline_eval(const FsGrid& g, double y0, double dy, double c0, double c1,
+                                                 double dx) {
+    const double bq = fma(dy, g.ih, -(g.h * (1.0 / 3.0)) * fma(2.0, c0, c1));
+    const double d = (c1 - c0) * (g.ih * (1.0 / 3.0));
+    return fma(dx, fma(dx, fma(dx, d, c0), bq), y0);
+}
+static __device__ __noinline__ NodeTerms dnu_node_terms(const Background* B, const double* fs_y, const double* fs_c,
+                                                        const FsGrid& g, const double* kx, int na, double x) {
     NodeTerms t;
-    int i = (int)((x - fs_x0) * fs_inv);
-    i = i < 0 ? 0 : (i > nfs - 2 ? nfs - 2 : i);
-    while (i > 0 && x < fs_x[i]) i--;
-    while (i < nfs - 2 && x >= fs_x[i + 1]) i++;
-    t.fsl = fs_spline_eval(fs_x[i], fs_x[i + 1], fs_y[i], fs_y[i + 1], fs_c[i], fs_c[i + 1], x);
+    const int i = g.segment(x);
+    t.fsl = fs_spline_eval(g, fs_y[i], fs_y[i + 1] - fs_y[i], fs_c[i], fs_c[i + 1], x - g.node(i));
     t.j = seg_bsearch(kx, na, x);
     t.dx = x - kx[t.j];
     t.g = t.fsl * node_inv_aH(B, x);
@@ -1038,7 +1062,7 @@ struct NodeCache {
 struct DnuIntegrandC {
     const Background* B;
     double k_over_m, qc, nfl;
-    const double* fs_x; const double* fs_y; const double* fs_c; int nfs; double fs_x0, fs_inv;
+    const double* fs_y; const double* fs_c; FsGrid fs;
     const double* kx; const double* ky; const double* kc; int na;
     const double* sb; const double* sd;  // seg_poly of (ky, kc)
     KnotSeg ks;
@@ -1053,7 +1077,7 @@ struct DnuIntegrandC {
             t.j = __ldg(nc.j + q);
             return t;
         }
-        return dnu_node_terms(B, fs_x, fs_y, fs_c, nfs, fs_x0, fs_inv, kx, na, x);
+        return dnu_node_terms(B, fs_y, fs_c, fs, kx, na, x);
     }
 };
 
@@ -1066,9 +1090,9 @@ struct DnuIntegrandC {
 struct NodeWeights {
     double a, b, c, d;
 };
-__device__ __forceinline__ NodeWeights node_weights(double g, double dx, double h, int na) {
+__device__ __forceinline__ NodeWeights node_weights(double g, double dx, double h, double ih, int na) {
     NodeWeights w;
-    const double s = dx / h;
+    const double s = dx * ih;
     const double gs = __dmul_rn(g, s);
     w.a = __dsub_rn(g, gs);
     w.b = gs;
@@ -1099,7 +1123,7 @@ struct DnuIntegrandW {
     const double* kc;
     NodeTable nc;
     // for intervals that are not in the node table
-    const double* fs_x; const double* fs_y; const double* fs_c; const double* kx;
+    const double* fs_y; const double* fs_c; const double* kx; const double* kih;
     const StepScalars* S;
     int na;
     __device__ __forceinline__ double value(const NodeWeights& w, double fsl, float fslf, int j) const {

@@ -264,7 +264,8 @@ struct GL4 { double x[2], w[2]; };  // positive half of the 4-point Gauss-Legend
 struct PrepArgs {
     StepScalars S;                 // the call's scalars
     double loga, loga0;
-    int Na, Nfs, nodes;            // Nfs, nodes: 0 without a table
+    FsGrid fs;                     // its n, nodes: 0 without a table
+    int Na, nodes;
     int start_row, write_knot;
     int knot_blocks, fs_blocks, node_blocks, hyb_blocks;  // hyb_blocks: per species
 };
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, 
     }
     b -= P.knot_blocks;
     if (b < P.fs_blocks) {
-        fs_eval_block(*I.B, P.Nfs, P.loga0, P.loga, b, gl.x[0], gl.x[1], gl.w[0], gl.w[1], f, sg, I.fs_seg, I.fs_suf,
+        fs_eval_block(*I.B, P.fs, P.loga, b, gl.x[0], gl.x[1], gl.w[0], gl.w[1], f, sg, I.fs_seg, I.fs_suf,
                       I.fs_tot);
         return;
     }
@@ -375,29 +376,20 @@ __global__ void __launch_bounds__(kTableThreads, 8)
         return;
     }
     b -= nrow;
-    const FsTable F = fs_table(I, P.Nfs, P.loga0, P.loga, P.S.light, tsuf);
-    const int table_blocks = (P.Nfs + kTableThreads - 1) / kTableThreads;
+    const FsTable F = fs_table(I, P.fs, P.S.light, tsuf);
+    const int table_blocks = fs_table_blocks(P.fs.n, kTableThreads);
     if (b < table_blocks) {
-        const int i = b * kTableThreads + t;
-        if (i >= P.Nfs) return;
-        I.fs_x[i] = fs_node(i, P.Nfs, P.loga0, P.loga);
-        const double y = fs_table_y(F, i);
-        I.fs_y[i] = y;
-        I.fs_c[i] = fs_table_c(F, i);
-        if (i == 0) {
-            I.sc->fsl_A0a = y;
-            I.sc->Nfs = P.Nfs;
-        }
+        fs_table_store(I, F, b * kTableThreads + t);
         return;
     }
     const int q = (b - table_blocks) * kTableThreads + t;
     if (q >= P.nodes) return;
     double half;
     const double x = nc_node_x(q, P.loga0, P.loga, &half);
-    const double fsl = fs_table_at(F, P.loga0, P.loga, x);
+    const double fsl = fs_table_at(F, x);
     const double* kx = I.scalefact;
     const int j = seg_bsearch(kx, Na, x);
-    nc_store(I, q, fsl, I.nc_inv[q], x - kx[j], j, kx[j + 1] - kx[j], Na, half);
+    nc_store(I, q, fsl, I.nc_inv[q], x - kx[j], j, kx[j + 1] - kx[j], I.knot_invh[j], Na, half);
 }
 
 // block per bin: this bin's delta_cdm (a deferred normalisation), the provisional row
@@ -742,15 +734,15 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
     }
     P.knot_blocks = (Na - 1 + kPrepThreads - 1) / kPrepThreads;
     if (loga > loga0) {  // the fslength table also gives fslength(log a0, log a)
-        P.Nfs = 16 * (Na > 1 ? Na : 1);
-        P.fs_blocks = fs_blocks(P.Nfs, loga0, loga);
+        P.fs = fs_grid(16 * (Na > 1 ? Na : 1), loga0, loga);
+        P.fs_blocks = fs_blocks(P.fs);
         P.nodes = Na > 1 ? I.nc_slots * 61 : 0;
         P.node_blocks = (P.nodes + kPrepThreads - 1) / kPrepThreads;
         if (I.hyb && P.S.partnu > 0 && !P.S.skip_integral) P.hyb_blocks = kHybPieces / 8;
     }
     k_prep_eval<<<1 + P.knot_blocks + P.fs_blocks + kNuSpecies * P.hyb_blocks + P.node_blocks, kPrepThreads, 0, st>>>(I, P, gl);
     const int nrow = rows == kRowsBase ? nk + 1 : (rows == kRowsFull && (Na > 2 || update_row >= 0) ? nk : 0);
-    const int blocks = nrow + (P.Nfs + kTableThreads - 1) / kTableThreads +
+    const int blocks = nrow + fs_table_blocks(P.fs.n, kTableThreads) +
                        (P.nodes + kTableThreads - 1) / kTableThreads;
     if (blocks > 0)
         k_prep_tables<<<blocks, kTableThreads, 0, st>>>(I, P, nrow > 0 ? (int)rows : (int)kRowsNone, nk, update_row,

@@ -23,6 +23,7 @@ struct StepScalars {
     double relerr;                   // 1e-6, loosened for hybrid neutrinos (:547)
     double partnu_now;               // particle_nu_fraction(a, 0) (:539)
     double kspace_prefac;            // interface_common.c:139-145
+    double fs_h, fs_ih;              // spacing of the fslength table's nodes, and its inverse
     int skip_integral;               // particles carry everything (:542-543)
     int Na, Nfs;
 };
@@ -58,7 +59,6 @@ struct IntegratorDev {
     const double* jt;                // J's fine table (one per device)
     double* hyb;                     // optional: [kNuSpecies][kHybTable] the tables of J with a cut
     int nc_slots;                    // slots of the node table in use (1 + 2 levels, 0 = none)
-    double* fs_x;                    // [fs_cap]
     double* fs_y;                    // [fs_cap]
     double* fs_c;                    // [fs_cap]
     double* fs_seg;                  // [fs_cap] integrals of 1/(a^2 H) over the table's segments
@@ -231,16 +231,15 @@ __device__ __forceinline__ void spline_solve_scan(const IntegratorDev& I, int m,
 // The delta_nu integrand of one (species, bin) with the instance's node table; knots,
 // row and rc may be staged copies (shared memory) of the instance's arrays.
 // sb, sd: seg_poly of (row, rc), filled by the caller
-// k_over_m = k / (m / kT) and fs_inv = (Nfs - 1) / (log a - log a0) given: the integral
+// k_over_m = k / (m / kT) given: the integral
 // kernels form those divisions on one lane per task and broadcast them
 __device__ __forceinline__ DnuIntegrandC dnu_integrand_pre(const IntegratorDev& I, const StepScalars& S,
-                                                           double k_over_m, double fs_inv, double qc,
+                                                           double k_over_m, double qc,
                                                            const double* knots, const double* row, const double* rc,
                                                            const double* sb, const double* sd, int Na) {
     DnuIntegrandC f;
     f.B = I.B; f.k_over_m = k_over_m; f.qc = qc; f.nfl = I.B->nufrac_low[0];
-    f.fs_x = I.fs_x; f.fs_y = I.fs_y; f.fs_c = I.fs_c; f.nfs = S.Nfs; f.fs_x0 = S.loga0;
-    f.fs_inv = fs_inv;
+    f.fs_y = I.fs_y; f.fs_c = I.fs_c; f.fs = FsGrid{S.Nfs, S.loga0, S.fs_h, S.fs_ih};
     f.kx = knots; f.ky = row; f.kc = rc; f.na = Na;
     f.sb = sb; f.sd = sd;
     f.ks = KnotSeg{I.knot_invh, I.knot_h3, I.knot_ih3};
@@ -251,7 +250,7 @@ __device__ __forceinline__ DnuIntegrandC dnu_integrand(const IntegratorDev& I, c
                                                        double mnubykT, double qc, const double* knots,
                                                        const double* row, const double* rc, const double* sb,
                                                        const double* sd, int Na) {
-    return dnu_integrand_pre(I, S, k / mnubykT, (S.Nfs - 1.) / (S.loga - S.loga0), qc, knots, row, rc, sb, sd, Na);
+    return dnu_integrand_pre(I, S, k / mnubykT, qc, knots, row, rc, sb, sd, Na);
 }
 // The integrand of one (species mi, bin) from its row and spline coefficients (shared memory).
 __device__ __forceinline__ DnuIntegrandW dnu_integrand_w(const IntegratorDev& I, const StepScalars& S, int mi, double kom,
@@ -262,21 +261,22 @@ __device__ __forceinline__ DnuIntegrandW dnu_integrand_w(const IntegratorDev& I,
     f.hyb = I.hyb ? I.hyb + (size_t)mi * kHybTable : nullptr;
     f.ky = row; f.kc = rc;
     f.nc = NodeTable{I.nc_ab, I.nc_cd, I.nc_fsl, I.nc_jf, I.nc_half, I.nc_slots};
-    f.fs_x = I.fs_x; f.fs_y = I.fs_y; f.fs_c = I.fs_c; f.kx = I.scalefact;
+    f.fs_y = I.fs_y; f.fs_c = I.fs_c; f.kx = I.scalefact; f.kih = I.knot_invh;
     f.S = &S; f.na = Na;
     return f;
 }
 // A node outside the node table: its terms evaluated here, then the same arithmetic.
 __device__ __noinline__ inline double DnuIntegrandW::slow(double x) const {
-    const NodeTerms t = dnu_node_terms(B, fs_x, fs_y, fs_c, S->Nfs, S->loga0, (S->Nfs - 1.) / (S->loga - S->loga0), kx, na, x);
-    return value(node_weights(t.g, t.dx, kx[t.j + 1] - kx[t.j], na), t.fsl, (float)t.fsl, t.j);
+    const FsGrid g{S->Nfs, S->loga0, S->fs_h, S->fs_ih};
+    const NodeTerms t = dnu_node_terms(B, fs_y, fs_c, g, kx, na, x);
+    return value(node_weights(t.g, t.dx, kx[t.j + 1] - kx[t.j], kih[t.j], na), t.fsl, (float)t.fsl, t.j);
 }
 // Node q of the node table, in an interval of half-width `half`.
 __device__ __forceinline__ void nc_store(const IntegratorDev& I, int q, double fsl, double inv_aH, double dx, int j,
-                                         double h, int Na, double half) {
+                                         double h, double ih, int Na, double half) {
     if (q % 61 == 0) I.nc_half[q / 61] = half;
     const double g = fsl * inv_aH;
-    const NodeWeights w = node_weights(g, dx, h, Na);
+    const NodeWeights w = node_weights(g, dx, h, ih, Na);
     I.nc_g[q] = g;
     I.nc_fsl[q] = fsl;
     I.nc_dx[q] = dx;

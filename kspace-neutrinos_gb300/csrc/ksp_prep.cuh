@@ -28,15 +28,16 @@ constexpr int kPrepThreads = 64;
 // square root, two divisions and the rho_nu tables, ~100 FP64 operations.
 constexpr double kFsNodeRule = 1.5e-3, kFsGauss2 = 5e-3;
 constexpr int kFsNodeSegs = kPrepThreads - 7;  // segments of a block by the node rule
-__host__ __device__ inline int fs_block_segs(int Nfs, double loga0, double loga) {
-    const double h = (loga - loga0) / (Nfs - 1.);
+__host__ __device__ inline int fs_block_segs(double h) {
     return h < kFsNodeRule ? kFsNodeSegs : (h < kFsGauss2 ? kPrepThreads / 2 : kPrepThreads / 4);
 }
-// blocks of a table of Nfs nodes (segments 0 .. Nfs - 2, and a last one of zero)
-__host__ __device__ inline int fs_blocks(int Nfs, double loga0, double loga) {
-    const int per = fs_block_segs(Nfs, loga0, loga);
-    return (Nfs + per - 1) / per;
+// blocks of a table (segments 0 .. n - 2, and a last one of zero)
+__host__ __device__ inline int fs_blocks(const FsGrid& g) {
+    const int per = fs_block_segs(g.h);
+    return (g.n + per - 1) / per;
 }
+// nodes per block of the second kernel: two a thread
+constexpr int fs_table_blocks(int n, int threads) { return (n + 2 * threads - 1) / (2 * threads); }
 
 #ifdef __CUDACC__
 // integrals over [o, o + 1], o = 0..3, of the Lagrange basis on the nodes 0..7, x 120960
@@ -49,18 +50,13 @@ static __constant__ double kNodeRule[4][8] = {
 
 __device__ __noinline__ static double fsl_integrand_call(const Background& B, double x) { return fsl_integrand(B, x); }
 
-// Node i of the table.
-__device__ __forceinline__ double fs_node(int i, int Nfs, double loga0, double loga) {
-    return loga0 + i * (loga - loga0) / (Nfs - 1.);
-}
-
 // Block `blk` of the segments, by 64 threads: fs_seg[v] = s_v, fs_suf[v] = the sum of the
 // block's s from v on, fs_tot[blk] = the block's.  f: 64 doubles of shared memory, sg: 64.
-__device__ __forceinline__ void fs_eval_block(const Background& B, int Nfs, double loga0, double loga, int blk,
+__device__ __forceinline__ void fs_eval_block(const Background& B, const FsGrid& g, double loga, int blk,
                                               double gx0, double gx1, double gw0, double gw1, double* f, double* sg,
                                               double* fs_seg, double* fs_suf, double* fs_tot) {
-    const int t = threadIdx.x;
-    const double h = (loga - loga0) / (Nfs - 1.);
+    const int t = threadIdx.x, Nfs = g.n;
+    const double h = g.h;
     int per, v;
     double s = 0;
     if (h < kFsNodeRule) {
@@ -70,7 +66,7 @@ __device__ __forceinline__ void fs_eval_block(const Background& B, int Nfs, doub
         int base = first - 3;
         base = base > Nfs - kPrepThreads ? Nfs - kPrepThreads : base;
         base = base < 0 ? 0 : base;
-        f[t] = base + t < Nfs ? fsl_integrand_call(B, fs_node(base + t, Nfs, loga0, loga)) : 0.0;
+        f[t] = base + t < Nfs ? fsl_integrand_call(B, g.node(base + t)) : 0.0;
         __syncthreads();
         v = first + t;
         if (t < per && v < Nfs - 1) {
@@ -93,7 +89,7 @@ __device__ __forceinline__ void fs_eval_block(const Background& B, int Nfs, doub
         const int u = blk * per + t / w, q = t % w;
         double x = 0;
         if (u < Nfs - 1) {
-            const double xa = fs_node(u, Nfs, loga0, loga), xb = u + 1 == Nfs - 1 ? loga : fs_node(u + 1, Nfs, loga0, loga);
+            const double xa = g.node(u), xb = u + 1 == Nfs - 1 ? loga : g.node(u + 1);
             const double c = 0.5 * (xa + xb), hh = 0.5 * (xb - xa);
             const double gx = two ? 0.57735026918962576451 : ((q & 1) ? gx1 : gx0);  // 1 / sqrt 3
             const double gw = two ? 1.0 : ((q & 1) ? gw1 : gw0);
@@ -156,8 +152,9 @@ struct FsTable {  // what the second kernel reads
     const double* suf;
     const double* tot;
     const double* tsuf;  // fs_totals_suffix
-    int Nfs, nblk, per;
-    double light, h;     // h: node spacing
+    FsGrid g;
+    int nblk, per;
+    double light;
     double cscale;       // light * 3 / h^2 / (2 sqrt 3)
 };
 
@@ -176,55 +173,59 @@ __device__ __forceinline__ double fs_table_y(const FsTable& F, int i) {
 // that is, the s evenly: s_{-1-k} = s_k, s_{n+k} = s_{n-1-k}, n = Nfs - 1.  The sums over the
 // neighbours are taken over the s themselves (summation by parts: one multiply-add per
 // term), D to a side: 20 where h < 0.02 (nu^20 = 4e-12 of a term below 4e-4 of fslength), 28
-// elsewhere (Nfs >= 16: one continuation reaches).
+// elsewhere (n >= 15: the second end's continuation may reach back past the first).
+//
+// The two sums at a node follow from those of its neighbour by one multiply-add each, so a pair
+// of nodes i, i + 1 takes the left sum of the first and the right sum of the second: c[0], c[1].
 __device__ __forceinline__ double fs_table_s(const FsTable& F, int i) {
-    const int n = F.Nfs - 1;
+    const int n = F.g.n - 1;
     i = i < 0 ? -1 - i : i;
     i = i >= n ? 2 * n - 1 - i : i;
+    i = i < 0 ? -1 - i : i;
     return F.seg[i];
 }
-__device__ __forceinline__ double fs_table_c(const FsTable& F, int i) {
-    if (i == 0 || i == F.Nfs - 1) return 0.0;
+__device__ __forceinline__ void fs_table_c2(const FsTable& F, int i, double* c) {
     const double nu = -0.26794919243112270647, k = 0.78867513459481288225;  // 1 / (1 - nu)
-    double l, r;
-    if (F.h < 0.02) {
+    double l, r;  // left sum of node i, right sum of node i + 1
+    if (F.g.h < 0.02) {
         constexpr int D = 20;
         l = fs_table_s(F, i - D - 1) * k;
-        r = fs_table_s(F, i + D) * k;
+        r = fs_table_s(F, i + 1 + D) * k;
 #pragma unroll
         for (int d = D; d >= 2; d--) {
             l = fma(nu, l, fs_table_s(F, i - d));
-            r = fma(nu, r, fs_table_s(F, i + d - 1));
+            r = fma(nu, r, fs_table_s(F, i + d));
         }
     } else {
         constexpr int D = 28;
         l = fs_table_s(F, i - D - 1) * k;
-        r = fs_table_s(F, i + D) * k;
+        r = fs_table_s(F, i + 1 + D) * k;
         for (int d = D; d >= 2; d--) {
             l = fma(nu, l, fs_table_s(F, i - d));
-            r = fma(nu, r, fs_table_s(F, i + d - 1));
+            r = fma(nu, r, fs_table_s(F, i + d));
         }
     }
-    const double s0 = F.seg[i], s1 = F.seg[i - 1];
-    const double q = fma(1.0 - nu, l - r, s0 - s1);  // the two sides' sums of nu^(d-1) D^2 y
-    return F.cscale * fma(nu, q, s1 - s0);
+    const double sm = fs_table_s(F, i - 1), s0 = fs_table_s(F, i), s1 = fs_table_s(F, i + 1);
+    const double r0 = fma(nu, r, s1), l1 = fma(nu, l, sm);
+    // the two sides' sums of nu^(d-1) D^2 y
+    const double q0 = fma(1.0 - nu, l - r0, s0 - sm), q1 = fma(1.0 - nu, l1 - r, s1 - s0);
+    c[0] = i == 0 ? 0.0 : F.cscale * fma(nu, q0, sm - s0);
+    c[1] = i + 1 >= F.g.n - 1 ? 0.0 : F.cscale * fma(nu, q1, s0 - s1);
 }
 
 // The table of a call as the second kernel's blocks read it.  Called by a whole block of at
 // least kPrepThreads threads; tsuf: kPrepThreads + 1 doubles of shared memory.
-__device__ __forceinline__ FsTable fs_table(const IntegratorDev& I, int Nfs, double loga0, double loga, double light,
-                                            double* tsuf) {
+__device__ __forceinline__ FsTable fs_table(const IntegratorDev& I, const FsGrid& g, double light, double* tsuf) {
     FsTable F;
     F.seg = I.fs_seg;
     F.suf = I.fs_suf;
     F.tot = I.fs_tot;
     F.tsuf = tsuf;
-    F.Nfs = Nfs;
-    F.nblk = fs_blocks(Nfs, loga0, loga);
-    F.per = fs_block_segs(Nfs, loga0, loga);
+    F.g = g;
+    F.nblk = fs_blocks(g);
+    F.per = fs_block_segs(g.h);
     F.light = light;
-    F.h = (loga - loga0) / (Nfs - 1.);
-    F.cscale = light * (3.0 / (F.h * F.h) / (2.0 * 1.7320508075688772935));
+    F.cscale = light * (g.ih * g.ih) * 0.86602540378443864676;
     if (threadIdx.x < kPrepThreads) {
         fs_totals_suffix(I.fs_tot, F.nblk, tsuf);
     } else {
@@ -234,14 +235,33 @@ __device__ __forceinline__ FsTable fs_table(const IntegratorDev& I, int Nfs, dou
     return F;
 }
 
-// fslength at x, from the spline of the table
-__device__ __forceinline__ double fs_table_at(const FsTable& F, double loga0, double loga, double x) {
-    int i = (int)((x - loga0) * ((F.Nfs - 1.) / (loga - loga0)));
-    i = i < 0 ? 0 : (i > F.Nfs - 2 ? F.Nfs - 2 : i);
-    while (i > 0 && x < fs_node(i, F.Nfs, loga0, loga)) i--;
-    while (i < F.Nfs - 2 && x >= fs_node(i + 1, F.Nfs, loga0, loga)) i++;
-    return fs_spline_eval(fs_node(i, F.Nfs, loga0, loga), fs_node(i + 1, F.Nfs, loga0, loga), fs_table_y(F, i),
-                          fs_table_y(F, i + 1), fs_table_c(F, i), fs_table_c(F, i + 1), x);
+// Nodes i = 2 u, i + 1 of the table to memory; the first also to the call's scalars.
+__device__ __forceinline__ void fs_table_store(const IntegratorDev& I, const FsTable& F, int u) {
+    const int i = 2 * u;
+    if (i >= F.g.n) return;
+    double c[2];
+    fs_table_c2(F, i, c);
+    const double y = fs_table_y(F, i);
+    I.fs_y[i] = y;
+    I.fs_c[i] = c[0];
+    if (i + 1 < F.g.n) {
+        I.fs_y[i + 1] = i + 1 == F.g.n - 1 ? 0.0 : fs_table_y(F, i + 1);
+        I.fs_c[i + 1] = c[1];
+    }
+    if (i == 0) {
+        I.sc->fsl_A0a = y;
+        I.sc->Nfs = F.g.n;
+        I.sc->fs_h = F.g.h;
+        I.sc->fs_ih = F.g.ih;
+    }
+}
+
+// fslength at x, from the spline of the table (which falls by light s_i from node i to i + 1)
+__device__ __forceinline__ double fs_table_at(const FsTable& F, double x) {
+    const int i = F.g.segment(x);
+    double c[2];
+    fs_table_c2(F, i, c);
+    return fs_spline_eval(F.g, fs_table_y(F, i), -F.light * F.seg[i], c[0], c[1], x - F.g.node(i));
 }
 
 // ------------------------------------------------------------------ knots

@@ -406,20 +406,34 @@ void batch_set_attributes() {
     raise_dynamic_smem_limit(reinterpret_cast<const void*>(kb_dtot_coeffs));
 }
 
-void launch_batch_update(const BatchDev& b, cudaStream_t st) {
-    static GL4b gl;
-    static bool init = false;
-    if (!init) {
-        gl_nodes_b(4, gl.x, gl.w);
-        init = true;
-    }
+// The tables keep the FP64 pipes busy, the prologue and the row splines wait for their serial
+// chains: side by side, segments | prologue (and the binning of bound grids before it), then
+// tables | splines (a call of 256 members: 3853 us one after the other, 3720 so).
+cudaError_t launch_batch_segments(const BatchDev& b, const BatchStreams& s) {
+    static const GL4b gl = [] {
+        GL4b g;
+        gl_nodes_b(4, g.x, g.w);
+        return g;
+    }();
+    cudaError_t e = cudaEventRecord(s.start, s.main);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s.side, s.start, 0);
+    if (e == cudaSuccess) kb_fs_eval<<<4 * kBatchSmallBlocks, kPrepThreads, 0, s.side>>>(b, gl);
+    return e;
+}
+cudaError_t launch_batch_update(const BatchDev& b, const BatchStreams& s) {
     const int nb = kBatchSmallBlocks;
+    const cudaStream_t st = s.main;
     kb_prologue<<<b.M < nb ? b.M : nb, 128, 0, st>>>(b);
-    kb_fs_eval<<<4 * nb, kPrepThreads, 0, st>>>(b, gl);
-    kb_tables<<<2 * nb, kBatchTable, 0, st>>>(b);
+    cudaError_t e = cudaEventRecord(s.prologue, st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s.side, s.prologue, 0);
+    kb_tables<<<2 * nb, kBatchTable, 0, s.side>>>(b);
+    if (e == cudaSuccess) e = cudaEventRecord(s.tables, s.side);
     kb_dtot_coeffs<<<nb, 32 * kRowWarps, kRowWarps * sizeof(RowSmem), st>>>(b);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, s.tables, 0);
+    if (e != cudaSuccess) return e;
     kb_dnu_qag<<<b.qag_blocks, 32 * b.wpb, batch_qag_smem(b.ldmax, b.wpb), st>>>(b);
     kb_finish<<<nb, 256, 0, st>>>(b);
+    return cudaPeekAtLastError();
 }
 
 void launch_batch_corr(const BatchDev& b, const BatchGridCorr* g, int ngrid, cudaStream_t st) {

@@ -61,7 +61,14 @@ struct BatchGridCorr {
 
 size_t batch_qag_smem(int ldmax, int wpb);
 void batch_set_attributes();
-void launch_batch_update(const BatchDev& b, cudaStream_t st);
+// A step's streams; the events order the two.
+struct BatchStreams {
+    cudaStream_t main = nullptr, side = nullptr;
+    cudaEvent_t start = nullptr, prologue = nullptr, tables = nullptr;
+};
+// the fslength segments, on the side stream after what the main one holds so far; then the rest
+cudaError_t launch_batch_segments(const BatchDev& b, const BatchStreams& s);
+cudaError_t launch_batch_update(const BatchDev& b, const BatchStreams& s);
 void launch_batch_corr(const BatchDev& b, const BatchGridCorr* g, int ngrid, cudaStream_t st);
 
 }  // namespace ksp

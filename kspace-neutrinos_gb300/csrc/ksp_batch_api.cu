@@ -55,6 +55,8 @@ struct kspace_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaStream_t side = nullptr;  // beside it (launch_batch_segments)
+    cudaEvent_t ev_start = nullptr, ev_prologue = nullptr, ev_tables = nullptr;
     float last_ms = 0;
     std::vector<int> last_status;
     int sm_count = 152;
@@ -95,6 +97,10 @@ extern "C" int kspace_gpu_batch_create(kspace_batch** out, kspace_ctx* const* ct
     b->ctx.assign(ctxs, ctxs + M);
     cudaDeviceGetAttribute(&b->sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->ev_start, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->ev_prologue, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->ev_tables, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreate(&b->ev0) != cudaSuccess || cudaEventCreate(&b->ev1) != cudaSuccess ||
         cudaMalloc(&b->status_d, sizeof(unsigned) * M) != cudaSuccess ||
         cudaMallocHost(&b->status_h, sizeof(unsigned) * M) != cudaSuccess ||
@@ -121,6 +127,7 @@ extern "C" int kspace_gpu_batch_create(kspace_batch** out, kspace_ctx* const* ct
 extern "C" int kspace_gpu_batch_destroy(kspace_batch* b) {
     if (!b) return KSPACE_OK;
     cudaSetDevice(b->device);
+    if (b->side) cudaStreamSynchronize(b->side);
     if (b->stream) cudaStreamSynchronize(b->stream);
     drop_graph(b);
     cudaFree(b->insts_d);
@@ -133,6 +140,9 @@ extern "C" int kspace_gpu_batch_destroy(kspace_batch* b) {
     cudaFree(b->gcorr_d);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
+    for (cudaEvent_t e : {b->ev_start, b->ev_prologue, b->ev_tables})
+        if (e) cudaEventDestroy(e);
+    if (b->side) cudaStreamDestroy(b->side);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return KSPACE_OK;
@@ -250,6 +260,7 @@ static int enqueue_bin(kspace_batch* b, const BoundGrid& g) {
     gg.slab0 = 0;
     gg.nslab = g.N;
     gg.nmodes = (long long)g.N * g.N * (g.N / 2 + 1);
+    gg.beside = true;  // the fslength segments run beside
     const int nb = gg.nrbins;
     CKB(cudaMemsetAsync(c->bin_sum_d, 0, sizeof(double) * (nb + 1), b->stream));
     if (launch_bin_power(gg, g.grid, c->bin_sum_d, c->bin_sum_d + nb, b->status_d + g.inst, c->tma, c->rows,
@@ -277,12 +288,14 @@ static int enqueue_correct(kspace_batch* b, const BoundGrid& g) {
 
 // The whole step's device work in stream order.
 static int enqueue_step(kspace_batch* b, bool correct) {
+    const BatchDev d = dev_view(b);
+    const BatchStreams s{b->stream, b->side, b->ev_start, b->ev_prologue, b->ev_tables};
+    CKB(launch_batch_segments(d, s));
     for (const BoundGrid& g : b->grids) {
         const int st = enqueue_bin(b, g);
         if (st) return st;
     }
-    const BatchDev d = dev_view(b);
-    launch_batch_update(d, b->stream);
+    CKB(launch_batch_update(d, s));
     if (correct && !b->grids.empty()) {
         launch_batch_corr(d, b->gcorr_d, (int)b->grids.size(), b->stream);
         for (const BoundGrid& g : b->grids) {

@@ -276,6 +276,7 @@ struct PrepArgs {
 // where hybrid neutrinos cut it, and the part of the node table that needs no fslength.
 __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, PrepArgs P, GL4 gl) {
     __shared__ double f[kPrepThreads], sg[kPrepThreads];
+    ptx::dep_launch();
     const int t = threadIdx.x, Na = P.Na;
     int b = blockIdx.x;
     if (b == 0) {
@@ -338,6 +339,8 @@ constexpr int kTableThreads = 128;
 __global__ void __launch_bounds__(kTableThreads, 8)
     k_prep_tables(IntegratorDev I, PrepArgs P, int rows, int nk, int update_row, FinalizeArgs fin) {
     __shared__ double tsuf[kPrepThreads + 1], sh[2 * kTableThreads / 32];
+    ptx::dep_wait();
+    ptx::dep_launch();
     const int t = threadIdx.x, Na = P.Na;
     int b = blockIdx.x;
     const int nrow = rows == kRowsBase ? nk + 1 : (rows == kRowsFull ? nk : 0);
@@ -511,6 +514,8 @@ __global__ void __launch_bounds__(SPEC ? 256 : 128, SPEC ? 2 : 4)
     k_dnu_qag_blk(IntegratorDev I, int nk, int Na, int nspec, int4 spec_ids, RowUpdate upd) {
     typedef typename QagBlkSmemOf<SPEC>::type Smem;
     extern __shared__ __align__(16) unsigned char sm[];
+    ptx::dep_wait();
+    ptx::dep_launch();
     Gk61Nodes& N = *reinterpret_cast<Gk61Nodes*>(sm);
     size_t off = (sizeof(Gk61Nodes) + 15) & ~size_t(15);
     double* row = reinterpret_cast<double*>(sm + off);
@@ -745,8 +750,8 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
     const int blocks = nrow + fs_table_blocks(P.fs.n, kTableThreads) +
                        (P.nodes + kTableThreads - 1) / kTableThreads;
     if (blocks > 0)
-        k_prep_tables<<<blocks, kTableThreads, 0, st>>>(I, P, nrow > 0 ? (int)rows : (int)kRowsNone, nk, update_row,
-                                                     fin ? *fin : FinalizeArgs{});
+        launch_dependent(k_prep_tables, blocks, kTableThreads, 0, st, I, P, nrow > 0 ? (int)rows : (int)kRowsNone, nk,
+                         update_row, fin ? *fin : FinalizeArgs{});
 }
 
 // The rest, after the rows' splines: the integrals, the species sum.
@@ -802,8 +807,8 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
                 blk_attr = true;
             }
             const int4 sp = make_int4(spec_ids[0], spec_ids[1], spec_ids[2], 0);
-            if (spec) k_dnu_qag_blk<true><<<ntask, 256, bsmem, st>>>(I, nk, Na, nspec, sp, upd);
-            else k_dnu_qag_blk<false><<<ntask, split >= 4 ? 128 : 64, bsmem, st>>>(I, nk, Na, nspec, sp, upd);
+            if (spec) launch_dependent(k_dnu_qag_blk<true>, ntask, 256, bsmem, st, I, nk, Na, nspec, sp, upd);
+            else launch_dependent(k_dnu_qag_blk<false>, ntask, split >= 4 ? 128 : 64, bsmem, st, I, nk, Na, nspec, sp, upd);
         } else {
             if (upd.row >= 0) k_row_update<<<nk, 128, 0, st>>>(I, nk, Na, upd.row, upd.fin);
             const int blocks = (ntask + wpb - 1) / wpb;
@@ -822,6 +827,8 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
 __global__ void k_finish(IntegratorDev I, int nk, int commit_row, double a, double loga, const double* keff,
                          double* dnu_out, double* logk_out, double* ratio_out, CorrTable corr, double* norm_out,
                          int combine, int logk_ready) {
+    ptx::dep_wait();
+    ptx::dep_launch();
     const StepScalars& S = *I.sc;
     const bool pass = commit_row == -2;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -879,9 +886,8 @@ __global__ void k_finish(IntegratorDev I, int nk, int commit_row, double a, doub
 void launch_finish_update(const IntegratorDev& I, int nk, int commit_row, double a, double loga,
                           const double* keff, double* dnu_out, double* logk_out, double* ratio_out,
                           CorrTable corr, double* norm_out, cudaStream_t st, bool combine, bool logk_ready) {
-    k_finish<<<(nk + 31) / 32 > 0 ? (nk + 31) / 32 : 1, 32, 0, st>>>(I, nk, commit_row, a, loga, keff, dnu_out,
-                                                                     logk_out, ratio_out, corr, norm_out,
-                                                                     combine ? 1 : 0, logk_ready ? 1 : 0);
+    launch_dependent(k_finish, (nk + 31) / 32 > 0 ? (nk + 31) / 32 : 1, 32, 0, st, I, nk, commit_row, a, loga, keff,
+                     dnu_out, logk_out, ratio_out, corr, norm_out, combine ? 1 : 0, logk_ready ? 1 : 0);
 }
 
 }  // namespace ksp

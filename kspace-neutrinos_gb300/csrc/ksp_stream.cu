@@ -462,6 +462,8 @@ __global__ void __launch_bounds__(WARPS * 32)
             ptx::tma_load_2d_hint(my_stage + s * kTileBytes, &tmap, &my_bar[s], 0, (int)((gw + s * TW) * kRowsPerWarp), pol);
         }
     }
+    // the grid itself was complete before the kernel before this one began
+    ptx::dep_wait();
     // an error of the step so far (the reference terminates before the multiply): the
     // grid stays as it is, and goes to another output unchanged
     if (tid == 0) s_abort = (*reinterpret_cast<volatile unsigned*>(status) & kStAbort) != 0u;
@@ -1755,8 +1757,10 @@ int run_corr_stream(const GridArgs& a, const float* grid, float* out, CorrTable 
     const long long ntiles = (a.nrows16 + kRowsPerWarp - 1) / kRowsPerWarp;
     int grid_n = 1, adv_r = 0, adv_z = 0;
     if (!stream_grid(kern, WARPS, P.total, ntiles, a.nz, grid_n, adv_r, adv_z)) return -1;
-    kern<<<grid_n, WARPS * 32, P.total, st>>>(map, omap, a, corr, grid, out, status, ntiles, adv_r, adv_z);
-    return cudaPeekAtLastError() == cudaSuccess ? 0 : -2;
+    return launch_dependent(kern, grid_n, WARPS * 32, P.total, st, map, omap, a, corr, grid, out, status, ntiles, adv_r,
+                            adv_z) == cudaSuccess
+               ? 0
+               : -2;
 }
 
 // KSPACE_GPU_MIRROR=0: the row pass only (read once)

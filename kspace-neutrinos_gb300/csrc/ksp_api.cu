@@ -56,9 +56,10 @@ int ksp::map_status(unsigned s) {
 }
 
 // Synchronise with the stream and convert the device status word.  Results that a call has
-// queued for pinned memory before it are then there too.
-static int sync_status(kspace_ctx* c) {
-    CK(cudaMemcpyAsync(c->status_h, c->status_d, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+// queued for pinned memory before it are then there too.  delivered: the call's last kernel
+// writes the status word there itself.
+static int sync_status(kspace_ctx* c, bool delivered = false) {
+    if (!delivered) CK(cudaMemcpyAsync(c->status_h, c->status_d, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     const unsigned s = *c->status_h;
     if (s & kStKWarn)
@@ -460,8 +461,9 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
     };
     for (int pass = 0; pass < 2; pass++) {
         at = 0;
-        take(&I.dtot, nk * ld);  // first: these two are cleared
+        take(&I.dtot, nk * ld);  // first: these three are cleared
         take(&I.coef, nk * ld);
+        take(&I.done, 1);
         take(&I.scalefact, ld);
         take(&I.coef_unit, ld);
         take(&I.nu_init, nk);
@@ -514,7 +516,7 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
             base = static_cast<char*>(c->arena_d);
         }
     }
-    CK(cudaMemset(c->arena_d, 0, reinterpret_cast<char*>(I.scalefact) - base));  // dtot, coef
+    CK(cudaMemset(c->arena_d, 0, reinterpret_cast<char*>(I.scalefact) - base));  // dtot, coef, done
     I.jt = jfine_table();
     NEED(I.jt, KSPACE_ERR_CUDA);
     I.status = c->status_d;
@@ -528,7 +530,7 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
     CK(cudaMemcpy(I.sc, &S, sizeof(S), cudaMemcpyHostToDevice));
     c->buf_nb = nk_alloc;
     c->F0sq_d = c->bin_sum_d + nk;
-    CK(cudaMallocHost(reinterpret_cast<void**>(&c->ar_h), sizeof(double) * (3 * nk + 1)));
+    CK(cudaMallocHost(reinterpret_cast<void**>(&c->ar_h), sizeof(double) * (4 * nk + 1)));
     c->io_h = c->ar_h + nk + 1;
     c->TimeTransfer = TimeTransfer;
     c->loga0 = log(TimeTransfer);
@@ -736,7 +738,7 @@ extern "C" int kspace_gpu_save_nu_power(kspace_ctx* c, double Time, int snapnum,
 // A call's preparation with Na knots at scale factor a (launch_integrator_prepare).
 static void prepare_call(kspace_ctx* c, int Na, double a, double loga, int start_row, int write_knot, RowsMode rows,
                          int nk, int update_row, cudaStream_t st, bool scalars_only = false,
-                         const FinalizeArgs* fin = nullptr) {
+                         const FinalizeArgs* fin = nullptr, const CallInput& in = CallInput{}) {
     // hybrid neutrinos: room for J's tables, with the first call that can need them (without it
     // the integrals evaluate the series)
     if (c->hB.hyb_enabled && !c->I.hyb && dalloc(&c->I.hyb, (size_t)kNuSpecies * kHybTable) != cudaSuccess) {
@@ -744,7 +746,7 @@ static void prepare_call(kspace_ctx* c, int Na, double a, double loga, int start
         c->I.hyb = nullptr;
     }
     launch_integrator_prepare(c->I, c->hB, c->S0, Na, a, loga, c->loga0, c->TimeTransfer, start_row, write_knot,
-                              scalars_only, rows, nk, update_row, fin, st);
+                              scalars_only, rows, nk, update_row, fin, st, in);
 }
 
 // delta_tot_table.c:79-149 (host bookkeeping; numbers on the device)
@@ -790,7 +792,8 @@ static int delta_tot_init(kspace_ctx* c, int nk_in, const double* keff_d, const 
 // at the end; the correction pass reads the status word itself and leaves the grid as it
 // is after an error, which the step's final status check reports.
 static int update_device(kspace_ctx* c, double a, int nk_in, const double* keff_d, const double* dcdm_d,
-                         double* dnu_out_d, bool want_corr, const FinalizeArgs* fin = nullptr, bool sync = true) {
+                         double* dnu_out_d, bool want_corr, const FinalizeArgs* fin = nullptr, bool sync = true,
+                         const CallInput& in = CallInput{}, unsigned* status_out = nullptr) {
     NEED(c->table_ready && c->hubble_ready, KSPACE_ERR_ORDER);
     IntegratorDev& I = c->I;
     // side-stream work queued by start_prep writes the integrator's tables (the row
@@ -834,7 +837,7 @@ static int update_device(kspace_ctx* c, double a, int nk_in, const double* keff_
             CK(cudaMemcpyAsync(I.dnu, I.nu_last, sizeof(double) * c->nk, cudaMemcpyDeviceToDevice, c->stream));
             launch_finish_update(I, c->nk, -2, a, loga, want_corr ? keff_d : nullptr, dnu_out_d,
                                  want_corr ? c->logk_d : nullptr, want_corr ? c->ratio_d : nullptr,
-                                 want_corr ? c->corr : CorrTable{}, c->norm_d, c->stream);
+                                 want_corr ? c->corr : CorrTable{}, c->norm_d, c->stream, false, false, status_out);
             g_launches += 2;
         }
         return sync ? sync_status(c) : KSPACE_OK;
@@ -852,7 +855,7 @@ static int update_device(kspace_ctx* c, double a, int nk_in, const double* keff_
         launch_integrator_rest(I, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, prov_row,
                                true, fin, c->prep_base);
     } else {
-        prepare_call(c, Na, a, loga, c->fact_valid, 1, kRowsFull, c->nk, prov_row, c->stream);
+        prepare_call(c, Na, a, loga, c->fact_valid, 1, kRowsFull, c->nk, prov_row, c->stream, false, nullptr, in);
         launch_integrator_rest(I, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, -1, true);
     }
     I.kq = nullptr;
@@ -862,7 +865,7 @@ static int update_device(kspace_ctx* c, double a, int nk_in, const double* keff_
     const bool commit = a >= exp(c->h_scalefact[Na - 2]) + 0.009;
     launch_finish_update(I, c->nk, commit ? Na - 1 : -1, a, loga, want_corr ? keff_d : nullptr, dnu_out_d,
                          want_corr ? c->logk_d : nullptr, want_corr ? c->ratio_d : nullptr,
-                         want_corr ? c->corr : CorrTable{}, c->norm_d, c->stream, true, logk_ready);
+                         want_corr ? c->corr : CorrTable{}, c->norm_d, c->stream, true, logk_ready, status_out);
     g_launches += prepared ? 2 : 4;
     if (commit) {
         c->fact_valid = Na - 2 > 0 ? Na - 2 : 0;
@@ -880,28 +883,40 @@ extern "C" int kspace_gpu_get_delta_nu_update(kspace_ctx* c, double a, int nk, c
     NEED(nk <= c->I.nk_alloc, KSPACE_ERR_NK_ALLOC);
     double* kd = c->io_d;
     const size_t n = nk;
-    // through pinned memory: one copy in, one wait for the result and the status (copies from
-    // and to the caller's pageable memory took a wait of their own).  Anything else than plain
-    // host memory is left to the copies themselves.
+    // Through pinned memory, which the call's own kernels read and write: the preparation takes
+    // the inputs, the last kernel leaves the result and the status, and the call waits once
+    // (copies of either took 2-4 us each: 64 bins x 16 rows 72 -> 64 us).  The first call's initialisation
+    // and a repeated scale factor need the inputs earlier; anything else than plain host memory
+    // is left to the copies themselves.
     const bool pinned = !is_device_ptr(keff) && !is_device_ptr(P_cdm_sqrt) && !is_device_ptr(delta_nu);
-    if (pinned) {
-        memcpy(c->io_h, keff, sizeof(double) * n);
-        memcpy(c->io_h + n, P_cdm_sqrt, sizeof(double) * n);
-        CK(cudaMemcpyAsync(kd, c->io_h, sizeof(double) * 2 * n, cudaMemcpyHostToDevice, c->stream));
-    } else {
+    if (!pinned) {
         CK(cudaMemcpyAsync(kd, keff, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
-        CK(cudaMemcpyAsync(kd + n, P_cdm_sqrt, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(c->I.dcdm, P_cdm_sqrt, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
+        const int st = update_device(c, a, nk, kd, c->I.dcdm, c->dnu_out_d, false);
+        if (st) return st;
+        CK(cudaMemcpy(delta_nu, c->dnu_out_d, sizeof(double) * n, cudaMemcpyDeviceToHost));
+        return KSPACE_OK;
     }
-    int st = update_device(c, a, nk, kd, kd + n, c->dnu_out_d, false, nullptr, false);
+    memcpy(c->io_h, keff, sizeof(double) * n);
+    memcpy(c->io_h + n, P_cdm_sqrt, sizeof(double) * n);
+    double* out = c->io_h + 2 * n;
+    CallInput in;
+    if (c->hubble_ready && c->init_done && nk == c->nk && nk >= 2 && c->ia >= 1 && c->ia < c->I.namax &&
+        !c->prep_valid && !(log(a) - c->h_scalefact[c->ia - 1] < kFloatAcc)) {
+        in = CallInput{c->io_h, kd, c->I.dcdm, nk};
+    } else {
+        CK(cudaMemcpyAsync(kd, c->io_h, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(c->I.dcdm, c->io_h + n, sizeof(double) * n, cudaMemcpyHostToDevice, c->stream));
+    }
+    *c->status_h = kStTimeout;  // until the last kernel writes it
+    int st = update_device(c, a, nk, kd, c->I.dcdm, out, false, nullptr, false, in, c->status_h);
     if (st) {
         cudaStreamSynchronize(c->stream);  // the inputs are free again
         return st;
     }
-    if (pinned) CK(cudaMemcpyAsync(c->io_h, c->dnu_out_d, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
-    st = sync_status(c);
+    st = sync_status(c, true);
     if (st) return st;
-    if (pinned) memcpy(delta_nu, c->io_h, sizeof(double) * n);
-    else CK(cudaMemcpy(delta_nu, c->dnu_out_d, sizeof(double) * n, cudaMemcpyDeviceToHost));
+    memcpy(delta_nu, out, sizeof(double) * n);
     return KSPACE_OK;
 }
 

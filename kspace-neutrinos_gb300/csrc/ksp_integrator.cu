@@ -268,6 +268,8 @@ struct PrepArgs {
     int Na, nodes;
     int start_row, write_knot;
     int knot_blocks, fs_blocks, node_blocks, hyb_blocks;  // hyb_blocks: per species
+    int in_blocks;
+    CallInput in;
 };
 
 // Block 0: the call's scalars to the device.  Then the knots' spacings and factorised spline system
@@ -289,6 +291,13 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, 
         return;
     }
     b--;
+    if (b < P.in_blocks) {  // the call's inputs, across the host's link
+        const int i = b * kPrepThreads + t;
+        if (i < P.in.n) P.in.k[i] = P.in.src[i];
+        else if (i < 2 * P.in.n) P.in.dcdm[i - P.in.n] = P.in.src[i];
+        return;
+    }
+    b -= P.in_blocks;
     if (b < P.knot_blocks) {
         const double* x = I.scalefact;
         auto knot = [&](int j) { return P.write_knot && j == Na - 1 ? P.loga : x[j]; };
@@ -723,7 +732,7 @@ size_t dnu_qag_smem(int ld, int wpb) {
 void launch_integrator_prepare(const IntegratorDev& I, const Background& B, const StepScalars& S, int Na, double a,
                                double loga, double loga0, double TimeTransfer, int start_row, int write_knot,
                                bool scalars_only, RowsMode rows, int nk, int update_row, const FinalizeArgs* fin,
-                               cudaStream_t st) {
+                               cudaStream_t st, const CallInput& in) {
     static const GL4 gl = gl4_host();
     PrepArgs P{};
     P.S = S;
@@ -737,6 +746,8 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
         k_prep_eval<<<1, kPrepThreads, 0, st>>>(I, P, gl);
         return;
     }
+    P.in = in;
+    P.in_blocks = (2 * in.n + kPrepThreads - 1) / kPrepThreads;
     P.knot_blocks = (Na - 1 + kPrepThreads - 1) / kPrepThreads;
     if (loga > loga0) {  // the fslength table also gives fslength(log a0, log a)
         P.fs = fs_grid(16 * (Na > 1 ? Na : 1), loga0, loga);
@@ -745,7 +756,8 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
         P.node_blocks = (P.nodes + kPrepThreads - 1) / kPrepThreads;
         if (I.hyb && P.S.partnu > 0 && !P.S.skip_integral) P.hyb_blocks = kHybPieces / 8;
     }
-    k_prep_eval<<<1 + P.knot_blocks + P.fs_blocks + kNuSpecies * P.hyb_blocks + P.node_blocks, kPrepThreads, 0, st>>>(I, P, gl);
+    const int roles = P.in_blocks + P.knot_blocks + P.fs_blocks + kNuSpecies * P.hyb_blocks + P.node_blocks;
+    k_prep_eval<<<1 + roles, kPrepThreads, 0, st>>>(I, P, gl);
     const int nrow = rows == kRowsBase ? nk + 1 : (rows == kRowsFull && (Na > 2 || update_row >= 0) ? nk : 0);
     const int blocks = nrow + fs_table_blocks(P.fs.n, kTableThreads) +
                        (P.nodes + kTableThreads - 1) / kTableThreads;
@@ -826,7 +838,7 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
 // -3: a differentiable step: like -1 but delta_nu_last is left unchanged.
 __global__ void k_finish(IntegratorDev I, int nk, int commit_row, double a, double loga, const double* keff,
                          double* dnu_out, double* logk_out, double* ratio_out, CorrTable corr, double* norm_out,
-                         int combine, int logk_ready) {
+                         int combine, int logk_ready, unsigned* status_out) {
     ptx::dep_wait();
     ptx::dep_launch();
     const StepScalars& S = *I.sc;
@@ -881,13 +893,22 @@ __global__ void k_finish(IntegratorDev I, int nk, int commit_row, double a, doub
             }
         }
     }
+    if (status_out) {  // the call's status to the host, from the last block (of one warp) to end
+        __threadfence();
+        __syncwarp();
+        if (threadIdx.x == 0 && atomicInc(I.done, gridDim.x - 1) == gridDim.x - 1) {
+            __threadfence();
+            *status_out = *reinterpret_cast<volatile unsigned*>(I.status);
+        }
+    }
 }
 
 void launch_finish_update(const IntegratorDev& I, int nk, int commit_row, double a, double loga,
                           const double* keff, double* dnu_out, double* logk_out, double* ratio_out,
-                          CorrTable corr, double* norm_out, cudaStream_t st, bool combine, bool logk_ready) {
+                          CorrTable corr, double* norm_out, cudaStream_t st, bool combine, bool logk_ready,
+                          unsigned* status_out) {
     launch_dependent(k_finish, (nk + 31) / 32 > 0 ? (nk + 31) / 32 : 1, 32, 0, st, I, nk, commit_row, a, loga, keff,
-                     dnu_out, logk_out, ratio_out, corr, norm_out, combine ? 1 : 0, logk_ready ? 1 : 0);
+                     dnu_out, logk_out, ratio_out, corr, norm_out, combine ? 1 : 0, logk_ready ? 1 : 0, status_out);
 }
 
 }  // namespace ksp

@@ -56,6 +56,7 @@ struct IntegratorDev {
     double2* nc_cd;
     int2* nc_jf;
     double* nc_half;                 // [kNcMaxSlots]
+    unsigned* done;                  // blocks of k_finish that are through (0 between calls)
     const double* jt;                // J's fine table (one per device)
     double* hyb;                     // optional: [kNuSpecies][kHybTable] the tables of J with a cut
     int nc_slots;                    // slots of the node table in use (1 + 2 levels, 0 = none)
@@ -389,12 +390,19 @@ enum RowsMode {
     kRowsFull   // every row's spline; update_row >= 0: after writing the provisional row
                 // `update_row` (update_delta_tot, from delta_nu_last and delta_cdm)
 };
+// in: a call's k and delta_cdm in pinned host memory, read by the preparation itself
+struct CallInput {
+    const double* src = nullptr;  // [n] k, then [n] delta_cdm
+    double* k = nullptr;
+    double* dcdm = nullptr;
+    int n = 0;
+};
 // S: the table's scalars (light, prefac, Omeganonu); B: the background's host copy
 // fin (kRowsBase): the binning pass's normalisation, whose geometry part (keff) is formed here
 void launch_integrator_prepare(const IntegratorDev& I, const Background& B, const StepScalars& S, int Na, double a,
                                double loga, double loga0, double TimeTransfer, int start_row, int write_knot,
                                bool scalars_only, RowsMode rows, int nk, int update_row, const FinalizeArgs* fin,
-                               cudaStream_t st);
+                               cudaStream_t st, const CallInput& in = CallInput{});
 // The rest: the integrals and the species sum (get_delta_nu_combined,
 // delta_tot_table.c:153-172, writes I.dnu).
 // update_row >= 0: with a prepared step's provisional row first (base_ready: kRowsBase ran);
@@ -411,7 +419,7 @@ size_t dnu_qag_smem(int ld, int wpb);
 void launch_finish_update(const IntegratorDev& I, int nk, int commit_row, double a, double loga,
                           const double* keff, double* dnu_out, double* logk_out, double* ratio_out,
                           CorrTable corr, double* norm_out, cudaStream_t st, bool combine = false,
-                          bool logk_ready = false);
+                          bool logk_ready = false, unsigned* status_out = nullptr);
 
 // ---- adjoint (ksp_adjoint.cu)
 struct AdjBinsHost {

@@ -1321,7 +1321,7 @@ static int start_prep(kspace_ctx* c, const Geo* G, double Time) {
 // units), dcdm and keff (physical) for the integrator.  prep_time > 0: start the
 // integrator's preparation for that scale factor once the binning pass is queued.
 static int bin_grid(kspace_ctx* c, Geo* G, const float* gd, int pmgrid, int slab0, int nslab, double BoxSize,
-                    const SlabChunks* ch = nullptr, double prep_time = 0) {
+                    const SlabChunks* ch = nullptr, double prep_time = 0, const SpectrumOut& host = SpectrumOut{}) {
     NEED(c->table_ready && c->buf_nb >= G->g.nrbins, KSPACE_ERR_ORDER);
     const int nb = G->g.nrbins;
     G->g.slab0 = slab0;
@@ -1370,7 +1370,7 @@ static int bin_grid(kspace_ctx* c, Geo* G, const float* gd, int pmgrid, int slab
     if (!(prep_time > 0 && c->prep_valid)) {
         // a prepared step does it in its integral kernel instead (update_device)
         launch_finalize_power(c->bin_sum_d, c->F0sq_d, G->count_d, G->ksum_d, G->compact_d, G->nk, BoxSize,
-                              c->power_d, c->keffg_d, c->I.dcdm, c->keff_d, c->stream);
+                              c->power_d, c->keffg_d, c->I.dcdm, c->keff_d, c->stream, host);
         g_launches += 1;
         c->fin.active = 0;
     }
@@ -1390,12 +1390,13 @@ extern "C" int kspace_gpu_total_powerspectrum(kspace_ctx* c, int dims, const voi
     bool staged;
     st = grid_in(c, grid, bytes, &gd, &staged);
     if (st) return st;
-    st = bin_grid(c, G, gd, dims, startslab, nslab, 1.0);
+    // the normalisation writes the spectrum and the status to pinned memory
+    *c->status_h = kStTimeout;
+    st = bin_grid(c, G, gd, dims, startslab, nslab, 1.0, nullptr, 0,
+                  SpectrumOut{c->io_h, c->status_h, c->status_d, c->I.done});
     if (st) return st;
     const size_t n = G->nk;
-    CK(cudaMemcpyAsync(c->io_h, c->power_d, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(c->io_h + n, c->keffg_d, sizeof(double) * n, cudaMemcpyDeviceToHost, c->stream));
-    st = sync_status(c);
+    st = sync_status(c, true);
     if (st) return st;
     memcpy(power, c->io_h, sizeof(double) * n);
     memcpy(keffs, c->io_h + n, sizeof(double) * n);

@@ -412,20 +412,27 @@ void launch_k2_histogram(int N, int slab0, int nslab, unsigned long long* hist, 
 __global__ void k_finalize_power(const double* bin_sum, const double* F0sq, const long long* count,
                                  const double* ksum, const int* compact_bins, int nk, double BoxSize,
                                  double* power_out, double* keff_out, double* dcdm_out, double* keffphys_out,
-                                 double scale, double kfac) {
+                                 double scale, double kfac, SpectrumOut host) {
+    ptx::dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nk) return;
-    const FinalizeArgs f{bin_sum, F0sq,   count,   ksum,         compact_bins, BoxSize, power_out,
-                         keff_out, dcdm_out, keffphys_out, 1, scale, kfac};
-    finalize_bin(f, c);
+    if (c < nk) {
+        const FinalizeArgs f{bin_sum, F0sq,   count,   ksum,         compact_bins, BoxSize, power_out,
+                             keff_out, dcdm_out, keffphys_out, 1, scale, kfac};
+        finalize_bin(f, c);
+        if (host.out) {
+            host.out[c] = power_out[c];
+            host.out[nk + c] = keff_out[c];
+        }
+    }
+    if (host.status_out) deliver_status(host.status, host.done, host.status_out);
 }
 void launch_finalize_power(const double* bin_sum, const double* F0sq, const long long* count, const double* ksum,
                            const int* compact_bins, int nk, double BoxSize, double* power_out, double* keff_out,
-                           double* dcdm_out, double* keffphys_out, cudaStream_t st) {
+                           double* dcdm_out, double* keffphys_out, cudaStream_t st, const SpectrumOut& host) {
     // a warp per block: the FP64 pow, sqrt and divisions of the bins spread over SMs
-    k_finalize_power<<<(nk + 31) / 32, 32, 0, st>>>(bin_sum, F0sq, count, ksum, compact_bins, nk, BoxSize, power_out,
-                                                    keff_out, dcdm_out, keffphys_out, pow(BoxSize, -3.0),
-                                                    2 * 3.14159265358979323846 / BoxSize);
+    launch_dependent(k_finalize_power, (nk + 31) / 32, 32, 0, st, bin_sum, F0sq, count, ksum, compact_bins, nk, BoxSize,
+                     power_out, keff_out, dcdm_out, keffphys_out, pow(BoxSize, -3.0),
+                     2 * 3.14159265358979323846 / BoxSize, host);
 }
 
 // ------------------------------------------------------------------ host launchers

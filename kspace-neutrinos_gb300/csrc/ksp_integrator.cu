@@ -893,14 +893,7 @@ __global__ void k_finish(IntegratorDev I, int nk, int commit_row, double a, doub
             }
         }
     }
-    if (status_out) {  // the call's status to the host, from the last block (of one warp) to end
-        __threadfence();
-        __syncwarp();
-        if (threadIdx.x == 0 && atomicInc(I.done, gridDim.x - 1) == gridDim.x - 1) {
-            __threadfence();
-            *status_out = *reinterpret_cast<volatile unsigned*>(I.status);
-        }
-    }
+    if (status_out) deliver_status(I.status, I.done, status_out);
 }
 
 void launch_finish_update(const IntegratorDev& I, int nk, int commit_row, double a, double loga,

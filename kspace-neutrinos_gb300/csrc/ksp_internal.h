@@ -316,7 +316,24 @@ struct FinalizeArgs {
     double scale, kfac;
     double* logk_out;  // log of the physical keff (finalize_keff)
 };
+// A spectrum in pinned host memory: [nk] power, then [nk] keff, and the status word from the last
+// of the kernel's blocks to end (they count themselves in done, 0 between calls).
+struct SpectrumOut {
+    double* out = nullptr;
+    unsigned* status_out = nullptr;
+    const unsigned* status = nullptr;
+    unsigned* done = nullptr;
+};
 #ifdef __CUDACC__
+// The status word to the host from the last block (of one warp) of a kernel to end.
+__device__ __forceinline__ void deliver_status(const unsigned* status, unsigned* done, unsigned* out) {
+    __threadfence();
+    __syncwarp();
+    if (threadIdx.x == 0 && atomicInc(done, gridDim.x - 1) == gridDim.x - 1) {
+        __threadfence();
+        *out = *reinterpret_cast<const volatile unsigned*>(status);
+    }
+}
 // the part that depends on the sums, and the part that is the geometry's alone (a prepared
 // step forms the latter beside the binning pass); p: the bin's power, returned: delta_cdm
 __device__ __forceinline__ double finalize_power(const FinalizeArgs& f, int c, double* p_out) {
@@ -461,7 +478,8 @@ int launch_apply_correction(const GridGeom& g, float* grid, CorrTable corr, floa
 // interface_gadget.c:96-100)
 void launch_finalize_power(const double* bin_sum, const double* F0sq, const long long* count, const double* ksum,
                            const int* compact_bins, int nk, double BoxSize, double* power_out, double* keff_out,
-                           double* dcdm_out, double* keffphys_out, cudaStream_t st);
+                           double* dcdm_out, double* keffphys_out, cudaStream_t st,
+                           const SpectrumOut& host = SpectrumOut{});
 
 struct GridGeom;
 void launch_adj_reduce(const GridGeom& gg, CorrTable corr, float lnscale, const float* gbar, const float* x,

@@ -1269,6 +1269,7 @@ __global__ void __launch_bounds__(WHOLE ? mirror_max_warps(K, true) * 32 : 512)
                  const unsigned* __restrict__ runtab) {
     typedef typename SpillOf<EXACT>::type Spill;
     extern __shared__ unsigned char sm_raw[];
+    ptx::dep_launch();
     const int W = blockDim.x >> 5;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const StreamPlan Pl = plan_bin_mirror(W, g.nrbins, g.nz, EXACT, T);

@@ -805,54 +805,65 @@ __device__ QagResult qag_block_c(const F& f, const Gk61Nodes& N, QagList& L, dou
 }
 
 // ------------------------------------------------------------------ block QAG with look-ahead
-// qag_block_c with one level of look-ahead.  On these integrands QAG nearly always
+// qag_block_c with G - 1 levels of look-ahead.  On these integrands QAG nearly always
 // bisects next the right half it has just made (the late-time end, where delta_tot and
 // the free-streaming kernel change fastest).  A round that evaluates the halves of
-// interval k therefore also evaluates the halves of k's right half; when the next round
-// picks that half, its rule results are already there and the round is bookkeeping only,
-// so the sequential evaluation rounds are halved.  Node values come from the same
+// interval k therefore also evaluates the halves of k's right half, and so on down G levels
+// (the first round: the whole interval and G - 1 levels); while the next rounds pick those
+// halves, their rule results are already there and the rounds are bookkeeping only, so that
+// the sequential evaluation rounds are 1/G as many.  Node values come from the same
 // node_at, and each interval's sums are formed by one warp in the lane layout of a
 // two-interval gk61_block_c call, so every rule result is that of qag_block_c (to the
 // last bits, which the compiler's multiply-add contraction may change from kernel to
-// kernel) and so is every decision.  blockDim.x = 256: the 244 node slots of a round in
-// one pass.  Shared scratch: QagSpecSmem.
+// kernel) and so is every decision.  blockDim.x = 128 G: a round's 122 G nodes in one pass.
+template <int G>
 struct QagSpecSmem {
-    double fv[244];  // group A: slots [0, 122), group B: [122, 244)
-    GkOut out[4];    // group A intervals 0, 1 | group B intervals 0, 1
-    GkOut pg[2];     // rule results of the halves of list entry pre_k
-    double ic[4], ih[4];  // centre and half-width of the intervals of the next evaluation
-    int isl[4];           // and their node-table slots
-    int k, hit, cont, ok, pre_k;
+    double fv[122 * G];          // group (level) g: slots [122 g, 122 g + 122)
+    GkOut out[2 * G];            // group g: intervals 2 g, 2 g + 1
+    double ic[2 * G], ih[2 * G]; // centre and half-width of the intervals of the next evaluation
+    int isl[2 * G];              // and their node-table slots
+    int k, hit, cont, ok;
+    int pre_k, pre_g;            // the list entry whose halves group pre_g holds (-1: none)
     double errsum;
 };
 
 // Interval q of the next evaluation: its slot, or its geometry, formed once (one thread).
-__device__ __forceinline__ void spec_set_interval(QagSpecSmem& sh, int q, double a, double b, int slot) {
+template <int G>
+__device__ __forceinline__ void spec_set_interval(QagSpecSmem<G>& sh, int q, double a, double b, int slot) {
     sh.isl[q] = slot;
     if (slot >= 0) return;
     sh.ic[q] = __dmul_rn(0.5, __dadd_rn(a, b));
     sh.ih[q] = __dmul_rn(0.5, __dsub_rn(b, a));
 }
+// Groups g0 .. G - 1: the halves of [a, b] (slot), of its right half, ...
+template <int G>
+__device__ __forceinline__ void spec_set_halves(QagSpecSmem<G>& sh, int g0, double a, double b, int slot, int ns) {
+    for (int g = g0; g < G; g++) {
+        const double m = 0.5 * (a + b);
+        spec_set_interval(sh, 2 * g, a, m, nc_child(slot, 0, ns));
+        slot = nc_child(slot, 1, ns);
+        spec_set_interval(sh, 2 * g + 1, m, b, slot);
+        a = m;
+    }
+}
 
-// Rule results of two groups of intervals, nA in {1, 2} (intervals 0, 1) and nB in
-// {0, 1, 2} (intervals 2, 3), whose geometry is in sh.ic / sh.ih / sh.isl.  Warp 0 sums
-// group A, warp 1 group B, each as gk61_block_c sums a call of that many intervals.
-template <class F>
-__device__ __forceinline__ void gk61_block_groups(const F& f, const Gk61Nodes& N, int nA, int nB, QagSpecSmem& sh) {
+// Rule results of the groups' intervals (n0 in {1, 2} of group 0), whose geometry is in
+// sh.ic / sh.ih / sh.isl.  Warp g sums group g as gk61_block_c sums a call of that many
+// intervals.
+template <int G, class F>
+__device__ __forceinline__ void gk61_block_groups(const F& f, const Gk61Nodes& N, int n0, QagSpecSmem<G>& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int s = tid; s < 244; s += blockDim.x) {
-        const int g = s >= 122 ? 1 : 0;
-        const int u = s - 122 * g;
-        const int t = u >= 61 ? 1 : 0;
-        const int j = u - 61 * t;
-        if (t < (g ? nB : nA)) {
+    if (tid < 122 * G) {
+        const int g = tid / 122, u = tid - 122 * g;
+        const int t = u >= 61 ? 1 : 0, j = u - 61 * t;
+        if (g > 0 || t < n0) {
             const int q = 2 * g + t;
-            sh.fv[s] = f.node_at(sh.isl[q], j, sh.ic[q], sh.ih[q], N.x[j]);
+            sh.fv[tid] = f.node_at(sh.isl[q], j, sh.ic[q], sh.ih[q], N.x[j]);
         }
     }
     __syncthreads();
-    const int ng = warp == 0 ? nA : (warp == 1 ? nB : 0);
-    if (ng > 0) {  // warp-uniform
+    if (warp < G) {
+        const int ng = warp == 0 ? n0 : 2;
         const double* fvg = sh.fv + 122 * warp;
         double fv[4];
 #pragma unroll
@@ -876,25 +887,23 @@ __device__ __forceinline__ void gk61_block_groups(const F& f, const Gk61Nodes& N
     __syncthreads();
 }
 
-template <class F>
+template <int G, class F>
 __device__ QagResult qag_block_spec_c(const F& f, const Gk61Nodes& N, QagList& L, double a, double b, double epsabs,
-                                      double epsrel, int limit, QagSpecSmem& sh) {
+                                      double epsrel, int limit, QagSpecSmem<G>& sh) {
     const int tid = threadIdx.x, lane = tid & 31;
     const int ns = f.nc.nslots;
     QagResult R;
     const int s0 = ns > 0 ? 0 : -1;
-    if (tid == 0) {  // the root, and its halves ahead
-        const double m = 0.5 * (a + b);
+    if (tid == 0) {  // the root, and halves ahead
         spec_set_interval(sh, 0, a, b, s0);
-        spec_set_interval(sh, 2, a, m, nc_child(s0, 0, ns));
-        spec_set_interval(sh, 3, m, b, nc_child(s0, 1, ns));
+        spec_set_halves(sh, 1, a, b, s0, ns);
     }
     __syncthreads();
-    gk61_block_groups(f, N, 1, 2, sh);
+    gk61_block_groups(f, N, 1, sh);
     const GkOut g0 = sh.out[0];
     if (tid == 0) {
         L.a[0] = a; L.b[0] = b; L.r[0] = g0.result; L.e[0] = g0.abserr; L.slot[0] = s0;
-        sh.pre_k = 0; sh.pg[0] = sh.out[2]; sh.pg[1] = sh.out[3];
+        sh.pre_k = 0; sh.pre_g = 1;
     }
     __syncthreads();
     double tol = fmax(epsabs, epsrel * fabs(g0.result));
@@ -910,46 +919,31 @@ __device__ QagResult qag_block_spec_c(const F& f, const Gk61Nodes& N, QagList& L
     do {
         // warp 0 finds the interval of largest error (lowest index on ties); its lane 0
         // notes whether the halves are already evaluated and, if not, lays out the halves
-        // of k and of k's right half
+        // of k, of k's right half, ...
         if (tid < 32) {
             const int bk = warp_argmax_err(L.e, n);
             if (lane == 0) {
                 const bool hit = bk == sh.pre_k;
                 sh.k = bk;
                 sh.hit = hit;
-                if (!hit) {
-                    const double a_i = L.a[bk], b_i = L.b[bk];
-                    const int s_i = L.slot[bk];
-                    const double b1 = 0.5 * (a_i + b_i);
-                    const double m2 = 0.5 * (b1 + b_i);
-                    const int c1 = nc_child(s_i, 1, ns);
-                    spec_set_interval(sh, 0, a_i, b1, nc_child(s_i, 0, ns));
-                    spec_set_interval(sh, 1, b1, b_i, c1);
-                    spec_set_interval(sh, 2, b1, m2, nc_child(c1, 0, ns));
-                    spec_set_interval(sh, 3, m2, b_i, nc_child(c1, 1, ns));
-                }
+                if (!hit) spec_set_halves(sh, 0, L.a[bk], L.b[bk], L.slot[bk], ns);
             }
         }
         __syncthreads();
         const int k = sh.k;
-        if (!sh.hit) gk61_block_groups(f, N, 2, 2, sh);  // block-uniform
+        if (!sh.hit) gk61_block_groups(f, N, 2, sh);  // block-uniform
         // QUADPACK's bookkeeping on thread 0
         if (tid == 0) {
-            const bool hit = sh.hit;
+            const int gi = sh.hit ? sh.pre_g : 0;
             const double a_i = L.a[k], b_i = L.b[k], r_i = L.r[k], e_i = L.e[k];
             const int s_i = L.slot[k];
             const double a1 = a_i, b1 = 0.5 * (a_i + b_i), a2 = b1, b2 = b_i;
-            const GkOut g[2] = {hit ? sh.pg[0] : sh.out[0], hit ? sh.pg[1] : sh.out[1]};
+            const GkOut g[2] = {sh.out[2 * gi], sh.out[2 * gi + 1]};
             sh.cont = qag_account(q, g, r_i, e_i, a1, a2, b2, epsabs, epsrel, limit);
             L.b[k] = b1; L.r[k] = g[0].result; L.e[k] = g[0].abserr; L.slot[k] = nc_child(s_i, 0, ns);
             L.a[n] = a2; L.b[n] = b2; L.r[n] = g[1].result; L.e[n] = g[1].abserr; L.slot[n] = nc_child(s_i, 1, ns);
-            if (hit) {
-                sh.pre_k = -1;
-            } else {
-                sh.pre_k = n;
-                sh.pg[0] = sh.out[2];
-                sh.pg[1] = sh.out[3];
-            }
+            sh.pre_k = gi + 1 < G ? n : -1;
+            sh.pre_g = gi + 1;
             sh.errsum = q.errsum;
             sh.ok = q.errsum <= q.tol;
         }

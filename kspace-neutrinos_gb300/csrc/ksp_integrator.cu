@@ -500,12 +500,12 @@ __global__ void __launch_bounds__(128) k_dnu_qag(IntegratorDev I, int nk, int Na
     }
 }
 
-// One (species, bin) task per block of 8 warps: the same integral as k_dnu_qag with the
-// GK61 nodes of each step spread over the block and one bisection level evaluated ahead
+// One (species, bin) task per block of 4 G warps: the same integral as k_dnu_qag with the
+// GK61 nodes of each step spread over the block and G - 1 bisection levels evaluated ahead
 // (qag_block_spec_c: the same decisions, sums equal to the last bits).  For calls with few tasks, where one warp
 // per task leaves the SMs' FP64 pipes idle between the long dependent chains of a single
 // warp and the sequential QAG rounds set the time.
-// SPEC = false: blocks of 4 warps and qag_block_c (no look-ahead).
+// G: levels of a round (0: blocks of 2 or 4 warps and qag_block_c, no look-ahead).
 // upd.row >= 0: a prepared step's provisional row (k_row_update's arithmetic, per task, while
 // the row is on its way, instead of a launch of its own before this one: 7 us).
 // Shared memory: Gk61Nodes | row[ld] | coef[ld] | QagList | QagSpecSmem or QagBlockSmem | mbarrier
@@ -513,15 +513,16 @@ struct RowUpdate {
     int row;
     FinalizeArgs fin;
 };
-template <bool SPEC>
-struct QagBlkSmemOf { typedef QagSpecSmem type; };
+constexpr int qag_blk_threads(int G) { return G > 0 ? 128 * G : 128; }
+template <int G>
+struct QagBlkSmemOf { typedef QagSpecSmem<G> type; };
 template <>
-struct QagBlkSmemOf<false> { typedef QagBlockSmem type; };
+struct QagBlkSmemOf<0> { typedef QagBlockSmem type; };
 
-template <bool SPEC>
-__global__ void __launch_bounds__(SPEC ? 256 : 128, SPEC ? 2 : 4)
+template <int G>
+__global__ void __launch_bounds__(qag_blk_threads(G), 512 / qag_blk_threads(G))
     k_dnu_qag_blk(IntegratorDev I, int nk, int Na, int nspec, int4 spec_ids, RowUpdate upd) {
-    typedef typename QagBlkSmemOf<SPEC>::type Smem;
+    typedef typename QagBlkSmemOf<G>::type Smem;
     extern __shared__ __align__(16) unsigned char sm[];
     ptx::dep_wait();
     ptx::dep_launch();
@@ -610,7 +611,7 @@ __global__ void __launch_bounds__(SPEC ? 256 : 128, SPEC ? 2 : 4)
         const double kom = (I.kq ? I.kq[ik] : I.wavenum[ik]) * S.inv_m[mi];
         const DnuIntegrandW f = dnu_integrand_w(I, S, mi, kom, row, rc, Na);
         QagResult r;
-        if constexpr (SPEC) r = qag_block_spec_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
+        if constexpr (G > 0) r = qag_block_spec_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
         else r = qag_block_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
         if (I.ivals) {  // keep the final subdivision for the adjoint
             double* dst = I.ivals + ((size_t)mi * I.nk_alloc + ik) * kQagLimit * 2;
@@ -632,9 +633,10 @@ __global__ void __launch_bounds__(SPEC ? 256 : 128, SPEC ? 2 : 4)
     }
 }
 
-size_t dnu_qag_blk_smem(int ld, bool spec) {
+template <int G>
+static size_t dnu_qag_blk_smem(int ld) {
     return ((sizeof(Gk61Nodes) + 15) & ~size_t(15)) + 2 * sizeof(double) * ld + ((sizeof(QagList) + 15) & ~size_t(15)) +
-           (((spec ? sizeof(QagSpecSmem) : sizeof(QagBlockSmem)) + 15) & ~size_t(15)) + sizeof(uint64_t);
+           ((sizeof(typename QagBlkSmemOf<G>::type) + 15) & ~size_t(15)) + sizeof(uint64_t);
 }
 
 // delta_tot_table.c:155-170: combine the species
@@ -767,6 +769,17 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
 }
 
 // The rest, after the rows' splines: the integrals, the species sum.
+// One block per task; false: the history row does not fit shared memory.
+template <int G>
+static bool launch_dnu_qag_blk(const IntegratorDev& I, int nk, int Na, int nspec, int4 spec_ids, const RowUpdate& upd,
+                               int threads, cudaStream_t st) {
+    const size_t smem = dnu_qag_blk_smem<G>(I.ld);
+    if (smem > 227 * 1024 - 256) return false;
+    raise_dynamic_smem_limit(reinterpret_cast<const void*>(k_dnu_qag_blk<G>));
+    launch_dependent(k_dnu_qag_blk<G>, nspec * nk, threads, smem, st, I, nk, Na, nspec, spec_ids, upd);
+    return true;
+}
+
 void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, const int* spec_ids,
                             int warps_per_block, cudaStream_t st, int qag_split, int update_row, bool defer_combine,
                             const FinalizeArgs* fin, bool base_ready, bool rows_stored) {
@@ -803,25 +816,24 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
             if (nsm <= 0) nsm = 1;
         }
-        // a block per task: 8 warps with look-ahead (split 8) below 4 tasks per SM, 4 warps
-        // without up to 6 tasks per SM, 2 warps from there (at 128 registers a thread, 4
-        // blocks of 4 warps fit an SM: 1221 tasks of 3 species x 407 bins take two waves
-        // of 4-warp blocks and one of 2-warp blocks, measured 0.211 against 0.223 ms; a
+        // a block per task: with no more tasks than SMs 12 warps and two levels of look-ahead
+        // (split 12; a call of 64, 100, 150 bins 62, 71, 78 us, with 8 warps and one level 64, 74,
+        // 82; three levels 65, 75, 77; but 200 bins 86 against 82, and hybrid neutrinos' nodes,
+        // off the table, are too dear to guess), 8 warps and one level (split 8) below 4 tasks
+        // per SM, 4 warps without look-ahead up to 6, 2 warps from there (at 128 registers a
+        // thread, 4 blocks of 4 warps fit an SM: 1221 tasks of 3 species x 407 bins take two
+        // waves of 4-warp blocks and one of 2-warp blocks, measured 0.211 against 0.223 ms; a
         // warp per task, split 1, 0.231 ms)
-        const int split = qag_split > 0 ? qag_split : (ntask < 4 * nsm ? 8 : (ntask < 6 * nsm ? 4 : 2));
-        const bool spec = split >= 8;
-        const size_t bsmem = dnu_qag_blk_smem(I.ld, spec);
-        if (split > 1 && bsmem <= 227 * 1024 - 256) {
-            static bool blk_attr = false;
-            if (!blk_attr) {
-                raise_dynamic_smem_limit(reinterpret_cast<const void*>(k_dnu_qag_blk<true>));
-                raise_dynamic_smem_limit(reinterpret_cast<const void*>(k_dnu_qag_blk<false>));
-                blk_attr = true;
-            }
-            const int4 sp = make_int4(spec_ids[0], spec_ids[1], spec_ids[2], 0);
-            if (spec) launch_dependent(k_dnu_qag_blk<true>, ntask, 256, bsmem, st, I, nk, Na, nspec, sp, upd);
-            else launch_dependent(k_dnu_qag_blk<false>, ntask, split >= 4 ? 128 : 64, bsmem, st, I, nk, Na, nspec, sp, upd);
-        } else {
+        const int split = qag_split > 0       ? qag_split
+                          : ntask <= nsm && !I.hyb ? 12
+                                              : (ntask < 4 * nsm ? 8 : (ntask < 6 * nsm ? 4 : 2));
+        const int4 sp = make_int4(spec_ids[0], spec_ids[1], spec_ids[2], 0);
+        const bool done =
+            split >= 12 ? launch_dnu_qag_blk<3>(I, nk, Na, nspec, sp, upd, 384, st)
+            : split >= 8 ? launch_dnu_qag_blk<2>(I, nk, Na, nspec, sp, upd, 256, st)
+            : split > 1  ? launch_dnu_qag_blk<0>(I, nk, Na, nspec, sp, upd, split >= 4 ? 128 : 64, st)
+                         : false;
+        if (!done) {
             if (upd.row >= 0) k_row_update<<<nk, 128, 0, st>>>(I, nk, Na, upd.row, upd.fin);
             const int blocks = (ntask + wpb - 1) / wpb;
             k_dnu_qag<<<blocks, 32 * wpb, smem, st>>>(I, nk, Na, nspec,

@@ -312,11 +312,11 @@ struct DnuAdjArgs {
 // its spline second derivatives), and its mass derivative to mder (per lane).
 __device__ __forceinline__ void adj_interval(const DnuIntegrandC& fi, const Gk61Nodes& N, const double* knots,
                                              const double* row, const double* rc, int Na, double qc, double a_i,
-                                             double b_i, double loga0, double loga, int nc_slots, double ckm,
+                                             double b_i, double loga0, double loga, NcLayout lay, double ckm,
                                              double* ybar, double* cbar, double& mder, int lane) {
     const double c = __dmul_rn(0.5, __dadd_rn(a_i, b_i));
     const double h = __dmul_rn(0.5, __dsub_rn(b_i, a_i));
-    const int slot = nc_slot_of(a_i, b_i, loga0, loga, nc_slots);
+    const int slot = nc_slot_of(a_i, b_i, loga0, loga, lay);
     // nodes in ascending x (lane order): the history segments grow with the
     // lane, so a segmented warp sum per segment replaces atomic updates
     for (int m = 0; m < 2; m++) {
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(128) k_dnu_adj(IntegratorDev I, DnuAdjArgs A, 
             const double ckm = -sbar * S.prefac * fi.k_over_m / mnu;  // d(J's argument)/dm per fsl
             for (int q = 0; q < nint; q++)
                 adj_interval(fi, N, knots, row, rc, Na, qc, iv ? iv[2 * q] : L.a[q], iv ? iv[2 * q + 1] : L.b[q],
-                             S.loga0, S.loga, I.nc_slots, ckm, ybar, cbar, mder, lane);
+                             S.loga0, S.loga, NcLayout{I.nc_slots, I.nc_tree}, ckm, ybar, cbar, mder, lane);
             __syncwarp();
             if (Na > 2) {
                 // z = A^-1 cbar_int with the shared factorisation (A is symmetric, so the
@@ -673,7 +673,7 @@ __global__ void __launch_bounds__(128) k_dnu_adj_blk(IntegratorDev I, DnuAdjArgs
             double* cb = wc + (size_t)warp * I.ld;
             for (int q = warp; q < nint; q += nw)
                 adj_interval(fi, N, knots, row, rc, Na, qc, iv ? iv[2 * q] : L.a[q], iv ? iv[2 * q + 1] : L.b[q],
-                             S.loga0, S.loga, I.nc_slots, ckm, yb, cb, mder, lane);
+                             S.loga0, S.loga, NcLayout{I.nc_slots, I.nc_tree}, ckm, yb, cb, mder, lane);
             __syncthreads();
             for (int j = tid; j < Na; j += blockDim.x) {
                 double y = wy[j], c = wc[j];

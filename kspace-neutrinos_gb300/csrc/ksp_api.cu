@@ -449,6 +449,7 @@ extern "C" int kspace_gpu_alloc_table(kspace_ctx* c, int nk_alloc, double TimeTr
     I.ld = (I.namax + 1) & ~1;  // even: every row starts on a 16-byte boundary
     const size_t nk = nk_alloc, ld = I.ld;
     I.nc_slots = c->nc_levels > 0 ? 1 + 2 * c->nc_levels : 0;
+    I.nc_tree = 1;
     I.fs_cap = 16 * (int)ld + 16;
     // all of the table's arrays and the step's buffers in one allocation, each from a 256-byte
     // boundary (one call each, they were two thirds of closing an instance)
@@ -735,16 +736,45 @@ extern "C" int kspace_gpu_save_nu_power(kspace_ctx* c, double Time, int snapnum,
 }
 
 // ------------------------------------------------------------------ integrator
+// One allocation for the tables of a cut J and the node table of all shallow intervals.
+static void hyb_alloc(kspace_ctx* c) {
+    constexpr size_t n = (size_t)kNcTreeSlots * 61, nh = (size_t)kNuSpecies * kHybTable;
+    double* p = nullptr;  // (16-byte arrays first)
+    if (dalloc(&p, nh + 10 * n + kNcTreeSlots) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    c->I.hyb = p;
+    p += nh;
+    c->nc_plain = c->I.nodes();
+    NcNodes& t = c->nc_cut;
+    auto take = [&](size_t k) {
+        double* q = p;
+        p += k;
+        return q;
+    };
+    t.ab = reinterpret_cast<double2*>(take(2 * n));
+    t.cd = reinterpret_cast<double2*>(take(2 * n));
+    t.jf = reinterpret_cast<int2*>(take(n));
+    t.g = take(n);
+    t.fsl = take(n);
+    t.dx = take(n);
+    t.inv = take(n);
+    t.j = reinterpret_cast<int*>(take(n));
+    t.half = take(kNcTreeSlots);
+    t.slots = kNcTreeSlots;
+    t.tree = kNcTree;
+}
+
 // A call's preparation with Na knots at scale factor a (launch_integrator_prepare).
 static void prepare_call(kspace_ctx* c, int Na, double a, double loga, int start_row, int write_knot, RowsMode rows,
                          int nk, int update_row, cudaStream_t st, bool scalars_only = false,
                          const FinalizeArgs* fin = nullptr, const CallInput& in = CallInput{}) {
-    // hybrid neutrinos: room for J's tables, with the first call that can need them (without it
-    // the integrals evaluate the series)
-    if (c->hB.hyb_enabled && !c->I.hyb && dalloc(&c->I.hyb, (size_t)kNuSpecies * kHybTable) != cudaSuccess) {
-        cudaGetLastError();
-        c->I.hyb = nullptr;
-    }
+    // hybrid neutrinos: room for J's tables and the larger node table, with the first call that
+    // needs them (without it the integrals evaluate the series, off the smaller one)
+    const bool cut = c->hB.hyb_enabled && particle_nu_fraction(c->hB, a, 0) > 0;
+    if (cut && !c->I.hyb) hyb_alloc(c);
+    if (c->I.hyb) c->I.set_nodes(cut && c->nc_levels == kNcMaxLevels ? c->nc_cut : c->nc_plain);
     launch_integrator_prepare(c->I, c->hB, c->S0, Na, a, loga, c->loga0, c->TimeTransfer, start_row, write_knot,
                               scalars_only, rows, nk, update_row, fin, st, in);
 }
@@ -1795,20 +1825,24 @@ extern "C" int kspace_gpu_diff_forward(kspace_ctx* c, double Time, double BoxSiz
     if (st) return st;
     if (G->nk != c->nk) return KSPACE_ERR_NK_MISMATCH;
     if (c->ia >= c->I.namax) return KSPACE_ERR_NAMAX;
-    IntegratorDev Is = I;
-    if (store_intervals) {
-        Is.ivals = c->ivals_d;
-        Is.nivals = c->nivals_d;
-    }
+    auto stored = [&] {  // (after the preparation, which chooses the node table)
+        IntegratorDev Is = I;
+        if (store_intervals) {
+            Is.ivals = c->ivals_d;
+            Is.nivals = c->nivals_d;
+        }
+        return Is;
+    };
     // the adjoint reads the rows and their splines: stored before the integrals
     bool logk_ready = false;
     if (prepared) {
         logk_ready = c->fin.active && c->prep_base;
-        launch_integrator_rest(Is, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, c->ia,
+        launch_integrator_rest(stored(), c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, c->ia,
                                true, c->fin.active ? &c->fin : nullptr, c->prep_base, true);
     } else {
         prepare_call(c, Na, Time, loga, start, 1, kRowsFull, c->nk, c->ia, c->stream);
-        launch_integrator_rest(Is, c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, -1, true);
+        launch_integrator_rest(stored(), c->nk, Na, c->nspec, c->spec_ids, c->qag_warps, c->stream, c->qag_split, -1,
+                               true);
     }
     c->fin.active = 0;
     launch_finish_update(I, c->nk, -3, Time, loga, c->keff_d, c->dnu_out_d, c->logk_d, c->ratio_d, c->corr,

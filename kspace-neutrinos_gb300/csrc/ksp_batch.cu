@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kBatchTable) kb_tables(BatchDev b) {
         const int q = (blk - table_blocks) * kBatchTable + threadIdx.x;
         if (q >= b.nc_slots * 61) continue;
         double half;
-        const double x = nc_node_x(q, P.loga0, P.loga, &half);
+        const double x = nc_node_x(q, NcLayout{b.nc_slots, 1}, P.loga0, P.loga, &half);
         const double fsl = fs_table_at(F, x);
         const int j = seg_bsearch(I.scalefact, P.Na, x);
         nc_store(I, q, fsl, node_inv_aH(I.B, x), x - I.scalefact[j], j, I.scalefact[j + 1] - I.scalefact[j],

@@ -234,6 +234,7 @@ static int lay_out(kspace_batch* b, const int* nk_in) {
         desc[i].ivals = nullptr;
         desc[i].nivals = nullptr;
         desc[i].nc_slots = b->nc_slots;
+        desc[i].nc_tree = 1;
     }
     CKB(cudaMemcpy(b->insts_d, desc.data(), sizeof(IntegratorDev) * M, cudaMemcpyHostToDevice));
     if (!b->grids.empty()) {

@@ -600,20 +600,31 @@ __device__ QagResult qag_warp(const F& f, const Gk61Nodes& N, QagList& L, double
 // QAG only ever bisects, so its intervals are dyadic subintervals of [a, b].  For the
 // delta_nu integral it refines toward the upper end (log a, where J -> 1 and the newest
 // history rows are): at every depth the intervals it evaluates are the two children of
-// the rightmost interval of the depth above.  Those are numbered: slot 0 = [a, b]; at
-// depth d >= 1, slot 2d-1 the left and slot 2d the right child of the depth-(d-1)
-// rightmost interval.  A functor with node(slot, j, x) may serve the 61 nodes of such an
-// interval from a table built once; the others pass slot -1.
+// the rightmost interval of the depth above.  Those are numbered, and a functor's node_at
+// serves the 61 nodes of a numbered interval from a table built once; the others pass slot -1.
+// Where hybrid neutrinos cut J it oscillates, and the bisections go anywhere: all intervals
+// down to some depth are numbered then.  A table of `tree` = 2^(D+1) - 1 slots down to depth D
+// numbers them as a heap (slot 0 = [a, b], slot s has children 2 s + 1 and 2 s + 2), and then
+// left and right child of the rightmost interval, depth after depth; D = 0 without the cut.
 constexpr int kNcMaxLevels = 12;
 constexpr int kNcMaxSlots = 1 + 2 * kNcMaxLevels;  // 25 intervals
 constexpr int kNcNodes = kNcMaxSlots * 61;         // capacity of a node table
+constexpr int kNcTreeDepth = 6, kNcTree = (2 << kNcTreeDepth) - 1;
+constexpr int kNcTreeSlots = kNcTree + 2 * (kNcMaxLevels - kNcTreeDepth);
 
-// child slot of s (right = 0, 1) in a table of nslots = 1 + 2 levels slots
-__device__ __forceinline__ int nc_child(int s, int right, int nslots) {
-    if (s < 0 || (s > 0 && (s & 1))) return -1;  // only the rightmost intervals have cached children
-    const int d = s / 2 + 1;                      // depth of the children
-    const int c = 2 * d - 1 + right;
-    return c < nslots ? c : -1;
+struct NcLayout {
+    int nslots, tree;
+};
+// child slot of s (right = 0, 1)
+__device__ __forceinline__ int nc_child(int s, int right, NcLayout t) {
+    if (s < 0) return -1;
+    int c = 2 * s + 1 + right;
+    if (c >= t.tree) {  // past the heap only the rightmost intervals have children
+        if (s == t.tree - 1) c = t.tree + right;
+        else if (s >= t.tree && ((s - t.tree) & 1)) c = s + 1 + right;
+        else return -1;
+    }
+    return c < t.nslots ? c : -1;
 }
 
 // Centre and half-width of an interval.  A cached one's nodes need no centre, and its half-width
@@ -656,7 +667,7 @@ __device__ QagResult qag_warp_c(const F& f, const Gk61Nodes& N, QagList& L, doub
     QagResult R;
     GkOut g[2];
     double aa[2] = {a, a}, bb[2] = {b, b};
-    int ss[2] = {f.nc.nslots > 0 ? 0 : -1, -1};
+    int ss[2] = {f.nc.lay.nslots > 0 ? 0 : -1, -1};
     gk61_warp_c(f, N, 1, aa, bb, ss, g);
     if (lane == 0) { L.a[0] = a; L.b[0] = b; L.r[0] = g[0].result; L.e[0] = g[0].abserr; L.slot[0] = ss[0]; }
     __syncwarp();
@@ -676,8 +687,8 @@ __device__ QagResult qag_warp_c(const F& f, const Gk61Nodes& N, QagList& L, doub
         const int s_i = L.slot[k];
         const double a1 = a_i, b1 = 0.5 * (a_i + b_i), a2 = b1, b2 = b_i;
         aa[0] = a1; bb[0] = b1; aa[1] = a2; bb[1] = b2;
-        ss[0] = nc_child(s_i, 0, f.nc.nslots);
-        ss[1] = nc_child(s_i, 1, f.nc.nslots);
+        ss[0] = nc_child(s_i, 0, f.nc.lay);
+        ss[1] = nc_child(s_i, 1, f.nc.lay);
         gk61_warp_c(f, N, 2, aa, bb, ss, g);
         // QUADPACK's bookkeeping on lane 0 (its FP64 is not repeated on 32 lanes)
         cont = 0;
@@ -753,7 +764,7 @@ __device__ QagResult qag_block_c(const F& f, const Gk61Nodes& N, QagList& L, dou
     QagResult R;
     GkOut g[2];
     double aa[2] = {a, a}, bb[2] = {b, b};
-    int ss[2] = {f.nc.nslots > 0 ? 0 : -1, -1};
+    int ss[2] = {f.nc.lay.nslots > 0 ? 0 : -1, -1};
     gk61_block_c(f, N, 1, aa, bb, ss, g, sh);
     if (tid == 0) { L.a[0] = a; L.b[0] = b; L.r[0] = g[0].result; L.e[0] = g[0].abserr; L.slot[0] = ss[0]; }
     __syncthreads();
@@ -779,8 +790,8 @@ __device__ QagResult qag_block_c(const F& f, const Gk61Nodes& N, QagList& L, dou
         const int s_i = L.slot[k];
         const double a1 = a_i, b1 = 0.5 * (a_i + b_i), a2 = b1, b2 = b_i;
         aa[0] = a1; bb[0] = b1; aa[1] = a2; bb[1] = b2;
-        ss[0] = nc_child(s_i, 0, f.nc.nslots);
-        ss[1] = nc_child(s_i, 1, f.nc.nslots);
+        ss[0] = nc_child(s_i, 0, f.nc.lay);
+        ss[1] = nc_child(s_i, 1, f.nc.lay);
         gk61_block_c(f, N, 2, aa, bb, ss, g, sh);
         // QUADPACK's bookkeeping on thread 0
         if (tid == 0) {
@@ -828,8 +839,8 @@ struct QagSpecSmem {
 };
 
 // Interval q of the next evaluation: its slot, or its geometry, formed once (one thread).
-template <int G>
-__device__ __forceinline__ void spec_set_interval(QagSpecSmem<G>& sh, int q, double a, double b, int slot) {
+template <class S>
+__device__ __forceinline__ void spec_set_interval(S& sh, int q, double a, double b, int slot) {
     sh.isl[q] = slot;
     if (slot >= 0) return;
     sh.ic[q] = __dmul_rn(0.5, __dadd_rn(a, b));
@@ -837,7 +848,7 @@ __device__ __forceinline__ void spec_set_interval(QagSpecSmem<G>& sh, int q, dou
 }
 // Groups g0 .. G - 1: the halves of [a, b] (slot), of its right half, ...
 template <int G>
-__device__ __forceinline__ void spec_set_halves(QagSpecSmem<G>& sh, int g0, double a, double b, int slot, int ns) {
+__device__ __forceinline__ void spec_set_halves(QagSpecSmem<G>& sh, int g0, double a, double b, int slot, NcLayout ns) {
     for (int g = g0; g < G; g++) {
         const double m = 0.5 * (a + b);
         spec_set_interval(sh, 2 * g, a, m, nc_child(slot, 0, ns));
@@ -847,13 +858,13 @@ __device__ __forceinline__ void spec_set_halves(QagSpecSmem<G>& sh, int g0, doub
     }
 }
 
-// Rule results of the groups' intervals (n0 in {1, 2} of group 0), whose geometry is in
+// Rule results of ng groups' intervals (n0 in {1, 2} of group 0), whose geometry is in
 // sh.ic / sh.ih / sh.isl.  Warp g sums group g as gk61_block_c sums a call of that many
 // intervals.
-template <int G, class F>
-__device__ __forceinline__ void gk61_block_groups(const F& f, const Gk61Nodes& N, int n0, QagSpecSmem<G>& sh) {
+template <class S, class F>
+__device__ __forceinline__ void gk61_block_groups(const F& f, const Gk61Nodes& N, int n0, int ng, S& sh) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid < 122 * G) {
+    if (tid < 122 * ng) {
         const int g = tid / 122, u = tid - 122 * g;
         const int t = u >= 61 ? 1 : 0, j = u - 61 * t;
         if (g > 0 || t < n0) {
@@ -862,26 +873,26 @@ __device__ __forceinline__ void gk61_block_groups(const F& f, const Gk61Nodes& N
         }
     }
     __syncthreads();
-    if (warp < G) {
-        const int ng = warp == 0 ? n0 : 2;
+    if (warp < ng) {
+        const int ni = warp == 0 ? n0 : 2;
         const double* fvg = sh.fv + 122 * warp;
         double fv[4];
 #pragma unroll
         for (int m = 0; m < 4; m++) {
             const int j = lane + 32 * (m & 1), t = m >> 1;
-            fv[m] = t < ng && j < 61 ? fvg[61 * t + j] : 0.0;
+            fv[m] = t < ni && j < 61 ? fvg[61 * t + j] : 0.0;
         }
         double hh[2];
 #pragma unroll
         for (int t = 0; t < 2; t++) {
-            const int q = 2 * warp + t, slot = t < ng ? sh.isl[q] : -1;
+            const int q = 2 * warp + t, slot = t < ni ? sh.isl[q] : -1;
             hh[t] = slot >= 0 ? __ldg(f.nc.half + slot) : sh.ih[q];
         }
         GkOut o[2];
-        gk61_lane_sums(N, fv, ng, hh, o);
+        gk61_lane_sums(N, fv, ni, hh, o);
         if (lane == 0) {
             sh.out[2 * warp] = o[0];
-            if (ng > 1) sh.out[2 * warp + 1] = o[1];
+            if (ni > 1) sh.out[2 * warp + 1] = o[1];
         }
     }
     __syncthreads();
@@ -891,15 +902,15 @@ template <int G, class F>
 __device__ QagResult qag_block_spec_c(const F& f, const Gk61Nodes& N, QagList& L, double a, double b, double epsabs,
                                       double epsrel, int limit, QagSpecSmem<G>& sh) {
     const int tid = threadIdx.x, lane = tid & 31;
-    const int ns = f.nc.nslots;
+    const NcLayout ns = f.nc.lay;
     QagResult R;
-    const int s0 = ns > 0 ? 0 : -1;
+    const int s0 = ns.nslots > 0 ? 0 : -1;
     if (tid == 0) {  // the root, and halves ahead
         spec_set_interval(sh, 0, a, b, s0);
         spec_set_halves(sh, 1, a, b, s0, ns);
     }
     __syncthreads();
-    gk61_block_groups(f, N, 1, sh);
+    gk61_block_groups(f, N, 1, G, sh);
     const GkOut g0 = sh.out[0];
     if (tid == 0) {
         L.a[0] = a; L.b[0] = b; L.r[0] = g0.result; L.e[0] = g0.abserr; L.slot[0] = s0;
@@ -931,7 +942,7 @@ __device__ QagResult qag_block_spec_c(const F& f, const Gk61Nodes& N, QagList& L
         }
         __syncthreads();
         const int k = sh.k;
-        if (!sh.hit) gk61_block_groups(f, N, 2, sh);  // block-uniform
+        if (!sh.hit) gk61_block_groups(f, N, 2, G, sh);  // block-uniform
         // QUADPACK's bookkeeping on thread 0
         if (tid == 0) {
             const int gi = sh.hit ? sh.pre_g : 0;
@@ -944,6 +955,145 @@ __device__ QagResult qag_block_spec_c(const F& f, const Gk61Nodes& N, QagList& L
             L.a[n] = a2; L.b[n] = b2; L.r[n] = g[1].result; L.e[n] = g[1].abserr; L.slot[n] = nc_child(s_i, 1, ns);
             sh.pre_k = gi + 1 < G ? n : -1;
             sh.pre_g = gi + 1;
+            sh.errsum = q.errsum;
+            sh.ok = q.errsum <= q.tol;
+        }
+        __syncthreads();
+        n++;
+    } while (sh.cont);
+    double sum = 0;
+    if (lane == 0)
+        for (int i = 0; i < n; i++) sum += L.r[i];
+    R.result = bcast0(sum);
+    R.abserr = sh.errsum;
+    R.nint = n;
+    R.ok = sh.ok;
+    __syncthreads();
+    return R;
+}
+
+// ------------------------------------------------------------------ block QAG, several intervals a round
+// qag_block_c for integrands that oscillate (J with a momentum cut): which interval is next is
+// anyone's guess, but those with a large error all have their turn.  A round that needs the halves
+// of interval k evaluates those of the up to G - 1 intervals of the next largest errors as well
+// and keeps their rule results until QAG picks them: next to no evaluation is wasted, and the
+// sequence of decisions is qag_block_c's.  blockDim.x = 128 G.
+template <int G>
+struct QagMultiSmem {
+    double fv[122 * G];          // as QagSpecSmem
+    GkOut out[2 * G];
+    double ic[2 * G], ih[2 * G];
+    int isl[2 * G];
+    GkOut kept[2 * 32];          // rule results of halves evaluated ahead
+    signed char have[kQagLimit]; // where a list entry's are kept (-1: nowhere)
+    int gk[G];                   // the groups' list entries
+    int k, ng, cont, ok;
+    double errsum, tol;
+};
+
+template <int G, class F>
+__device__ QagResult qag_block_multi_c(const F& f, const Gk61Nodes& N, QagList& L, double a, double b, double epsabs,
+                                       double epsrel, int limit, QagMultiSmem<G>& sh) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const NcLayout ns = f.nc.lay;
+    QagResult R;
+    const int s0 = ns.nslots > 0 ? 0 : -1;
+    auto set_halves = [&](int g, double a, double b, int slot) {
+        const double m = 0.5 * (a + b);
+        spec_set_interval(sh, 2 * g, a, m, nc_child(slot, 0, ns));
+        spec_set_interval(sh, 2 * g + 1, m, b, nc_child(slot, 1, ns));
+    };
+    if (tid == 0) {  // the root, and its halves
+        spec_set_interval(sh, 0, a, b, s0);
+        set_halves(1, a, b, s0);
+    }
+    __syncthreads();
+    gk61_block_groups(f, N, 1, 2, sh);
+    const GkOut g0 = sh.out[0];
+    double tol = fmax(epsabs, epsrel * fabs(g0.result));
+    unsigned spare = ~1u;  // (thread 0) free places of sh.kept
+    if (tid == 0) {
+        L.a[0] = a; L.b[0] = b; L.r[0] = g0.result; L.e[0] = g0.abserr; L.slot[0] = s0;
+        sh.kept[0] = sh.out[2];
+        sh.kept[1] = sh.out[3];
+        sh.have[0] = 0;
+        sh.tol = tol;
+    }
+    __syncthreads();
+    const double round_off = 50 * DBL_EPSILON * g0.resabs;
+    R.nint = 1;
+    R.result = g0.result;
+    R.abserr = g0.abserr;
+    if (g0.abserr <= round_off && g0.abserr > tol) { R.ok = 0; return R; }
+    if ((g0.abserr <= tol && g0.abserr != g0.resasc) || g0.abserr == 0.0) { R.ok = 1; return R; }
+    if (limit == 1) { R.ok = 0; return R; }
+    QagSums q = {g0.result, g0.abserr, tol, 1, 0, 0, 0};
+    int n = 1;
+    do {
+        if (tid < 32) {
+            const int bk = warp_argmax_err(L.e, n);
+            int ng = 0;
+            if (sh.have[bk] < 0) {
+                if (lane == 0) sh.gk[0] = bk;
+                ng = 1;
+                const int room = __popc(__shfl_sync(0xffffffffu, spare, 0));
+                // (an error below tol / 2 n is small enough to stay)
+                const long long least = bits_of(sh.tol * (0.5 / n));
+                while (ng < G && ng <= room) {
+                    __syncwarp();
+                    long long best = least;
+                    int at = -1;
+                    for (int i = lane; i < n; i += 32) {
+                        bool taken = sh.have[i] >= 0;
+                        for (int u = 0; u < ng; u++) taken = taken || sh.gk[u] == i;
+                        const long long v = err_key(L.e[i]);
+                        if (!taken && v > best) { best = v; at = i; }
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const long long ob = __shfl_down_sync(0xffffffffu, best, o);
+                        const int oa = __shfl_down_sync(0xffffffffu, at, o);
+                        if (ob > best) { best = ob; at = oa; }
+                    }
+                    at = __shfl_sync(0xffffffffu, at, 0);
+                    if (at < 0) break;
+                    if (lane == 0) sh.gk[ng] = at;
+                    ng++;
+                }
+                __syncwarp();
+                if (lane < ng) {  // a lane per group
+                    const int i = sh.gk[lane];
+                    set_halves(lane, L.a[i], L.b[i], L.slot[i]);
+                }
+            }
+            if (lane == 0) {
+                sh.k = bk;
+                sh.ng = ng;
+            }
+        }
+        __syncthreads();
+        const int k = sh.k, ng = sh.ng;
+        if (ng > 0) gk61_block_groups(f, N, 2, ng, sh);  // block-uniform
+        // QUADPACK's bookkeeping on thread 0
+        if (tid == 0) {
+            const double a_i = L.a[k], b_i = L.b[k], r_i = L.r[k], e_i = L.e[k];
+            const int s_i = L.slot[k];
+            const double a1 = a_i, b1 = 0.5 * (a_i + b_i), a2 = b1, b2 = b_i;
+            for (int u = 1; u < ng; u++) {
+                const int p = __ffs(spare) - 1;
+                spare &= spare - 1;
+                sh.kept[2 * p] = sh.out[2 * u];
+                sh.kept[2 * p + 1] = sh.out[2 * u + 1];
+                sh.have[sh.gk[u]] = (signed char)p;
+            }
+            const int p = sh.have[k];
+            const GkOut g[2] = {p >= 0 ? sh.kept[2 * p] : sh.out[0], p >= 0 ? sh.kept[2 * p + 1] : sh.out[1]};
+            if (p >= 0) spare |= 1u << p;
+            sh.cont = qag_account(q, g, r_i, e_i, a1, a2, b2, epsabs, epsrel, limit);
+            L.b[k] = b1; L.r[k] = g[0].result; L.e[k] = g[0].abserr; L.slot[k] = nc_child(s_i, 0, ns);
+            L.a[n] = a2; L.b[n] = b2; L.r[n] = g[1].result; L.e[n] = g[1].abserr; L.slot[n] = nc_child(s_i, 1, ns);
+            sh.have[k] = sh.have[n] = -1;
+            sh.tol = q.tol;
             sh.errsum = q.errsum;
             sh.ok = q.errsum <= q.tol;
         }
@@ -1049,7 +1199,7 @@ struct NodeCache {
     double* fsl;
     double* dx;
     int* j;
-    int nslots;
+    NcLayout lay;
 };
 
 // The integrand's terms at the nodes, for the adjoint.
@@ -1104,7 +1254,7 @@ struct NodeTable {
     const double* fsl;
     const int2* jf;
     const double* half;  // half-width of a slot's interval
-    int nslots;
+    NcLayout lay;
 };
 struct DnuIntegrandW {
     const Background* B;
@@ -1137,18 +1287,19 @@ struct DnuIntegrandW {
     __device__ __noinline__ double slow(double x) const;  // (ksp_internal.h)
 };
 
-// Slot of the dyadic interval [a, b] of [lo, hi] in a node table of nslots slots (-1: not
-// one of them), by the bisections QAG performs.
-__device__ __forceinline__ int nc_slot_of(double a, double b, double lo, double hi, int nslots) {
-    if (nslots <= 0) return -1;
-    if (a == lo && b == hi) return 0;
-    for (int d = 1; 2 * d < nslots + 1; d++) {
+// Slot of the dyadic interval [a, b] of [lo, hi] in a node table (-1: not one of them), by the
+// bisections QAG performs.
+__device__ __forceinline__ int nc_slot_of(double a, double b, double lo, double hi, NcLayout t) {
+    int s = t.nslots > 0 ? 0 : -1;
+    while (s >= 0 && !(a == lo && b == hi)) {
         const double m = 0.5 * (lo + hi);
-        if (a == lo && b == m) return 2 * d - 1;
-        if (a == m && b == hi) return 2 * d;
-        lo = m;
+        const int right = a >= m ? 1 : 0;
+        if (!right && b > m) return -1;
+        if (right) lo = m;
+        else hi = m;
+        s = nc_child(s, right, t);
     }
-    return -1;
+    return s;
 }
 
 // Segmented sums over the lanes of a warp: runs of equal key (in lane order) are summed
@@ -1169,12 +1320,22 @@ __device__ __forceinline__ void warp_seg_sum4(int key, double& a, double& b, dou
 }
 
 // End points of cache slot s of [a, b], by the bisections QAG performs (b1 = (a+b)/2).
-__device__ __forceinline__ void nc_interval(int s, double a, double b, double* lo, double* hi) {
-    if (s == 0) { *lo = a; *hi = b; return; }
-    const int d = (s + 1) / 2;
-    for (int k = 1; k < d; k++) a = 0.5 * (a + b);  // the rightmost interval of depth k
-    const double m = 0.5 * (a + b);
-    if (s & 1) { *lo = a; *hi = m; } else { *lo = m; *hi = b; }
+__device__ __forceinline__ void nc_interval(int s, NcLayout t, double a, double b, double* lo, double* hi) {
+    const int u = s - t.tree;                   // past the heap: its number there
+    const int h = u < 0 ? s + 1 : t.tree;       // the heap's node (from 1) to start from
+    for (int k = 30 - __clz(h); k >= 0; k--) {  // the bits after the leading one: left or right
+        const double m = 0.5 * (a + b);
+        if ((h >> k) & 1) a = m;
+        else b = m;
+    }
+    if (u >= 0) {
+        for (int k = 0; k < u / 2; k++) a = 0.5 * (a + b);
+        const double m = 0.5 * (a + b);
+        if (u & 1) a = m;
+        else b = m;
+    }
+    *lo = a;
+    *hi = b;
 }
 #endif  // __CUDACC__
 

@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, 
     const int q = b * kPrepThreads + t;
     if (q >= P.nodes) return;
     double half;
-    I.nc_inv[q] = node_inv_aH(I.B, nc_node_x(q, P.loga0, P.loga, &half));
+    I.nc_inv[q] = node_inv_aH(I.B, nc_node_x(q, NcLayout{I.nc_slots, I.nc_tree}, P.loga0, P.loga, &half));
 }
 
 // The fslength table, the node table, and the row splines.
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kTableThreads, 8)
     const int q = (b - table_blocks) * kTableThreads + t;
     if (q >= P.nodes) return;
     double half;
-    const double x = nc_node_x(q, P.loga0, P.loga, &half);
+    const double x = nc_node_x(q, NcLayout{I.nc_slots, I.nc_tree}, P.loga0, P.loga, &half);
     const double fsl = fs_table_at(F, x);
     const double* kx = I.scalefact;
     const int j = seg_bsearch(kx, Na, x);
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(128) k_dnu_qag(IntegratorDev I, int nk, int Na
 // (qag_block_spec_c: the same decisions, sums equal to the last bits).  For calls with few tasks, where one warp
 // per task leaves the SMs' FP64 pipes idle between the long dependent chains of a single
 // warp and the sequential QAG rounds set the time.
-// G: levels of a round (0: blocks of 2 or 4 warps and qag_block_c, no look-ahead).
+// G: levels of a round; -G: intervals of a round (qag_block_multi_c; 0: blocks of 2 or 4 warps and qag_block_c, no look-ahead).
 // upd.row >= 0: a prepared step's provisional row (k_row_update's arithmetic, per task, while
 // the row is on its way, instead of a launch of its own before this one: 7 us).
 // Shared memory: Gk61Nodes | row[ld] | coef[ld] | QagList | QagSpecSmem or QagBlockSmem | mbarrier
@@ -513,11 +513,13 @@ struct RowUpdate {
     int row;
     FinalizeArgs fin;
 };
-constexpr int qag_blk_threads(int G) { return G > 0 ? 128 * G : 128; }
-template <int G>
+constexpr int qag_blk_threads(int G) { return G > 0 ? 128 * G : (G < 0 ? -128 * G : 128); }
+template <int G, bool MULTI = (G < 0)>
 struct QagBlkSmemOf { typedef QagSpecSmem<G> type; };
+template <int G>
+struct QagBlkSmemOf<G, true> { typedef QagMultiSmem<-G> type; };
 template <>
-struct QagBlkSmemOf<0> { typedef QagBlockSmem type; };
+struct QagBlkSmemOf<0, false> { typedef QagBlockSmem type; };
 
 template <int G>
 __global__ void __launch_bounds__(qag_blk_threads(G), 512 / qag_blk_threads(G))
@@ -611,7 +613,8 @@ __global__ void __launch_bounds__(qag_blk_threads(G), 512 / qag_blk_threads(G))
         const double kom = (I.kq ? I.kq[ik] : I.wavenum[ik]) * S.inv_m[mi];
         const DnuIntegrandW f = dnu_integrand_w(I, S, mi, kom, row, rc, Na);
         QagResult r;
-        if constexpr (G > 0) r = qag_block_spec_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
+        if constexpr (G < 0) r = qag_block_multi_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
+        else if constexpr (G > 0) r = qag_block_spec_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
         else r = qag_block_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
         if (I.ivals) {  // keep the final subdivision for the adjoint
             double* dst = I.ivals + ((size_t)mi * I.nk_alloc + ik) * kQagLimit * 2;
@@ -818,18 +821,21 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
         }
         // a block per task: with no more tasks than SMs 12 warps and two levels of look-ahead
         // (split 12; a call of 64, 100, 150 bins 62, 71, 78 us, with 8 warps and one level 64, 74,
-        // 82; three levels 65, 75, 77; but 200 bins 86 against 82, and hybrid neutrinos' nodes,
-        // off the table, are too dear to guess), 8 warps and one level (split 8) below 4 tasks
+        // 82; three levels 65, 75, 77; but 200 bins 86 against 82), 8 warps and one level (split 8) below 4 tasks
         // per SM, 4 warps without look-ahead up to 6, 2 warps from there (at 128 registers a
         // thread, 4 blocks of 4 warps fit an SM: 1221 tasks of 3 species x 407 bins take two
         // waves of 4-warp blocks and one of 2-warp blocks, measured 0.211 against 0.223 ms; a
-        // warp per task, split 1, 0.231 ms)
-        const int split = qag_split > 0       ? qag_split
-                          : ntask <= nsm && !I.hyb ? 12
-                                              : (ntask < 4 * nsm ? 8 : (ntask < 6 * nsm ? 4 : 2));
+        // warp per task, split 1, 0.231 ms).  Where hybrid neutrinos cut J the next interval is
+        // anyone's guess: two intervals a round by their errors (151 bins 228 us; one 256, one
+        // and a level of look-ahead 310, three 222 but 60 bins 216 against 214)
+        const int split = qag_split > 0   ? qag_split
+                          : ntask <= nsm ? 12
+                                         : (ntask < 4 * nsm ? 8 : (ntask < 6 * nsm ? 4 : 2));
+        const bool cut = qag_split <= 0 && I.nc_tree > 1;
         const int4 sp = make_int4(spec_ids[0], spec_ids[1], spec_ids[2], 0);
         const bool done =
-            split >= 12 ? launch_dnu_qag_blk<3>(I, nk, Na, nspec, sp, upd, 384, st)
+            cut          ? launch_dnu_qag_blk<-2>(I, nk, Na, nspec, sp, upd, 256, st)
+            : split >= 12 ? launch_dnu_qag_blk<3>(I, nk, Na, nspec, sp, upd, 384, st)
             : split >= 8 ? launch_dnu_qag_blk<2>(I, nk, Na, nspec, sp, upd, 256, st)
             : split > 1  ? launch_dnu_qag_blk<0>(I, nk, Na, nspec, sp, upd, split >= 4 ? 128 : 64, st)
                          : false;

@@ -28,8 +28,25 @@ struct StepScalars {
     int Na, Nfs;
 };
 
+// The arrays of a node table.
+struct NcNodes {
+    double2 *ab, *cd;
+    int2* jf;
+    double *g, *fsl, *dx, *inv;
+    int* j;
+    double* half;
+    int slots, tree;
+};
+
 // One integrator instance (the reference's delta_tot_table + omega_nu + transfer table).
 struct IntegratorDev {
+    NcNodes nodes() const {
+        return NcNodes{nc_ab, nc_cd, nc_jf, nc_g, nc_fsl, nc_dx, nc_inv, nc_j, nc_half, nc_slots, nc_tree};
+    }
+    void set_nodes(const NcNodes& t) {
+        nc_ab = t.ab; nc_cd = t.cd; nc_jf = t.jf; nc_g = t.g; nc_fsl = t.fsl; nc_dx = t.dx; nc_inv = t.inv;
+        nc_j = t.j; nc_half = t.half; nc_slots = t.slots; nc_tree = t.tree;
+    }
     Background* B;                   // device
     int nk_alloc, namax, ld;         // ld: padded row length of the history table
     double* scalefact;               // [namax]
@@ -59,7 +76,7 @@ struct IntegratorDev {
     unsigned* done;                  // blocks of k_finish that are through (0 between calls)
     const double* jt;                // J's fine table (one per device)
     double* hyb;                     // optional: [kNuSpecies][kHybTable] the tables of J with a cut
-    int nc_slots;                    // slots of the node table in use (1 + 2 levels, 0 = none)
+    int nc_slots, nc_tree;           // slots of the node table in use (0 = none), and its heap's (NcLayout)
     double* fs_y;                    // [fs_cap]
     double* fs_c;                    // [fs_cap]
     double* fs_seg;                  // [fs_cap] integrals of 1/(a^2 H) over the table's segments
@@ -244,7 +261,7 @@ __device__ __forceinline__ DnuIntegrandC dnu_integrand_pre(const IntegratorDev& 
     f.kx = knots; f.ky = row; f.kc = rc; f.na = Na;
     f.sb = sb; f.sd = sd;
     f.ks = KnotSeg{I.knot_invh, I.knot_h3, I.knot_ih3};
-    f.nc = NodeCache{I.nc_g, I.nc_fsl, I.nc_dx, I.nc_j, I.nc_slots};
+    f.nc = NodeCache{I.nc_g, I.nc_fsl, I.nc_dx, I.nc_j, {I.nc_slots, I.nc_tree}};
     return f;
 }
 __device__ __forceinline__ DnuIntegrandC dnu_integrand(const IntegratorDev& I, const StepScalars& S, double k,
@@ -261,7 +278,7 @@ __device__ __forceinline__ DnuIntegrandW dnu_integrand_w(const IntegratorDev& I,
     f.qc = S.qc[mi]; f.nfl = I.B->nufrac_low[0];
     f.hyb = I.hyb ? I.hyb + (size_t)mi * kHybTable : nullptr;
     f.ky = row; f.kc = rc;
-    f.nc = NodeTable{I.nc_ab, I.nc_cd, I.nc_fsl, I.nc_jf, I.nc_half, I.nc_slots};
+    f.nc = NodeTable{I.nc_ab, I.nc_cd, I.nc_fsl, I.nc_jf, I.nc_half, {I.nc_slots, I.nc_tree}};
     f.fs_y = I.fs_y; f.fs_c = I.fs_c; f.kx = I.scalefact; f.kih = I.knot_invh;
     f.S = &S; f.na = Na;
     return f;

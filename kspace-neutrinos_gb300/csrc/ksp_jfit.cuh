@@ -87,7 +87,7 @@ __device__ __forceinline__ double specialJ_node(const double* jt, double fsl, fl
 // octave, degree 6 (the interpolant's error 2e-17): 11200 evaluations of the series instead of
 // one per node, and a node costs a sine, a cosine and 12 multiply-adds.  (151 bins x 100
 // rows: the integrals took 3074 us term by term, 1134 with the series' sine and cosine taken
-// once.)  Piece: centre, 7 coefficients of A, 7 of B, both over 1.5 zeta(3) (1 - nufrac_low).
+// once.)  Piece: centre, 7 coefficients of A / x, 7 of B, both over 1.5 zeta(3) (1 - nufrac_low).
 constexpr int kHybE0 = -12, kHybSubBits = 6, kHybPieces = 25 << kHybSubBits, kHybStride = 16;
 constexpr int kHybTable = kHybPieces * kHybStride;
 
@@ -106,7 +106,7 @@ static __device__ __noinline__ double specialJ_cut(const double* hyb, double x, 
     }
     double sn, cs;
     sincos(qc * x, &sn, &cs);
-    return A * (sn / x) + B * cs;
+    return A * sn + B * cs;
 }
 
 // Pieces blk * 8 .. + 7 of the table of one species, by 64 threads: eight per piece, seven of
@@ -131,7 +131,7 @@ __device__ __forceinline__ void hyb_table_block(double* hyb, int blk, double qc,
     double A, B;
     specialJ_sums(x * x, qc, exp(-qc), &A, &B);
     const double norm = 1.0 / (1.5 * kZeta3 * (1 - nfl));
-    A *= norm;
+    A *= norm / x;
     B *= norm;
     const unsigned all = 0xffffffffu;
     const double A3 = __shfl_sync(all, A, 3, 8), B3 = __shfl_sync(all, B, 3, 8);

@@ -297,10 +297,10 @@ __device__ __forceinline__ void knot_row(const X& knot, int i, double* invdiag, 
 
 // ------------------------------------------------------------------ nodes
 // Node q = 61 slot + jn of the node table: its log a, and the half-width of its interval.
-__device__ __forceinline__ double nc_node_x(int q, double loga0, double loga, double* half) {
+__device__ __forceinline__ double nc_node_x(int q, NcLayout lay, double loga0, double loga, double* half) {
     const int slot = q / 61, jn = q - 61 * slot;
     double lo, hi;
-    nc_interval(slot, loga0, loga, &lo, &hi);
+    nc_interval(slot, lay, loga0, loga, &lo, &hi);
     const double c = __dmul_rn(0.5, __dadd_rn(lo, hi));
     const double h = __dmul_rn(0.5, __dsub_rn(hi, lo));
     *half = h;

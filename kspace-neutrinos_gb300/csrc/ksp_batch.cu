@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kBatchTable) kb_tables(BatchDev b) {
 // and the backward one c_k = g_k + V_k c_{k+1}, the factors of a knot formed by one lane for
 // all rows: five FP64 operations per knot and row, which is the bound (a row by the warp's
 // scans costs twice that, a thread per row with its row in global memory waits for every
-// knot: 24 members, 446 us, now 197; 256 members, 687 us, now 374).
+// knot: 256 members 687 us, now 329; with the operands of a step read when they are needed 374).
 constexpr int kRowTile = 32, kRowPitch = kRowTile + 1, kRowWarps = 4;
 struct RowSmem {
     double y[2][32 * kRowPitch];  // [row][knot of the tile], a pitch free of bank conflicts
@@ -165,18 +165,23 @@ __global__ void __launch_bounds__(32 * kRowWarps) kb_dtot_coeffs(BatchDev b) {
             if (later) asm volatile("cp.async.wait_group 1;" ::: "memory");
             else asm volatile("cp.async.wait_group 0;" ::: "memory");
         };
-        // the factors of unknown k (of a tile, by its lane; zero past the last)
+        // the factors of unknown k (of a tile, by its lane; zero past the last): what they are made
+        // of is read a tile ahead
+        double kinv, kih0, kih1, kx0, kx1, kx2;
+        auto knots = [&](int t) {
+            const int k = min(max(kRowTile * t + lane, 0), m - 1);
+            kinv = I.knot_invdiag[k];
+            kih0 = I.knot_invh[k];
+            kih1 = I.knot_invh[k + 1];
+            kx0 = I.scalefact[k];
+            kx1 = I.scalefact[k + 1];
+            kx2 = I.scalefact[k + 2];
+        };
         auto factors = [&](int t) {
-            const int k = kRowTile * t + lane;
-            double2 ab = make_double2(0.0, 0.0), wv = ab;
-            if (k < m) {
-                const double inv = I.knot_invdiag[k], i3 = 3.0 * inv;
-                const double h0 = I.scalefact[k + 1] - I.scalefact[k], h1 = I.scalefact[k + 2] - I.scalefact[k + 1];
-                ab = make_double2(i3 * I.knot_invh[k + 1], -i3 * I.knot_invh[k]);
-                wv = make_double2(-h0 * inv, -h1 * inv);
-            }
-            sh.ab[lane] = ab;
-            sh.wv[lane] = wv;
+            const bool in = kRowTile * t + lane < m;
+            const double i3 = 3.0 * kinv;
+            sh.ab[lane] = in ? make_double2(i3 * kih1, -i3 * kih0) : make_double2(0.0, 0.0);
+            sh.wv[lane] = in ? make_double2((kx0 - kx1) * kinv, (kx1 - kx2) * kinv) : make_double2(0.0, 0.0);
         };
         auto store = [&](int t, int buf) {
             const int k = kRowTile * t + lane;
@@ -186,32 +191,45 @@ __global__ void __launch_bounds__(32 * kRowWarps) kb_dtot_coeffs(BatchDev b) {
         };
         __syncwarp();  // the previous group's reads
         fetch(0, y, 2, 0);
+        knots(0);
         const double* yr = y + (size_t)my * I.ld;
         double y1 = yr[1], d0 = y1 - yr[0], gp = 0.0;
         for (int t = 0; t < nt; t++) {
             const int buf = t & 1, n = min(kRowTile, m - kRowTile * t);
             if (t + 1 < nt) fetch(t + 1, y, 2, buf ^ 1);
             factors(t);
+            knots(t + 1 < nt ? t + 1 : t - 1);  // (the last tile turns round)
             arrived(t + 1 < nt);
             __syncwarp();
             double* q = sh.y[buf] + my * kRowPitch;
             if (lane < nr) {
-                for (int k = 0; k < n; k += 4) {
-                    double2 ab[4];
-                    double w[4], y2[4];
+                // (four knots' operands are read while the four before are worked on)
+                double2 ab[4];
+                double w[4], y2[4];
+                auto operands = [&](int k) {
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         ab[u] = sh.ab[k + u];
                         w[u] = sh.wv[k + u].x;
                         y2[u] = q[k + u];
                     }
+                };
+                operands(0);
+                for (int k = 0; k < n; k += 4) {
+                    double r[4], v[4];
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         const double d1 = y2[u] - y1;
-                        gp = fma(w[u], gp, fma(ab[u].x, d1, ab[u].y * d0));
-                        q[k + u] = k + u < n ? gp : 0.0;
+                        r[u] = fma(ab[u].x, d1, ab[u].y * d0);
+                        v[u] = w[u];
                         y1 = y2[u];
                         d0 = d1;
+                    }
+                    operands(k + 4 < kRowTile ? k + 4 : 0);
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        gp = fma(v[u], gp, r[u]);
+                        q[k + u] = k + u < n ? gp : 0.0;
                     }
                 }
             }
@@ -223,21 +241,34 @@ __global__ void __launch_bounds__(32 * kRowWarps) kb_dtot_coeffs(BatchDev b) {
         for (int t = nt - 1; t >= 0; t--) {
             const int buf = t & 1, n = min(kRowTile, m - kRowTile * t);
             if (t > 0) fetch(t - 1, c, 1, buf ^ 1);
-            if (t < nt - 1) factors(t);
+            if (t < nt - 1) {
+                factors(t);
+                knots(t - 1);
+            }
             arrived(t > 0);
             __syncwarp();
             double* q = sh.y[buf] + my * kRowPitch;
             if (lane < nr) {
-                for (int k = (n - 1) & ~3; k >= 0; k -= 4) {
-                    double v[4], gk[4];
+                double v[4], gk[4];
+                auto operands = [&](int k) {
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         v[u] = sh.wv[k + u].y;
                         gk[u] = q[k + u];
                     }
+                };
+                operands((n - 1) & ~3);
+                for (int k = (n - 1) & ~3; k >= 0; k -= 4) {
+                    double r[4], p[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        p[u] = v[u];
+                        r[u] = gk[u];
+                    }
+                    operands(k >= 4 ? k - 4 : 0);
 #pragma unroll
                     for (int u = 3; u >= 0; u--) {
-                        next = fma(v[u], next, gk[u]);
+                        next = fma(p[u], next, r[u]);
                         q[k + u] = next;
                     }
                 }

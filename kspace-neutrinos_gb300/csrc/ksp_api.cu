@@ -1351,7 +1351,7 @@ static int start_prep(kspace_ctx* c, const Geo* G, double Time) {
 // units), dcdm and keff (physical) for the integrator.  prep_time > 0: start the
 // integrator's preparation for that scale factor once the binning pass is queued.
 static int bin_grid(kspace_ctx* c, Geo* G, const float* gd, int pmgrid, int slab0, int nslab, double BoxSize,
-                    const SlabChunks* ch = nullptr, double prep_time = 0, const SpectrumOut& host = SpectrumOut{}) {
+                    const SlabChunks* ch = nullptr, double prep_time = 0, const HostOut& host = HostOut{}) {
     NEED(c->table_ready && c->buf_nb >= G->g.nrbins, KSPACE_ERR_ORDER);
     const int nb = G->g.nrbins;
     G->g.slab0 = slab0;
@@ -1423,7 +1423,7 @@ extern "C" int kspace_gpu_total_powerspectrum(kspace_ctx* c, int dims, const voi
     // the normalisation writes the spectrum and the status to pinned memory
     *c->status_h = kStTimeout;
     st = bin_grid(c, G, gd, dims, startslab, nslab, 1.0, nullptr, 0,
-                  SpectrumOut{c->io_h, c->status_h, c->status_d, c->I.done});
+                  HostOut{c->io_h, c->status_h, c->status_d, c->I.done});
     if (st) return st;
     const size_t n = G->nk;
     st = sync_status(c, true);
@@ -1441,16 +1441,22 @@ extern "C" int kspace_gpu_total_powerspectrum(kspace_ctx* c, int dims, const voi
     return KSPACE_OK;
 }
 
-// in: the grid to read where it is not gd itself.
+// in: the grid to read where it is not gd itself.  delivered: the status word is to come with the
+// pass, and whether it does (sync_status).
 static int correct_grid(kspace_ctx* c, Geo* G, float* gd, double BoxSize, int nk, const SlabChunks* ch = nullptr,
-                        void* host = nullptr, const float* in = nullptr) {
+                        void* host = nullptr, const float* in = nullptr, bool* delivered = nullptr) {
     CorrTable corr = c->corr;
     corr.nk = nk;
     const float lnscale = (float)log(2 * kPi / BoxSize);
     if (c->prof) cudaEventRecord(c->ev[2], c->stream);
     if (!ch) {
-        if (launch_apply_correction(G->g, gd, corr, lnscale, c->status_d, c->tma, c->rows, c->stages, c->stream, in) <
-            0)
+        HostOut out;
+        if (delivered) {
+            *c->status_h = kStTimeout;  // until the pass writes it
+            out = HostOut{nullptr, c->status_h, c->status_d, c->I.done};
+        }
+        if (launch_apply_correction(G->g, gd, corr, lnscale, c->status_d, c->tma, c->rows, c->stages, c->stream, in,
+                                    out, delivered) < 0)
             return KSPACE_ERR_CUDA;
         g_launches += 1;
     } else {
@@ -1527,9 +1533,11 @@ extern "C" int kspace_gpu_add_nu_power_to_rhogrid(kspace_ctx* c, double Time, do
                        false);
     c->fin.active = 0;
     if (st) return st;
-    st = correct_grid(c, G, gd, BoxSize, G->nk, staged ? &ch : nullptr, staged ? grid : nullptr);
+    bool delivered = false;
+    st = correct_grid(c, G, gd, BoxSize, G->nk, staged ? &ch : nullptr, staged ? grid : nullptr, nullptr,
+                      staged ? nullptr : &delivered);
     if (st) return st;
-    st = sync_status(c);
+    st = sync_status(c, delivered);
     if (st == KSPACE_OK) {
         c->last_nk = G->nk;
         c->last_BoxSize = BoxSize;
@@ -1849,10 +1857,11 @@ extern "C" int kspace_gpu_diff_forward(kspace_ctx* c, double Time, double BoxSiz
                          c->norm_d, c->stream, true, logk_ready);
     k_square<<<(c->nk + 127) / 128, 128, 0, c->stream>>>(c->dnu_out_d, pnu_out, c->nk);
     g_launches += 5;
+    bool delivered = false;
     st = correct_grid(c, G, reinterpret_cast<float*>(grid_out), BoxSize, c->nk, nullptr, nullptr,
-                      reinterpret_cast<const float*>(grid_in));
+                      reinterpret_cast<const float*>(grid_in), &delivered);
     if (st) return st;
-    st = sync_status(c);
+    st = sync_status(c, delivered);
     if (st) return st;
     c->diff_ready = true;
     c->diff_ia = c->ia;

@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kBatchTable) kb_tables(BatchDev b) {
 // and the backward one c_k = g_k + V_k c_{k+1}, the factors of a knot formed by one lane for
 // all rows: five FP64 operations per knot and row, which is the bound (a row by the warp's
 // scans costs twice that, a thread per row with its row in global memory waits for every
-// knot: 256 members 687 us, now 329; with the operands of a step read when they are needed 374).
+// knot: 256 members 687 us, now 330 to 380).
 constexpr int kRowTile = 32, kRowPitch = kRowTile + 1, kRowWarps = 4;
 struct RowSmem {
     double y[2][32 * kRowPitch];  // [row][knot of the tile], a pitch free of bank conflicts

@@ -412,7 +412,7 @@ void launch_k2_histogram(int N, int slab0, int nslab, unsigned long long* hist, 
 __global__ void k_finalize_power(const double* bin_sum, const double* F0sq, const long long* count,
                                  const double* ksum, const int* compact_bins, int nk, double BoxSize,
                                  double* power_out, double* keff_out, double* dcdm_out, double* keffphys_out,
-                                 double scale, double kfac, SpectrumOut host) {
+                                 double scale, double kfac, HostOut host) {
     ptx::dep_wait();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < nk) {
@@ -428,7 +428,7 @@ __global__ void k_finalize_power(const double* bin_sum, const double* F0sq, cons
 }
 void launch_finalize_power(const double* bin_sum, const double* F0sq, const long long* count, const double* ksum,
                            const int* compact_bins, int nk, double BoxSize, double* power_out, double* keff_out,
-                           double* dcdm_out, double* keffphys_out, cudaStream_t st, const SpectrumOut& host) {
+                           double* dcdm_out, double* keffphys_out, cudaStream_t st, const HostOut& host) {
     // a warp per block: the FP64 pow, sqrt and divisions of the bins spread over SMs
     launch_dependent(k_finalize_power, (nk + 31) / 32, 32, 0, st, bin_sum, F0sq, count, ksum, compact_bins, nk, BoxSize,
                      power_out, keff_out, dcdm_out, keffphys_out, pow(BoxSize, -3.0),
@@ -569,10 +569,13 @@ static int corr_variant(const GridGeom& g, const GridArgs& a, float* grid, CorrT
 }
 
 int launch_apply_correction(const GridGeom& g, float* grid, CorrTable corr, float lnscale, unsigned* status, int tma,
-                            int rows_per_cta, int stages, cudaStream_t st, const float* in) {
+                            int rows_per_cta, int stages, cudaStream_t st, const float* in, const HostOut& host,
+                            bool* delivered) {
+    if (delivered) *delivered = false;
     const GridArgs a = make_grid_args(g, corr.nk, lnscale);
     if (tma >= 3) {
-        const int r = launch_correct_stream(a, in ? in : grid, grid, corr, status, rows_per_cta / 32, stages, st);
+        const int r = launch_correct_stream(a, in ? in : grid, grid, corr, status, rows_per_cta / 32, stages, st, host);
+        if (r == 0 && delivered) *delivered = host.status_out != nullptr;
         if (r == 0) return 0;
         if (r == -2) return -2;
     }

@@ -333,9 +333,10 @@ struct FinalizeArgs {
     double scale, kfac;
     double* logk_out;  // log of the physical keff (finalize_keff)
 };
-// A spectrum in pinned host memory: [nk] power, then [nk] keff, and the status word from the last
-// of the kernel's blocks to end (they count themselves in done, 0 between calls).
-struct SpectrumOut {
+// What a call's last kernel leaves in pinned host memory: a spectrum ([nk] power, then [nk]
+// keff), and the status word from the last of its blocks to end (they count themselves in done,
+// 0 between calls).
+struct HostOut {
     double* out = nullptr;
     unsigned* status_out = nullptr;
     const unsigned* status = nullptr;
@@ -490,13 +491,14 @@ int launch_bin_power(const GridGeom& g, const float* grid, double* bin_sum, doub
 // K3: grid *= 1 + norm * interp(log k)
 // Every variant leaves the grid as it is when the status word holds an error (kStAbort).
 int launch_apply_correction(const GridGeom& g, float* grid, CorrTable corr, float lnscale, unsigned* status, int tma,
-                            int rows_per_cta, int stages, cudaStream_t st, const float* in = nullptr);
+                            int rows_per_cta, int stages, cudaStream_t st, const float* in = nullptr,
+                            const HostOut& host = HostOut{}, bool* delivered = nullptr);
 // normalisation of K1's sums into P(k), delta_cdm, keff (powerspectrum.c:98-115,
 // interface_gadget.c:96-100)
 void launch_finalize_power(const double* bin_sum, const double* F0sq, const long long* count, const double* ksum,
                            const int* compact_bins, int nk, double BoxSize, double* power_out, double* keff_out,
                            double* dcdm_out, double* keffphys_out, cudaStream_t st,
-                           const SpectrumOut& host = SpectrumOut{});
+                           const HostOut& host = HostOut{});
 
 struct GridGeom;
 void launch_adj_reduce(const GridGeom& gg, CorrTable corr, float lnscale, const float* gbar, const float* x,

@@ -437,7 +437,7 @@ template <int WARPS, int STAGES>
 __global__ void __launch_bounds__(WARPS * 32)
     k_correct_stream(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap omap, GridArgs g,
                      CorrTable corr, const float* grid, float* out, unsigned* status, long long ntiles, int adv_r,
-                     int adv_z) {
+                     int adv_z, HostOut host) {
     extern __shared__ unsigned char sm_raw[];
     __shared__ int s_gap, s_abort;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -481,10 +481,21 @@ __global__ void __launch_bounds__(WARPS * 32)
         s_gap = -1;
     }
     __syncthreads();
+    // the status word to the host, from the last block to end
+    auto deliver = [&] {
+        if (!host.status_out) return;
+        __threadfence();
+        __syncthreads();
+        if (tid == 0 && atomicInc(host.done, gridDim.x - 1) == gridDim.x - 1) {
+            __threadfence();
+            *host.status_out = *reinterpret_cast<volatile unsigned*>(status);
+        }
+    };
     const bool keep = s_abort;
     if (keep && out == grid) {
         if (lane == 0)
             for (int s = 0; s < STAGES - 1 && s < my_n; s++) ptx::mbar_wait_bounded(&my_bar[s], 0);
+        deliver();
         return;
     }
     for (int s = tid; s <= nk; s += blockDim.x) {
@@ -642,6 +653,7 @@ __global__ void __launch_bounds__(WARPS * 32)
         }
     }
     if (flags) atomicOr(status, flags);
+    deliver();
 }
 
 // ------------------------------------------------------------------ K1, row-aligned runs
@@ -1747,7 +1759,7 @@ int run_bin_mirror_any(const GridGeom& g, const GridArgs& a, const float* grid, 
 
 template <int WARPS, int STAGES>
 int run_corr_stream(const GridArgs& a, const float* grid, float* out, CorrTable corr, unsigned* status,
-                    cudaStream_t st) {
+                    cudaStream_t st, const HostOut& host) {
     CUtensorMap map, omap;
     if (!grid_tmap_cached(&map, grid, a.nrows16, kRowsPerWarp)) return -1;
     if (out == grid) omap = map;
@@ -1759,7 +1771,7 @@ int run_corr_stream(const GridArgs& a, const float* grid, float* out, CorrTable 
     int grid_n = 1, adv_r = 0, adv_z = 0;
     if (!stream_grid(kern, WARPS, P.total, ntiles, a.nz, grid_n, adv_r, adv_z)) return -1;
     return launch_dependent(kern, grid_n, WARPS * 32, P.total, st, map, omap, a, corr, grid, out, status, ntiles, adv_r,
-                            adv_z) == cudaSuccess
+                            adv_z, host) == cudaSuccess
                ? 0
                : -2;
 }
@@ -1896,13 +1908,13 @@ int launch_bin_rows(const GridGeom& g, const GridArgs& a, const float* grid, dou
 }
 
 int launch_correct_stream(const GridArgs& a, const float* grid, float* out, CorrTable corr, unsigned* status,
-                          int warps, int stages, cudaStream_t st) {
+                          int warps, int stages, cudaStream_t st, const HostOut& host) {
     if (a.nrows16 <= 0 || a.nk < 2 || a.N >= 32768) return -1;
 #define KSP_CS(W, S) \
-    if (warps == W && stages == S) return run_corr_stream<W, S>(a, grid, out, corr, status, st);
+    if (warps == W && stages == S) return run_corr_stream<W, S>(a, grid, out, corr, status, st, host);
     KSP_CS(4, 2) KSP_CS(4, 3) KSP_CS(4, 4) KSP_CS(8, 2) KSP_CS(8, 3) KSP_CS(8, 4)
 #undef KSP_CS
-    return run_corr_stream<8, 2>(a, grid, out, corr, status, st);
+    return run_corr_stream<8, 2>(a, grid, out, corr, status, st, host);
 }
 
 }  // namespace ksp

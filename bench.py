@@ -414,7 +414,7 @@ def run_gb300(args, cfg):
         "hbm_frac_step": 3 * bytes_grid / (ms_per_step * 1e-3) / 1e9 / hbm,
         "stage_ms": {"binning_K1": k1_ms, "integrator_K2": k2_ms, "correction_K3": k3_ms, "whole_call": stage[3]},
         "stage_gbs": {"K1": k1_gbs, "K3": k3_gbs},
-        "stage_kernels": {"K1": k1_name, "K2": "k_dnu_qag_blk (+ k_dtot_coeffs, k_combine, k_finish)", "K3": k3_name},
+        "stage_kernels": {"K1": k1_name, "K2": "k_dnu_qag_blk (+ k_finish)", "K3": k3_name},
         "stage_frac": {"K1": (k1_gbs / hbm) if k1_gbs else None, "K3": (k3_gbs / hbm) if k3_gbs else None},
         "roofline": {"bound": "hbm", "kernel": dom["kernel"], "achieved": dom["gbs"], "peak": hbm,
                      "peak_kind": peak_kind, "unit": "GB/s", "frac": (dom["gbs"] / hbm) if dom["gbs"] else None,

@@ -21,7 +21,7 @@ int launch_bin_stream(const struct GridGeom& g, const GridArgs& a, const float* 
                       unsigned* status, int warps, int stages, bool exact, cudaStream_t st);
 int launch_correct_stream(const GridArgs& a, const float* grid, float* out, struct CorrTable corr, unsigned* status,
                           int warps, int stages, cudaStream_t st, const struct HostOut& host);
-// K1 over row-aligned runs of 17 modes (ksp_stream.cu): same return codes
+// K1 over mirrored rows or row-aligned runs (ksp_stream.cu): same return codes
 int launch_bin_rows(const struct GridGeom& g, const GridArgs& a, const float* grid, double* bin_sum, double* F0sq,
                     unsigned* status, int warps, int stages, bool exact, cudaStream_t st);
 

@@ -1,6 +1,6 @@
 // ksp_integrator.cu -- the linear-response neutrino integrator on the GPU.
 //
-//   k_rho_points / k_spline1    Omega_nu(a) tables (omega_nu_single.c:117-153)
+//   k_rho_points / k_rho_splines  Omega_nu(a) tables (omega_nu_single.c:117-153)
 //   k_nufrac_low                hybrid-neutrino fractions (omega_nu_single.c:214-240)
 //   k_update_row                update_delta_tot (delta_tot_table.c:177-191)
 //   k_delta_tot_init            delta_tot_init's per-bin part (delta_tot_table.c:94-129)
@@ -9,14 +9,15 @@
 //                               table (delta_tot_table.c:574-591: sums of fixed-order
 //                               segment integrals over the 16*Na uniform nodes replace 16*Na
 //                               adaptive integrals), the integrand's bin-independent terms on
-//                               QAG's right spine, the natural spline of every history row
+//                               QAG's right spine (hybrid neutrinos: on all shallow intervals),
+//                               the natural spline of every history row
 //   k_row_update                a prepared step's provisional row, with the binning pass's
 //                               normalisation
 //   k_dnu_qag                   one warp per (species, bin): history row staged into
 //                               shared memory by a TMA bulk copy, then QAG/GK61 of the
 //                               delta_nu time integral (delta_tot_table.c:492-500,592-599)
-//   k_dnu_qag_blk               the same with a block per task (few tasks), one bisection
-//                               level evaluated ahead
+//   k_dnu_qag_blk               the same with a block per task (few tasks), bisection levels
+//                               or intervals evaluated ahead
 //   k_combine / k_finish        species sum, row commit, NaN check, clamp, ratio table
 #include <cuda_runtime.h>
 #include <stdio.h>

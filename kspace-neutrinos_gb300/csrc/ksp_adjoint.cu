@@ -324,7 +324,7 @@ __device__ __forceinline__ void adj_interval(const DnuIntegrandC& fi, const Gk61
         double ya = 0.0, yb = 0.0, ca = 0.0, cb = 0.0;
         int key = -1;
         if (sidx < 61) {
-            const int jn = sidx < 30 ? sidx : (sidx == 30 ? 60 : 90 - sidx);
+            const int jn = gk61_ascending(sidx);
             const double xn = __dadd_rn(c, __dmul_rn(h, N.x[jn]));
             const NodeTerms t = fi.terms(slot, jn, xn);
             double J, Jd;

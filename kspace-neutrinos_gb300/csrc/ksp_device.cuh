@@ -358,8 +358,11 @@ __device__ __forceinline__ int warp_argmax_err(const double* e, int n) {
 
 // ------------------------------------------------------------------ QAG (GK61)
 #ifdef __CUDACC__
-struct Gk61Nodes {  // expanded 61-node table: slot j<30: -x_j, 30<=j<60: +x_{j-30}, 60: centre
-    double x[61], wk[61], wg[61];
+// The expanded 61-node table, the nodes of the embedded Gauss rule (odd i of the rule's table)
+// first: slots 0-14 -x_1, -x_3, ..., 15-29 +x_1, ..., 30-44 -x_0, -x_2, ..., 45-59 +x_0, ..., 60 the
+// centre.  A lane's second node (slots 32 on) then has no part in the Gauss sum.
+struct Gk61Nodes {
+    double x[61], wk[61], wg[32];
 };
 
 // the rule in memory: as arrays of the functions that index them they were copied to every
@@ -367,15 +370,24 @@ struct Gk61Nodes {  // expanded 61-node table: slot j<30: -x_j, 30<=j<60: +x_{j-
 static __device__ const double kGkXK[31] = KSP_GK61_XK_INIT;
 static __device__ const double kGkWK[31] = KSP_GK61_WK_INIT;
 static __device__ const double kGkWG[31] = KSP_GK61_WG_INIT;
+__device__ __forceinline__ int gk61_index(int j) {  // i of slot j's +-x_i
+    return j < 30 ? 2 * (j < 15 ? j : j - 15) + 1 : 2 * (j < 45 ? j - 30 : j - 45);  // 60: i = 30
+}
 __device__ __forceinline__ double gk61_x(int j) {  // abscissa of slot j
-    return j < 30 ? -__ldg(kGkXK + j) : (j < 60 ? __ldg(kGkXK + j - 30) : 0.0);
+    const double x = __ldg(kGkXK + gk61_index(j));
+    return j == 60 ? 0.0 : (j < 15 || (j >= 30 && j < 45) ? -x : x);
+}
+// slot of the s-th node in ascending x
+__device__ __forceinline__ int gk61_ascending(int s) {
+    const int i = s <= 30 ? s : 60 - s, up = s > 30 ? 1 : 0;
+    return s == 30 ? 60 : ((i & 1) ? (i >> 1) + 15 * up : 30 + (i >> 1) + 15 * up);
 }
 __device__ __forceinline__ void gk61_fill(Gk61Nodes& n, int tid, int nthreads) {
     for (int j = tid; j < 61; j += nthreads) {
-        const int i = j < 30 ? j : j - 30;  // slot 60: the centre, i = 30
+        const int i = gk61_index(j);
         n.x[j] = gk61_x(j);
         n.wk[j] = __ldg(kGkWK + i);
-        n.wg[j] = j < 60 ? __ldg(kGkWG + i) : 0.0;
+        if (j < 32) n.wg[j] = j < 30 ? __ldg(kGkWG + i) : 0.0;
     }
 }
 
@@ -429,13 +441,13 @@ __device__ __forceinline__ void gk61_lane_sums(const Gk61Nodes& N, const double*
     const int lane = threadIdx.x & 31;
     const bool two = lane < 29;  // the lane has a second node
     const double k0 = N.wk[lane], k1 = two ? N.wk[32 + lane] : 0.0;
-    const double g0 = N.wg[lane], g1 = two ? N.wg[32 + lane] : 0.0;
+    const double g0 = N.wg[lane];
     const int b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
     double rk[2], rg[2];
 #pragma unroll
     for (int t = 0; t < 2; t++) {
         rk[t] = fma(k1, fv[2 * t + 1], k0 * fv[2 * t]);
-        rg[t] = fma(g1, fv[2 * t + 1], g0 * fv[2 * t]);
+        rg[t] = g0 * fv[2 * t];
     }
     const int signs = __double2hiint(fv[0]) | __double2hiint(fv[1]) | __double2hiint(fv[2]) | __double2hiint(fv[3]);
     const bool negative = __any_sync(0xffffffffu, signs < 0);

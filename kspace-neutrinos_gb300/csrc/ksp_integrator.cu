@@ -87,7 +87,9 @@ __global__ void __launch_bounds__(kSplineThreads) k_rho_splines(Background* B) {
 
 void launch_background_tables(Background* dB, double a0, cudaStream_t st, unsigned* status) {
     (void)a0;
-    const int warps = 4;
+    // a warp per block: the 200 integrals of one mass state spread over the SMs' FP64 pipes (four
+    // warps per block used 50 of 152 SMs: 52 us, 47 so)
+    const int warps = 1;
     const int tasks = kNuSpecies * kNRhoTab;
     k_rho_points<<<(tasks + warps - 1) / warps, 32 * warps, warps * sizeof(QagList), st>>>(dB, status);
     k_rho_splines<<<kNuSpecies, kSplineThreads, 0, st>>>(dB);

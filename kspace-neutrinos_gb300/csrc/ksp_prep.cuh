@@ -265,19 +265,23 @@ __device__ __forceinline__ double fs_table_at(const FsTable& F, double x) {
 }
 
 // ------------------------------------------------------------------ knots
-// Row i of the factorised natural-spline system of the knots x[0..Na-1]: the pivot
+// Rows i0 .. i1 - 1 of the factorised natural-spline system of the knots x[0..Na-1]: the pivot
 // d_i = b_i - h_i^2 / d_{i-1}, b_i = 2 (h_i + h_{i+1}), h_i = x_{i+1} - x_i, as a quotient
-// of two-term recurrences p / q carried from 28 rows before (an error in a pivot shrinks
-// by 4 or more per row, so the start does not show), with two divisions at the end instead
-// of one per row.  knot(j): knot j.
+// of two-term recurrences p / q carried from 28 rows before i0 (an error in a pivot shrinks
+// by 4 or more per row, so the start does not show), with two divisions per row at its end.
+// knot(j): knot j.
 template <class X>
-__device__ __forceinline__ void knot_row(const X& knot, int i, double* invdiag, double* fac) {
-    int r = i > 28 ? i - 28 : 0;
+__device__ __forceinline__ void knot_rows(const X& knot, int i0, int i1, double* invdiag, double* fac) {
+    int r = i0 > 28 ? i0 - 28 : 0;
     double x1 = knot(r + 1), x2 = knot(r + 2);
     double h0 = x1 - knot(r), h1 = x2 - x1;
     double p = 2.0 * (h0 + h1), q = 1.0, pp = 0, qp = 0;
-    while (r < i) {
-        r++;
+    for (;;) {
+        if (r >= i0) {
+            invdiag[r] = q / p;
+            if (r > 0) fac[r] = h0 * (qp / pp);
+        }
+        if (++r >= i1) return;
         pp = p;
         qp = q;
         x1 = x2;
@@ -291,8 +295,10 @@ __device__ __forceinline__ void knot_row(const X& knot, int i, double* invdiag, 
             q = 1.0;
         }
     }
-    invdiag[i] = q / p;
-    if (i > 0) fac[i] = h0 * (qp / pp);
+}
+template <class X>
+__device__ __forceinline__ void knot_row(const X& knot, int i, double* invdiag, double* fac) {
+    knot_rows(knot, i, i + 1, invdiag, fac);
 }
 
 // ------------------------------------------------------------------ nodes
@@ -392,8 +398,11 @@ __device__ __forceinline__ void natural_spline_block(const double* x, const doub
                                                      double* invdiag, double* sh) {
     const int t = threadIdx.x;
     auto knot = [&](int j) { return x[j]; };
+    // a thread's rows side by side: one run-up for them (a row at a time, strided, 300 knots are 10
+    // run-ups of 28 steps on one FP64 pipe)
+    const int per = (n - 2 + T - 1) / T, u0 = t * per, u1 = min(u0 + per, n - 2);
+    if (u0 < u1) knot_rows(knot, u0, u1, invdiag, fac);
     for (int u = t; u < n - 2; u += T) {
-        knot_row(knot, u, invdiag, fac);
         c[u + 1] = 3.0 * ((y[u + 2] - y[u + 1]) / (x[u + 2] - x[u + 1]) - (y[u + 1] - y[u]) / (x[u + 1] - x[u]));
     }
     __syncthreads();

@@ -10,12 +10,12 @@
 //   y_m    = x_m (1 + norm interp_r(log|k_m|))                (correction, K3)
 // Adjoint (subdivision of every QAG held fixed, background Omega_nu(a), H(a) fixed):
 //   B1  k_adj_reduce8        rbar_j = norm sum_m (gbar_m . x_m) dinterp/dr_j   (reads gbar, x)
-//   B2a k_adj_bins           dnubar_b from rbar and the P_nu cotangent
-//   B2  k_dnu_adj            warp per (species, bin): history row and spline
-//                            coefficients staged by TMA bulk copies; the GK61 nodes of the
-//                            stored (or recomputed) final QAG intervals give
-//                            d/d(row) through the spline (cubic basis + transposed
+//   B2  k_dnu_adj            (needs no cotangent: beside B1) per (species, bin): history row
+//                            and spline coefficients staged by TMA bulk copies; the GK61 nodes
+//                            of the stored (or recomputed) final QAG intervals give d delta_nu /
+//                            d(row) through the spline (cubic basis + transposed
 //                            natural-spline solve) and d/dm through J's argument
+//   B2a k_adj_rows           dnubar_b from rbar and the P_nu cotangent, times B2's derivatives
 //   B2c k_adj_bins2          dcdm/P cotangents -> per-bin Q_b and the DC term
 //   B3  k_adj_grid           xbar_m = gbar_m smth_m + Q_b w_m W_m^4 x_m   (reads gbar, x; writes xbar)
 #include <cuda_runtime.h>
@@ -254,24 +254,13 @@ struct AdjBins {
     const long long* count;  // mode count per bin (indexed by bin)
     const int* compact;      // compact -> bin
     const double* F0sq;
-    double* dnu_bar;         // out [nk]
-    const double* dprov_bar; // provisional-row cotangent (from k_dnu_adj), stride ld
+    const double* dprov_bar; // provisional-row cotangent (from k_adj_rows), stride ld
     double* rbar;            // out [nk]
     double* Q;               // out: 2 Pbar_b / (F0 C_b), indexed by bin [nrbins]
     double* dc_sum;          // out: sum_b Pbar_b P_b (DC term)
     double norm, L3, fcdm;
     int ld;
 };
-
-__global__ void k_adj_bins(AdjBins A, int nk) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nk) return;
-    const double rb = A.norm * A.node_sum[b];
-    A.rbar[b] = rb;
-    const double v = A.dnu[b];
-    const double out = v < 0 ? 0.0 : v;
-    A.dnu_bar[b] = v > 0 ? (2.0 * out * A.pnu_bar[b] + rb / A.dcdm[b]) : 0.0;
-}
 
 __global__ void k_adj_bins2(AdjBins A, int nk) {
     __shared__ double red[8];
@@ -298,9 +287,8 @@ __global__ void k_adj_bins2(AdjBins A, int nk) {
 
 // ------------------------------------------------------------------ B2
 struct DnuAdjArgs {
-    const double* dnu_bar;   // [nk]
-    double* Dbar;            // [nk][ld] history cotangent (columns < Na)
-    double* mbar;            // [kNuSpecies]
+    double* unit;            // [nspec][nk][ld] d delta_nu of a (species, bin) / d row (columns < Na)
+    double* umass;           // [nspec][nk] and / d mass
     const double* ivals;     // stored intervals [kNuSpecies][nk][kQagLimit][2] or null
     const int* nivals;       // [kNuSpecies][nk]
     int recompute;
@@ -395,13 +383,12 @@ __global__ void __launch_bounds__(128) k_dnu_adj(IntegratorDev I, DnuAdjArgs A, 
         const double mnu = B->mnu_J[mi];
         const double mnubykT = mnu / B->kBtnu;
         const double k = I.wavenum[ik];
-        const double sbar = A.dnu_bar[ik] * S.omeganu[mi] / S.Omega_nu_tot;
-        if (sbar == 0.0) continue;
+        double* unit = A.unit + (size_t)task * I.ld;
         double mder = 0.0;
         // initial-condition piece (delta_tot_table.c:525-535)
         if (lane == 0 && mnubykT > 0) {
             const double x0 = k * S.fsl_A0a / mnubykT;
-            mder += sbar * specialJ_fit_deriv(x0) * (-x0 / mnu) * I.nu_init[ik] * (1. + S.deriv_prefac * S.fsl_A0a);
+            mder += specialJ_fit_deriv(x0) * (-x0 / mnu) * I.nu_init[ik] * (1. + S.deriv_prefac * S.fsl_A0a);
         }
         const bool integrate = !S.skip_integral && Na > 1 && mnubykT > 0;
         if (integrate) {
@@ -438,7 +425,7 @@ __global__ void __launch_bounds__(128) k_dnu_adj(IntegratorDev I, DnuAdjArgs A, 
                 nint = r.nint;
             }
             const DnuIntegrandC fi = dnu_integrand(I, S, k, mnubykT, qc, knots, row, rc, sb, sd, Na);
-            const double ckm = -sbar * S.prefac * fi.k_over_m / mnu;  // d(J's argument)/dm per fsl
+            const double ckm = -S.prefac * fi.k_over_m / mnu;  // d(J's argument)/dm per fsl
             for (int q = 0; q < nint; q++)
                 adj_interval(fi, N, knots, row, rc, Na, qc, iv ? iv[2 * q] : L.a[q], iv ? iv[2 * q + 1] : L.b[q],
                              S.loga0, S.loga, NcLayout{I.nc_slots, I.nc_tree}, ckm, ybar, cbar, mder, lane);
@@ -460,10 +447,41 @@ __global__ void __launch_bounds__(128) k_dnu_adj(IntegratorDev I, DnuAdjArgs A, 
             }
             __syncwarp();
             for (int j = lane; j < Na; j += 32)  // column Na-1: the provisional row
-                atomicAdd(&A.Dbar[(size_t)ik * I.ld + j], S.prefac * sbar * ybar[j]);
+                unit[j] = S.prefac * ybar[j];
+        } else {
+            for (int j = lane; j < Na; j += 32) unit[j] = 0.0;
         }
         mder = warp_sum_to0(mder);
-        if (lane == 0 && mder != 0.0) atomicAdd(&A.mbar[mi], mder);
+        if (lane == 0) A.umass[task] = mder;
+    }
+}
+
+// The history's and the masses' gradients, a block per bin: delta_nu's cotangent (B2a) times the
+// derivatives that k_dnu_adj made beside B1 (42 us of it at 128 bins x 128 rows), summed over the
+// species.
+__global__ void __launch_bounds__(128) k_adj_rows(IntegratorDev I, AdjBins A, const double* unit, const double* umass,
+                                                  double* Dbar, double* mbar, int nk, int Na, int nspec,
+                                                  int4 spec_ids) {
+    __shared__ double sbar[kNuSpecies];
+    const int ik = blockIdx.x, tid = threadIdx.x;
+    const StepScalars& S = *I.sc;
+    if (tid < nspec) {
+        const double rb = A.norm * A.node_sum[ik];
+        if (tid == 0) A.rbar[ik] = rb;
+        const double v = A.dnu[ik];
+        const double db = v > 0 ? 2.0 * v * A.pnu_bar[ik] + rb / A.dcdm[ik] : 0.0;
+        const int mi = tid == 0 ? spec_ids.x : (tid == 1 ? spec_ids.y : spec_ids.z);
+        const double s = db * S.omeganu[mi] / S.Omega_nu_tot;
+        sbar[tid] = s;
+        const double m = s != 0.0 ? s * umass[(size_t)tid * nk + ik] : 0.0;
+        if (m != 0.0) atomicAdd(&mbar[mi], m);
+    }
+    __syncthreads();
+    for (int j = tid; j < Na; j += blockDim.x) {
+        double v = 0.0;
+        for (int si = 0; si < nspec; si++)
+            if (sbar[si] != 0.0) v += sbar[si] * unit[((size_t)si * nk + ik) * I.ld + j];
+        Dbar[(size_t)ik * I.ld + j] = v;
     }
 }
 
@@ -622,13 +640,12 @@ __global__ void __launch_bounds__(128) k_dnu_adj_blk(IntegratorDev I, DnuAdjArgs
         const double mnu = B->mnu_J[mi];
         const double mnubykT = mnu / B->kBtnu;
         const double k = I.wavenum[ik];
-        const double sbar = A.dnu_bar[ik] * S.omeganu[mi] / S.Omega_nu_tot;
-        if (sbar == 0.0) continue;  // block-uniform
+        double* unit = A.unit + (size_t)task * I.ld;
         double mder = 0.0;
         // initial-condition piece (delta_tot_table.c:525-535)
         if (tid == 0 && mnubykT > 0) {
             const double x0 = k * S.fsl_A0a / mnubykT;
-            mder += sbar * specialJ_fit_deriv(x0) * (-x0 / mnu) * I.nu_init[ik] * (1. + S.deriv_prefac * S.fsl_A0a);
+            mder += specialJ_fit_deriv(x0) * (-x0 / mnu) * I.nu_init[ik] * (1. + S.deriv_prefac * S.fsl_A0a);
         }
         const bool integrate = !S.skip_integral && Na > 1 && mnubykT > 0;
         if (integrate) {
@@ -668,7 +685,7 @@ __global__ void __launch_bounds__(128) k_dnu_adj_blk(IntegratorDev I, DnuAdjArgs
             }
             __syncthreads();
             const DnuIntegrandC fi = dnu_integrand(I, S, k, mnubykT, qc, knots, row, rc, sb, sd, Na);
-            const double ckm = -sbar * S.prefac * fi.k_over_m / mnu;
+            const double ckm = -S.prefac * fi.k_over_m / mnu;
             double* yb = wy + (size_t)warp * I.ld;
             double* cb = wc + (size_t)warp * I.ld;
             for (int q = warp; q < nint; q += nw)
@@ -696,8 +713,10 @@ __global__ void __launch_bounds__(128) k_dnu_adj_blk(IntegratorDev I, DnuAdjArgs
                     if (j >= 1 && j <= m) v -= 3 * wc[j] * (ih[j - 1] + ih[j]);
                     if (j < m) v += 3 * wc[j + 1] * ih[j];
                 }
-                atomicAdd(&A.Dbar[(size_t)ik * I.ld + j], S.prefac * sbar * v);
+                unit[j] = S.prefac * v;
             }
+        } else {
+            for (int j = tid; j < Na; j += blockDim.x) unit[j] = 0.0;
         }
         mder = warp_sum_to0(mder);
         if (lane == 0) s_red[warp] = mder;
@@ -705,7 +724,7 @@ __global__ void __launch_bounds__(128) k_dnu_adj_blk(IntegratorDev I, DnuAdjArgs
         if (tid == 0) {
             double t = 0.0;
             for (int w = 0; w < nw; w++) t += s_red[w];
-            if (t != 0.0) atomicAdd(&A.mbar[mi], t);
+            A.umass[task] = t;
         }
         __syncthreads();
     }
@@ -770,22 +789,26 @@ void launch_adj_reduce(const GridGeom& gg, CorrTable corr, float lnscale, const 
                                                                           node_sum);
 }
 
-void launch_adj_bins(const AdjBinsHost& h, cudaStream_t st) {
-    AdjBins A{h.node_sum, h.pnu_bar, h.dnu, h.dcdm, h.power, h.count, h.compact, h.F0sq, h.dnu_bar, h.dprov_bar,
-              h.rbar, h.Q, h.dc_sum, h.norm, h.L3, h.fcdm, h.ld};
-    k_adj_bins<<<(h.nk + 127) / 128, 128, 0, st>>>(A, h.nk);
+static AdjBins adj_bins(const AdjBinsHost& h) {
+    return AdjBins{h.node_sum, h.pnu_bar, h.dnu,  h.dcdm, h.power, h.count, h.compact, h.F0sq,
+                   h.dprov_bar, h.rbar, h.Q, h.dc_sum, h.norm, h.L3, h.fcdm, h.ld};
+}
+
+void launch_adj_rows(const IntegratorDev& I, const AdjBinsHost& h, const double* unit, const double* umass,
+                     double* Dbar, double* mbar, int nk, int Na, int nspec, const int* spec_ids, cudaStream_t st) {
+    k_adj_rows<<<nk, 128, 0, st>>>(I, adj_bins(h), unit, umass, Dbar, mbar, nk, Na, nspec,
+                                   make_int4(spec_ids[0], spec_ids[1], spec_ids[2], 0));
 }
 
 void launch_adj_bins2(const AdjBinsHost& h, cudaStream_t st) {
-    AdjBins A{h.node_sum, h.pnu_bar, h.dnu, h.dcdm, h.power, h.count, h.compact, h.F0sq, h.dnu_bar, h.dprov_bar,
-              h.rbar, h.Q, h.dc_sum, h.norm, h.L3, h.fcdm, h.ld};
+    const AdjBins A = adj_bins(h);
     k_adj_bins2<<<1, 256, 0, st>>>(A, h.nk);
 }
 
-void launch_dnu_adj(const IntegratorDev& I, const double* dnu_bar, double* Dbar, double* mbar, const double* ivals,
+void launch_dnu_adj(const IntegratorDev& I, double* unit, double* umass, const double* ivals,
                     const int* nivals, int recompute, int nk, int Na, int nspec, const int* spec_ids, int wpb,
                     cudaStream_t st) {
-    DnuAdjArgs A{dnu_bar, Dbar, mbar, ivals, nivals, recompute};
+    DnuAdjArgs A{unit, umass, ivals, nivals, recompute};
     wpb = wpb < 1 ? 1 : (wpb > 4 ? 4 : wpb);
     while (wpb > 1 && dnu_adj_smem(I.ld, wpb) > 227 * 1024 - 256) wpb--;
     const size_t smem = dnu_adj_smem(I.ld, wpb);

@@ -151,11 +151,11 @@ static void free_table(kspace_ctx* c) {
     if (c->ar_h) cudaFreeHost(c->ar_h);
     c->ar_h = c->io_h = nullptr;
     void* adj[] = {c->ivals_d, c->adj_node_d, c->adj_Dbar_d, c->adj_mbar_d, c->adj_Q_d, c->adj_dcsum_d,
-                   c->adj_dnubar_d, c->adj_rbar_d, c->nivals_d};
+                   c->adj_unit_d, c->adj_rbar_d, c->nivals_d};
     for (void* p : adj)
         if (p) cudaFree(p);
     c->ivals_d = c->adj_node_d = c->adj_Dbar_d = c->adj_mbar_d = c->adj_Q_d = c->adj_dcsum_d = nullptr;
-    c->adj_dnubar_d = c->adj_rbar_d = nullptr;
+    c->adj_unit_d = c->adj_rbar_d = nullptr;
     c->nivals_d = nullptr;
     c->adj_cap_nb = 0;
     c->diff_ready = false;
@@ -1793,7 +1793,7 @@ static int ensure_adj_buffers(kspace_ctx* c, int nrbins) {
         CK(dalloc(&c->adj_Dbar_d, nk * ld));
         CK(dalloc(&c->adj_mbar_d, kNuSpecies));
         CK(dalloc(&c->adj_dcsum_d, 1));
-        CK(dalloc(&c->adj_dnubar_d, nk));
+        CK(dalloc(&c->adj_unit_d, kNuSpecies * nk * (ld + 1)));
         CK(dalloc(&c->adj_rbar_d, nk));
     }
     if (c->adj_cap_nb < nrbins) {
@@ -1906,8 +1906,14 @@ extern "C" int kspace_gpu_diff_backward(kspace_ctx* c, const void* gbar_out, con
     IntegratorDev& I = c->I;
     const int nk = c->diff_nk, Na = c->diff_Na;
     const double a = c->diff_time, L = c->diff_box;
+    // the integrals' derivatives need no cotangent: beside the pass over the grid (B1)
+    double* umass = c->adj_unit_d + (size_t)kNuSpecies * I.nk_alloc * I.ld;
+    CK(cudaEventRecord(c->ev_fork, c->stream));
+    CK(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
+    launch_dnu_adj(I, c->adj_unit_d, umass, c->ivals_d, c->nivals_d, recompute, nk, Na, c->nspec, c->spec_ids,
+                   c->qag_warps, c->side);
+    CK(cudaEventRecord(c->ev_join, c->side));
     CK(cudaMemsetAsync(c->adj_node_d, 0, sizeof(double) * nk, c->stream));
-    CK(cudaMemsetAsync(c->adj_Dbar_d, 0, sizeof(double) * (size_t)I.nk_alloc * I.ld, c->stream));
     CK(cudaMemsetAsync(c->adj_mbar_d, 0, sizeof(double) * kNuSpecies, c->stream));
     CK(cudaMemsetAsync(c->adj_Q_d, 0, sizeof(double) * G->g.nrbins, c->stream));
     CorrTable corr = c->corr;
@@ -1932,7 +1938,6 @@ extern "C" int kspace_gpu_diff_backward(kspace_ctx* c, const void* gbar_out, con
     h.count = G->count_d;
     h.compact = G->compact_d;
     h.F0sq = c->F0sq_d;
-    h.dnu_bar = c->adj_dnubar_d;
     h.dprov_bar = c->adj_Dbar_d + (Na - 1);  // provisional column, stride ld
     h.rbar = c->adj_rbar_d;
     h.Q = c->adj_Q_d;
@@ -1942,9 +1947,8 @@ extern "C" int kspace_gpu_diff_backward(kspace_ctx* c, const void* gbar_out, con
     h.fcdm = 1 - OmegaNua3 / (c->Omeganonu + OmegaNu1);
     h.nk = nk;
     h.ld = I.ld;
-    launch_adj_bins(h, c->stream);
-    launch_dnu_adj(I, c->adj_dnubar_d, c->adj_Dbar_d, c->adj_mbar_d, c->ivals_d, c->nivals_d, recompute, nk, Na,
-                   c->nspec, c->spec_ids, c->qag_warps, c->stream);
+    CK(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+    launch_adj_rows(I, h, c->adj_unit_d, umass, c->adj_Dbar_d, c->adj_mbar_d, nk, Na, c->nspec, c->spec_ids, c->stream);
     launch_adj_bins2(h, c->stream);
     launch_adj_grid(G->g, corr, lnscale, reinterpret_cast<const float*>(gbar_out),
                     reinterpret_cast<const float*>(grid_in), reinterpret_cast<float*>(gbar_in), c->adj_Q_d,

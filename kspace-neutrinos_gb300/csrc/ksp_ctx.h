@@ -75,7 +75,7 @@ struct kspace_ctx {
     // differentiable step
     double Omeganonu = 0;
     double *ivals_d = nullptr, *adj_node_d = nullptr, *adj_Dbar_d = nullptr, *adj_mbar_d = nullptr;
-    double *adj_Q_d = nullptr, *adj_dcsum_d = nullptr, *adj_dnubar_d = nullptr, *adj_rbar_d = nullptr;
+    double *adj_Q_d = nullptr, *adj_dcsum_d = nullptr, *adj_unit_d = nullptr, *adj_rbar_d = nullptr;
     int* nivals_d = nullptr;
     int adj_cap_nb = 0;
     bool diff_ready = false;

@@ -460,7 +460,7 @@ void launch_finish_update(const IntegratorDev& I, int nk, int commit_row, double
 struct AdjBinsHost {
     const double* node_sum; const double* pnu_bar; const double* dnu; const double* dcdm; const double* power;
     const long long* count; const int* compact; const double* F0sq;
-    double* dnu_bar; double* dprov_bar; double* rbar; double* Q; double* dc_sum;
+    double* dprov_bar; double* rbar; double* Q; double* dc_sum;
     double norm, L3, fcdm;
     int nk, ld;  // dprov_bar has stride ld
 };
@@ -503,9 +503,10 @@ void launch_finalize_power(const double* bin_sum, const double* F0sq, const long
 struct GridGeom;
 void launch_adj_reduce(const GridGeom& gg, CorrTable corr, float lnscale, const float* gbar, const float* x,
                        double* node_sum, cudaStream_t st);
-void launch_adj_bins(const AdjBinsHost& h, cudaStream_t st);
+void launch_adj_rows(const IntegratorDev& I, const AdjBinsHost& h, const double* unit, const double* umass,
+                     double* Dbar, double* mbar, int nk, int Na, int nspec, const int* spec_ids, cudaStream_t st);
 void launch_adj_bins2(const AdjBinsHost& h, cudaStream_t st);
-void launch_dnu_adj(const IntegratorDev& I, const double* dnu_bar, double* Dbar, double* mbar, const double* ivals,
+void launch_dnu_adj(const IntegratorDev& I, double* unit, double* umass, const double* ivals,
                     const int* nivals, int recompute, int nk, int Na, int nspec, const int* spec_ids, int wpb,
                     cudaStream_t st);
 void launch_adj_grid(const GridGeom& gg, CorrTable corr, float lnscale, const float* gbar, const float* x, float* xbar,

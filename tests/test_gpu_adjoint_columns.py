@@ -48,3 +48,21 @@ def test_output_beside_the_input(gpu, oracle, N, nb, Na):
     assert torch.equal(g, g0) and torch.equal(out, work)
     assert out[0, 0, 0] == g[0, 0, 0] and not torch.equal(out, g)
     k.close()
+
+
+@pytest.mark.parametrize("N,nb", [(30, 20), (48, 500)])
+@pytest.mark.parametrize("recompute", [False, True])
+def test_history_gradient_of_three_mass_states(gpu, oracle, N, nb, recompute):
+    """The derivatives of the integrals, made without the cotangent and summed over the species
+    afterwards: a block per (species, bin) and, from 608 of them up, a warp."""
+    c, ref, k, a = setup(oracle, gpu, N, nb, 16, (0.02, 0.03, 0.06), seed=N)
+    assert (3 * c["nk"] >= 608) == (nb == 500)
+    wb = np.random.default_rng(N).random(c["nk"])
+    xg, Dg, mg, out, pnu = gpu_grads(k, c, a, wb, recompute=recompute)
+    adj = ref.adjoint(c["grid"].astype(np.complex128), c["delta_tot"], np.array(c["MNu"]), wb)
+    xr, Dr = adj["xbar"], adj["Dbar"]
+    assert np.max(np.abs(xg - xr)) <= 1e-5 * np.max(np.abs(xr))
+    assert np.max(np.abs(Dg - Dr)) <= 1e-5 * np.max(np.abs(Dr))
+    for i in range(3):
+        assert abs(mg[i] / adj["mbar"][i] - 1) < 1e-5
+    k.close()

@@ -782,7 +782,13 @@ static bool launch_dnu_qag_blk(const IntegratorDev& I, int nk, int Na, int nspec
     const size_t smem = dnu_qag_blk_smem<G>(I.ld);
     if (smem > 227 * 1024 - 256) return false;
     raise_dynamic_smem_limit(reinterpret_cast<const void*>(k_dnu_qag_blk<G>));
-    launch_dependent(k_dnu_qag_blk<G>, nspec * nk, threads, smem, st, I, nk, Na, nspec, spec_ids, upd);
+    // Small blocks not as dependents: the up to eight an SM takes spread unevenly over the SMs if
+    // they come up while the kernel before is still there (1221 tasks of 2 warps: a call of 138 us
+    // as dependents, 125 so; of 8 warps, two to an SM, 4-5 us are won instead).
+    if constexpr (G == 0)
+        k_dnu_qag_blk<G><<<nspec * nk, threads, smem, st>>>(I, nk, Na, nspec, spec_ids, upd);
+    else
+        launch_dependent(k_dnu_qag_blk<G>, nspec * nk, threads, smem, st, I, nk, Na, nspec, spec_ids, upd);
     return true;
 }
 
@@ -824,16 +830,13 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
         }
         // a block per task: with no more tasks than SMs 12 warps and two levels of look-ahead
         // (split 12; a call of 64, 100, 150 bins 62, 71, 78 us, with 8 warps and one level 64, 74,
-        // 82; three levels 65, 75, 77; but 200 bins 86 against 82), 8 warps and one level (split 8) below 4 tasks
-        // per SM, 4 warps without look-ahead up to 6, 2 warps from there (at 128 registers a
-        // thread, 4 blocks of 4 warps fit an SM: 1221 tasks of 3 species x 407 bins take two
-        // waves of 4-warp blocks and one of 2-warp blocks, measured 0.211 against 0.223 ms; a
-        // warp per task, split 1, 0.231 ms).  Where hybrid neutrinos cut J the next interval is
-        // anyone's guess: two intervals a round by their errors (151 bins 228 us; one 256, one
-        // and a level of look-ahead 310, three 222 but 60 bins 216 against 214)
-        const int split = qag_split > 0   ? qag_split
-                          : ntask <= nsm ? 12
-                                         : (ntask < 4 * nsm ? 8 : (ntask < 6 * nsm ? 4 : 2));
+        // 82; three levels 65, 75, 77; but 200 bins 86 against 82), 8 warps and one level (split 8)
+        // below 4 tasks per SM (512 tasks 105 us; 4 warps without look-ahead 115, 2 117), 2 warps
+        // from there (750, 900, 1221, 1536 tasks 103, 107, 125, 137 us; 4 warps 115, 126, 139, 160;
+        // a warp per task, split 1, 108, 107, 127, 140).  Where hybrid neutrinos cut J the next
+        // interval is anyone's guess: two intervals a round by their errors (151 bins 228 us; one
+        // 256, one and a level of look-ahead 310, three 222 but 60 bins 216 against 214)
+        const int split = qag_split > 0 ? qag_split : (ntask <= nsm ? 12 : (ntask < 4 * nsm ? 8 : 2));
         const bool cut = qag_split <= 0 && I.nc_tree > 1;
         const int4 sp = make_int4(spec_ids[0], spec_ids[1], spec_ids[2], 0);
         const bool done =

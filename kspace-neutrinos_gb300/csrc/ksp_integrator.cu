@@ -736,6 +736,16 @@ size_t dnu_qag_smem(int ld, int wpb) {
            wpb * sizeof(uint64_t);
 }
 
+static int sm_count_i() {
+    static const int n = [] {
+        int dev = 0, c = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
+        return c > 0 ? c : 1;
+    }();
+    return n;
+}
+
 // Blocks per role of a call's preparation.
 void launch_integrator_prepare(const IntegratorDev& I, const Background& B, const StepScalars& S, int Na, double a,
                                double loga, double loga0, double TimeTransfer, int start_row, int write_knot,
@@ -769,9 +779,16 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
     const int nrow = rows == kRowsBase ? nk + 1 : (rows == kRowsFull && (Na > 2 || update_row >= 0) ? nk : 0);
     const int blocks = nrow + fs_table_blocks(P.fs.n, kTableThreads) +
                        (P.nodes + kTableThreads - 1) / kTableThreads;
-    if (blocks > 0)
-        launch_dependent(k_prep_tables, blocks, kTableThreads, 0, st, I, P, nrow > 0 ? (int)rows : (int)kRowsNone, nk,
-                         update_row, fin ? *fin : FinalizeArgs{});
+    if (blocks <= 0) return;
+    const int mode = nrow > 0 ? (int)rows : (int)kRowsNone;
+    const FinalizeArgs f = fin ? *fin : FinalizeArgs{};
+    // As a dependent the kernel starts 2-3 us earlier, but several blocks to an SM then spread
+    // unevenly (as launch_dnu_qag_blk's): calls of 400 to 512 bins, 430 to 560 blocks, 101, 125,
+    // 137 us as dependents and 98, 122, 131 after it; of 200 to 300 bins 85 and 84 to 87.
+    if (2 * blocks > 5 * sm_count_i())
+        k_prep_tables<<<blocks, kTableThreads, 0, st>>>(I, P, mode, nk, update_row, f);
+    else
+        launch_dependent(k_prep_tables, blocks, kTableThreads, 0, st, I, P, mode, nk, update_row, f);
 }
 
 // The rest, after the rows' splines: the integrals, the species sum.
@@ -821,13 +838,7 @@ void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, c
     }
     const int ntask = nspec * nk;
     if (ntask > 0) {
-        static int nsm = 0;
-        if (!nsm) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-            if (nsm <= 0) nsm = 1;
-        }
+        const int nsm = sm_count_i();
         // a block per task: with no more tasks than SMs 12 warps and two levels of look-ahead
         // (split 12; a call of 64, 100, 150 bins 62, 71, 78 us, with 8 warps and one level 64, 74,
         // 82; three levels 65, 75, 77; but 200 bins 86 against 82), 8 warps and one level (split 8)

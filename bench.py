@@ -837,7 +837,7 @@ def run_batch(args, cfg):
         "autotune": {"warps_per_block_blocks_per_sm": tune[0], "ms": tune[1]} if tune else None,
         "e2e": {"value": e2e, "unit": "solves/s", "h2d_bytes_per_step": 8 * nbins_total,
                 "d2h_bytes_per_step": 8 * nbins_total},
-        "gpu_launches": args.steps * (8 + 3 * G),
+        "gpu_launches": args.steps * (6 + (1 + 3 * G if G else 0)),
         "setup_s": t_setup,
         "clocks": clk.summary(),
     }

@@ -334,7 +334,8 @@ KSP_HD double specialJ(double x, double qc, double nufrac_low) {
 // Index of the largest error among e[0..n) (lowest index on ties), on every lane of
 // the warp.  Errors are >= 0, so their IEEE bit patterns order as the numbers do: the
 // comparisons run on the integer pipe (a NaN, never chosen by the floating-point
-// comparison, gets key -1).
+// comparison, gets key -1; with nothing else in the list it is entry 0, as in QUADPACK's
+// search, whose first candidate that is).
 __device__ __forceinline__ long long err_key(double e) {
     const long long b = __double_as_longlong(e);
     return (b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL ? -1LL : b;
@@ -342,7 +343,7 @@ __device__ __forceinline__ long long err_key(double e) {
 __device__ __forceinline__ int warp_argmax_err(const double* e, int n) {
     const int lane = threadIdx.x & 31;
     long long best = -1;
-    int bk = 0x7fffffff;
+    int bk = lane;
     for (int i = lane; i < n; i += 32) {
         const long long v = err_key(e[i]);
         if (v > best) { best = v; bk = i; }

@@ -53,7 +53,10 @@ __global__ void kb_prologue(BatchDev b) {
         const int Na = P.Na;
         const bool integrate = P.commit_row != -2;
         if (threadIdx.x < 32) call_scalars_warp(*I.B, a, P.loga, P.loga0, P.TimeTransfer, integrate ? Na : 1, S);
-        if (threadIdx.x == 0 && integrate) I.scalefact[Na - 1] = P.loga;
+        if (threadIdx.x == 0 && integrate) {
+            I.scalefact[Na - 1] = P.loga;
+            if (Na > 1 && no_number(P.loga)) atomicOr(I.status, kStGsl);
+        }
         __syncthreads();
         if (!integrate) continue;
         const double OmegaNua3 = S.OmegaNua3, OmegaNu1 = S.OmegaNu1, partnu = S.partnu, Omeganonu = S.Omeganonu;

@@ -415,7 +415,7 @@ static int plan_call(kspace_batch* b, const double* a, bool dry, std::vector<int
                 const int Na = c->ia + 1;
                 P.Na = Na;
                 P.start_row = c->fact_valid;
-                P.fs = fs_grid(loga > c->loga0 ? 16 * Na : 0, c->loga0, loga);
+                P.fs = fs_grid(no_interval(c->loga0, loga) ? 0 : 16 * Na, c->loga0, loga);
                 const bool commit = a[i] >= exp(c->h_scalefact[Na - 2]) + 0.009;  // :229-237
                 P.commit_row = commit ? Na - 1 : -1;
                 after[i] = dry ? 0 : (commit ? 1 : 2);

@@ -290,6 +290,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_eval(IntegratorDev I, 
             *I.qag_max = 0;  // this call's QAG statistics start from zero
             *I.qag_total = 0;
             if (P.write_knot) I.scalefact[Na - 1] = P.loga;  // the provisional knot
+            if (Na > 1 && no_number(P.loga)) atomicOr(I.status, kStGsl);  // as QAG would end
         }
         return;
     }
@@ -767,7 +768,7 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
     P.in = in;
     P.in_blocks = (2 * in.n + kPrepThreads - 1) / kPrepThreads;
     P.knot_blocks = (Na - 1 + kPrepThreads - 1) / kPrepThreads;
-    if (loga > loga0) {  // the fslength table also gives fslength(log a0, log a)
+    if (!no_interval(loga0, loga)) {  // the fslength table also gives fslength(log a0, log a)
         P.fs = fs_grid(16 * (Na > 1 ? Na : 1), loga0, loga);
         P.fs_blocks = fs_blocks(P.fs);
         P.nodes = Na > 1 ? I.nc_slots * 61 : 0;

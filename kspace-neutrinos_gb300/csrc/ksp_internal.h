@@ -24,7 +24,7 @@ struct StepScalars {
     double partnu_now;               // particle_nu_fraction(a, 0) (:539)
     double kspace_prefac;            // interface_common.c:139-145
     double fs_h, fs_ih;              // spacing of the fslength table's nodes, and its inverse
-    int skip_integral;               // particles carry everything (:542-543)
+    int skip_integral;               // particles carry everything (:542-543), or no_interval
     int Na, Nfs;
 };
 
@@ -98,6 +98,13 @@ struct IntegratorDev {
                                      // the other knots zero (kRowsBase)
 };
 
+// Whether a call at log a has nothing to integrate: at a0 the interval is empty, before a0
+// fslength, a factor of the integrand, is zero (delta_tot_table.c:394-396), and an end that is no
+// finite number is refused (no_number).  No fslength table and no node table is made then, and
+// the integrals read neither.
+KSP_HD bool no_number(double loga) { return !isfinite(loga); }
+KSP_HD bool no_interval(double loga0, double loga) { return !(loga > loga0) || no_number(loga); }
+
 // What the integrals and the species sum need of a species, from its omeganu, Omega_nu_tot and
 // partnu.
 KSP_HD void species_scalars(const Background& B, int mi, StepScalars& S) {
@@ -128,7 +135,7 @@ inline void call_scalars(const Background& B, double a, double loga, double loga
     S.deriv_prefac = TT * (hubble(B, TT) / S.light) * TT;
     S.relerr = 1e-6;
     S.partnu_now = partnu;
-    S.skip_integral = 0;
+    S.skip_integral = no_interval(loga0, loga) ? 1 : 0;
     if (S.partnu_now > 0) {
         if (1 - S.partnu_now < 1e-3) S.skip_integral = 1;
         S.relerr /= (1. + 1e-5 - S.partnu_now);
@@ -173,7 +180,7 @@ __device__ __forceinline__ void call_scalars_warp(const Background& B, double a,
     S.deriv_prefac = TT * (h_tt / S.light) * TT;
     S.relerr = 1e-6;
     S.partnu_now = partnu;
-    S.skip_integral = 0;
+    S.skip_integral = no_interval(loga0, loga) ? 1 : 0;
     if (S.partnu_now > 0) {
         if (1 - S.partnu_now < 1e-3) S.skip_integral = 1;
         S.relerr /= (1. + 1e-5 - S.partnu_now);

@@ -1761,21 +1761,15 @@ extern "C" int kspace_gpu_set_vectors(kspace_ctx* c, const double* nu_init, cons
     return KSPACE_OK;
 }
 
-// The values travel as kernel arguments: nothing of the host's is read after the call.
-__global__ void k_set_jmass(Background* B, double m0, double m1, double m2) {
-    B->mnu_J[0] = m0;
-    B->mnu_J[1] = m1;
-    B->mnu_J[2] = m2;
-}
-
+// Waits: a batch reads the masses on its own streams, and the context's stream may be another one
+// by the next call (set_stream).
 extern "C" int kspace_gpu_set_jmass(kspace_ctx* c, const double* MNu) {
     NEED(c, KSPACE_ERR_ARG);
     NEED(c->bg_ready, KSPACE_ERR_ORDER);
     for (int i = 0; i < kNuSpecies; i++) c->hB.mnu_J[i] = MNu ? MNu[i] : c->hB.mnu[i];
-    static_assert(kNuSpecies == 3, "one argument per species");
-    k_set_jmass<<<1, 1, 0, c->stream>>>(c->dB, c->hB.mnu_J[0], c->hB.mnu_J[1], c->hB.mnu_J[2]);
-    g_launches += 1;
-    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&c->dB->mnu_J[0], &c->hB.mnu_J[0], sizeof(double) * kNuSpecies, cudaMemcpyHostToDevice,
+                       c->stream));
+    CK(cudaStreamSynchronize(c->stream));
     return KSPACE_OK;
 }
 

@@ -768,17 +768,23 @@ void launch_adj_reduce(const GridGeom& gg, CorrTable corr, float lnscale, const 
     GridArgs a = make_grid_args(gg, corr.nk, lnscale);
     const bool aligned = ((reinterpret_cast<uintptr_t>(gbar) | reinterpret_cast<uintptr_t>(x)) & 15) == 0;
     if (aligned && corr.nk >= 2) {
+        // eight warps up to 5811 nodes (a float per node and warp, two for the table); above, as
+        // many as the shared memory has room for
+        auto smem_of = [&](int nw) { return sizeof(float) * corr.nk * (2 + nw); };
+        int nw = 8;
+        while (nw > 1 && smem_of(nw) > 227 * 1024) nw--;
+        const size_t smem = smem_of(nw);
+        const int threads = 32 * nw;
         const long long nchunks = (gg.nmodes + 7) / 8;
-        long long blocks = (nchunks + 255) / 256;
+        long long blocks = (nchunks + threads - 1) / threads;
         if (blocks > 4LL * sm_count_a()) blocks = 4LL * sm_count_a();
         if (blocks < 1) blocks = 1;
-        const long long adv = blocks * 256 * 8;  // modes per grid stride
+        const long long adv = blocks * threads * 8;  // modes per grid stride
         const int nz = gg.N / 2 + 1;
-        const size_t smem = sizeof(float) * corr.nk * (2 + 8);
         cudaFuncSetAttribute(k_adj_reduce8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         const long long adv_rows = adv / nz;
-        k_adj_reduce8<<<(int)blocks, 256, smem, st>>>(a, corr, gbar, x, node_sum, nchunks, (int)(adv_rows / gg.N),
-                                                      (int)(adv_rows % gg.N), (int)(adv % nz));
+        k_adj_reduce8<<<(int)blocks, threads, smem, st>>>(a, corr, gbar, x, node_sum, nchunks, (int)(adv_rows / gg.N),
+                                                          (int)(adv_rows % gg.N), (int)(adv % nz));
         return;
     }
     const size_t smem = sizeof(double) * corr.nk + sizeof(int) * (2 * gg.nrbins + 1) + sizeof(float) * 3 * corr.nk + 64;

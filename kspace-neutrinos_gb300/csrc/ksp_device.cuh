@@ -110,10 +110,6 @@ KSP_HD double cspline_seg(const double* x, const double* y, const double* c, int
     return y[i] + dx * (b + dx * (c[i] + dx * d));
 }
 
-KSP_HD double linear_seg(const double* x, const double* y, int i, double v) {
-    return y[i] + (v - x[i]) * ((y[i + 1] - y[i]) / (x[i + 1] - x[i]));
-}
-
 // ------------------------------------------------------------------ background
 // omega_nu_single.c:100-114 (rho_nu conversion factor)
 KSP_HD double rho_nu_conversion() {

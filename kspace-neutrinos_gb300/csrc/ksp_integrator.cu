@@ -542,20 +542,25 @@ __global__ void __launch_bounds__(qag_blk_threads(G), 512 / qag_blk_threads(G))
     Smem& sh = *reinterpret_cast<Smem*>(sm + off);
     off += (sizeof(Smem) + 15) & ~size_t(15);
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + off);
-    __shared__ double s_y, s_dy;  // the current task's provisional value, and what it adds
+    __shared__ double s_y, s_dy;  // the provisional value, and what it adds
     const int tid = threadIdx.x;
     const StepScalars& S = *I.sc;
-    const int ntask = nspec * nk;
-    const unsigned row_bytes = (unsigned)(((Na + 1) & ~1) * sizeof(double));
-    // Thread 0 starts a task: the copies of its history row and spline coefficients, then the
-    // provisional value while they land; another warp's first thread leaves the
+    // Blocks take the tasks from the last: the high-k bins of the last species, among the
+    // deepest QAG subdivisions, start first, and the blocks that wait for a free slot
+    // (more tasks than resident blocks) get the shallow low-k bins of the first species.
+    const int task = nspec * nk - 1 - (int)blockIdx.x, si = task / nk, ik = task % nk;
+    const int mi = si == 0 ? spec_ids.x : (si == 1 ? spec_ids.y : spec_ids.z);
+    const double k = I.kq ? I.kq[ik] : I.wavenum[ik];
+    const bool integrate = !S.skip_integral && Na > 1 && S.inv_m[mi] > 0;  // block-uniform
+    // Thread 0: the copies of the history row and its spline coefficients, in flight while the
+    // block fills its tables, and the provisional value; another warp's first thread leaves the
     // initial-condition term where the integral will be added.
-    auto start_task = [&](int task) {
-        const int si = task / nk, ik = task % nk;
-        const int mi = si == 0 ? spec_ids.x : (si == 1 ? spec_ids.y : spec_ids.z);
-        if (tid == 32) I.dnu_s[(size_t)mi * I.nk_alloc + ik] = dnu_initial(I, S, ik, mi, I.kq ? I.kq[ik] : I.wavenum[ik]);
-        if (tid != 0) return;
-        if (!S.skip_integral && Na > 1 && S.inv_m[mi] > 0) {
+    if (tid == 32) I.dnu_s[(size_t)mi * I.nk_alloc + ik] = dnu_initial(I, S, ik, mi, k);
+    if (tid == 0) {
+        ptx::mbar_init(bar, 1);
+        ptx::mbar_init_fence();
+        if (integrate) {
+            const unsigned row_bytes = (unsigned)(((Na + 1) & ~1) * sizeof(double));
             ptx::fence_async_smem();
             ptx::mbar_expect_tx(bar, Na > 2 ? 2 * row_bytes : row_bytes);
             ptx::bulk_g2s(row, I.dtot + (size_t)ik * I.ld, row_bytes, bar);
@@ -577,66 +582,40 @@ __global__ void __launch_bounds__(qag_blk_threads(G), 512 / qag_blk_threads(G))
             s_y = get_delta_tot(I.nu_last[ik], d, S.OmegaNua3, S.Omeganonu, S.OmegaNu1, S.partnu);
             s_dy = s_y - I.dtot[(size_t)ik * I.ld + Na - 2];
         }
-    };
-    // the first task's copies are in flight while the block fills its tables
-    if (tid == 0) {
-        ptx::mbar_init(bar, 1);
-        ptx::mbar_init_fence();
     }
-    if (blockIdx.x < ntask) start_task(ntask - 1 - (int)blockIdx.x);
     gk61_fill(N, tid, blockDim.x);
     __syncthreads();
-    unsigned phase = 0;
-    int my_max = 0;
-    long long my_tot = 0;
-    // Blocks take the tasks from the last: the high-k bins of the last species, among the
-    // deepest QAG subdivisions, start first, and the blocks that wait for a free slot
-    // (more tasks than resident blocks) get the shallow low-k bins of the first species.
-    for (int task = blockIdx.x; task < ntask; task += gridDim.x) {
-        const int si = (ntask - 1 - task) / nk, ik = (ntask - 1 - task) % nk;
-        const int mi = si == 0 ? spec_ids.x : (si == 1 ? spec_ids.y : spec_ids.z);
-        if (task != (int)blockIdx.x) {  // later tasks: after the previous task's reads of row / rc
-            __syncthreads();
-            start_task(ntask - 1 - task);
-            __syncthreads();
-        }
-        if (S.skip_integral || Na <= 1 || !(S.inv_m[mi] > 0)) continue;  // block-uniform
-        const bool got = __syncthreads_and(ptx::mbar_wait_bounded(bar, phase));  // block-uniform
-        phase ^= 1;
-        if (!got) {
-            if (tid == 0) atomicOr(I.status, kStTimeout);
-            ptx::mbar_wait_bounded(bar, phase ^ 1);
-            return;
-        }
-        if (upd.row >= 0) {
-            const double dy = s_dy;
-            for (int j = 1 + tid; j < Na - 1; j += blockDim.x) rc[j] = fma(dy, __ldg(I.coef_unit + j), rc[j]);
-            if (tid == 0) row[Na - 1] = s_y;
-            __syncthreads();
-        }
-        const double kom = (I.kq ? I.kq[ik] : I.wavenum[ik]) * S.inv_m[mi];
-        const DnuIntegrandW f = dnu_integrand_w(I, S, mi, kom, row, rc, Na);
-        QagResult r;
-        if constexpr (G < 0) r = qag_block_multi_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
-        else if constexpr (G > 0) r = qag_block_spec_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
-        else r = qag_block_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
-        if (I.ivals) {  // keep the final subdivision for the adjoint
-            double* dst = I.ivals + ((size_t)mi * I.nk_alloc + ik) * kQagLimit * 2;
-            for (int q = tid; q < r.nint; q += blockDim.x) {
-                dst[2 * q] = L.a[q];
-                dst[2 * q + 1] = L.b[q];
-            }
-            if (tid == 0) I.nivals[(size_t)mi * I.nk_alloc + ik] = r.nint;
-        }
-        if (!r.ok && tid == 0) atomicOr(I.status, kStGsl);
-        my_max = max(my_max, r.nint);
-        my_tot += r.nint;
-        // (the same block wrote the initial-condition term, before a barrier)
-        if (tid == 0) I.dnu_s[(size_t)mi * I.nk_alloc + ik] += S.prefac * r.result;
+    if (!integrate) return;
+    if (!__syncthreads_and(ptx::mbar_wait_bounded(bar, 0))) {
+        if (tid == 0) atomicOr(I.status, kStTimeout);
+        ptx::mbar_wait_bounded(bar, 0);  // the copies still in flight
+        return;
     }
-    if (tid == 0 && my_tot) {
-        atomicMax(I.qag_max, my_max);
-        atomicAdd(reinterpret_cast<unsigned long long*>(I.qag_total), (unsigned long long)my_tot);
+    if (upd.row >= 0) {
+        const double dy = s_dy;
+        for (int j = 1 + tid; j < Na - 1; j += blockDim.x) rc[j] = fma(dy, __ldg(I.coef_unit + j), rc[j]);
+        if (tid == 0) row[Na - 1] = s_y;
+        __syncthreads();
+    }
+    const DnuIntegrandW f = dnu_integrand_w(I, S, mi, k * S.inv_m[mi], row, rc, Na);
+    QagResult r;
+    if constexpr (G < 0) r = qag_block_multi_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
+    else if constexpr (G > 0) r = qag_block_spec_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
+    else r = qag_block_c(f, N, L, S.loga0, S.loga, 0.0, S.relerr, kQagLimit, sh);
+    if (I.ivals) {  // keep the final subdivision for the adjoint
+        double* dst = I.ivals + ((size_t)mi * I.nk_alloc + ik) * kQagLimit * 2;
+        for (int q = tid; q < r.nint; q += blockDim.x) {
+            dst[2 * q] = L.a[q];
+            dst[2 * q + 1] = L.b[q];
+        }
+        if (tid == 0) I.nivals[(size_t)mi * I.nk_alloc + ik] = r.nint;
+    }
+    if (tid == 0) {
+        // (thread 32 wrote the initial-condition term, before a barrier)
+        I.dnu_s[(size_t)mi * I.nk_alloc + ik] += S.prefac * r.result;
+        if (!r.ok) atomicOr(I.status, kStGsl);
+        atomicMax(I.qag_max, r.nint);
+        atomicAdd(reinterpret_cast<unsigned long long*>(I.qag_total), (unsigned long long)r.nint);
     }
 }
 

@@ -158,9 +158,4 @@ __device__ __forceinline__ void hyb_table_block(double* hyb, int blk, double qc,
     p[8 + k] = k == 0 ? B3 : cb * ih;
 }
 
-// specialJ (delta_tot_table.c:442-463) with the tabulated fit
-__device__ __forceinline__ double specialJ_tab(double x, double qc, double nufrac_low) {
-    return qc > 0 ? specialJ(x, qc, nufrac_low) : specialJ_fit_tab(x);
-}
-
 }  // namespace ksp

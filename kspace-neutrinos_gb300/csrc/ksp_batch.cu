@@ -11,8 +11,8 @@
 //   kb_tables       the fslength tables and the node tables of the integrand
 //   kb_dtot_coeffs  warp per 32 bins of an instance: history-row spline coefficients
 //   kb_dnu_qag      persistent warps that pull (instance, species, bin) tasks from an
-//                   atomic queue; knots, row and coefficients staged into shared memory
-//                   by TMA bulk copies; QAG with the 61-point Gauss-Kronrod rule
+//                   atomic queue; row and coefficients staged into shared memory by
+//                   TMA bulk copies; QAG with the 61-point Gauss-Kronrod rule
 //   kb_finish       thread per (instance, bin): species sum, commit, NaN check, clamp
 //   kb_corr         block per bound grid: correction table (interface_common.c:134-146)
 // All kernels run on fixed launch shapes and read the call's totals from device memory,

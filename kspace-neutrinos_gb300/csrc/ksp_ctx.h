@@ -36,7 +36,7 @@ struct kspace_ctx {
     int tma = 5, rows = 256, stages = 2, qag_warps = 1;
     ksp::NcNodes nc_plain{}, nc_cut{};  // the node tables of hybrid neutrinos' calls (with I.hyb)
     int nc_levels = 12;  // depths of QAG's rightmost bisections kept in the integrand node table (all)
-    int qag_split = 0;  // warps per (species, bin) integral: 1, 2, 4, 8 (8: with look-ahead); 0 = by the task count
+    int qag_split = 0;  // warps per (species, bin) integral: 1, 2, 4, 8, 12 (8, 12: with look-ahead); 0 = by the task count
     // background
     bool bg_ready = false, hubble_ready = false;
     Background hB;
@@ -63,7 +63,7 @@ struct kspace_ctx {
     unsigned* status_d = nullptr;
     unsigned* status_h = nullptr;
     void* arena_d = nullptr;   // the table's device arrays (alloc_table), one allocation
-    double* ar_h = nullptr;    // pinned: [nk_alloc + 1] for the exchange, then [2 nk_alloc] for a call's in- and outputs
+    double* ar_h = nullptr;    // pinned: [nk_alloc + 1] for the exchange, then [3 nk_alloc] for a call's in- and outputs
     double* io_h = nullptr;
     int last_nk = 0;
     double last_BoxSize = 0;

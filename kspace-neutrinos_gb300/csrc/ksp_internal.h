@@ -448,7 +448,7 @@ void launch_integrator_prepare(const IntegratorDev& I, const Background& B, cons
 // The rest: the integrals and the species sum (get_delta_nu_combined,
 // delta_tot_table.c:153-172, writes I.dnu).
 // update_row >= 0: with a prepared step's provisional row first (base_ready: kRowsBase ran);
-// qag_split: warps per (species, bin) task (1, 2, 4 or 8; 0 = chosen by the task count)
+// qag_split: warps per (species, bin) task (1, 2, 4, 8 or 12; 0 = chosen by the task count)
 // defer_combine: leave the species sum to launch_finish_update(..., combine = true)
 void launch_integrator_rest(const IntegratorDev& I, int nk, int Na, int nspec, const int* spec_ids,
                             int warps_per_block, cudaStream_t st, int qag_split, int update_row = -1,

@@ -9,8 +9,9 @@
 // Two kernels make it: the first evaluates the segments, a block per stretch of them,
 // with their suffix sums within the stretch and the stretch's total; the second adds the
 // totals of the later stretches and forms the coefficients.  Nothing in it is serial in
-// N, and no block is larger than 64 threads or 128 registers a thread, so that the blocks
-// find room beside the binning pass, which holds most of every SM.
+// N, and no block is larger than 64 threads (128 in the second kernel) at a register cap of eight
+// such blocks to an SM, so that the blocks find room beside the binning pass, which holds most
+// of every SM.
 #pragma once
 #include "ksp_internal.h"
 
@@ -25,7 +26,7 @@ constexpr int kPrepThreads = 64;
 // evaluation per node, a segment being the integral of the degree-7 interpolant through 8
 // neighbouring nodes (7e-13; at wider spacings the kinks of the rho_nu tables, a knot every
 // ~0.016, spread over its 8 segments: 2e-10 at h = 0.019).  An evaluation is an exp, a
-// square root, two divisions and the rho_nu tables, ~100 FP64 operations.
+// reciprocal square root and the rho_nu tables, ~60 FP64 operations (fsl_integrand).
 constexpr double kFsNodeRule = 1.5e-3, kFsGauss2 = 5e-3;
 constexpr int kFsNodeSegs = kPrepThreads - 7;  // segments of a block by the node rule
 __host__ __device__ inline int fs_block_segs(double h) {

@@ -27,7 +27,10 @@
 // copies with their run-table rows, the two modes of a pair summed exactly before they
 // are binned, and the sums of up to four row pairs of the same bins flushed together.
 // k_bin_rows, over tiles of whole grid rows and runs of one row, works without a run table
-// (the allocation-free entry point).
+// (the allocation-free entry point, KSPACE_GPU_MIRROR=0, and grids whose run table would be over
+// 1 GiB, N > 3262), where the warps of its tiles divide the CTA's eight: rows of up to 32 runs
+// (N <= 1086), of 49 to 64 (N = 1632 to 2174) and of 113 to 128.  Other rows go to the plain
+// kernel of ksp_grid.cu, which took 45.5 ms at N=1280 where the mirrored rows take 1.6.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -984,17 +987,18 @@ __global__ void __launch_bounds__(WARPS * 32)
 // integrator's preparation runs beside the pass): a store to a spill slot no longer holds up
 // the next modes' loads, and with the whole run in registers the stage is on its way again
 // during the sums.
-// Together, kernel alone: N=1024 889 -> 697 us (0.92 of the measured copy bandwidth, 534
-// million warp instructions, issue slots 63 % busy: 11 warps by shared memory, mostly
-// waiting for fixed latencies; in two stretches 735), N=512 137 -> 124 us.  Two steps' arithmetic packed
-// (f32x2) took fewer instructions and more time (N=1024 +80 us): the chain of the run sum
-// stays, and the packing's register pairs lengthen the rest.
+// Together, kernel alone: N=1024 889 -> 697 us (0.92 of the measured copy bandwidth; in two
+// stretches 735), N=512 137 -> 124 us.  N=768 under ncu 439 -> 333 us: 3.16e8 -> 2.51e8 warp
+// instructions, issue slots 65 % busy, 12 warps by shared memory and registers, waiting for fixed
+// latencies first of all.  Two steps' arithmetic packed (f32x2) took fewer instructions and more
+// time (N=1024 +80 us): the chain of the run sum stays, and the packing's register pairs
+// lengthen the rest.
 //
 // A tile is P consecutive |ky| = q of one plane (P = 32 / runs per row) and its rows'
 // mirrors: two copies where the rows are neighbours in memory (tiles 0 and 1), a copy per
 // row for the exchanged tiles (2 and 3), whose rows lie in P planes.  Rows of more than
-// 32 runs (N > 1086) are cut into parts, a part per warp (the row kernel's stages do not
-// fit shared memory there, and the plain kernel that was left took 45.5 ms at N=1280).
+// 32 runs (N > 1086) are cut into parts, a part per warp (the row kernel refuses the three
+// warps a tile of them takes, and the plain kernel that was left took 45.5 ms at N=1280).
 // Rows q = 0 and q = N/2 are their own mirrors: their lanes pair the row with zeros (the
 // stage's zeroed tail).  A copy starts at the 16-byte boundary at or below its first mode
 // and ends at the one at or above its last (a row is 8 (N/2+1) bytes, so odd rows start
@@ -1089,7 +1093,7 @@ inline MirrorTiling make_mirror_tiling(int K, int N, int nz, int slab0, int nsla
 }
 
 // stage rings (two stages per warp) | mbarriers | per-warp spill slots | float-pair bin
-// totals (T.copies copies) | thresholds | {w1[z], multiplicity} for z < nz + 17 Rt (zero past nz)
+// totals (T.copies copies) | thresholds | {w1[z], multiplicity} for z < nz + K (zero past nz)
 __host__ __device__ inline StreamPlan plan_bin_mirror(int warps, int nrbins, int nz, bool exact,
                                                       const MirrorTiling& T) {
     StreamPlan p{};
